@@ -189,3 +189,36 @@ def test_acceptance_case_of_the_kernel_microbenchmark_matches_the_oracle():
     lb.free(); qb.free()
     stream.destroy()
     dev.close()
+
+
+@pytest.mark.parametrize("B,V", [(2, 1000), (2, 4099), (2, 8192), (3, 32767), (2, 32768), (40, 65536), (80, 65538), (2, 262147)])
+def test_rejection_walk_at_the_vocabulary_sizes_where_the_launch_changes(B, V):
+    """One CTA, two, four and eight CTAs per sequence, vocabularies that 16-byte loads do not divide: trees of 17
+    rows, bit for bit the oracle's."""
+    parent, T = synth.tree_16(), 0.8
+    N = parent.size
+    dev = cuda.Device(0)
+    stream = dev.stream()
+    rng = np.random.default_rng(V)
+    logits = (3.0 * rng.standard_normal((B, N, V), dtype=np.float32)).astype(np.float32)
+    q, tokens = np.zeros((B, N, V), np.float32), np.zeros((B, N), np.int32)
+    for b in range(B):
+        if b >= 3:  # (many sequences: copies of the first three)
+            logits[b], q[b], tokens[b] = logits[b % 3], q[b % 3], tokens[b % 3]
+            continue
+        for c in range(1, N):
+            q[b, c] = softmax32((logits[b, parent[c]] + rng.standard_normal(V, dtype=np.float32)) / T)
+            tokens[b, c] = int(np.argmax(q[b, c])) if (b + c) % 2 else rng.integers(0, V)
+    uniforms = np.minimum(rng.random((B, N, 2), dtype=np.float32), np.float32(0.99999994))
+    lb, qb = dev.upload(logits), dev.upload(q)
+    for _ in range(2):  # the second call reuses what the first left in the stream's scratch
+        acc, em, path = cuda.accept_tree(stream, lb, tokens, V, parent=np.tile(parent, (B, 1)), mode=cuda.ACCEPT_REJECTION,
+                                         temperature=T, draft_probs=qb, uniforms=uniforms)
+        for b in (range(B) if B < 4 else (0, 1, 2, B - 1)):
+            a, p_o, e_o = yo.accept_rejection_tree(logits[b], q[b], tokens[b], parent, T, uniforms[b])
+            assert int(acc[b]) == a, b
+            assert path[b, :a].tolist() == p_o.tolist() and em[b, :a + 1].tolist() == e_o.tolist()
+            assert (path[b, a:] == -1).all() and (em[b, a + 1:] == -1).all()
+    lb.free(); qb.free()
+    stream.destroy()
+    dev.close()

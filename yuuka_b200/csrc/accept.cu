@@ -6,6 +6,8 @@
 // cur the wanted token is argmax(logits[cur]); the lowest-numbered child of
 // cur that carries it is accepted and becomes cur; otherwise the wanted token
 // is emitted as the correction and the walk ends.
+#include <cstring>
+#include <mutex>
 #include <vector>
 
 #include "layers.cuh"
@@ -32,7 +34,22 @@ __global__ void __launch_bounds__(256) argmax_partial_kernel(const float * __res
     const int begin = c * ARGMAX_CHUNK, end = min(vocab, begin + ARGMAX_CHUNK);
     float bv = -INFINITY;
     int bi = 0x7fffffff;
-    for (int i = begin + threadIdx.x; i < end; i += blockDim.x) best_of(bv, bi, row[i], i);
+    if (end - begin == ARGMAX_CHUNK && ((uintptr_t)(row + begin) & 15) == 0) {
+        // a whole chunk: all of a thread's loads are in flight at once (bound by DRAM: 64 x 9 x 248320 logits)
+        float4 v[ARGMAX_CHUNK / 1024];
+#pragma unroll
+        for (int u = 0; u < ARGMAX_CHUNK / 1024; u++) v[u] = __ldcs(reinterpret_cast<const float4 *>(row + begin) + u * 256 + threadIdx.x);
+#pragma unroll
+        for (int u = 0; u < ARGMAX_CHUNK / 1024; u++) {
+            const int i = begin + (u * 256 + (int)threadIdx.x) * 4;
+            best_of(bv, bi, v[u].x, i);
+            best_of(bv, bi, v[u].y, i + 1);
+            best_of(bv, bi, v[u].z, i + 2);
+            best_of(bv, bi, v[u].w, i + 3);
+        }
+    } else {
+        for (int i = begin + threadIdx.x; i < end; i += blockDim.x) best_of(bv, bi, row[i], i);
+    }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
         float ov = __shfl_xor_sync(0xffffffffu, bv, o);
@@ -137,178 +154,262 @@ int launch_accept_greedy(cudaStream_t s, const float * logits, int vocab, const 
 //   no child accepted: t = min((uint64)((double)U[2 cur + 1] * (double)R), R - 1);
 //     emit the smallest j with sum_{i <= j} r_i > t.
 
-__device__ __forceinline__ float exp_det(float x) {
-    if (x < -87.0f) return 0.0f;
-    if (x > 88.0f) x = 88.0f;
-    const float n = rintf(x * 1.44269504f);
-    float r = fmaf(n, -0.693359375f, x);
-    r = fmaf(n, 2.12194440e-4f, r);
-    float p = 1.9875691500e-4f;
-    p = fmaf(p, r, 1.3981999507e-3f);
-    p = fmaf(p, r, 8.3334519073e-3f);
-    p = fmaf(p, r, 4.1665795894e-2f);
-    p = fmaf(p, r, 1.6666665459e-1f);
-    p = fmaf(p, r, 5.0000001201e-1f);
-    const float r2 = __fmul_rn(r, r);
-    const float e = __fadd_rn(fmaf(p, r2, r), 1.0f);
-    const float scale = __uint_as_float((uint32_t)((int)n + 127) << 23);
-    return __fmul_rn(e, scale);
+// Packed fp32 pairs (fma / mul / add.rn.f32x2): the IEEE results of the scalar forms in half the instructions.
+__device__ __forceinline__ unsigned long long pack2(float x, float y) {
+    unsigned long long r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(x), "f"(y));
+    return r;
+}
+__device__ __forceinline__ float2 unpack2(unsigned long long v) {
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+    return r;
+}
+__device__ __forceinline__ unsigned long long fma_p(unsigned long long a, unsigned long long b, unsigned long long c) {
+    unsigned long long d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+    return d;
+}
+__device__ __forceinline__ unsigned long long mul_p(unsigned long long a, unsigned long long b) {
+    unsigned long long d;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+__device__ __forceinline__ unsigned long long add_p(unsigned long long a, unsigned long long b) {
+    unsigned long long d;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+// Weights of two logits: w = (uint64)(exp_det((L - mx) / T) * 2^40) with
+//   exp_det(x): n = rint(x * 1.44269504), r = x - n ln 2 in two parts, a degree-5 polynomial, times 2^n; 0 below -87.
+// rint is an addition and subtraction of 1.5 * 2^23 (|x log2 e| < 2^22), whose low bits are n; 2^n * 2^40 is one
+// exact multiplication; x is clamped at -87, where the weight is 0 as well (anything below 2^-40 is).
+__device__ __forceinline__ void target_weights2(float l0, float l1, float mx, float inv_t, unsigned long long & w0, unsigned long long & w1) {
+    const float2 xs = unpack2(mul_p(add_p(pack2(l0, l1), pack2(-mx, -mx)), pack2(inv_t, inv_t)));
+    const unsigned long long x = pack2(fmaxf(xs.x, -87.0f), fmaxf(xs.y, -87.0f));
+    const unsigned long long shifted = add_p(mul_p(x, pack2(1.44269504f, 1.44269504f)), pack2(12582912.0f, 12582912.0f));
+    const unsigned long long n = add_p(shifted, pack2(-12582912.0f, -12582912.0f));
+    unsigned long long r = fma_p(n, pack2(-0.693359375f, -0.693359375f), x);
+    r = fma_p(n, pack2(2.12194440e-4f, 2.12194440e-4f), r);
+    unsigned long long q = fma_p(pack2(1.9875691500e-4f, 1.9875691500e-4f), r, pack2(1.3981999507e-3f, 1.3981999507e-3f));
+    q = fma_p(q, r, pack2(8.3334519073e-3f, 8.3334519073e-3f));
+    q = fma_p(q, r, pack2(4.1665795894e-2f, 4.1665795894e-2f));
+    q = fma_p(q, r, pack2(1.6666665459e-1f, 1.6666665459e-1f));
+    q = fma_p(q, r, pack2(5.0000001201e-1f, 5.0000001201e-1f));
+    const unsigned long long e = add_p(fma_p(q, mul_p(r, r), r), pack2(1.0f, 1.0f));
+    const float2 ns = unpack2(shifted);
+    // (low bits of the shifted value + 127 + 40, moved into the exponent: the upper bits drop out)
+    const float s0 = __uint_as_float((__float_as_uint(ns.x) + 167u) << 23), s1 = __uint_as_float((__float_as_uint(ns.y) + 167u) << 23);
+    const float2 v = unpack2(mul_p(e, pack2(s0, s1)));
+    w0 = (unsigned long long)v.x;
+    w1 = (unsigned long long)v.y;
 }
 
-__device__ __forceinline__ unsigned long long target_weight(float logit, float mx, float inv_t) {
-    const float e = exp_det(__fmul_rn(__fsub_rn(logit, mx), inv_t));
-    return (unsigned long long)__fmul_rn(e, 1099511627776.0f);
-}
-
-constexpr int REJ_THREADS = 1024;
-constexpr int REJ_CLUSTER = 8;          // CTAs that share one sequence's vocabulary when it is large
-constexpr int REJ_CLUSTER_MIN_VOCAB = 32768;
+constexpr int REJ_THREADS = 512;
+constexpr int REJ_WARPS = REJ_THREADS / 32;
+constexpr int REJ_MAX_CLUSTER = 8;   // CTAs that share one sequence's vocabulary
+constexpr int REJ_MAX_NODES = 64;
 
 struct RejectParams {
     const float * logits;   // [batch][nodes][vocab]
     const float * q;        // [batch][nodes][vocab]
     const float * u;        // [batch][nodes][2]
-    unsigned long long * r; // [batch][vocab]
     int vocab;
     float inv_t;
     RowMeta rows;
     AcceptOut out;
 };
 
-// Sums and maxima over the CL CTAs that walk one sequence together. Every CTA reduces its own slice, leaves the
-// result in one of two shared-memory slots (alternating: a CTA can only be one exchange ahead of the slowest,
-// because the hardware barrier of exchange k + 1 needs every CTA to have finished reading exchange k), and reads
-// all CL slots after the cluster barrier. Integer sums and float maxima do not depend on the order, so every
-// CTA holds the same value and takes the same branches. CL = 1 degenerates to the block reduction.
-template <int CL> struct RejectExchange {
-    unsigned long long * red;   // [REJ_THREADS / 32]
-    unsigned long long * slot;  // [2]
-    int turn = 0;
+__device__ __forceinline__ void st_cluster_u64(unsigned long long * p, unsigned rank, unsigned long long v) {
+    const uint32_t local = (uint32_t)__cvta_generic_to_shared(p);
+    uint32_t remote;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(local), "r"(rank));
+    asm volatile("st.shared::cluster.u64 [%0], %1;" ::"r"(remote), "l"(v) : "memory");
+}
+// four consecutive values from p + i, `fill` beyond n (VEC: p is 16-byte aligned, i and n are multiples of four)
+template <bool VEC>
+__device__ __forceinline__ float4 load4(const float * p, int i, int n, float fill) {
+    if (VEC) return i < n ? *reinterpret_cast<const float4 *>(p + i) : make_float4(fill, fill, fill, fill);
+    return make_float4(i < n ? p[i] : fill, i + 1 < n ? p[i + 1] : fill, i + 2 < n ? p[i + 2] : fill, i + 3 < n ? p[i + 3] : fill);
+}
+__device__ __forceinline__ unsigned long long take_away(unsigned long long r, float q, double R) {
+    const unsigned long long qr = (unsigned long long)__dmul_rn((double)q, R);
+    return r > qr ? r - qr : 0ull;
+}
 
-    __device__ unsigned long long block_sum(unsigned long long v) {
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-        __syncthreads();  // red may still be read from the previous use
-        if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
-        __syncthreads();
-        unsigned long long t = 0;
-        for (int w = 0; w < REJ_THREADS / 32; w++) t += red[w];
-        return t;
-    }
-    __device__ float block_max(float v) {
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
-        __syncthreads();
-        if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = (unsigned long long)__float_as_uint(v);
-        __syncthreads();
-        for (int w = 0; w < REJ_THREADS / 32; w++) v = fmaxf(v, __uint_as_float((uint32_t)red[w]));
-        return v;
-    }
-    // total over the cluster; *before (if given) receives the sum over the CTAs of lower rank
-    __device__ unsigned long long sum(unsigned long long v, unsigned long long * before = nullptr) {
-        const unsigned long long mine = block_sum(v);
-        if constexpr (CL == 1) {
-            if (before) *before = 0;
-            return mine;
-        } else {
-            if (threadIdx.x == 0) slot[turn] = mine;
-            cluster_sync_all();
-            unsigned long long tot = 0, low = 0;
-            const unsigned me = cluster_cta_rank();
-            for (unsigned c = 0; c < (unsigned)CL; c++) {
-                const unsigned long long x = ld_cluster_u64(slot + turn, c);
-                if (c < me) low += x;
-                tot += x;
-            }
-            if (before) *before = low;
-            turn ^= 1;
-            return tot;
-        }
-    }
-    __device__ float max(float v) {
-        v = block_max(v);
-        if constexpr (CL == 1) {
-            return v;
-        } else {
-            if (threadIdx.x == 0) slot[turn] = (unsigned long long)__float_as_uint(v);
-            cluster_sync_all();
-            for (unsigned c = 0; c < (unsigned)CL; c++) v = fmaxf(v, __uint_as_float((uint32_t)ld_cluster_u64(slot + turn, c)));
-            turn ^= 1;
-            return v;
-        }
-    }
-    // orders this cluster's global writes (the residual weights) before the reads that follow in other CTAs
-    __device__ void sync() {
-        if constexpr (CL == 1) __syncthreads();
-        else cluster_sync_all();
-    }
-};
-
-// One sequence per cluster of CL CTAs; CTA c of the cluster owns the vocabulary slice [c * slice, (c + 1) * slice).
-// All CTAs of a cluster walk the tree together: the deciding quantities (R, r[x], q[x], the uniforms) are the
-// same everywhere, so they take the same turns; only rank 0 writes the path.
-template <int CL>
-__global__ void __launch_bounds__(REJ_THREADS) rejection_walk_kernel(const RejectParams p) {
+// One sequence per cluster of CL CTAs; CTA c owns the vocabulary slice [c * slice, (c + 1) * slice), a warp of it a
+// contiguous run of `run` tokens. All CTAs of a cluster walk the tree together: the deciding quantities (the
+// maximum, R, r[x], the uniforms) are the same everywhere, so they take the same turns; rank 0 writes the path.
+//
+// The residual weights are never stored. They are elementwise functions of a row of logits and of the draft rows
+// rejected at the node so far, so each pass recomputes them from those rows, which the first pass has left in L2:
+// 4 bytes read per token and pass, where keeping them moved 16. What bounds the walk is then latency (two
+// passes, two exchanges a node, each behind the one before), so the grid is chosen for one wave of all sequences
+// (rejection_cluster), with two CTAs to an SM to overlap one's exchanges with another's passes.
+// 64 sequences x 9 rows x 248,320 tokens at T = 0.7 (1.6 accepted a sequence): 361 -> 181 us, one sequence 39 us; all
+// eight drafts accepted 262 us, of which 9 x 64 MB of logits are 90 us at the measured copy rate.
+// Sums and maxima cross the cluster by stores into every CTA's slots and one hardware barrier; slots alternate
+// between two sets (a CTA can only be one exchange ahead of the slowest).
+template <int CL, bool VEC>
+__global__ void __launch_bounds__(REJ_THREADS, 2) rejection_walk_kernel(const RejectParams p, int slice, int run) {
     pdl_entry();
-    __shared__ unsigned long long red[REJ_THREADS / 32];
-    __shared__ unsigned long long slot[2];
-    __shared__ int flag;
-    RejectExchange<CL> ex{red, slot};
+    __shared__ unsigned long long red[REJ_WARPS];
+    __shared__ unsigned long long slots[2][CL];
+    __shared__ int rejected[REJ_MAX_NODES];   // draft rows taken away from the weights at this node, in order
+    __shared__ double rejected_R[REJ_MAX_NODES];
     const unsigned rank = CL == 1 ? 0u : cluster_cta_rank();
-    const int seq = blockIdx.x / CL, N = p.rows.nodes, V = p.vocab, tid = threadIdx.x;
-    const int slice = CL == 1 ? V : (((V + CL - 1) / CL + 3) & ~3);
-    const int v0 = min(V, (int)rank * slice), v1 = min(V, v0 + slice);
+    const int seq = blockIdx.x / CL, N = p.rows.nodes, V = p.vocab, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int v1 = min(V, ((int)rank + 1) * slice);
+    const int s0 = min(v1, (int)rank * slice + warp * run), s1 = min(v1, s0 + run);
     const int32_t * tokens = p.rows.tokens + (int64_t)seq * N;
     const int32_t * parent = p.rows.parent + (int64_t)seq * N;
     const float * U = p.u + (int64_t)seq * N * 2;
-    unsigned long long * r = p.r + (int64_t)seq * V;
+    const float * Q = p.q + (int64_t)seq * N * V;
     int32_t * path = p.out.path + (int64_t)seq * N;
     int32_t * emitted = p.out.emitted + (int64_t)seq * N;
+    if constexpr (CL > 1) cluster_sync_all();  // every CTA of the cluster has started before another stores into it
+    int turn = 0;
+    // every warp's value (in all its lanes) -> red, every CTA's -> slots[turn ^ 1] after the return
+    auto exchange = [&](unsigned long long v, bool is_max) {
+        auto join = [&](unsigned long long x, unsigned long long y) {
+            return is_max ? (unsigned long long)__float_as_uint(fmaxf(__uint_as_float((uint32_t)x), __uint_as_float((uint32_t)y))) : x + y;
+        };
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) v = join(v, __shfl_xor_sync(0xffffffffu, v, o));
+        if (lane == 0) red[warp] = v;
+        __syncthreads();
+        if (warp == 0) {
+            v = red[lane & (REJ_WARPS - 1)];
+#pragma unroll
+            for (int o = REJ_WARPS / 2; o > 0; o >>= 1) v = join(v, __shfl_xor_sync(0xffffffffu, v, o));
+            if constexpr (CL == 1) {
+                if (lane == 0) slots[turn][0] = v;
+            } else {
+                if (lane < CL) st_cluster_u64(&slots[turn][rank], (unsigned)lane, v);
+            }
+        }
+        if constexpr (CL == 1) __syncthreads();
+        else cluster_sync_all();
+        turn ^= 1;
+    };
     int cur = 0, a = 0;
     for (;;) {
         const float * L = p.logits + ((int64_t)seq * N + cur) * V;
-        // max of the row (order-independent)
         float mx = -INFINITY;
-        for (int i = v0 + tid; i < v1; i += REJ_THREADS) mx = fmaxf(mx, L[i]);
-        mx = ex.max(mx);
-        // target weights
-        unsigned long long z = 0;
-        for (int i = v0 + tid; i < v1; i += REJ_THREADS) {
-            const unsigned long long w = target_weight(L[i], mx, p.inv_t);
-            r[i] = w;
-            z += w;
+        for (int i0 = s0 + lane * 4; i0 < s1; i0 += 8 * 128) {
+            float4 l[8];
+#pragma unroll
+            for (int u = 0; u < 8; u++) l[u] = load4<VEC>(L, i0 + u * 128, s1, -INFINITY);
+#pragma unroll
+            for (int u = 0; u < 8; u++) mx = fmaxf(mx, fmaxf(fmaxf(l[u].x, l[u].y), fmaxf(l[u].z, l[u].w)));
         }
-        const unsigned long long Z = ex.sum(z);  // (its barrier also publishes r)
-        unsigned long long R = Z;
-        int next = -1;
-        for (int c = cur + 1; c < N && next < 0; c++) {
-            if (parent[c] != cur) continue;
-            const float * q = p.q + ((int64_t)seq * N + c) * V;
-            __syncthreads();  // flag of the previous child has been read
-            if (tid == 0) {
-                const int32_t x = tokens[c];
-                const float lhs = __fmul_rn(U[2 * c], q[x]);
-                flag = __dmul_rn((double)lhs, (double)R) <= (double)__ldcg(r + x);
+        exchange((unsigned long long)__float_as_uint(mx), true);
+#pragma unroll
+        for (int c = 0; c < CL; c++) mx = fmaxf(mx, __uint_as_float((uint32_t)slots[turn ^ 1][c]));
+        int n_rej = 0;
+        // weights of tokens i .. i + 3, zero from `end` on
+        auto weights_at4 = [&](int i, int end, unsigned long long (&w)[4]) {
+            const float4 l = load4<VEC>(L, i, end, -INFINITY);
+            target_weights2(l.x, l.y, mx, p.inv_t, w[0], w[1]);
+            target_weights2(l.z, l.w, mx, p.inv_t, w[2], w[3]);
+            for (int j = 0; j < n_rej; j++) {
+                const float4 q = load4<VEC>(Q + (int64_t)rejected[j] * V, i, end, 0.0f);
+                const double Rj = rejected_R[j];
+                w[0] = take_away(w[0], q.x, Rj);
+                w[1] = take_away(w[1], q.y, Rj);
+                w[2] = take_away(w[2], q.z, Rj);
+                w[3] = take_away(w[3], q.w, Rj);
             }
-            __syncthreads();
-            if (flag) {
+        };
+        // sum of the weights of this warp's run
+        auto run_sum = [&]() {
+            unsigned long long sum = 0;
+            if (n_rej == 0) {
+                for (int i0 = s0 + lane * 4; i0 < s1; i0 += 4 * 128) {
+                    float4 l[4];
+#pragma unroll
+                    for (int u = 0; u < 4; u++) l[u] = load4<VEC>(L, i0 + u * 128, s1, -INFINITY);
+#pragma unroll
+                    for (int u = 0; u < 4; u++) {
+                        unsigned long long w[4];
+                        target_weights2(l[u].x, l[u].y, mx, p.inv_t, w[0], w[1]);
+                        target_weights2(l[u].z, l[u].w, mx, p.inv_t, w[2], w[3]);
+                        sum += (w[0] + w[1]) + (w[2] + w[3]);
+                    }
+                }
+                return sum;
+            }
+            if (n_rej == 1) {  // (the usual case on its own: its row and its R stay in registers)
+                const float * q = Q + (int64_t)rejected[0] * V;
+                const double R0 = rejected_R[0];
+                for (int i0 = s0 + lane * 4; i0 < s1; i0 += 4 * 128) {
+                    float4 l[4], d[4];
+#pragma unroll
+                    for (int u = 0; u < 4; u++) {
+                        l[u] = load4<VEC>(L, i0 + u * 128, s1, -INFINITY);
+                        d[u] = load4<VEC>(q, i0 + u * 128, s1, 0.0f);
+                    }
+#pragma unroll
+                    for (int u = 0; u < 4; u++) {
+                        unsigned long long w0, w1;
+                        target_weights2(l[u].x, l[u].y, mx, p.inv_t, w0, w1);
+                        sum += take_away(w0, d[u].x, R0) + take_away(w1, d[u].y, R0);
+                        target_weights2(l[u].z, l[u].w, mx, p.inv_t, w0, w1);
+                        sum += take_away(w0, d[u].z, R0) + take_away(w1, d[u].w, R0);
+                    }
+                }
+                return sum;
+            }
+            for (int i0 = s0 + lane * 4; i0 < s1; i0 += 128) {
+                unsigned long long w[4];
+                weights_at4(i0, s1, w);
+                sum += (w[0] + w[1]) + (w[2] + w[3]);
+            }
+            return sum;
+        };
+        auto weight_at = [&](int x) {
+            unsigned long long w, unused;
+            target_weights2(L[x], mx, mx, p.inv_t, w, unused);
+            for (int j = 0; j < n_rej; j++) w = take_away(w, Q[(int64_t)rejected[j] * V + x], rejected_R[j]);
+            return w;
+        };
+        unsigned long long below, mine;
+        auto total = [&]() {
+            unsigned long long tot = 0;
+            below = 0;
+#pragma unroll
+            for (int c = 0; c < CL; c++) {
+                const unsigned long long x = slots[turn ^ 1][c];
+                if (c < (int)rank) below += x;
+                if (c == (int)rank) mine = x;
+                tot += x;
+            }
+            return tot;
+        };
+        exchange(run_sum(), false);
+        unsigned long long R = total();
+        int next = -1;
+        for (int c = cur + 1; c < N; c++) {
+            if (parent[c] != cur) continue;
+            const int32_t x = tokens[c];
+            // (every thread of every CTA works this out for itself: no exchange)
+            if (__dmul_rn((double)__fmul_rn(U[2 * c], Q[(int64_t)c * V + x]), (double)R) <= (double)weight_at(x)) {
                 next = c;
                 break;
             }
-            if constexpr (CL > 1) ex.sync();  // every CTA has read r[x] before its owner rewrites it
-            unsigned long long sum = 0;
-            for (int i = v0 + tid; i < v1; i += REJ_THREADS) {
-                const unsigned long long qr = (unsigned long long)__dmul_rn((double)q[i], (double)R);
-                const unsigned long long ri = r[i];
-                const unsigned long long nr = ri > qr ? ri - qr : 0ull;
-                r[i] = nr;
-                sum += nr;
+            __syncthreads();  // the list may still be in use
+            if (tid == 0) {
+                rejected[n_rej] = c;
+                rejected_R[n_rej] = (double)R;
             }
-            R = ex.sum(sum);
-            if (R == 0) {
-                for (int i = v0 + tid; i < v1; i += REJ_THREADS) r[i] = target_weight(L[i], mx, p.inv_t);
-                R = Z;
-                ex.sync();
+            n_rej++;
+            __syncthreads();
+            exchange(run_sum(), false);
+            R = total();
+            if (R == 0) {  // nothing is left: the target's own weights again
+                n_rej = 0;
+                exchange(run_sum(), false);
+                R = total();
             }
         }
         if (next >= 0) {
@@ -318,37 +419,46 @@ __global__ void __launch_bounds__(REJ_THREADS) rejection_walk_kernel(const Rejec
             }
             a++;
             cur = next;
-            if constexpr (CL > 1) ex.sync();  // r[x] has been read everywhere before the next node rewrites r
             continue;
         }
-        // residual draw: the smallest j whose inclusive prefix sum over r exceeds t. Thread tid of CTA c owns the
-        // contiguous range [lo, hi) of c's slice.
+        // residual draw: the smallest j whose inclusive prefix sum over r exceeds t, by the warp whose run holds it
         unsigned long long t = (unsigned long long)__dmul_rn((double)U[2 * cur + 1], (double)R);
         if (t >= R) t = R - 1;
-        const int per = (v1 - v0 + REJ_THREADS - 1) / REJ_THREADS;
-        const int lo = min(v1, v0 + tid * per), hi = min(v1, lo + per);
-        unsigned long long mine = 0;
-        for (int i = lo; i < hi; i++) mine += r[i];
-        unsigned long long below = 0;
-        ex.sum(mine, &below);  // total of the slices of lower rank
-        // exclusive prefix of the per-thread sums: inside the warp, then across warps
-        unsigned long long incl = mine;
+        if (t < below || t - below >= mine) break;  // (no exchange follows: every CTA may leave)
+        t -= below;
+        int owner = 0;
+        unsigned long long before = 0;
+        while (t - before >= red[owner]) before += red[owner++];
+        t -= before;
+        // the CTA shares out that warp's run, a few consecutive tokens to a thread: which thread's, then which token
+        const int r0 = min(v1, (int)rank * slice + owner * run), r1 = min(v1, r0 + run);
+        const int part = ((run + REJ_THREADS - 1) / REJ_THREADS + 3) & ~3;
+        const int p0 = min(r1, r0 + tid * part), p1 = min(r1, p0 + part);
+        unsigned long long own = 0;
+        for (int i = p0; i < p1; i += 4) {
+            unsigned long long w[4];
+            weights_at4(i, p1, w);
+            own += (w[0] + w[1]) + (w[2] + w[3]);
+        }
+        unsigned long long incl = own;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
             const unsigned long long v = __shfl_up_sync(0xffffffffu, incl, o);
-            if ((tid & 31) >= o) incl += v;
+            if (lane >= o) incl += v;
         }
+        __syncthreads();  // red has been read
+        if (lane == 31) red[warp] = incl;
         __syncthreads();
-        if ((tid & 31) == 31) red[tid >> 5] = incl;
-        __syncthreads();
-        unsigned long long before = below + incl - mine;
-        for (int w = 0; w < (tid >> 5); w++) before += red[w];
-        if (before <= t && t < before + mine) {
-            unsigned long long acc = before;
-            for (int i = lo; i < hi; i++) {
-                acc += r[i];
-                if (acc > t) {
-                    emitted[a] = i;  // exactly one thread of the cluster: t < R = the total
+        for (int w = 0; w < warp; w++) incl += red[w];
+        if (incl - own <= t && t < incl) {  // exactly one thread: t is below the run's total
+            unsigned long long acc = incl - own;
+            for (int i = p0; i < p1; i += 4) {
+                unsigned long long w[4];
+                weights_at4(i, p1, w);
+                int e = 0;
+                for (; e < 4 && acc + w[e] <= t; e++) acc += w[e];
+                if (e < 4) {
+                    emitted[a] = i + e;
                     break;
                 }
             }
@@ -360,18 +470,36 @@ __global__ void __launch_bounds__(REJ_THREADS) rejection_walk_kernel(const Rejec
         for (int i = a + 1 + tid; i < N; i += REJ_THREADS) emitted[i] = -1;
         if (tid == 0) p.out.accepted[seq] = a;
     }
-    if constexpr (CL > 1) cluster_sync_all();  // no CTA leaves while another may still read its slots
 }
 
-int launch_accept_rejection(cudaStream_t s, const float * logits, const float * draft_probs, const float * uniforms,
-                            unsigned long long * residual, int vocab, float temperature, const RowMeta & rows,
-                            const AcceptOut & out) {
+// CTAs per sequence: as many as let all sequences run at once (two CTAs on each of 148 SMs), as long as a CTA keeps
+// at least 4,096 tokens (two loads per thread and pass; below that the exchanges cost more than the passes they cut).
+static int rejection_cluster(int batch, int vocab) {
+    int cl = REJ_MAX_CLUSTER;
+    while (cl > 1 && (batch * cl > 2 * 148 || vocab < cl * 4096)) cl >>= 1;
+    return cl;
+}
+
+template <int CL>
+static void launch_rejection(cudaStream_t s, const RejectParams & p) {
+    const int slice = ((p.vocab + CL - 1) / CL + 3) & ~3, run = ((slice + REJ_WARPS - 1) / REJ_WARPS + 3) & ~3;
+    const bool vec = (p.vocab & 3) == 0 && (((uintptr_t)p.logits | (uintptr_t)p.q) & 15) == 0;
+    auto kern = vec ? rejection_walk_kernel<CL, true> : rejection_walk_kernel<CL, false>;
+    if (CL > 1) launch_k_cluster(kern, dim3(p.rows.batch * CL), REJ_THREADS, 0, s, CL, p, slice, run);
+    else launch_k(kern, p.rows.batch, REJ_THREADS, 0, s, p, slice, run);
+}
+
+int launch_accept_rejection(cudaStream_t s, const float * logits, const float * draft_probs, const float * uniforms, int vocab,
+                            float temperature, const RowMeta & rows, const AcceptOut & out) {
     YK_REQUIRE(temperature > 0.0f, YUUKA_ERR_INVALID_ARGUMENT, "rejection sampling needs a temperature above zero");
-    RejectParams p{logits, draft_probs, uniforms, residual, vocab, 1.0f / temperature, rows, out};
-    if (vocab >= REJ_CLUSTER_MIN_VOCAB)
-        launch_k_cluster(rejection_walk_kernel<REJ_CLUSTER>, dim3(rows.batch * REJ_CLUSTER), REJ_THREADS, 0, s, REJ_CLUSTER, p);
-    else
-        launch_k(rejection_walk_kernel<1>, rows.batch, REJ_THREADS, 0, s, p);
+    YK_REQUIRE(rows.nodes <= REJ_MAX_NODES, YUUKA_ERR_UNSUPPORTED, "rejection sampling: at most %d rows per sequence", REJ_MAX_NODES);
+    RejectParams p{logits, draft_probs, uniforms, vocab, 1.0f / temperature, rows, out};
+    switch (rejection_cluster(rows.batch, vocab)) {
+    case 8: launch_rejection<8>(s, p); break;
+    case 4: launch_rejection<4>(s, p); break;
+    case 2: launch_rejection<2>(s, p); break;
+    default: launch_rejection<1>(s, p); break;
+    }
     YK_CUDA(cudaGetLastError());
     return 1;
 }
@@ -437,41 +565,39 @@ extern "C" yuuka_status yuuka_accept_tree(yuuka_stream * stream, const yuuka_buf
             }
         set_device(stream->dev);
         const int chunks = argmax_chunks(vocab);
-        // one allocation: anc | tokens | parent | depth | accepted | path | emitted | uniforms | argmax val, idx | residual
-        const size_t o_anc = 0, o_tok = o_anc + R * 8, o_par = o_tok + R * 4, o_dep = o_par + R * 4, o_acc = o_dep + R * 4,
-                     o_path = o_acc + (size_t)batch * 4, o_em = o_path + R * 4, o_uni = o_em + R * 4, o_val = o_uni + R * 8,
-                     o_idx = o_val + R * chunks * 4, o_res = ((o_idx + R * chunks * 4 + 255) / 256) * 256,
-                     total = o_res + (mode == YUUKA_ACCEPT_REJECTION ? (size_t)batch * vocab * 8 : 0);
-        uint8_t * d = nullptr;
-        YK_REQUIRE(cudaMalloc((void **)&d, total) == cudaSuccess, YUUKA_ERR_ALLOCATION, "accept_tree: scratch allocation of %llu bytes failed",
-                   (unsigned long long)total);
-        try {
-            cudaStream_t st = stream->s;
-            YK_CUDA(cudaMemcpyAsync(d + o_anc, anc.data(), R * 8, cudaMemcpyHostToDevice, st));
-            YK_CUDA(cudaMemcpyAsync(d + o_tok, tokens, R * 4, cudaMemcpyHostToDevice, st));
-            YK_CUDA(cudaMemcpyAsync(d + o_par, par.data(), R * 4, cudaMemcpyHostToDevice, st));
-            YK_CUDA(cudaMemcpyAsync(d + o_dep, dep.data(), R * 4, cudaMemcpyHostToDevice, st));
-            if (mode == YUUKA_ACCEPT_REJECTION) YK_CUDA(cudaMemcpyAsync(d + o_uni, uniforms, R * 8, cudaMemcpyHostToDevice, st));
-            RowMeta rows{(const int32_t *)(d + o_tok), (const int32_t *)(d + o_par), (const int32_t *)(d + o_dep),
-                         (const uint64_t *)(d + o_anc), nullptr, batch, nodes};
-            AcceptOut out{(int32_t *)(d + o_acc), (int32_t *)(d + o_path), (int32_t *)(d + o_em)};
-            if (begin) YK_CUDA(cudaEventRecord(begin->e, st));
-            if (mode == YUUKA_ACCEPT_GREEDY) {
-                ArgmaxScratch sc{(float *)(d + o_val), (int32_t *)(d + o_idx), chunks};
-                launch_accept_greedy(st, (const float *)logits->ptr, vocab, rows, sc, out);
-            } else {
-                launch_accept_rejection(st, (const float *)logits->ptr, (const float *)draft_probs->ptr, (const float *)(d + o_uni),
-                                        (unsigned long long *)(d + o_res), vocab, temperature, rows, out);
-            }
-            if (end) YK_CUDA(cudaEventRecord(end->e, st));
-            YK_CUDA(cudaMemcpyAsync(accepted, d + o_acc, (size_t)batch * 4, cudaMemcpyDeviceToHost, st));
-            YK_CUDA(cudaMemcpyAsync(emitted, d + o_em, R * 4, cudaMemcpyDeviceToHost, st));
-            if (path) YK_CUDA(cudaMemcpyAsync(path, d + o_path, R * 4, cudaMemcpyDeviceToHost, st));
-            YK_CUDA(cudaStreamSynchronize(st));
-        } catch (...) {
-            cudaFree(d);
-            throw;
+        const bool reject = mode == YUUKA_ACCEPT_REJECTION;
+        // inputs, filled by one copy: anc | uniforms | tokens | parent | depth; results, read by one copy: accepted |
+        // path | emitted; then scratch: argmax val, idx
+        const size_t o_anc = 0, o_uni = o_anc + R * 8, o_tok = o_uni + (reject ? R * 8 : 0), o_par = o_tok + R * 4, o_dep = o_par + R * 4,
+                     o_acc = o_dep + R * 4, o_path = o_acc + (size_t)batch * 4, o_em = o_path + R * 4, staged = o_em + R * 4,
+                     o_val = (staged + 255) / 256 * 256, o_idx = o_val + (reject ? 0 : R * chunks * 4),
+                     total = o_idx + (reject ? 0 : R * chunks * 4);
+        std::lock_guard<std::mutex> lock(stream->scratch.mutex);
+        StreamScratchUse use(stream->scratch, total, staged);
+        uint8_t * d = use.device, * h = use.host;
+        memcpy(h + o_anc, anc.data(), R * 8);
+        memcpy(h + o_tok, tokens, R * 4);
+        memcpy(h + o_par, par.data(), R * 4);
+        memcpy(h + o_dep, dep.data(), R * 4);
+        if (reject) memcpy(h + o_uni, uniforms, R * 8);
+        cudaStream_t st = stream->s;
+        YK_CUDA(cudaMemcpyAsync(d, h, o_acc, cudaMemcpyHostToDevice, st));
+        RowMeta rows{(const int32_t *)(d + o_tok), (const int32_t *)(d + o_par), (const int32_t *)(d + o_dep),
+                     (const uint64_t *)(d + o_anc), nullptr, batch, nodes};
+        AcceptOut out{(int32_t *)(d + o_acc), (int32_t *)(d + o_path), (int32_t *)(d + o_em)};
+        if (begin) YK_CUDA(cudaEventRecord(begin->e, st));
+        if (!reject) {
+            ArgmaxScratch sc{(float *)(d + o_val), (int32_t *)(d + o_idx), chunks};
+            launch_accept_greedy(st, (const float *)logits->ptr, vocab, rows, sc, out);
+        } else {
+            launch_accept_rejection(st, (const float *)logits->ptr, (const float *)draft_probs->ptr, (const float *)(d + o_uni),
+                                    vocab, temperature, rows, out);
         }
-        cudaFree(d);
+        if (end) YK_CUDA(cudaEventRecord(end->e, st));
+        YK_CUDA(cudaMemcpyAsync(h + o_acc, d + o_acc, staged - o_acc, cudaMemcpyDeviceToHost, st));
+        YK_CUDA(cudaStreamSynchronize(st));
+        memcpy(accepted, h + o_acc, (size_t)batch * 4);
+        memcpy(emitted, h + o_em, R * 4);
+        if (path) memcpy(path, h + o_path, R * 4);
     });
 }

@@ -158,6 +158,7 @@ void yuuka_stream_destroy(yuuka_stream * stream) {
     if (stream->s) {
         cudaSetDevice(stream->dev->index);
         cudaStreamDestroy(stream->s);
+        stream->scratch.release();
     }
     delete stream;
 }

@@ -8,6 +8,7 @@
 #include <cstdint>
 #include <cstdio>
 #include <exception>
+#include <mutex>
 #include <new>
 #include <string>
 #include <utility>
@@ -86,9 +87,78 @@ struct yuuka_buffer {
     uint64_t bytes = 0;
 };
 
+namespace yk {
+// Small device and page-locked host areas that a stream keeps for the synchronous calls made on it (a call used to
+// allocate and free its own: about a millisecond of cudaMalloc and cudaFree). Freed with the stream; what a call
+// needs beyond KEEP is allocated for that call alone. `mutex` is held for the length of a call, so host threads may
+// share a stream.
+struct StreamScratch {
+    static constexpr size_t KEEP = 16u << 20;
+    std::mutex mutex;
+    uint8_t * device = nullptr;
+    uint8_t * host = nullptr;
+    size_t device_bytes = 0, host_bytes = 0;
+    void release() {
+        if (device) cudaFree(device);
+        if (host) cudaFreeHost(host);
+        device = host = nullptr;
+        device_bytes = host_bytes = 0;
+    }
+};
+// Areas of at least the given sizes for one call; the caller holds the mutex and has set the device.
+struct StreamScratchUse {
+    uint8_t * device = nullptr;
+    uint8_t * host = nullptr;
+    bool own_device = false, own_host = false;
+    StreamScratchUse(StreamScratch & sc, size_t device_bytes, size_t host_bytes) {
+        try {
+            device = take(sc.device, sc.device_bytes, device_bytes, own_device, false);
+            host = take(sc.host, sc.host_bytes, host_bytes, own_host, true);
+        } catch (...) {
+            drop();
+            throw;
+        }
+    }
+    ~StreamScratchUse() { drop(); }
+    StreamScratchUse(const StreamScratchUse &) = delete;
+    StreamScratchUse & operator=(const StreamScratchUse &) = delete;
+
+private:
+    void drop() {
+        if (own_device && device) cudaFree(device);
+        if (own_host && host) cudaFreeHost(host);
+    }
+    static uint8_t * take(uint8_t *& kept, size_t & have, size_t need, bool & own, bool pinned) {
+        if (need <= have) return kept;
+        own = need > StreamScratch::KEEP;
+        size_t size = need;
+        if (!own) {
+            size = 64u << 10;
+            while (size < need) size *= 2;
+            if (kept) (void)(pinned ? cudaFreeHost(kept) : cudaFree(kept));
+            kept = nullptr;
+            have = 0;
+        }
+        void * ptr = nullptr;
+        const cudaError_t err = pinned ? cudaMallocHost(&ptr, size) : cudaMalloc(&ptr, size);
+        if (err != cudaSuccess) {
+            cudaGetLastError();
+            own = false;
+            YK_REQUIRE(false, YUUKA_ERR_ALLOCATION, "scratch allocation of %llu bytes failed", (unsigned long long)size);
+        }
+        if (!own) {
+            kept = (uint8_t *)ptr;
+            have = size;
+        }
+        return (uint8_t *)ptr;
+    }
+};
+}  // namespace yk
+
 struct yuuka_stream {
     yuuka_device * dev = nullptr;
     cudaStream_t s = nullptr;
+    yk::StreamScratch scratch;
 };
 
 struct yuuka_event {
