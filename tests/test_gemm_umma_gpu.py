@@ -54,3 +54,20 @@ def test_umma_route_accumulates(dev):
     got = run_gemm(dev, w, dtype, n_out, n_in, x, cuda.PATH_MMA, accumulate=base)
     err, cos = stats(got, want)
     assert err <= 4e-3 and cos >= 0.999999, (err, cos)
+
+
+@pytest.mark.parametrize("n_out,n_in,rows", [
+    (128, 256, 48),      # one CTA of the pair has no rows of its own; one superblock
+    (257, 512, 255), (257, 512, 257),   # a row beyond the first pair; a tile one short of full and one row over
+    (1001, 1536, 97),    # K split with rows that 16-byte stores do not divide
+    (1000, 2560, 289),   # K split, two tiles of rows
+    (2560, 768, 513),
+])
+@pytest.mark.parametrize("dtype", [synth.Q4_K, synth.Q6_K])
+def test_umma_route_at_the_edges_of_its_tiles(dev, n_out, n_in, rows, dtype):
+    w = synth.normal_quant(n_out, n_in, dtype, 0.02, 5 + n_out)
+    x = synth.normal_f32(rows * n_in, 1.0, rows).reshape(rows, n_in)
+    want = yo.matmul(w, dtype, n_out, n_in, x)
+    got = run_gemm(dev, w, dtype, n_out, n_in, x, cuda.PATH_MMA)
+    err, cos = stats(got, want)
+    assert err <= 6e-3 and cos >= 0.999999, (err, cos)

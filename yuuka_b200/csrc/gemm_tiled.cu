@@ -23,6 +23,7 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <type_traits>
 
 #include "gemm_tiled.cuh"
 #include "quant.cuh"
@@ -61,6 +62,11 @@ __device__ __forceinline__ uint32_t h2_fma(uint32_t a, uint32_t b, uint32_t c) {
 __device__ __forceinline__ uint32_t h2_mul(uint32_t a, uint32_t b) {
     uint32_t d;
     asm("mul.rn.f16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
+    return d;
+}
+__device__ __forceinline__ uint32_t h2_add(uint32_t a, uint32_t b) {
+    uint32_t d;
+    asm("add.rn.f16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
     return d;
 }
 __device__ __forceinline__ uint32_t h2_sub(uint32_t a, uint32_t b) {
@@ -140,7 +146,6 @@ __device__ __forceinline__ int pos6(int t, int b) { return b < 4 ? 4 * t + b : 1
 
 template <> struct Codec<YUUKA_DTYPE_Q4_K> {
     static constexpr int SB = 144, REC = 16 * SB;
-    static constexpr int SCL_STRIDE = 80, MN_STRIDE = 48, MN_OFF = 16 * SCL_STRIDE, TAB = MN_OFF + 16 * MN_STRIDE;
     struct Regs { uint4 q[4]; uint4 hdr; };
     __device__ static void map(int p, int & r, int & o) {
         if (p < 2048) {
@@ -160,7 +165,6 @@ template <> struct Codec<YUUKA_DTYPE_Q4_K> {
 
 template <> struct Codec<YUUKA_DTYPE_Q5_K> {
     static constexpr int SB = 176, REC = 16 * SB;
-    static constexpr int SCL_STRIDE = 80, MN_STRIDE = 48, MN_OFF = 16 * SCL_STRIDE, TAB = MN_OFF + 16 * MN_STRIDE;
     struct Regs { uint4 q[4]; uint4 qh; uint4 hdr; };
     __device__ static void map(int p, int & r, int & o) {
         if (p < 2048) {
@@ -185,7 +189,6 @@ template <> struct Codec<YUUKA_DTYPE_Q5_K> {
 
 template <> struct Codec<YUUKA_DTYPE_Q6_K> {
     static constexpr int SB = 210, REC = 16 * SB;
-    static constexpr int SCL_STRIDE = 144, MN_STRIDE = 80, MN_OFF = 16 * SCL_STRIDE, TAB = MN_OFF + 16 * MN_STRIDE;
     struct Regs { uint4 ql[4]; uint4 qh[2]; uint4 sc; uint32_t d; };
     __device__ static void map(int p, int & r, int & o) {
         if (p < 2048) {
@@ -212,7 +215,6 @@ template <> struct Codec<YUUKA_DTYPE_Q6_K> {
 
 template <> struct Codec<YUUKA_DTYPE_Q8_0> {
     static constexpr int SB = 272, REC = 16 * SB;
-    static constexpr int SCL_STRIDE = 48, MN_OFF = 0, TAB = 16 * SCL_STRIDE;
     struct Regs { uint4 q[8]; uint4 d; };
     __device__ static void map(int p, int & r, int & o) {
         if (p < 4096) {
@@ -296,28 +298,7 @@ static void launch_xprep(cudaStream_t s, __half * xh, __half * xl, __half2 * xs1
 }
 
 // ===========================================================================
-// header decode -> per-warp tables, and the per-superblock MMA sequence
-
-// Q4_K / Q5_K header: hdr.x = d | dmin << 16, hdr.y/z/w = 12 scale bytes.
-// scl[row][pair j] = {s_lo, -1024 s_lo, s_hi/16, -64 s_hi} (half2 each); mn2[row][sub] = (-min, -min).
-template <typename C>
-__device__ __forceinline__ void header_k4(const uint4 & hdr, int lane, uint8_t * tab) {
-    const int r = lane & 15, hf = lane >> 4;  // hf: pairs 2hf, 2hf+1
-    const uint32_t d2 = dup_lo(hdr.x), dm2 = dup_hi(hdr.x);
-    const uint32_t w0 = hdr.y, w1 = hdr.z, w2 = hdr.w;
-    const uint32_t sc4 = hf ? ((w2 & 0x0f0f0f0fu) | ((w0 >> 2) & 0x30303030u)) : (w0 & 0x3f3f3f3fu);
-    const uint32_t mn4 = hf ? (((w2 >> 4) & 0x0f0f0f0fu) | ((w1 >> 2) & 0x30303030u)) : (w1 & 0x3f3f3f3fu);
-    uint4 * scl = reinterpret_cast<uint4 *>(tab + r * C::SCL_STRIDE) + hf * 2;
-    uint2 * mn2 = reinterpret_cast<uint2 *>(tab + C::MN_OFF + r * C::MN_STRIDE) + hf * 2;
-#pragma unroll
-    for (int jl = 0; jl < 2; jl++) {
-        const uint32_t sp = h2_mul(h2_sub(jl ? bytes23_h2(sc4) : bytes01_h2(sc4), H2_1024), d2);
-        const uint32_t mp = h2_mul(h2_sub(jl ? bytes23_h2(mn4) : bytes01_h2(mn4), H2_1024), dm2);
-        const uint32_t slo = dup_lo(sp), shi = dup_hi(sp);
-        scl[jl] = make_uint4(slo, h2_mul(slo, H2_NEG1024), h2_mul(shi, H2_INV16), h2_mul(shi, H2_NEG64));
-        mn2[jl] = make_uint2(h2_mul(dup_lo(mp), H2_NEG1), h2_mul(dup_hi(mp), H2_NEG1));
-    }
-}
+// decode
 
 // Bit masks and the fp16 "1024" pattern as run-time values (kernel parameters). A LOP3 takes one
 // immediate only; with two compile-time constants in (v & mask) | 0x6400'6400 the compiler emits two
@@ -337,82 +318,6 @@ inline DecodeConsts decode_consts(uint32_t dtype) {
     }
     return c;
 }
-
-// ---------------------------------------------------------------------------
-// Scaled decode (tensor-memory route, gemm_umma.cuh): block headers become per-warp tables of fp16
-// scales with which a packed weight turns into fp16(s * q) by one LOP3 and one fma.f16x2.
-
-template <int DT, int NT> struct Mma;
-
-template <int NT> struct Mma<YUUKA_DTYPE_Q4_K, NT> {
-    using C = Codec<YUUKA_DTYPE_Q4_K>;
-    __device__ static void header(const typename C::Regs & r, int lane, uint8_t * tab) { header_k4<C>(r.hdr, lane, tab); }
-};
-
-template <int NT> struct Mma<YUUKA_DTYPE_Q5_K, NT> {
-    using C = Codec<YUUKA_DTYPE_Q5_K>;
-    __device__ static void header(const typename C::Regs & r, int lane, uint8_t * tab) { header_k4<C>(r.hdr, lane, tab); }
-    // bit k of every byte of hb -> bit `tgt` of bytes 0 and 2 (shift_bytes13: of bytes 1 and 3 moved down)
-    // ... merged with the fp16 1024 pattern: ((hb shifted) & bit) | magic is one LOP3
-    template <int K, int TGT, bool B13> __device__ static uint32_t hibit(uint32_t hb, uint32_t bit, uint32_t magic) {
-        constexpr int from = K + (B13 ? 8 : 0);
-        if constexpr (from >= TGT) return and_or(hb >> (from - TGT), bit, magic);
-        else return and_or(hb << (TGT - from), bit, magic);
-    }
-    template <int K> __device__ static void sub(uint32_t vg, uint32_t vh, uint32_t hg, uint32_t hh, uint32_t s_g, uint32_t c_g,
-                                                uint32_t s_h, uint32_t c_h, uint32_t (&a)[4], const DecodeConsts & kc) {
-        constexpr bool hi = (K & 1) != 0;
-        constexpr int tgt = hi ? 8 : 4;
-        const uint32_t mask = hi ? kc.mf0 : kc.m0f, bit = hi ? kc.h8 : kc.h4;
-        a[0] = h2_fma(and_or(vg, mask, hibit<K, tgt, false>(hg, bit, kc.magic)), s_g, c_g);
-        a[1] = h2_fma(and_or(vh, mask, hibit<K, tgt, false>(hh, bit, kc.magic)), s_h, c_h);
-        a[2] = h2_fma(and_or(vg >> 8, mask, hibit<K, tgt, true>(hg, bit, kc.magic)), s_g, c_g);
-        a[3] = h2_fma(and_or(vh >> 8, mask, hibit<K, tgt, true>(hh, bit, kc.magic)), s_h, c_h);
-    }
-};
-
-// Q6_K: scl[row][s16] = {s', c'} with (s, -1024 s) where the value sits in a low nibble
-// (s16 % 8 < 4) and (s/16, -64 s) where it sits in a high nibble; mn2[row][s16] = (-32 s, -32 s).
-template <int NT> struct Mma<YUUKA_DTYPE_Q6_K, NT> {
-    using C = Codec<YUUKA_DTYPE_Q6_K>;
-    __device__ static void header(const typename C::Regs & r, int lane, uint8_t * tab) {
-        const int row = lane & 15, hf = lane >> 4;  // hf: groups 8hf .. 8hf+7
-        const uint32_t d2 = dup_lo(r.d);
-        const uint32_t wa = (hf ? r.sc.z : r.sc.x) ^ 0x80808080u;  // groups +0..3: low-nibble form
-        const uint32_t wb = (hf ? r.sc.w : r.sc.y) ^ 0x80808080u;  // groups +4..7: high-nibble form
-        uint2 * scl = reinterpret_cast<uint2 *>(tab + row * C::SCL_STRIDE) + hf * 8;
-        uint32_t * mn2 = reinterpret_cast<uint32_t *>(tab + C::MN_OFF + row * C::MN_STRIDE) + hf * 8;
-#pragma unroll
-        for (int q = 0; q < 4; q++) {
-            const uint32_t w = q < 2 ? wa : wb;
-            const uint32_t sp = h2_mul(h2_sub((q & 1) ? bytes23_h2(w) : bytes01_h2(w), H2_1152), d2);
-            const uint32_t s0 = dup_lo(sp), s1 = dup_hi(sp);
-            if (q < 2) {
-                scl[2 * q] = make_uint2(s0, h2_mul(s0, H2_NEG1024));
-                scl[2 * q + 1] = make_uint2(s1, h2_mul(s1, H2_NEG1024));
-            } else {
-                scl[2 * q] = make_uint2(h2_mul(s0, H2_INV16), h2_mul(s0, H2_NEG64));
-                scl[2 * q + 1] = make_uint2(h2_mul(s1, H2_INV16), h2_mul(s1, H2_NEG64));
-            }
-            mn2[2 * q] = h2_mul(s0, H2_NEG32);
-            mn2[2 * q + 1] = h2_mul(s1, H2_NEG32);
-        }
-    }
-};
-
-// Q8_0: scl[row][block] = (s, s).
-template <int NT> struct Mma<YUUKA_DTYPE_Q8_0, NT> {
-    using C = Codec<YUUKA_DTYPE_Q8_0>;
-    __device__ static void header(const typename C::Regs & r, int lane, uint8_t * tab) {
-        const int row = lane & 15, hf = lane >> 4;
-        const uint32_t da = hf ? r.d.z : r.d.x, db = hf ? r.d.w : r.d.y;
-        uint32_t * scl = reinterpret_cast<uint32_t *>(tab + row * C::SCL_STRIDE) + hf * 4;
-        scl[0] = dup_lo(da);
-        scl[1] = dup_hi(da);
-        scl[2] = dup_lo(db);
-        scl[3] = dup_hi(db);
-    }
-};
 
 // ---------------------------------------------------------------------------
 // Exact decode (register-fed route, 1..16 activation rows per launch). The fp16 operand of the tensor core
@@ -591,6 +496,23 @@ template <int NT> struct XMma<YUUKA_DTYPE_Q5_K, NT> {
     using C = Codec<YUUKA_DTYPE_Q5_K>;
     using X = XTab<YUUKA_DTYPE_Q5_K>;
     __device__ static void header(const typename C::Regs & r, int lane, uint8_t * tab) { header_k4_exact<X>(r.hdr, lane, tab); }
+    // bit k of every byte of hb -> bit `tgt` of bytes 0 and 2 (shift_bytes13: of bytes 1 and 3 moved down)
+    // ... merged with the fp16 1024 pattern: ((hb shifted) & bit) | magic is one LOP3
+    template <int K, int TGT, bool B13> __device__ static uint32_t hibit(uint32_t hb, uint32_t bit, uint32_t magic) {
+        constexpr int from = K + (B13 ? 8 : 0);
+        if constexpr (from >= TGT) return and_or(hb >> (from - TGT), bit, magic);
+        else return and_or(hb << (TGT - from), bit, magic);
+    }
+    template <int K> __device__ static void sub(uint32_t vg, uint32_t vh, uint32_t hg, uint32_t hh, uint32_t s_g, uint32_t c_g,
+                                                uint32_t s_h, uint32_t c_h, uint32_t (&a)[4], const DecodeConsts & kc) {
+        constexpr bool hi = (K & 1) != 0;
+        constexpr int tgt = hi ? 8 : 4;
+        const uint32_t mask = hi ? kc.mf0 : kc.m0f, bit = hi ? kc.h8 : kc.h4;
+        a[0] = h2_fma(and_or(vg, mask, hibit<K, tgt, false>(hg, bit, kc.magic)), s_g, c_g);
+        a[1] = h2_fma(and_or(vh, mask, hibit<K, tgt, false>(hh, bit, kc.magic)), s_h, c_h);
+        a[2] = h2_fma(and_or(vg >> 8, mask, hibit<K, tgt, true>(hg, bit, kc.magic)), s_g, c_g);
+        a[3] = h2_fma(and_or(vh >> 8, mask, hibit<K, tgt, true>(hh, bit, kc.magic)), s_h, c_h);
+    }
     template <int K>
     __device__ static void subblock(const typename C::Regs & r, const uint8_t * tg, const uint8_t * th,
                                     const uint8_t * const (&xrow)[NT], int sbl, float (&q)[NT][4], const DecodeConsts & kc) {
@@ -603,7 +525,7 @@ template <int NT> struct XMma<YUUKA_DTYPE_Q5_K, NT> {
         uint32_t a[2][4];
 #pragma unroll
         for (int h = 0; h < 2; h++)
-            Mma<YUUKA_DTYPE_Q5_K, 1>::template sub<K>(qg[2 * jl + h], qh[2 * jl + h], hg[h], hh[h], s_g, c_g, s_h, c_h, a[h], kc);
+            sub<K>(qg[2 * jl + h], qh[2 * jl + h], hg[h], hh[h], s_g, c_g, s_h, c_h, a[h], kc);
 #pragma unroll
         for (int jt = 0; jt < NT; jt++) {
             const uint4 b = *reinterpret_cast<const uint4 *>(xrow[jt] + (sbl * 256 + 32 * K) * 2);
@@ -1477,44 +1399,44 @@ static bool umma_enabled() {
     return on;
 }
 
-// K splits of the tensor-memory route: enough CTAs to fill the machine when the matrix has few
-// 128-row blocks, at least two superblocks each. `separate` (may be null: then the in-kernel sum is the only
-// choice) is set when the parts are summed by a kernel of their own.
-static bool umma_specialised();
-static int umma_ksplit(const yuuka_device * dev, int n_out, int n_in, int rows, bool * separate) {
+// How a launch of the tensor-memory kernel is cut: m activation rows into n_tiles tiles of n_tile rows, K into kparts.
+struct UmmaPlan {
+    int n_tile, n_tiles, kparts;
+};
+// K parts: enough pairs of CTAs to fill the machine when the matrix has few blocks of rows, at least two superblocks each.
+// Two parts do not pay for the launch that sums them (9216 x 2560 at 576 rows: 47 us against 39), and without 16-byte
+// stores that sum is four times the loads, so fewer parts pay. (The count does not depend on how the rows are tiled: the
+// sums, and with them the bits of a row's result, do not change with the rows that travel with it, up to 96 rows and
+// beyond where n_out is not a multiple of four.)
+static int umma_kparts(const yuuka_device * dev, int n_out, int n_in, int m) {
     const int n_blocks = (n_out + UM_ROWS - 1) / UM_ROWS, nsb = n_in / 256;
     int ks = dev->sm_count / n_blocks;
     if (ks > nsb / 2) ks = nsb / 2;
-    if (separate) *separate = false;
-    static const bool no_separate = [] { const char * e = getenv("YUUKA_CUDA_UMMA_INLINE_SUM"); return e && e[0] == '1'; }();
-    // The decode of a narrow matrix (20 blocks of a 2560-row one) is spread over the whole machine and the parts
-    // are summed by every SM in a second launch; the output must allow 16-byte stores. Measured on 2560 x 9216
-    // against the in-kernel sum below: 38 vs 53-62 us at 48-96 rows, 59 vs 192 us at 512.
-    if (separate && !no_separate && ks > 2 && (n_out & 3) == 0 && umma_specialised()) {
-        *separate = true;
-        return ks < 8 ? ks : 8;
-    }
-    // the last CTA of a block sums the parts alone: measured on 2560-row matrices, four parts pay up to
-    // about 96 activation rows and two beyond (the sum grows with rows x parts, the decode it hides does not)
-    const int cap = rows <= 96 ? 4 : 2;
+    const int cap = (n_out & 3) == 0 ? 8 : (m <= 96 ? 4 : 1);
     if (ks > cap) ks = cap;
-    return ks < 1 ? 1 : ks;
+    return ks <= 2 ? 1 : ks;
 }
-
-static bool umma_specialised() {
-    static const bool on = [] { const char * e = getenv("YUUKA_CUDA_UMMA_WS"); return !(e && e[0] == '0'); }();
-    return on;
-}
-
-// Activation rows of one tensor-memory launch. YUUKA_CUDA_UMMA_ROWS=256 keeps the warp-specialised kernel to one
-// accumulator.
-static int umma_rows_per_launch() {
-    static const int rows = [] {
-        const char * e = getenv("YUUKA_CUDA_UMMA_ROWS");
-        const int want = e ? atoi(e) : UM_MAX_N2;
-        return want > UM_MAX_N && umma_specialised() ? UM_MAX_N2 : UM_MAX_N;
-    }();
-    return rows;
+// The tiling of the rows with the lowest estimate of cycles: rounds of the pairs x (stages of a tile x cycles per stage +
+// a fixed cost for filling and draining the rings). A stage took 634 / 682 / 774 / 890 cycles at 64 / 128 / 192 / 256
+// activation rows per tile (248320 x 2560 Q6_K): the decode of 8192 weights and its barriers, and 1.3 cycles per row on top.
+constexpr double UMMA_STAGE = 540.0, UMMA_ROW = 1.3, UMMA_TILE = 4000.0;
+static UmmaPlan umma_plan(const yuuka_device * dev, int n_out, int n_in, int m) {
+    const int m_blocks = (n_out + 2 * UM_ROWS - 1) / (2 * UM_ROWS), nsb = n_in / 256, pairs = dev->sm_count / 2;
+    UmmaPlan best{0, 0, umma_kparts(dev, n_out, n_in, m)};
+    double best_cost = 1e30;
+    const int t0 = (m + UM_MAX_N - 1) / UM_MAX_N, stages = (nsb + best.kparts - 1) / best.kparts * 4;
+    for (int tiles = t0; tiles <= t0 + 4; tiles++) {
+        const int n_tile = ((m + tiles - 1) / tiles + 31) / 32 * 32;
+        if ((m + n_tile - 1) / n_tile != tiles) continue;  // the same cut as a smaller count
+        const int rounds = (m_blocks * tiles * best.kparts + pairs - 1) / pairs;
+        const double cost = rounds * (stages * (UMMA_STAGE + UMMA_ROW * n_tile) + UMMA_TILE);
+        if (cost < best_cost) {
+            best_cost = cost;
+            best.n_tile = n_tile;
+            best.n_tiles = tiles;
+        }
+    }
+    return best;
 }
 
 void gemm_tiled_scratch_need(const yuuka_device * dev, uint32_t w_dtype, int rows, int n_out, int n_in,
@@ -1522,26 +1444,10 @@ void gemm_tiled_scratch_need(const yuuka_device * dev, uint32_t w_dtype, int row
     *partial_floats = 0;
     *counters = 0;
     if (!tiled_supported(w_dtype, n_in)) return;
-    if (rows >= UMMA_EARLY_ROWS) {
-        const int per_launch = rows < umma_rows_per_launch() ? rows : umma_rows_per_launch();
-        // enough for this row count and for every smaller one (fewer rows may split K further)
-        int ks = 1, worst = 0;
-        for (int m = UMMA_EARLY_ROWS; m <= per_launch; m += (m < UMMA_MIN_ROWS ? UMMA_MIN_ROWS - m : 16)) {
-            bool sep;
-            const int k = umma_ksplit(dev, n_out, n_in, m, &sep);
-            if (k > ks) ks = k;
-            if (k * m > worst) worst = k * m;
-        }
-        {
-            bool sep;
-            const int k = umma_ksplit(dev, n_out, n_in, per_launch, &sep);
-            if (k > ks) ks = k;
-            if (k * per_launch > worst) worst = k * per_launch;
-        }
-        if (ks > 1) {
-            *partial_floats = (uint64_t)worst * n_out;
-            *counters = (n_out + UM_ROWS - 1) / UM_ROWS;
-        }
+    // enough for this row count and for every smaller one (fewer rows may split K further)
+    for (int m : {rows, rows < 96 ? rows : 96}) {
+        const int parts = rows >= UMMA_EARLY_ROWS ? umma_kparts(dev, n_out, n_in, m) : 1;
+        if (parts > 1 && (uint64_t)parts * m * n_out > *partial_floats) *partial_floats = (uint64_t)parts * m * n_out;
     }
     for (int m : {rows < MMA_ROWS ? rows : MMA_ROWS, MMA_ROWS < rows ? rows % MMA_ROWS : 0}) {
         if (m <= 0) continue;
@@ -1682,8 +1588,6 @@ typedef CUresult (*TensorMapEncodeFn)(CUtensorMap *, CUtensorMapDataType, cuuint
                                       CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
 static TensorMapEncodeFn tensor_map_encoder() {
     static const TensorMapEncodeFn fn = [] {
-        const char * e = getenv("YUUKA_CUDA_NO_TMA");
-        if (e && e[0] == '1') return (TensorMapEncodeFn) nullptr;
         void * f = nullptr;
         cudaDriverEntryPointQueryResult q;
         if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &f, cudaEnableDefault, &q) != cudaSuccess ||
@@ -1696,90 +1600,63 @@ static TensorMapEncodeFn tensor_map_encoder() {
     return fn;
 }
 
-// 2-D map over prepared activations [m][k] (fp16, row-major): boxes of 64 columns x npad rows, 128-byte swizzle.
-static bool make_x_map(CUtensorMap * map, const __half * xh, int m, int k, int npad) {
+// 2-D map over prepared activations [m][k] (fp16, row-major): boxes of 64 columns x box_rows, 128-byte swizzle, rows beyond
+// m read as zero.
+static void make_x_map(CUtensorMap * map, const __half * xh, int m, int k, int box_rows) {
     TensorMapEncodeFn enc = tensor_map_encoder();
-    if (!enc || ((uintptr_t)xh & 15) != 0) return false;
+    YK_REQUIRE(enc, YUUKA_ERR_DEVICE, "umma gemm: the driver has no tensor-map encoder");
     const cuuint64_t gdim[2] = {(cuuint64_t)k, (cuuint64_t)m};
     const cuuint64_t gstride[1] = {(cuuint64_t)k * 2};
-    const cuuint32_t box[2] = {(cuuint32_t)UM_KC, (cuuint32_t)npad};
+    const cuuint32_t box[2] = {(cuuint32_t)UM_KC, (cuuint32_t)box_rows};
     const cuuint32_t estr[2] = {1, 1};
-    return enc(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, (void *)xh, gdim, gstride, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-               CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+    YK_REQUIRE(enc(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, (void *)xh, gdim, gstride, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                   CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS,
+               YUUKA_ERR_INTERNAL, "umma gemm: the tensor map of the activations could not be encoded");
 }
 
 template <int DT>
 static int launch_umma_dt(const yuuka_device * dev, cudaStream_t s, const TiledGemmArgs & a, const __half * xh) {
-    int launches = 0;
-    const int n_blocks = (a.n_out + UM_ROWS - 1) / UM_ROWS;
-    // rows per launch: 512 (two accumulators) with tensor-map copies and the warp-specialised kernel, 256 with the
-    // one-accumulator kernel; the padded cp.async stages are larger, so fewer fit
-    const bool want_tma = tensor_map_encoder() != nullptr;
-    const bool ws = want_tma && umma_specialised();
-    int max_n = ws ? umma_rows_per_launch() : UM_MAX_N;
-    while (!want_tma && max_n > 16 &&
-           (size_t)(UM_STAGES - 1) * (UM_A_BYTES + (size_t)(max_n / 8) * UM_B_SBO) + (size_t)TW * Codec<DT>::TAB + 1024 >
-               dev->prop.sharedMemPerBlockOptin)
-        max_n -= 16;
-    for (int m0 = 0; m0 < a.rows; m0 += max_n) {
-        const int m = a.rows - m0 < max_n ? a.rows - m0 : max_n;
-        bool separate = false;
-        const int ksplit = umma_ksplit(dev, a.n_out, a.n_in, m, ws && (a.ldo & 3) == 0 && ((uintptr_t)a.out & 15) == 0 ? &separate : nullptr);
-        UParams p{};
-        p.kc = decode_consts(DT);
-        p.w = a.w;
-        p.N = a.n_out;
-        p.nsb = a.n_in / 256;
-        p.xh = xh + (int64_t)m0 * a.n_in;
-        p.M = m;
-        p.npad = (m + 15) / 16 * 16;
-        p.out = a.out + (int64_t)m0 * a.ldo;
-        p.ldo = a.ldo;
-        p.accumulate = (a.flags & YUUKA_GEMM_ACCUMULATE) ? 1 : 0;
-        p.tmem_cols = 32;
-        while ((int)p.tmem_cols < p.npad) p.tmem_cols *= 2;
-        // instruction descriptor: D f32, A and B f16, both K-major, N = rows of the accumulator, M = 128
-        const int n1 = p.npad < UM_MAX_N ? p.npad : UM_MAX_N;
-        p.idesc = (1u << 4) | ((uint32_t)(n1 >> 3) << 17) | ((uint32_t)(UM_ROWS >> 4) << 24);
-        p.idesc2 = p.npad > UM_MAX_N ? (1u << 4) | ((uint32_t)((p.npad - UM_MAX_N) >> 3) << 17) | ((uint32_t)(UM_ROWS >> 4) << 24) : 0u;
-        p.box_rows = (uint32_t)n1;
-        if (ksplit > 1) {
-            YK_REQUIRE(a.scratch && a.scratch->partial_floats >= (uint64_t)ksplit * m * a.n_out &&
-                           a.scratch->counter_count >= n_blocks,
-                       YUUKA_ERR_INTERNAL, "umma gemm: split-K scratch is too small");
-            p.partial = a.scratch->partial;
-            p.counters = separate ? nullptr : a.scratch->counters;
-        }
-        alignas(64) CUtensorMap xmap;
-        memset(&xmap, 0, sizeof(xmap));
-        const bool tma = want_tma && make_x_map(&xmap, p.xh, m, a.n_in, (int)p.box_rows);
-        YK_REQUIRE(tma || !want_tma, YUUKA_ERR_INTERNAL, "umma gemm: the tensor map of the activations could not be encoded");
-        const size_t b_bytes = tma ? (size_t)(p.idesc2 ? 2 : 1) * p.box_rows * 128 : (size_t)(p.npad / 8) * UM_B_SBO;
-        p.stages = UM_STAGES;
-        const size_t tab_bytes = (size_t)(ws ? UM_DW : TW) * Codec<DT>::TAB;
-        size_t smem = (size_t)p.stages * (UM_A_BYTES + b_bytes) + tab_bytes + 1024;
-        while (smem > dev->prop.sharedMemPerBlockOptin && p.stages > 2) {
-            p.stages--;
-            smem = (size_t)p.stages * (UM_A_BYTES + b_bytes) + tab_bytes + 1024;
-        }
-        YK_REQUIRE(smem <= dev->prop.sharedMemPerBlockOptin, YUUKA_ERR_INTERNAL, "umma gemm: stage buffers do not fit shared memory");
-        auto kern = ws ? gemm_umma_ws_kernel<DT> : (tma ? gemm_umma_kernel<DT, true> : gemm_umma_kernel<DT, false>);
-        YK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        const int per_split = dev->sm_count / ksplit > 0 ? dev->sm_count / ksplit : 1;
-        dim3 grid(n_blocks < per_split ? n_blocks : per_split, ksplit);
-        launch_k(kern, grid, ws ? UM_WS_THREADS : TW * 32, smem, s, p, xmap);
-        YK_CUDA(cudaGetLastError());
-        launches++;
-        if (separate && ksplit > 1) {
-            const int64_t quads = (int64_t)m * (a.n_out / 4);
-            const int64_t want = (quads + 255) / 256, most = (int64_t)dev->sm_count * 8;
-            launch_k(umma_reduce_kernel, (int)(want < most ? want : most), 256, 0, s, p.out, p.ldo, (const float *)p.partial, ksplit, m,
-                     a.n_out, p.accumulate);
-            YK_CUDA(cudaGetLastError());
-            launches++;
-        }
+    using S = UmmaStage<DT>;
+    const UmmaPlan pl = umma_plan(dev, a.n_out, a.n_in, a.rows);
+    UParams p{};
+    p.kc = decode_consts(DT);
+    p.w = a.w;
+    p.N = a.n_out;
+    p.nsb = a.n_in / 256;
+    p.M = a.rows;
+    p.out = a.out;
+    p.ldo = a.ldo;
+    p.accumulate = (a.flags & YUUKA_GEMM_ACCUMULATE) ? 1 : 0;
+    p.kparts = pl.kparts;
+    p.n_tile = pl.n_tile;
+    p.n_tiles = pl.n_tiles;
+    p.m_blocks = (a.n_out + 2 * UM_ROWS - 1) / (2 * UM_ROWS);
+    // instruction descriptor: D f32, A and B f16, both K-major, N = activation rows of the tile, M = 256 (the pair)
+    p.idesc = (1u << 4) | ((uint32_t)(pl.n_tile >> 3) << 17) | ((uint32_t)(2 * UM_ROWS >> 4) << 24);
+    if (pl.kparts > 1) {
+        YK_REQUIRE(a.scratch && a.scratch->partial_floats >= (uint64_t)pl.kparts * a.rows * a.n_out, YUUKA_ERR_INTERNAL,
+                   "umma gemm: split-K scratch is too small");
+        p.partial = a.scratch->partial;
     }
-    return launches;
+    alignas(64) CUtensorMap xmap;
+    make_x_map(&xmap, xh, a.rows, a.n_in, pl.n_tile / 2);
+    const size_t fixed = (size_t)UM_RAW_STAGES * S::RAW_BYTES + (size_t)UM_DW * HalfRecord<DT>::TAB + 1024,
+                 stage = (size_t)UM_A_BYTES + (size_t)pl.n_tile * 64;
+    p.stages = UM_MAX_STAGES;
+    while (fixed + p.stages * stage + 1024 > dev->prop.sharedMemPerBlockOptin && p.stages > 2) p.stages--;
+    const size_t smem = fixed + p.stages * stage;
+    YK_REQUIRE(smem + 1024 <= dev->prop.sharedMemPerBlockOptin, YUUKA_ERR_INTERNAL, "umma gemm: stage buffers do not fit shared memory");
+    YK_CUDA(cudaFuncSetAttribute(gemm_umma_kernel<DT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    const int items = p.m_blocks * p.n_tiles * p.kparts, pairs = dev->sm_count / 2;
+    launch_k_cluster(gemm_umma_kernel<DT>, dim3(2 * (items < pairs ? items : pairs)), UM_THREADS, smem, s, 2, p, xmap);
+    YK_CUDA(cudaGetLastError());
+    if (pl.kparts == 1) return 1;
+    const bool vec = (a.n_out & 3) == 0 && (a.ldo & 3) == 0 && ((uintptr_t)a.out & 15) == 0;
+    const int64_t want = ((int64_t)a.rows * (a.n_out / (vec ? 4 : 1)) + 255) / 256, most = (int64_t)dev->sm_count * 8;
+    launch_k(vec ? umma_reduce_kernel<4> : umma_reduce_kernel<1>, (int)(want < most ? want : most), 256, 0, s, p.out, p.ldo,
+             (const float *)p.partial, pl.kparts, a.rows, a.n_out, p.accumulate);
+    YK_CUDA(cudaGetLastError());
+    return 2;
 }
 
 template <int DT>
@@ -1909,9 +1786,7 @@ static void preload_dt() {
     YK_CUDA(cudaFuncGetAttributes(&fa, gemm_tiled_mma_kernel<DT, 4, false, false>));
     YK_CUDA(cudaFuncGetAttributes(&fa, gemm_tiled_fp32_kernel<DT, float>));
     YK_CUDA(cudaFuncGetAttributes(&fa, gemm_tiled_fp32_kernel<DT, __nv_bfloat16>));
-    YK_CUDA(cudaFuncGetAttributes(&fa, gemm_umma_ws_kernel<DT>));
-    YK_CUDA(cudaFuncGetAttributes(&fa, gemm_umma_kernel<DT, true>));
-    YK_CUDA(cudaFuncGetAttributes(&fa, gemm_umma_kernel<DT, false>));
+    YK_CUDA(cudaFuncGetAttributes(&fa, gemm_umma_kernel<DT>));
 }
 void gemm_tiled_preload_kernels() {
     cudaFuncAttributes fa;
@@ -1921,7 +1796,8 @@ void gemm_tiled_preload_kernels() {
     preload_dt<YUUKA_DTYPE_Q8_0>();
     YK_CUDA(cudaFuncGetAttributes(&fa, xprep_kernel<float>));
     YK_CUDA(cudaFuncGetAttributes(&fa, xprep_kernel<__nv_bfloat16>));
-    YK_CUDA(cudaFuncGetAttributes(&fa, umma_reduce_kernel));
+    YK_CUDA(cudaFuncGetAttributes(&fa, umma_reduce_kernel<4>));
+    YK_CUDA(cudaFuncGetAttributes(&fa, umma_reduce_kernel<1>));
     tensor_map_encoder();  // the driver entry point look-up happens once, here
 }
 

@@ -2,194 +2,257 @@
 // accumulator in tensor memory. Included by gemm_tiled.cu (it uses that file's
 // record codecs and header decoders).
 //
-// From 48 rows on (33 on request), re-decoding the packed weights for every 16-row pass of the
-// register-fed MMA kernel costs more than the arithmetic. Here a CTA owns 128 weight rows and up to
-// 256 activation rows (512 in the warp-specialised kernel, on two accumulators): eight warps decode one
-// 16-row tile each into fp16 (s * q - min, rounded: this route does not have the register-fed route's
-// exactness), 64 columns at a time, and store it into a shared-memory stage in the K-major core-matrix
-// layout (8 rows x 16 bytes, no swizzle); the matching 64 columns of the prepared activations (their fp16
-// hi halves) arrive in the same stage by a tensor-map copy (cp.async where the encoder is not available).
-// One thread then issues four tcgen05.mma (M = 128, N = rows padded to 16, K = 16 each) that accumulate
-// D[weight row][activation row] in tensor memory, and tcgen05.commit releases the stage through an
-// mbarrier when they have read it. The ring of stages lets decoding run ahead of the tensor pipe. The
-// epilogue reads the accumulator with tcgen05.ld (lane = weight row, column = activation row) and writes
-// out[row][n], 128 bytes per warp store.
+// From 48 rows on (33 on request), re-decoding the packed weights for every 16-row pass of the register-fed
+// kernel costs more than the arithmetic. Here two CTAs of a cluster form a pair on one tile of 256 weight rows x up to
+// 256 activation rows (cta_group::2, M = 256): each CTA decodes its own 128 weight rows into fp16 (s * q - min, rounded:
+// this route does not have the register-fed route's exactness), 64 columns at a time, and fetches half of the
+// tile's activation rows (their fp16 hi halves, a tensor-map copy). The even CTA issues the MMAs of both; each CTA reads its own half of D back.
 //
-// Every mbarrier wait is bounded; on expiry the device error word is set, the
-// kernel carries on (results are then garbage), frees its tensor memory and
-// returns.
+// What bounds it, and why this tile. At M = 128 per CTA a stage of 64 columns keeps the tensor pipe busy for two cycles
+// per activation row of the tile. Its activations come from L2, which feeds all SMs 46 bytes per cycle each
+// (13 TB/s measured): one CTA alone on 256 activation rows needs 64 bytes per cycle, a pair that shares them 32. The decode
+// of a stage (8192 weights per SM) takes 500 to 600 cycles with its barriers, so tiles
+// of up to about 200 rows are bound by the decode and wider ones by both. Tensor memory holds two accumulators of 256 columns: the
+// epilogue of a tile runs on warps of its own while the next tile is decoded and multiplied.
+// Calls on a B200, before (one CTA per 128 rows, 512 activation rows) and after: 9216 x 2560 Q4_K at 576 rows 115 -> 39 us,
+// 18432 x 2560 at 512 rows 55 -> 46 us; 248320 x 2560 Q6_K at 48 rows 367 -> 195 us (2.7 TB/s of weights), at 512 rows
+// 623 -> 530 us (1.2 PFLOP/s).
+//
+// Roles of a CTA's warps: sixteen decode warps (two per 16-row tile), four epilogue warps, one warp that copies packed
+// weights (one bulk copy per record, a superblock of all eight tiles per stage, ahead of everything else), one that copies
+// activations, one that issues the MMAs (even CTA) or passes on that the activations have landed (odd CTA).
+// Every mbarrier wait is bounded; on expiry the device error word is set, the kernel carries on (results are then
+// garbage), frees its tensor memory and returns.
 #pragma once
 
 namespace yk {
 
-constexpr int UM_ROWS = 128;   // weight rows per CTA = UMMA M
-constexpr int UM_KC = 64;      // columns per stage
-constexpr int UM_STAGES = 4;
-constexpr int UM_AHEAD = 2;    // chunks of activations in flight ahead of the decode
-constexpr int UM_MAX_N = 256;  // activation rows of one accumulator = UMMA N
-constexpr int UM_MAX_N2 = 512; // activation rows per launch of the warp-specialised kernel: two accumulators fill tensor memory
-// Weight stage: dense core matrices. Padding them to 160 bytes removes the four-way bank conflicts of the
-// decode warps' 16-byte stores and measured the same overall (56.3 vs 55.8 us on 18432 x 2560 at 256 rows),
-// so the smaller stage is kept; -DYK_UMMA_A_LBO=160 builds the padded form.
-#ifndef YK_UMMA_A_LBO
-#define YK_UMMA_A_LBO 128
-#endif
-constexpr int UM_A_LBO = YK_UMMA_A_LBO;
-constexpr int UM_A_SBO = 8 * UM_A_LBO;                // one group of eight rows
-constexpr int UM_A_BYTES = (UM_ROWS / 8) * UM_A_SBO;  // 16 KB
-// Activation stage: core matrices 144 bytes apart along K (16 bytes of padding each), so that the eight
-// 16-byte pieces of one row, copied by eight neighbouring lanes from 128 contiguous global bytes,
-// land in different banks.
-constexpr int UM_B_LBO = 144;
-constexpr int UM_B_SBO = 8 * UM_B_LBO;  // one group of eight rows
+constexpr int UM_ROWS = 128;     // weight rows per CTA; a pair has 256
+constexpr int UM_KC = 64;        // columns per stage
+constexpr int UM_MAX_N = 256;    // activation rows per tile
+constexpr int UM_MAX_STAGES = 6;
+constexpr int UM_RAW_STAGES = 2; // superblocks of packed weights in shared memory
+constexpr int UM_TILES = 8;      // 16-row tiles per CTA
+constexpr int UM_DW = 16;        // decode warps, two per tile: a half of every record each
+constexpr int UM_EW = 4;         // epilogue warps, one per quarter of the tensor-memory lanes
+constexpr int UM_WARP_RAW = UM_DW + UM_EW, UM_WARP_X = UM_WARP_RAW + 1, UM_WARP_MMA = UM_WARP_X + 1;
+constexpr int UM_THREADS = (UM_WARP_MMA + 1) * 32;
+static_assert(UM_TILES * 16 == UM_ROWS && UM_DW == 2 * UM_TILES, "two decode warps per tile");
+constexpr uint32_t H2_1024B = 0x64646464u, H2_ONE16 = 0x3C003C00u;
+
+constexpr int UM_A_BYTES = UM_ROWS * 128;      // a weight stage: 128 rows of 64 columns
+template <int DT> struct UmmaStage { static constexpr int RAW_BYTES = UM_TILES * Codec<DT>::REC; };
 
 struct UParams {
     DecodeConsts kc;
     const uint8_t * w;
     int N, nsb;           // weight rows, superblocks per row
-    const __half * xh;    // prepared activations [M][nsb * 256]
-    int M, npad;          // activation rows, padded to a multiple of 16
+    int M;                // activation rows
     float * out;
     int64_t ldo;
     int accumulate;
-    uint32_t tmem_cols;   // power of two >= npad, >= 32
+    float * partial;      // [kparts][M][N] when K is split across pairs
+    int kparts;
+    int n_tile, n_tiles;  // activation rows per tile (a multiple of 32), tiles
+    int m_blocks;         // blocks of 256 weight rows
     uint32_t idesc;
-    uint32_t idesc2;      // second accumulator (rows 256...), warp-specialised kernel with more than 256 rows; else 0
-    uint32_t box_rows;    // rows of one tensor-map box: npad, or 256 with two accumulators
-    uint32_t stages;      // ring depth: UM_STAGES, or fewer when four stages do not fit shared memory (at least 2)
-    float * partial;      // [gridDim.y][M][N] when K is split across CTAs
-    int * counters;       // one per block of 128 weight rows, zero between launches
+    uint32_t stages;      // ring depth
 };
 
-// K-major, 128-byte swizzle: rows of 64 halves (128 bytes), eight rows per 1024-byte atom, as a tensor-map
+// Both operands: K-major, 128-byte swizzle: rows of 64 halves (128 bytes), eight rows per 1024-byte atom, as a tensor-map
 // copy with CU_TENSOR_MAP_SWIZZLE_128B lays them out. 16 columns further along K = 32 bytes.
 __device__ __forceinline__ uint64_t umma_desc_sw128(uint32_t smem_addr) {
     return (uint64_t)((smem_addr >> 4) & 0x3fffu) | ((uint64_t)1u << 16) | ((uint64_t)(1024u >> 4) << 32) | (1ull << 46) |
            (2ull << 61);
 }
+// where 16-byte piece c (eight columns) of row r of a stage lies in that layout
+__device__ __forceinline__ uint32_t sw128(int r, int c) { return (uint32_t)(r * 128 + ((c ^ (r & 7)) << 4)); }
 
-// ---- scaled fragments of one 32-column sub-block K of a record, as the register-fed kernel forms
-// them: a[h][0], a[h][2] = row g, elements 8t + 4h + {0,1}, {2,3}; a[h][1], a[h][3] = row g + 8.
-// `mg`, `mh` receive the half2 that still has to be added (-min, or -32 * scale for Q6_K).
-__device__ __forceinline__ uint32_t h2_add(uint32_t a, uint32_t b) {
+// ---------------------------------------------------------------------------
+// Decode of half a record: 16 rows x 128 columns, two stages of 64, by one warp. fetch() takes the warp's share of a
+// record out of shared memory; header() turns the block headers into fp16 scales in the warp's own table; store<c>()
+// writes 64 columns (sub-blocks 2c, 2c + 1 of the half) as fp16(s * q - min): lane (g, t) holds rows g and g + 8 and eight
+// columns of each sub-block. Rows of odd g take the two sub-blocks in the other order: the lanes of a store then hit
+// every bank once in the swizzled layout (in the same order rows g and g + 1 would share theirs).
+// Two warps share a tile, a half each: a stage costs a warp about as much in barriers, fences and header work (400 cycles)
+// as in arithmetic (380), so that two warps per scheduler leave it idle half the time.
+
+// (v & mask) | magic is fp16 1024 + q (low nibble) or 1024 + 16 q (high nibble); times s plus -1024 s, or times s / 16 plus -64 s,
+// gives s * q; then the min is added
+__device__ __forceinline__ uint32_t nibble_h2(uint32_t v, uint32_t mask, uint32_t extra, uint32_t s, uint32_t c, uint32_t m) {
+    return h2_add(h2_fma(and_or(v, mask, extra), s, c), m);
+}
+
+template <int DT> struct HalfRecord;
+
+// Q4_K / Q5_K: table rows of 48 bytes: two pairs of sub-blocks (s_lo, -1024 s_lo, s_hi / 16, -64 s_hi); then rows of four (-min, -min)
+template <int DT> struct HalfRecordK4 {
+    static constexpr int DS = 48, MN_OFF = 16 * DS, TAB = MN_OFF + 16 * 16;
+    uint4 qg, qh, hdr;
+    __device__ void fetch_k4(const uint8_t * rec, int lane, int half, int hdr_at) {
+        const uint4 * p = reinterpret_cast<const uint4 *>(rec);
+        qg = p[half * 32 + lane];
+        qh = p[(2 + half) * 32 + lane];
+        hdr = p[hdr_at + (lane & 15)];
+    }
+    // hdr.x = d | dmin << 16, hdr.y/z/w = 12 scale bytes (getScaleMinK4, tensor/quant.go:96-103); lane: row, pair of sub-blocks
+    __device__ void header(int lane, int half, uint8_t * tab) const {
+        const int r = lane & 15, jl = lane >> 4;
+        const uint32_t w0 = hdr.y, w1 = hdr.z, w2 = hdr.w;
+        const uint32_t sc4 = half ? ((w2 & 0x0f0f0f0fu) | ((w0 >> 2) & 0x30303030u)) : (w0 & 0x3f3f3f3fu);
+        const uint32_t mn4 = half ? (((w2 >> 4) & 0x0f0f0f0fu) | ((w1 >> 2) & 0x30303030u)) : (w1 & 0x3f3f3f3fu);
+        const uint32_t sel = jl ? 0x4342u : 0x4140u;  // the pair's two bytes as fp16 1024 + b
+        const uint32_t sp = h2_mul(h2_sub(__byte_perm(sc4, H2_1024B, sel), H2_1024), dup_lo(hdr.x));
+        const uint32_t mp = h2_mul(h2_sub(__byte_perm(mn4, H2_1024B, sel), H2_1024), dup_hi(hdr.x));
+        const uint32_t slo = dup_lo(sp), shi = dup_hi(sp);
+        reinterpret_cast<uint4 *>(tab + r * DS)[jl] = make_uint4(slo, h2_mul(slo, H2_NEG1024), h2_mul(shi, H2_INV16), h2_mul(shi, H2_NEG64));
+        reinterpret_cast<uint2 *>(tab + MN_OFF + r * 16)[jl] = make_uint2(h2_mul(dup_lo(mp), H2_NEG1), h2_mul(dup_hi(mp), H2_NEG1));
+    }
+};
+template <> struct HalfRecord<YUUKA_DTYPE_Q4_K> : HalfRecordK4<YUUKA_DTYPE_Q4_K> {
+    __device__ void fetch(const uint8_t * rec, int lane, int half) { fetch_k4(rec, lane, half, 128); }
+    template <int C> __device__ void store(int lane, const uint8_t * tab, const DecodeConsts & kc, uint8_t * a_tile) const {
+        const int g = lane >> 2, t = lane & 3;
+        const uint32_t v[2][2] = {{C ? qg.z : qg.x, C ? qg.w : qg.y}, {C ? qh.z : qh.x, C ? qh.w : qh.y}};
+#pragma unroll
+        for (int k = 0; k < 2; k++) {
+            const int n = k ^ (g & 1);  // sub-block 2C + n: low or high nibbles
+            const uint32_t mask = n ? kc.mf0 : kc.m0f;
+#pragma unroll
+            for (int rr = 0; rr < 2; rr++) {
+                const uint2 s = reinterpret_cast<const uint2 *>(tab + (g + 8 * rr) * DS)[2 * C + n];
+                const uint32_t m = reinterpret_cast<const uint32_t *>(tab + MN_OFF + (g + 8 * rr) * 16)[2 * C + n];
+                const uint32_t v0 = v[rr][0], v1 = v[rr][1];
+                *reinterpret_cast<uint4 *>(a_tile + sw128(g + 8 * rr, 4 * n + t)) =
+                    make_uint4(nibble_h2(v0, mask, kc.magic, s.x, s.y, m), nibble_h2(v0 >> 8, mask, kc.magic, s.x, s.y, m),
+                               nibble_h2(v1, mask, kc.magic, s.x, s.y, m), nibble_h2(v1 >> 8, mask, kc.magic, s.x, s.y, m));
+            }
+        }
+    }
+};
+template <> struct HalfRecord<YUUKA_DTYPE_Q5_K> : HalfRecordK4<YUUKA_DTYPE_Q5_K> {
+    uint4 hi;  // bit k of byte b: fifth bit of column 8t + b of sub-block k of the half
+    __device__ void fetch(const uint8_t * rec, int lane, int half) {
+        fetch_k4(rec, lane, half, 160);
+        hi = reinterpret_cast<const uint4 *>(rec)[128 + lane];
+        if (half) hi = make_uint4(hi.x >> 4, hi.y >> 4, hi.z >> 4, hi.w >> 4);
+    }
+    template <int C> __device__ void store(int lane, const uint8_t * tab, const DecodeConsts & kc, uint8_t * a_tile) const {
+        const int g = lane >> 2, t = lane & 3;
+        const uint32_t v[2][2] = {{C ? qg.z : qg.x, C ? qg.w : qg.y}, {C ? qh.z : qh.x, C ? qh.w : qh.y}};
+        const uint32_t hb[2][2] = {{hi.x, hi.y}, {hi.z, hi.w}};
+#pragma unroll
+        for (int k = 0; k < 2; k++) {
+            const int n = k ^ (g & 1);  // sub-block 2C + n: low or high nibbles; its bit 2C + n of each byte goes to bit 4 or 8
+            const uint32_t mask = n ? kc.mf0 : kc.m0f, hm = n ? kc.h8 : kc.h4;
+            const int up = n ? 7 - 2 * C : 4 - 2 * C, down = n ? 1 + 2 * C : 4 + 2 * C;
+#pragma unroll
+            for (int rr = 0; rr < 2; rr++) {
+                const uint2 s = reinterpret_cast<const uint2 *>(tab + (g + 8 * rr) * DS)[2 * C + n];
+                const uint32_t m = reinterpret_cast<const uint32_t *>(tab + MN_OFF + (g + 8 * rr) * 16)[2 * C + n];
+                uint32_t o[4];
+#pragma unroll
+                for (int h = 0; h < 2; h++) {
+                    o[2 * h] = nibble_h2(v[rr][h], mask, and_or(hb[rr][h] << up, hm, kc.magic), s.x, s.y, m);
+                    o[2 * h + 1] = nibble_h2(v[rr][h] >> 8, mask, and_or(hb[rr][h] >> down, hm, kc.magic), s.x, s.y, m);
+                }
+                *reinterpret_cast<uint4 *>(a_tile + sw128(g + 8 * rr, 4 * n + t)) = make_uint4(o[0], o[1], o[2], o[3]);
+            }
+        }
+    }
+};
+// Q6_K: table rows of eight groups of 16 columns (s, -1024 s) or, for high nibbles (the last four), (s / 16, -64 s); then -32 s
+template <> struct HalfRecord<YUUKA_DTYPE_Q6_K> {
+    static constexpr int DS = 80, MN = 48, MN_OFF = 16 * DS, TAB = MN_OFF + 16 * MN;
+    uint4 lg, lh;
+    uint2 hg, hh, sc;
     uint32_t d;
-    asm("add.rn.f16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
-    return d;
-}
-
-template <int DT> struct SubBlock;
-
-template <> struct SubBlock<YUUKA_DTYPE_Q4_K> {
-    using C = Codec<YUUKA_DTYPE_Q4_K>;
-    template <int K>
-    __device__ static void frag(const typename C::Regs & r, int lane, const uint8_t * tab, const DecodeConsts & kc,
-                                uint32_t (&a)[2][4], uint32_t & mg, uint32_t & mh) {
-        constexpr int j = K >> 1, n = K & 1, jj = j >> 1, jl = j & 1;
-        const int g = lane >> 2;
-        const uint32_t qg[4] = {r.q[jj].x, r.q[jj].y, r.q[jj].z, r.q[jj].w};
-        const uint32_t qh[4] = {r.q[2 + jj].x, r.q[2 + jj].y, r.q[2 + jj].z, r.q[2 + jj].w};
-        const uint4 sg = reinterpret_cast<const uint4 *>(tab + g * C::SCL_STRIDE)[j];
-        const uint4 sh = reinterpret_cast<const uint4 *>(tab + (g + 8) * C::SCL_STRIDE)[j];
-        const uint32_t mask = n ? kc.mf0 : kc.m0f;
-        const uint32_t s_g = n ? sg.z : sg.x, c_g = n ? sg.w : sg.y, s_h = n ? sh.z : sh.x, c_h = n ? sh.w : sh.y;
+    __device__ void fetch(const uint8_t * rec, int lane, int half) {
+        const uint4 * p = reinterpret_cast<const uint4 *>(rec);
+        lg = p[half * 32 + lane];
+        lh = p[(2 + half) * 32 + lane];
+        hg = reinterpret_cast<const uint2 *>(p + 128 + lane)[half];
+        hh = reinterpret_cast<const uint2 *>(p + 160 + lane)[half];
+        sc = reinterpret_cast<const uint2 *>(p + 192 + (lane & 15))[half];
+        d = reinterpret_cast<const uint16_t *>(rec + 3328)[lane & 15];
+    }
+    __device__ void header(int lane, int, uint8_t * tab) const {
+        const int row = lane & 15, up = lane >> 4;  // groups 4 up .. 4 up + 3; the upper ones sit in high nibbles
+        const uint32_t w = (up ? sc.y : sc.x) ^ 0x80808080u, d2 = dup_lo(d);
+        const uint32_t f = up ? H2_INV16 : H2_ONE16, c = up ? H2_NEG64 : H2_NEG1024;
+        uint2 * scl = reinterpret_cast<uint2 *>(tab + row * DS) + 4 * up;
+        uint32_t s[4];
 #pragma unroll
-        for (int h = 0; h < 2; h++) {
-            const uint32_t vg = qg[2 * jl + h], vh = qh[2 * jl + h];
-            a[h][0] = h2_fma(and_or(vg, mask, kc.magic), s_g, c_g);
-            a[h][1] = h2_fma(and_or(vh, mask, kc.magic), s_h, c_h);
-            a[h][2] = h2_fma(and_or(vg >> 8, mask, kc.magic), s_g, c_g);
-            a[h][3] = h2_fma(and_or(vh >> 8, mask, kc.magic), s_h, c_h);
+        for (int q = 0; q < 2; q++) {
+            const uint32_t sp = h2_mul(h2_sub(q ? bytes23_h2(w) : bytes01_h2(w), H2_1152), d2);
+            s[2 * q] = dup_lo(sp);
+            s[2 * q + 1] = dup_hi(sp);
         }
-        mg = reinterpret_cast<const uint32_t *>(tab + C::MN_OFF + g * C::MN_STRIDE)[K];
-        mh = reinterpret_cast<const uint32_t *>(tab + C::MN_OFF + (g + 8) * C::MN_STRIDE)[K];
-    }
-};
-
-template <> struct SubBlock<YUUKA_DTYPE_Q5_K> {
-    using C = Codec<YUUKA_DTYPE_Q5_K>;
-    template <int K>
-    __device__ static void frag(const typename C::Regs & r, int lane, const uint8_t * tab, const DecodeConsts & kc,
-                                uint32_t (&a)[2][4], uint32_t & mg, uint32_t & mh) {
-        constexpr int j = K >> 1, n = K & 1, jj = j >> 1, jl = j & 1;
-        const int g = lane >> 2;
-        const uint32_t qg[4] = {r.q[jj].x, r.q[jj].y, r.q[jj].z, r.q[jj].w};
-        const uint32_t qh[4] = {r.q[2 + jj].x, r.q[2 + jj].y, r.q[2 + jj].z, r.q[2 + jj].w};
-        const uint32_t hg[2] = {r.qh.x, r.qh.y}, hh[2] = {r.qh.z, r.qh.w};
-        const uint4 sg = reinterpret_cast<const uint4 *>(tab + g * C::SCL_STRIDE)[j];
-        const uint4 sh = reinterpret_cast<const uint4 *>(tab + (g + 8) * C::SCL_STRIDE)[j];
-        const uint32_t s_g = n ? sg.z : sg.x, c_g = n ? sg.w : sg.y, s_h = n ? sh.z : sh.x, c_h = n ? sh.w : sh.y;
 #pragma unroll
-        for (int h = 0; h < 2; h++)
-            Mma<YUUKA_DTYPE_Q5_K, 1>::template sub<K>(qg[2 * jl + h], qh[2 * jl + h], hg[h], hh[h], s_g, c_g, s_h, c_h, a[h], kc);
-        mg = reinterpret_cast<const uint32_t *>(tab + C::MN_OFF + g * C::MN_STRIDE)[K];
-        mh = reinterpret_cast<const uint32_t *>(tab + C::MN_OFF + (g + 8) * C::MN_STRIDE)[K];
+        for (int q = 0; q < 4; q++) scl[q] = make_uint2(h2_mul(s[q], f), h2_mul(s[q], c));
+        reinterpret_cast<uint4 *>(tab + MN_OFF + row * MN)[up] =
+            make_uint4(h2_mul(s[0], H2_NEG32), h2_mul(s[1], H2_NEG32), h2_mul(s[2], H2_NEG32), h2_mul(s[3], H2_NEG32));
     }
-};
-
-template <> struct SubBlock<YUUKA_DTYPE_Q6_K> {
-    using C = Codec<YUUKA_DTYPE_Q6_K>;
-    // Q6_K records keep a lane's eight elements of a sub-block in two runs of four (pos6): a[0][*] are elements
-    // 4t + {0..3} (16-element group 2K), a[1][*] elements 16 + 4t + {0..3} (group 2K + 1). The offsets are added
-    // here, per group; mg / mh come back as zero.
-    template <int K>
-    __device__ static void frag(const typename C::Regs & r, int lane, const uint8_t * tab, const DecodeConsts & kc,
-                                uint32_t (&a)[2][4], uint32_t & mg, uint32_t & mh) {
-        constexpr int n6 = K >> 2, nib = (K >> 1) & 1, hsel = K & 1;
-        constexpr int lsh = 4 - 2 * hsel, rsh = 4 + 2 * hsel;
-        const int g = lane >> 2;
-        const uint32_t lg[4] = {r.ql[n6].x, r.ql[n6].y, r.ql[n6].z, r.ql[n6].w};
-        const uint32_t lh[4] = {r.ql[2 + n6].x, r.ql[2 + n6].y, r.ql[2 + n6].z, r.ql[2 + n6].w};
-        const uint32_t hg[2] = {n6 ? r.qh[0].z : r.qh[0].x, n6 ? r.qh[0].w : r.qh[0].y};
-        const uint32_t hh[2] = {n6 ? r.qh[1].z : r.qh[1].x, n6 ? r.qh[1].w : r.qh[1].y};
-        const uint32_t qm = nib ? kc.mf0 : kc.m0f, hm = nib ? kc.h8 : kc.h4;
+    template <int C> __device__ void store(int lane, const uint8_t * tab, const DecodeConsts & kc, uint8_t * a_tile) const {
+        const int g = lane >> 2, t = lane & 3;
+        const uint32_t qm = C ? kc.mf0 : kc.m0f, hm = C ? kc.h8 : kc.h4;
 #pragma unroll
-        for (int h = 0; h < 2; h++) {
-            const int s16 = 2 * K + h;
-            const uint2 eg = reinterpret_cast<const uint2 *>(tab + g * C::SCL_STRIDE)[s16];
-            const uint2 eh = reinterpret_cast<const uint2 *>(tab + (g + 8) * C::SCL_STRIDE)[s16];
-            const uint32_t og = reinterpret_cast<const uint32_t *>(tab + C::MN_OFF + g * C::MN_STRIDE)[s16];
-            const uint32_t oh = reinterpret_cast<const uint32_t *>(tab + C::MN_OFF + (g + 8) * C::MN_STRIDE)[s16];
-            const uint32_t vg = lg[2 * hsel + h], vh = lh[2 * hsel + h];
-            a[h][0] = h2_add(h2_fma(and_or(vg, qm, and_or(hg[h] << lsh, hm, kc.magic)), eg.x, eg.y), og);
-            a[h][1] = h2_add(h2_fma(and_or(vh, qm, and_or(hh[h] << lsh, hm, kc.magic)), eh.x, eh.y), oh);
-            a[h][2] = h2_add(h2_fma(and_or(vg >> 8, qm, and_or(hg[h] >> rsh, hm, kc.magic)), eg.x, eg.y), og);
-            a[h][3] = h2_add(h2_fma(and_or(vh >> 8, qm, and_or(hh[h] >> rsh, hm, kc.magic)), eh.x, eh.y), oh);
+        for (int k = 0; k < 2; k++) {
+            const int hsel = k ^ (g & 1);  // sub-block 2C + hsel
+            const int lsh = 4 - 2 * hsel, rsh = 4 + 2 * hsel;
+#pragma unroll
+            for (int rr = 0; rr < 2; rr++) {
+                const uint4 l4 = rr ? lh : lg;
+                const uint2 b2 = rr ? hh : hg, m2 = reinterpret_cast<const uint2 *>(tab + MN_OFF + (g + 8 * rr) * MN)[2 * C + hsel];
+                const uint4 s2 = reinterpret_cast<const uint4 *>(tab + (g + 8 * rr) * DS)[2 * C + hsel];
+#pragma unroll
+                for (int h = 0; h < 2; h++) {  // columns 32 hsel + 16 h + 4t .. + 3 of the stage
+                    const uint32_t v0 = h ? (hsel ? l4.w : l4.y) : (hsel ? l4.z : l4.x), b0 = h ? b2.y : b2.x;
+                    const uint32_t s = h ? s2.z : s2.x, c = h ? s2.w : s2.y, m = h ? m2.y : m2.x;
+                    *reinterpret_cast<uint2 *>(a_tile + sw128(g + 8 * rr, 4 * hsel + 2 * h + (t >> 1)) + (t & 1) * 8) =
+                        make_uint2(nibble_h2(v0, qm, and_or(b0 << lsh, hm, kc.magic), s, c, m),
+                                   nibble_h2(v0 >> 8, qm, and_or(b0 >> rsh, hm, kc.magic), s, c, m));
+                }
+            }
         }
-        mg = 0u;
-        mh = 0u;
     }
 };
-
-template <> struct SubBlock<YUUKA_DTYPE_Q8_0> {
-    using C = Codec<YUUKA_DTYPE_Q8_0>;
-    template <int K>
-    __device__ static void frag(const typename C::Regs & r, int lane, const uint8_t * tab, const DecodeConsts & kc,
-                                uint32_t (&a)[2][4], uint32_t & mg, uint32_t & mh) {
-        (void)kc;
-        constexpr int kk = K >> 1, kl = K & 1;
-        const int g = lane >> 2;
-        const uint32_t qg[4] = {r.q[kk].x, r.q[kk].y, r.q[kk].z, r.q[kk].w};
-        const uint32_t qh[4] = {r.q[4 + kk].x, r.q[4 + kk].y, r.q[4 + kk].z, r.q[4 + kk].w};
-        const uint32_t sg = reinterpret_cast<const uint32_t *>(tab + g * C::SCL_STRIDE)[K];
-        const uint32_t sh = reinterpret_cast<const uint32_t *>(tab + (g + 8) * C::SCL_STRIDE)[K];
+// Q8_0: table rows of four blocks of 32 columns (d, d)
+template <> struct HalfRecord<YUUKA_DTYPE_Q8_0> {
+    static constexpr int DS = 16, TAB = 16 * DS;
+    uint4 g0, g1, h0, h1;
+    uint2 d;
+    __device__ void fetch(const uint8_t * rec, int lane, int half) {
+        const uint4 * p = reinterpret_cast<const uint4 *>(rec);
+        g0 = p[(2 * half) * 32 + lane];
+        g1 = p[(2 * half + 1) * 32 + lane];
+        h0 = p[(4 + 2 * half) * 32 + lane];
+        h1 = p[(5 + 2 * half) * 32 + lane];
+        d = reinterpret_cast<const uint2 *>(p + 256 + (lane & 15))[half];
+    }
+    __device__ void header(int lane, int, uint8_t * tab) const {
+        const uint32_t v = lane < 16 ? d.x : d.y;
+        reinterpret_cast<uint2 *>(tab + (lane & 15) * DS)[lane >> 4] = make_uint2(dup_lo(v), dup_hi(v));
+    }
+    template <int C> __device__ void store(int lane, const uint8_t * tab, const DecodeConsts &, uint8_t * a_tile) const {
+        const int g = lane >> 2, t = lane & 3;
 #pragma unroll
-        for (int h = 0; h < 2; h++) {
-            const uint32_t vg = qg[2 * kl + h] ^ 0x80808080u, vh = qh[2 * kl + h] ^ 0x80808080u;
-            a[h][0] = h2_mul(h2_sub(bytes02_h2(vg), H2_1152), sg);
-            a[h][1] = h2_mul(h2_sub(bytes02_h2(vh), H2_1152), sh);
-            a[h][2] = h2_mul(h2_sub(bytes13_h2(vg), H2_1152), sg);
-            a[h][3] = h2_mul(h2_sub(bytes13_h2(vh), H2_1152), sh);
+        for (int k = 0; k < 2; k++) {
+            const int n = k ^ (g & 1);  // block 2C + n
+#pragma unroll
+            for (int rr = 0; rr < 2; rr++) {
+                const uint4 q = rr ? (C ? h1 : h0) : (C ? g1 : g0);
+                const uint32_t s = reinterpret_cast<const uint32_t *>(tab + (g + 8 * rr) * DS)[2 * C + n];
+                const uint32_t v0 = (n ? q.z : q.x) ^ 0x80808080u, v1 = (n ? q.w : q.y) ^ 0x80808080u;
+                *reinterpret_cast<uint4 *>(a_tile + sw128(g + 8 * rr, 4 * n + t)) =
+                    make_uint4(h2_mul(h2_sub(bytes02_h2(v0), H2_1152), s), h2_mul(h2_sub(bytes13_h2(v0), H2_1152), s),
+                               h2_mul(h2_sub(bytes02_h2(v1), H2_1152), s), h2_mul(h2_sub(bytes13_h2(v1), H2_1152), s));
+            }
         }
-        mg = 0u;
-        mh = 0u;
     }
 };
 
-// K-major, no swizzle: core matrix (8 rows x 16 bytes) at rowgroup * 1024 + kchunk * 128 inside a stage
-__device__ __forceinline__ uint64_t umma_desc(uint32_t smem_addr, uint32_t lbo = 128u, uint32_t sbo = 1024u) {
-    return (uint64_t)((smem_addr >> 4) & 0x3fffu) | ((uint64_t)(lbo >> 4) << 16) | ((uint64_t)(sbo >> 4) << 32) | (1ull << 46);
-}
-
+__device__ __forceinline__ uint32_t smem_u32(const void * p) { return (uint32_t)__cvta_generic_to_shared(p); }
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
     uint32_t ok = 0;
     for (uint32_t i = 0; i < (1u << 22) && !ok; i++) {
@@ -201,649 +264,334 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
     }
     return ok != 0;
 }
-
-template <int DT, int K>
-__device__ __forceinline__ void umma_store_subblock(const typename Codec<DT>::Regs & r, int lane, const uint8_t * tab,
-                                                    const DecodeConsts & kc, uint8_t * a_stage, int warp, int kblk_in_stage) {
-    uint32_t a[2][4], mg, mh;
-    SubBlock<DT>::template frag<K>(r, lane, tab, kc, a, mg, mh);
-    const int g = lane >> 2, t = lane & 3;
-    if constexpr (DT == YUUKA_DTYPE_Q6_K) {
-        // two runs of four columns: 4t.. (first half of the sub-block) and 16 + 4t..
-#pragma unroll
-        for (int h = 0; h < 2; h++) {
-            const int col = 16 * h + 4 * t, kchunk = 4 * kblk_in_stage + (col >> 3), off = g * 16 + (col & 7) * 2;
-            *reinterpret_cast<uint2 *>(a_stage + (2 * warp) * UM_A_SBO + kchunk * UM_A_LBO + off) = make_uint2(a[h][0], a[h][2]);
-            *reinterpret_cast<uint2 *>(a_stage + (2 * warp + 1) * UM_A_SBO + kchunk * UM_A_LBO + off) = make_uint2(a[h][1], a[h][3]);
-        }
-        return;
-    }
-    const int kchunk = 4 * kblk_in_stage + t;  // eight columns each
-    uint4 vg = make_uint4(a[0][0], a[0][2], a[1][0], a[1][2]);
-    uint4 vh = make_uint4(a[0][1], a[0][3], a[1][1], a[1][3]);
-    if (DT != YUUKA_DTYPE_Q8_0) {
-        vg = make_uint4(h2_add(vg.x, mg), h2_add(vg.y, mg), h2_add(vg.z, mg), h2_add(vg.w, mg));
-        vh = make_uint4(h2_add(vh.x, mh), h2_add(vh.y, mh), h2_add(vh.z, mh), h2_add(vh.w, mh));
-    }
-    *reinterpret_cast<uint4 *>(a_stage + (2 * warp) * UM_A_SBO + kchunk * UM_A_LBO + g * 16) = vg;
-    *reinterpret_cast<uint4 *>(a_stage + (2 * warp + 1) * UM_A_SBO + kchunk * UM_A_LBO + g * 16) = vh;
+__device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
+}
+__device__ __forceinline__ void mbar_arrive(uint32_t bar) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+__device__ __forceinline__ void mbar_expect(uint32_t bar, uint32_t bytes) {
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+}
+// One arrival on the barrier at this offset in the even CTA of the pair, from a thread of either CTA. Release at CTA scope
+// only: what the barrier announces are this CTA's own shared memory and tensor memory, which its own tensor core
+// reads, and a release at cluster scope stalls for some 900 cycles.
+__device__ __forceinline__ void mbar_arrive_leader(uint32_t bar) {
+    uint32_t remote;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(bar), "r"(0u));
+    asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(remote) : "memory");
+}
+// completion of this thread's MMAs so far -> one arrival on the barrier at this offset in both CTAs of the pair
+__device__ __forceinline__ void umma_commit_pair(uint32_t bar) {
+    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(bar), "h"((uint16_t)3)
+                 : "memory");
 }
 
-template <int DT, int Q>
-__device__ __forceinline__ void umma_store_chunk(const typename Codec<DT>::Regs & r, int lane, const uint8_t * tab,
-                                                 const DecodeConsts & kc, uint8_t * a_stage, int warp) {
-    umma_store_subblock<DT, 2 * Q>(r, lane, tab, kc, a_stage, warp, 0);
-    umma_store_subblock<DT, 2 * Q + 1>(r, lane, tab, kc, a_stage, warp, 1);
+__device__ __forceinline__ bool elect_one() {
+    uint32_t e;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(e));
+    return e != 0;
+}
+__device__ __forceinline__ void umma_f16_pair(uint32_t d, uint64_t da, uint64_t db, uint32_t idesc, uint32_t accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, {%5, %5, %5, %5, %5, %5, %5, %5}, p;\n\t}"
+        :
+        : "r"(d), "l"(da), "l"(db), "r"(idesc), "r"(accumulate), "r"(0u)
+        : "memory");
 }
 
-// TMA: the activation stage is filled by one cp.async.bulk.tensor per chunk (2-D map over the prepared
-// activations, box 64 columns x npad rows, 128-byte swizzle, rows beyond M zero-filled) that completes on
-// full_bar; otherwise by 16-byte cp.async copies into padded core matrices.
-template <int DT, bool TMA>
-__global__ void __launch_bounds__(TW * 32, 2) gemm_umma_kernel(const UParams p, const __grid_constant__ CUtensorMap xmap) {
-    using C = Codec<DT>;
-    extern __shared__ __align__(128) uint8_t smem_raw[];
-    // the swizzled stage needs 1024-byte alignment
-    uint8_t * smem = smem_raw + ((1024u - ((uint32_t)__cvta_generic_to_shared(smem_raw) & 1023u)) & 1023u);
-    __shared__ __align__(8) uint64_t empty_bar[UM_STAGES];
-    __shared__ __align__(8) uint64_t full_bar[UM_STAGES];
-    __shared__ __align__(8) uint64_t done_bar;
-    __shared__ uint32_t tmem_slot;
-    __shared__ int last_flag;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const uint32_t b_bytes = TMA ? (uint32_t)p.npad * 128u : (uint32_t)(p.npad >> 3) * UM_B_SBO;
-    const uint32_t stage_bytes = UM_A_BYTES + b_bytes;
-    uint8_t * tabs = smem + (size_t)p.stages * stage_bytes;
-    uint8_t * tab = tabs + warp * C::TAB;
-
-    if (threadIdx.x == 0) {
-        for (int s = 0; s < UM_STAGES; s++) {
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"((uint32_t)__cvta_generic_to_shared(&empty_bar[s])) : "memory");
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"((uint32_t)__cvta_generic_to_shared(&full_bar[s])) : "memory");
-        }
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"((uint32_t)__cvta_generic_to_shared(&done_bar)) : "memory");
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    }
-    if (warp == 0) {
-        __syncwarp();
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
-                         (uint32_t)__cvta_generic_to_shared(&tmem_slot)),
-                     "r"(p.tmem_cols)
-                     : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-    }
-    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    __syncthreads();
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    const uint32_t taddr = tmem_slot;
-    const uint32_t smem_base = (uint32_t)__cvta_generic_to_shared(smem);  // (1024-byte aligned)
-    const DecodeConsts kc = p.kc;
-
-    const int n_tiles = (p.N + 15) >> 4;
-    const int n_blocks = (p.N + UM_ROWS - 1) / UM_ROWS;
-    const size_t rec_row = (size_t)p.nsb * C::REC;
-    const int K = p.nsb * 256;
-    // this CTA's share of K (superblocks), when K is split across gridDim.y
-    const int sb_begin = (int)(((long long)p.nsb * blockIdx.y) / gridDim.y);
-    const int sb_end = (int)(((long long)p.nsb * (blockIdx.y + 1)) / gridDim.y);
-    const int chunks_per_block = (sb_end - sb_begin) * 4;
-    bool expired = false;
-
-    // activations of one chunk: columns [col0, col0 + 64) of every row into the stage
-    auto issue_x = [&](uint32_t stage, int col0) {
-        uint8_t * b_stage = smem + (size_t)stage * stage_bytes + UM_A_BYTES;
-        if constexpr (TMA) {
-            if (threadIdx.x == 0) {
-                const uint32_t bar = (uint32_t)__cvta_generic_to_shared(&full_bar[stage]);
-                asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(b_bytes) : "memory");
-                asm volatile(
-                    "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
-                    :
-                    : "r"((uint32_t)__cvta_generic_to_shared(b_stage)), "l"(&xmap), "r"(col0), "r"(0), "r"(bar)
-                    : "memory");
-            }
-        } else {
-            for (int i = threadIdx.x; i < p.npad * 8; i += TW * 32) {
-                const int tok = i >> 3, kch = i & 7;
-                const __half * src = p.xh + (size_t)min(tok, p.M - 1) * K + col0 + kch * 8;
-                const uint32_t dst =
-                    (uint32_t)__cvta_generic_to_shared(b_stage + (tok >> 3) * UM_B_SBO + kch * UM_B_LBO + (tok & 7) * 16);
-                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
-            }
-        }
-    };
-    // column offset of chunk number `ci` counted from this CTA's first chunk (blocks repeat the same columns)
-    auto chunk_col = [&](uint32_t ci) { return sb_begin * 256 + (int)(ci % (uint32_t)chunks_per_block) * UM_KC; };
-
-    pdl_trigger();
-    typename C::Regs cur, nxt;
-    {
-        const int rt = min(blockIdx.x * (UM_ROWS / 16) + warp, n_tiles - 1);
-        if (sb_begin < sb_end) C::load(p.w + rt * rec_row + (size_t)sb_begin * C::REC, lane, cur);
-    }
-    pdl_wait();
-
-    uint32_t chunk = 0;  // chunks started by this CTA so far (stage = chunk % p.stages)
-    uint32_t block_iter = 0;
-    // chunks this CTA will run in total, and the first UM_AHEAD activation copies
-    uint32_t total_chunks = 0;
-    if (chunks_per_block > 0 && (int)blockIdx.x < n_blocks)
-        total_chunks = (uint32_t)((n_blocks - 1 - (int)blockIdx.x) / (int)gridDim.x + 1) * (uint32_t)chunks_per_block;
-    for (uint32_t ci = 0; ci < UM_AHEAD; ci++) {
-        if (ci < total_chunks) issue_x(ci % p.stages, chunk_col(ci));
-        asm volatile("cp.async.commit_group;" ::: "memory");
-    }
-    for (int rb = blockIdx.x; rb < n_blocks && chunks_per_block > 0; rb += gridDim.x, block_iter++) {
-        const int rt = min(rb * (UM_ROWS / 16) + warp, n_tiles - 1);
-        const uint8_t * tile = p.w + rt * rec_row;
-        const bool more_blocks = rb + (int)gridDim.x < n_blocks;
-        for (int sb = sb_begin; sb < sb_end; sb++) {
-            if (sb + 1 < sb_end) {
-                C::load(tile + (size_t)(sb + 1) * C::REC, lane, nxt);
-            } else if (more_blocks) {
-                const int rtn = min((rb + (int)gridDim.x) * (UM_ROWS / 16) + warp, n_tiles - 1);
-                C::load(p.w + rtn * rec_row + (size_t)sb_begin * C::REC, lane, nxt);
-            }
-            Mma<DT, 1>::header(cur, lane, tab);
-            __syncwarp();
-#pragma unroll
-            for (int q = 0; q < 4; q++) {
-                const uint32_t stage = chunk % p.stages;
-                uint8_t * a_stage = smem + (size_t)stage * stage_bytes;
-                // start the activations of chunk + UM_AHEAD: the tensor pipe must have read that stage's previous contents
-                {
-                    const uint32_t nchunk = chunk + UM_AHEAD;
-                    if (nchunk < total_chunks) {
-                        const uint32_t nstage = nchunk % p.stages, nuse = nchunk / p.stages;
-                        if (nuse > 0 && !expired &&
-                            !mbar_wait((uint32_t)__cvta_generic_to_shared(&empty_bar[nstage]), (nuse - 1) & 1))
-                            expired = true;
-                        issue_x(nstage, chunk_col(nchunk));
-                    }
-                    asm volatile("cp.async.commit_group;" ::: "memory");
-                }
-                // this chunk's stage: free since the wait made when its activations were started (UM_AHEAD chunks ago)
-                // weights: this warp's 16 rows x 64 columns (the stage was waited for when its activations were started)
-                if (q == 0) umma_store_chunk<DT, 0>(cur, lane, tab, kc, a_stage, warp);
-                else if (q == 1) umma_store_chunk<DT, 1>(cur, lane, tab, kc, a_stage, warp);
-                else if (q == 2) umma_store_chunk<DT, 2>(cur, lane, tab, kc, a_stage, warp);
-                else umma_store_chunk<DT, 3>(cur, lane, tab, kc, a_stage, warp);
-                if constexpr (!TMA) asm volatile("cp.async.wait_group %0;" ::"n"(UM_AHEAD) : "memory");  // this chunk's have landed
-                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-                asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-                __syncthreads();
-                if (threadIdx.x == 0) {
-                    if constexpr (TMA) {
-                        if (!expired && !mbar_wait((uint32_t)__cvta_generic_to_shared(&full_bar[stage]), (chunk / p.stages) & 1))
-                            expired = true;
-                    }
-                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                    const uint64_t da = umma_desc(smem_base + stage * stage_bytes, UM_A_LBO, UM_A_SBO);
-                    const uint64_t db = TMA ? umma_desc_sw128(smem_base + stage * stage_bytes + UM_A_BYTES)
-                                            : umma_desc(smem_base + stage * stage_bytes + UM_A_BYTES, UM_B_LBO, UM_B_SBO);
-                    const uint32_t b_step = TMA ? 2u : (uint32_t)(2 * UM_B_LBO / 16);
-#pragma unroll
-                    for (int j = 0; j < UM_KC / 16; j++) {
-                        const uint32_t accumulate = (sb > sb_begin || q > 0 || j > 0) ? 1u : 0u;
-                        // 16 columns = two core matrices = 256 bytes further along K
-                        asm volatile(
-                            "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-                            "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, {%5, %5, %5, %5}, p;\n\t}"
-                            :
-                            : "r"(taddr), "l"(da + (uint64_t)(j * (2 * UM_A_LBO / 16))), "l"(db + (uint64_t)(j * b_step)), "r"(p.idesc), "r"(accumulate),
-                              "r"(0u)
-                            : "memory");
-                    }
-                    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-                                     (uint32_t)__cvta_generic_to_shared(&empty_bar[stage]))
-                                 : "memory");
-                }
-                chunk++;
-            }
-            __syncwarp();
-            cur = nxt;
-        }
-        // ---- epilogue of this block of 128 weight rows ----
-        if (threadIdx.x == 0)
-            asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-                             (uint32_t)__cvta_generic_to_shared(&done_bar))
-                         : "memory");
-        if (!expired && !mbar_wait((uint32_t)__cvta_generic_to_shared(&done_bar), block_iter & 1)) expired = true;
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        {
-            // warp w reads TMEM lanes 32 * (w % 4) ..; warps 0-3 take the even 32-column groups, 4-7 the odd ones
-            const int quad = warp & 3;
-            const int n = rb * UM_ROWS + quad * 32 + lane;
-            const bool split = gridDim.y > 1;
-            float * base = split ? p.partial + (size_t)blockIdx.y * p.M * p.N : p.out;
-            const int64_t ld = split ? p.N : p.ldo;
-            for (int c0 = (warp >> 2) * 32; c0 < p.npad; c0 += 64) {
-                uint32_t v[32];
-                const uint32_t src = taddr + ((uint32_t)(quad * 32) << 16) + (uint32_t)c0;
-                asm volatile(
-                    "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
-                    "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
-                    "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
-                    : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]),
-                      "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]), "=r"(v[16]),
-                      "=r"(v[17]), "=r"(v[18]), "=r"(v[19]), "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]), "=r"(v[24]),
-                      "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
-                    : "r"(src)
-                    : "memory");
-                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-                if (n < p.N) {
-#pragma unroll
-                    for (int i = 0; i < 32; i++) {
-                        const int tok = c0 + i;
-                        if (tok < p.M) {
-                            float * dst = base + (int64_t)tok * ld + n;
-                            const float val = __uint_as_float(v[i]);
-                            if (split) __stcg(dst, val);
-                            else *dst = p.accumulate ? *dst + val : val;
-                        }
-                    }
-                }
-            }
-        }
-        if (gridDim.y > 1) {
-            // K is split across CTAs: the last one to finish this block of rows sums the parts in a fixed order
-            __threadfence();
-            __syncthreads();
-            if (threadIdx.x == 0) last_flag = atomicAdd(&p.counters[rb], 1) == (int)gridDim.y - 1;
-            __syncthreads();
-            if (last_flag) {
-                __threadfence();
-                const int n0 = rb * UM_ROWS, nrows = min(UM_ROWS, p.N - n0);
-                // four outputs per thread and trip: all their loads are issued before the first sum is formed
-                const int total = p.M * nrows;
-                for (int i0 = threadIdx.x; i0 < total; i0 += 4 * TW * 32) {
-                    float sum[4] = {0.0f, 0.0f, 0.0f, 0.0f}, old[4];
-                    float * dst[4];
-#pragma unroll
-                    for (int u = 0; u < 4; u++) {
-                        const int i = min(i0 + u * TW * 32, total - 1);
-                        const int tok = i / nrows, n = n0 + i - tok * nrows;
-                        dst[u] = p.out + (int64_t)tok * p.ldo + n;
-                        old[u] = p.accumulate ? *dst[u] : 0.0f;
-                    }
-                    for (int part = 0; part < (int)gridDim.y; part++) {
-                        float v[4];
-#pragma unroll
-                        for (int u = 0; u < 4; u++) {
-                            const int i = min(i0 + u * TW * 32, total - 1);
-                            const int tok = i / nrows, n = n0 + i - tok * nrows;
-                            v[u] = __ldcg(p.partial + ((size_t)part * p.M + tok) * p.N + n);
-                        }
-#pragma unroll
-                        for (int u = 0; u < 4; u++) sum[u] += v[u];
-                    }
-#pragma unroll
-                    for (int u = 0; u < 4; u++)
-                        if (i0 + u * TW * 32 < total) *dst[u] = old[u] + sum[u];
-                }
-                if (threadIdx.x == 0) p.counters[rb] = 0;
-            }
-        }
-        // the next block overwrites the accumulator: everybody must have read it
-        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-        __syncthreads();
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    }
-    asm volatile("cp.async.wait_group 0;" ::: "memory");
-    if (expired) atomicExch(&g_gemm_wait_expired, 2);
-    // every MMA this CTA issued has completed (the last done_bar wait), nothing reads TMEM any more
-    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    __syncthreads();
-    if (warp == 0)
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(p.tmem_cols) : "memory");
-}
-
-// ---------------------------------------------------------------------------
-// Warp-specialised variant (tensor-map activations only): eight decode warps, a copy warp and an issue warp.
-// The decode warps never meet at a CTA-wide barrier inside a block of rows: each announces its
-// share of a stage on afull_bar (eight arrivals) and moves on to the next stage as soon as
-// empty_bar says the tensor pipe has drained it. Lane 0 of the copy warp starts the activation copy of
-// a stage as soon as it is free; lane 0 of the issue warp waits for (activations landed, weights
-// decoded), issues the MMAs and commits the stage back. tmem_free_bar (eight arrivals) tells it that
-// the epilogue has read the accumulator before the next block of rows overwrites it. (Sixteen decode
-// warps, two per tile on alternate chunks, measured slower on wide matrices: 96 registers per thread
-// spill and the doubled scale tables cost a ring stage.)
 // 32 accumulator values of one weight row (this lane's) for 32 consecutive activation rows, to out[row][n]:
-// MODE 0 stores, 1 adds to what is there, 2 stores a K part past L1. `lim` = rows that exist. One pointer step
-// per value: the per-value bounds, mode and 64-bit index arithmetic of a generic loop were a third of the
-// kernel's instructions at 256 rows and half of them at 512.
+// MODE 0 stores, 1 adds to what is there, 2 stores a K part past L1. `lim` = rows that exist. One pointer step per
+// value: per-value bounds, mode and 64-bit index arithmetic cost more than the stores.
 template <int MODE>
 __device__ __forceinline__ void umma_store_rows(float * dst, int64_t ld, const uint32_t (&v)[32], int lim) {
-    if (lim >= 32) {
 #pragma unroll
-        for (int i = 0; i < 32; i++) {
+    for (int i = 0; i < 32; i++) {
+        if (lim >= 32 || i < lim) {
             const float val = __uint_as_float(v[i]);
             if (MODE == 2) __stcg(dst, val);
             else if (MODE == 1) *dst += val;
             else *dst = val;
-            dst += ld;
         }
-    } else {
-#pragma unroll
-        for (int i = 0; i < 32; i++) {
-            if (i < lim) {
-                const float val = __uint_as_float(v[i]);
-                if (MODE == 2) __stcg(dst, val);
-                else if (MODE == 1) *dst += val;
-                else *dst = val;
-            }
-            dst += ld;
-        }
+        dst += ld;
     }
 }
 
-// Decode warps of the warp-specialised kernel: TW (one per 16-row tile), or 2 * TW: the two warps of a tile take
-// alternate 64-column chunks of every record (-DYK_UMMA_DECODE_WARPS=16). Measured with sixteen (112 registers,
-// 60-260 bytes of spills): Q4_K 18432 x 2560 at 256 / 512 rows 52.7 -> 50.4 / 70.6 -> 65.7 us, but the Q6_K
-// LM head 567 -> 745 us and a 64-row step 6.66 -> 6.96 ms, so eight stay. Asking the records four or eight
-// superblocks ahead into L2 changed nothing either: neither the latency of the weight loads nor the number of
-// decoding warps is what bounds the loop.
-#ifndef YK_UMMA_DECODE_WARPS
-#define YK_UMMA_DECODE_WARPS 8
-#endif
-constexpr int UM_DW = YK_UMMA_DECODE_WARPS;
-static_assert(UM_DW == TW || UM_DW == 2 * TW, "one or two decode warps per 16-row tile");
-constexpr int UM_WS_THREADS = (UM_DW + 2) * 32;
-
-__device__ __forceinline__ void mbar_arrive(uint32_t bar) {
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
+__device__ __forceinline__ void tmem_load32(uint32_t (&v)[32], uint32_t src) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
+        "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
+        "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
+        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]),
+          "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]), "=r"(v[16]),
+          "=r"(v[17]), "=r"(v[18]), "=r"(v[19]), "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]), "=r"(v[24]),
+          "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
+        : "r"(src)
+        : "memory");
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
+
+// Walks the work of a pair: tiles (256 weight rows x n_tile activation rows x a part of K) in steps of the number of
+// pairs, activation tiles of the same weights first, so that pairs next to each other read the same weights.
+struct UmmaWork {
+    int item, step, items;
+    __device__ UmmaWork(const UParams & p) {
+        item = blockIdx.x >> 1;
+        step = gridDim.x >> 1;
+        items = p.m_blocks * p.n_tiles * p.kparts;
+    }
+    __device__ bool valid() const { return item < items; }
+    __device__ void next() { item += step; }
+    __device__ int n0(const UParams & p) const { return (item % p.n_tiles) * p.n_tile; }
+    __device__ int part(const UParams & p) const { return (item / p.n_tiles) % p.kparts; }
+    __device__ int block(const UParams & p) const { return item / (p.n_tiles * p.kparts); }
+    __device__ int sb_begin(const UParams & p) const { return (int)((long long)p.nsb * part(p) / p.kparts); }
+    __device__ int sb_end(const UParams & p) const { return (int)((long long)p.nsb * (part(p) + 1) / p.kparts); }
+};
+// A position in a ring of `depth` stages: `phase` is the parity a consumer waits for, its inverse a producer's.
+struct Ring {
+    uint32_t at = 0, phase = 0;
+    __device__ void next(uint32_t depth) {
+        if (++at == depth) {
+            at = 0;
+            phase ^= 1u;
+        }
+    }
+};
 
 template <int DT>
-__global__ void __launch_bounds__(UM_WS_THREADS, 1) gemm_umma_ws_kernel(const UParams p, const __grid_constant__ CUtensorMap xmap) {
+__global__ void __launch_bounds__(UM_THREADS, 1) gemm_umma_kernel(const UParams p, const __grid_constant__ CUtensorMap xmap) {
     using C = Codec<DT>;
+    using S = UmmaStage<DT>;
     extern __shared__ __align__(128) uint8_t smem_raw[];
-    uint8_t * smem = smem_raw + ((1024u - ((uint32_t)__cvta_generic_to_shared(smem_raw) & 1023u)) & 1023u);
-    __shared__ __align__(8) uint64_t empty_bar[UM_STAGES];
-    __shared__ __align__(8) uint64_t xfull_bar[UM_STAGES];
-    __shared__ __align__(8) uint64_t afull_bar[UM_STAGES];
-    __shared__ __align__(8) uint64_t done_bar;
-    __shared__ __align__(8) uint64_t tmem_free_bar;
+    uint8_t * smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);  // the swizzled stages need 1024-byte alignment
+    __shared__ __align__(8) uint64_t empty_bar[UM_MAX_STAGES];  // the tensor pipe has read the stage
+    __shared__ __align__(8) uint64_t full_bar[UM_MAX_STAGES];   // (even CTA) both CTAs' weights and activations are in the stage
+    __shared__ __align__(8) uint64_t x_bar[UM_MAX_STAGES];      // (odd CTA) its activations have landed
+    __shared__ __align__(8) uint64_t raw_full[UM_RAW_STAGES], raw_empty[UM_RAW_STAGES];
+    __shared__ __align__(8) uint64_t acc_full[2], acc_empty[2]; // accumulators: finished by the MMAs, read by the epilogue
     __shared__ uint32_t tmem_slot;
-    __shared__ int last_flag;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const uint32_t halves = p.idesc2 ? 2u : 1u;
-    const uint32_t half_bytes = p.box_rows * 128u;
-    const uint32_t b_bytes = halves * half_bytes;
-    const uint32_t stage_bytes = UM_A_BYTES + b_bytes;
-    uint8_t * tabs = smem + (size_t)p.stages * stage_bytes;
+    const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;  // (uniform for the compiler too)
+    const uint32_t rank = blockIdx.x & 1u;  // clusters are pairs along x
+    const uint32_t half_n = (uint32_t)p.n_tile >> 1, b_bytes = half_n * 128u, stage_bytes = UM_A_BYTES + b_bytes;
+    uint8_t * raw = smem + (size_t)p.stages * stage_bytes;
+    uint8_t * tabs = raw + (size_t)UM_RAW_STAGES * S::RAW_BYTES;
 
     if (threadIdx.x == 0) {
-        for (int s = 0; s < UM_STAGES; s++) {
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"((uint32_t)__cvta_generic_to_shared(&empty_bar[s])) : "memory");
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"((uint32_t)__cvta_generic_to_shared(&xfull_bar[s])) : "memory");
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"((uint32_t)__cvta_generic_to_shared(&afull_bar[s])), "r"(TW)
-                         : "memory");
+        for (int s = 0; s < UM_MAX_STAGES; s++) {
+            mbar_init(smem_u32(&empty_bar[s]), 1);
+            mbar_init(smem_u32(&full_bar[s]), 2 * UM_TILES + 2);
+            mbar_init(smem_u32(&x_bar[s]), 1);
         }
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"((uint32_t)__cvta_generic_to_shared(&done_bar)) : "memory");
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"((uint32_t)__cvta_generic_to_shared(&tmem_free_bar)), "r"(UM_DW)
-                     : "memory");
+        for (int s = 0; s < UM_RAW_STAGES; s++) {
+            mbar_init(smem_u32(&raw_full[s]), 1);
+            mbar_init(smem_u32(&raw_empty[s]), UM_DW);
+        }
+        for (int s = 0; s < 2; s++) {
+            mbar_init(smem_u32(&acc_full[s]), 1);
+            mbar_init(smem_u32(&acc_empty[s]), 2 * UM_EW);
+        }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    if (warp == 0) {
-        __syncwarp();
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
-                         (uint32_t)__cvta_generic_to_shared(&tmem_slot)),
-                     "r"(p.tmem_cols)
-                     : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    if (warp == UM_WARP_MMA) {
+        asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_slot)), "r"(512u) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
+    cluster_sync_all();  // both CTAs' barriers are set up
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    const uint32_t taddr = tmem_slot;
-    const uint32_t smem_base = (uint32_t)__cvta_generic_to_shared(smem);
-
-    const int n_tiles = (p.N + 15) >> 4;
-    const int n_blocks = (p.N + UM_ROWS - 1) / UM_ROWS;
+    const uint32_t taddr = tmem_slot, smem_base = smem_u32(smem);
+    const int n_tiles16 = (p.N + 15) >> 4;
     const size_t rec_row = (size_t)p.nsb * C::REC;
-    const int sb_begin = (int)(((long long)p.nsb * blockIdx.y) / gridDim.y);
-    const int sb_end = (int)(((long long)p.nsb * (blockIdx.y + 1)) / gridDim.y);
-    const int chunks_per_block = (sb_end - sb_begin) * 4;
-    uint32_t my_blocks = 0;
-    if (chunks_per_block > 0 && (int)blockIdx.x < n_blocks) my_blocks = (uint32_t)((n_blocks - 1 - (int)blockIdx.x) / (int)gridDim.x + 1);
-    const uint32_t total_chunks = my_blocks * (uint32_t)chunks_per_block;
     bool expired = false;
+    auto wait = [&](const uint64_t & bar, uint32_t parity) {
+        if (!expired && !mbar_wait(smem_u32(&bar), parity)) expired = true;
+    };
 
     pdl_trigger();
-    if (warp == UM_DW) {
-        // ---------------- copy warp: starts the activation copy of a stage as soon as it is free ----------------
+    // (the copy and issue warps walk their loops whole, so that addresses and descriptors stay in uniform registers; one
+    // lane issues: a loop of that lane alone spent 85 cycles on each MMA)
+    if (warp == UM_WARP_RAW) {
+        // ---------------- packed weights: they do not depend on the previous kernel ----------------
+        Ring ring;
+        for (UmmaWork wk(p); wk.valid(); wk.next()) {
+            const int rt = min((wk.block(p) * 2 + (int)rank) * UM_TILES + (lane & (UM_TILES - 1)), n_tiles16 - 1), sb1 = wk.sb_end(p);
+            const uint8_t * src = p.w + rt * rec_row;
+            for (int sb = wk.sb_begin(p); sb < sb1; sb++) {
+                wait(raw_empty[ring.at], ring.phase ^ 1u);
+                const uint32_t bar = smem_u32(&raw_full[ring.at]);
+                if (lane == 0) mbar_expect(bar, S::RAW_BYTES);
+                __syncwarp();
+                if (lane < UM_TILES)
+                    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                                     smem_u32(raw + (size_t)ring.at * S::RAW_BYTES) + (uint32_t)(lane * C::REC)),
+                                 "l"(src + (size_t)sb * C::REC), "r"((uint32_t)C::REC), "r"(bar)
+                                 : "memory");
+                ring.next(UM_RAW_STAGES);
+            }
+        }
+    } else if (warp == UM_WARP_X) {
+        // ---------------- activations: this CTA's half of the tile's rows ----------------
         pdl_wait();
-        if (lane == 0) {
-            // ring positions are advanced by hand: the ring depth is a run-time value and a division per
-            // chunk on a single thread's critical path would cost more than the work it issues
-            uint32_t stage = 0, use = 0, in_block = 0;
-            for (uint32_t n = 0; n < total_chunks; n++) {
-                if (use > 0 && !expired && !mbar_wait((uint32_t)__cvta_generic_to_shared(&empty_bar[stage]), (use - 1) & 1))
-                    expired = true;
-                const uint32_t bar = (uint32_t)__cvta_generic_to_shared(&xfull_bar[stage]);
-                const int col0 = sb_begin * 256 + (int)in_block * UM_KC;
-                asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(b_bytes) : "memory");
-                for (uint32_t h = 0; h < halves; h++)
+        Ring ring;
+        for (UmmaWork wk(p); wk.valid(); wk.next()) {
+            const int row = wk.n0(p) + (int)(rank * half_n), sb1 = wk.sb_end(p);
+            for (int col = wk.sb_begin(p) * 256; col < sb1 * 256; col += UM_KC) {
+                wait(empty_bar[ring.at], ring.phase ^ 1u);
+                const uint32_t bar = smem_u32(rank == 0 ? &full_bar[ring.at] : &x_bar[ring.at]);
+                if (lane == 0) {
+                    mbar_expect(bar, b_bytes);
                     asm volatile(
                         "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
                         :
-                        : "r"(smem_base + stage * stage_bytes + UM_A_BYTES + h * half_bytes), "l"(&xmap), "r"(col0),
-                          "r"((int)(h * UM_MAX_N)), "r"(bar)
+                        : "r"(smem_base + ring.at * stage_bytes + UM_A_BYTES), "l"(&xmap), "r"(col), "r"(row), "r"(bar)
                         : "memory");
-                if (++stage == p.stages) { stage = 0; use++; }
-                if (++in_block == (uint32_t)chunks_per_block) in_block = 0;
-            }
-        }
-        __syncwarp();
-    } else if (warp == UM_DW + 1) {
-        // ---------------- issue warp: (activations landed, weights decoded) -> MMAs -> stage released ----------------
-        if (lane == 0) {
-            uint32_t stage = 0, use = 0, in_block = 0, blk = 0;
-            uint32_t a_addr = smem_base, b_addr = smem_base + UM_A_BYTES;
-            for (uint32_t c = 0; c < total_chunks; c++) {
-                // the epilogue of the previous block must have read the accumulator
-                if (in_block == 0 && blk > 0 && !expired &&
-                    !mbar_wait((uint32_t)__cvta_generic_to_shared(&tmem_free_bar), (blk - 1) & 1))
-                    expired = true;
-                if (!expired && !mbar_wait((uint32_t)__cvta_generic_to_shared(&xfull_bar[stage]), use & 1)) expired = true;
-                if (!expired && !mbar_wait((uint32_t)__cvta_generic_to_shared(&afull_bar[stage]), use & 1)) expired = true;
-                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                const uint64_t da = umma_desc(a_addr, UM_A_LBO, UM_A_SBO);
-                const uint64_t db = umma_desc_sw128(b_addr);
-                // rows 256... accumulate in tensor-memory columns 256...: the decoded weights are multiplied twice
-                for (uint32_t h = 0; h < halves; h++) {
-                    const uint32_t idesc = h ? p.idesc2 : p.idesc;
-                    const uint64_t dbh = db + (uint64_t)(h * (half_bytes >> 4));
-#pragma unroll
-                    for (int j = 0; j < UM_KC / 16; j++) {
-                        const uint32_t accumulate = (in_block > 0 || j > 0) ? 1u : 0u;
-                        asm volatile(
-                            "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-                            "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, {%5, %5, %5, %5}, p;\n\t}"
-                            :
-                            : "r"(taddr + h * (uint32_t)UM_MAX_N), "l"(da + (uint64_t)(j * (2 * UM_A_LBO / 16))),
-                              "l"(dbh + (uint64_t)(j * 2)), "r"(idesc), "r"(accumulate), "r"(0u)
-                            : "memory");
-                    }
                 }
-                asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-                                 (uint32_t)__cvta_generic_to_shared(&empty_bar[stage]))
-                             : "memory");
-                if (in_block == (uint32_t)chunks_per_block - 1)
-                    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-                                     (uint32_t)__cvta_generic_to_shared(&done_bar))
-                                 : "memory");
-                a_addr += stage_bytes;
-                b_addr += stage_bytes;
-                if (++stage == p.stages) {
-                    stage = 0;
-                    use++;
-                    a_addr = smem_base;
-                    b_addr = smem_base + UM_A_BYTES;
-                }
-                if (++in_block == (uint32_t)chunks_per_block) { in_block = 0; blk++; }
-            }
-        }
-        __syncwarp();
-    } else {
-        // ---------------- decode warps ----------------
-        uint8_t * tab = tabs + warp * C::TAB;
-        const DecodeConsts kc = p.kc;
-        const int tile = warp % TW, parity = warp / TW;  // with two warps per tile: chunks q with (q & 1) == parity
-        typename C::Regs cur, nxt;
-        if (my_blocks > 0) {
-            const int rt = min(blockIdx.x * (UM_ROWS / 16) + tile, n_tiles - 1);
-            C::load(p.w + rt * rec_row + (size_t)sb_begin * C::REC, lane, cur);
-        }
-        pdl_wait();
-        uint32_t stage = 0, use = 0, block_iter = 0;
-        for (int rb = blockIdx.x; rb < n_blocks && chunks_per_block > 0; rb += gridDim.x, block_iter++) {
-            const int rt = min(rb * (UM_ROWS / 16) + tile, n_tiles - 1);
-            const uint8_t * tile_w = p.w + rt * rec_row;
-            const bool more_blocks = rb + (int)gridDim.x < n_blocks;
-            for (int sb = sb_begin; sb < sb_end; sb++) {
-                if (sb + 1 < sb_end) {
-                    C::load(tile_w + (size_t)(sb + 1) * C::REC, lane, nxt);
-                } else if (more_blocks) {
-                    const int rtn = min((rb + (int)gridDim.x) * (UM_ROWS / 16) + tile, n_tiles - 1);
-                    C::load(p.w + rtn * rec_row + (size_t)sb_begin * C::REC, lane, nxt);
-                }
-                Mma<DT, 1>::header(cur, lane, tab);
                 __syncwarp();
+                ring.next(p.stages);
+            }
+        }
+    } else if (warp == UM_WARP_MMA && rank == 0) {
+        // ---------------- MMAs of the pair ----------------
+        Ring ring, acc;
+        const uint64_t da0 = umma_desc_sw128(smem_base), db0 = umma_desc_sw128(smem_base + UM_A_BYTES);
+        const uint32_t step = stage_bytes >> 4;
+        for (UmmaWork wk(p); wk.valid(); wk.next()) {
+            wait(acc_empty[acc.at], acc.phase ^ 1u);
+            const uint32_t d = taddr + acc.at * (uint32_t)UM_MAX_N;
+            const int chunks = (wk.sb_end(p) - wk.sb_begin(p)) * 4;
+            for (int c = 0; c < chunks; c++) {
+                wait(full_bar[ring.at], ring.phase);
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                const uint64_t da = da0 + (uint64_t)(ring.at * step), db = db0 + (uint64_t)(ring.at * step);
+                if (elect_one()) {
 #pragma unroll
-                for (int q = 0; q < 4; q++) {
-                    uint8_t * a_stage = smem + (size_t)stage * stage_bytes;
-                    if (UM_DW > TW && (q & 1) != parity) {
-                        if (++stage == p.stages) { stage = 0; use++; }
-                        continue;
-                    }
-                    if (use > 0 && !expired && !mbar_wait((uint32_t)__cvta_generic_to_shared(&empty_bar[stage]), (use - 1) & 1))
-                        expired = true;
-                    if (q == 0) umma_store_chunk<DT, 0>(cur, lane, tab, kc, a_stage, tile);
-                    else if (q == 1) umma_store_chunk<DT, 1>(cur, lane, tab, kc, a_stage, tile);
-                    else if (q == 2) umma_store_chunk<DT, 2>(cur, lane, tab, kc, a_stage, tile);
-                    else umma_store_chunk<DT, 3>(cur, lane, tab, kc, a_stage, tile);
+                    for (int j = 0; j < UM_KC / 16; j++)
+                        umma_f16_pair(d, da + (uint64_t)(j * 2), db + (uint64_t)(j * 2), p.idesc, (c > 0 || j > 0) ? 1u : 0u);
+                    umma_commit_pair(smem_u32(&empty_bar[ring.at]));
+                }
+                __syncwarp();
+                ring.next(p.stages);
+            }
+            if (elect_one()) umma_commit_pair(smem_u32(&acc_full[acc.at]));
+            __syncwarp();
+            acc.next(2);
+        }
+    } else if (warp == UM_WARP_MMA) {
+        // ---------------- odd CTA: its activations have landed -> the even CTA's barrier ----------------
+        Ring ring;
+        for (UmmaWork wk(p); wk.valid(); wk.next()) {
+            const int chunks = (wk.sb_end(p) - wk.sb_begin(p)) * 4;
+            for (int c = 0; c < chunks; c++) {
+                wait(x_bar[ring.at], ring.phase);
+                if (lane == 0) mbar_arrive_leader(smem_u32(&full_bar[ring.at]));
+                __syncwarp();
+                ring.next(p.stages);
+            }
+        }
+    } else if (warp < UM_DW) {
+        // ---------------- decode ----------------
+        const int tile = warp >> 1, half = warp & 1;  // stages 2 half, 2 half + 1 of every superblock
+        uint8_t * tab = tabs + warp * HalfRecord<DT>::TAB;
+        const DecodeConsts kc = p.kc;
+        Ring ring, rr;
+        if (half) {
+            ring.next(p.stages);
+            ring.next(p.stages);
+        }
+        for (UmmaWork wk(p); wk.valid(); wk.next()) {
+            for (int n = wk.sb_end(p) - wk.sb_begin(p); n > 0; n--) {
+                HalfRecord<DT> r;
+                wait(raw_full[rr.at], rr.phase);
+                r.fetch(raw + (size_t)rr.at * S::RAW_BYTES + tile * C::REC, lane, half);
+                r.header(lane, half, tab);
+                __syncwarp();  // the table is complete, and every lane has its part of the record
+                if (lane == 0) mbar_arrive(smem_u32(&raw_empty[rr.at]));
+                rr.next(UM_RAW_STAGES);
+                auto chunk = [&](auto c) {
+                    wait(empty_bar[ring.at], ring.phase ^ 1u);
+                    r.template store<decltype(c)::value>(lane, tab, kc, smem + (size_t)ring.at * stage_bytes + tile * 16 * 128);
                     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
                     __syncwarp();
-                    if (lane == 0) mbar_arrive((uint32_t)__cvta_generic_to_shared(&afull_bar[stage]));
-                    if (++stage == p.stages) { stage = 0; use++; }
-                }
-                __syncwarp();
-                cur = nxt;
+                    if (lane == 0) mbar_arrive_leader(smem_u32(&full_bar[ring.at]));
+                    ring.next(p.stages);
+                };
+                chunk(std::integral_constant<int, 0>());
+                chunk(std::integral_constant<int, 1>());
+                ring.next(p.stages);
+                ring.next(p.stages);
             }
-            // ---- epilogue of this block of 128 weight rows ----
-            if (!expired && !mbar_wait((uint32_t)__cvta_generic_to_shared(&done_bar), block_iter & 1)) expired = true;
+        }
+    } else {
+        // ---------------- epilogue: tensor-memory lane = weight row, column = activation row ----------------
+        pdl_wait();
+        const int quad = warp & 3;
+        Ring acc;
+        for (UmmaWork wk(p); wk.valid(); wk.next()) {
+            wait(acc_full[acc.at], acc.phase);
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            const bool split = gridDim.y > 1;
-            {
-                const int quad = warp & 3;
-                const int n = rb * UM_ROWS + quad * 32 + lane;
-                float * base = split ? p.partial + (size_t)blockIdx.y * p.M * p.N : p.out;
-                const int64_t ld = split ? p.N : p.ldo;
-                for (int c0 = (warp >> 2) * 32; c0 < p.npad; c0 += (UM_DW / 4) * 32) {
-                    uint32_t v[32];
-                    const uint32_t src = taddr + ((uint32_t)(quad * 32) << 16) + (uint32_t)c0;
-                    asm volatile(
-                        "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
-                        "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
-                        "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
-                        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]),
-                          "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]), "=r"(v[16]),
-                          "=r"(v[17]), "=r"(v[18]), "=r"(v[19]), "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]), "=r"(v[24]),
-                          "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
-                        : "r"(src)
-                        : "memory");
-                    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-                    if (n < p.N && c0 < p.M) {
-                        float * dst = base + (int64_t)c0 * ld + n;
-                        if (split) umma_store_rows<2>(dst, ld, v, p.M - c0);
-                        else if (p.accumulate) umma_store_rows<1>(dst, ld, v, p.M - c0);
-                        else umma_store_rows<0>(dst, ld, v, p.M - c0);
-                    }
+            const int n = (wk.block(p) * 2 + (int)rank) * UM_ROWS + quad * 32 + lane, m0 = wk.n0(p);
+            const bool split = p.kparts > 1;
+            float * base = split ? p.partial + (size_t)wk.part(p) * p.M * p.N : p.out;
+            const int64_t ld = split ? p.N : p.ldo;
+            for (int c0 = 0; c0 < p.n_tile && m0 + c0 < p.M; c0 += 32) {
+                uint32_t v[32];
+                tmem_load32(v, taddr + ((uint32_t)(quad * 32) << 16) + acc.at * (uint32_t)UM_MAX_N + (uint32_t)c0);
+                if (n < p.N) {
+                    float * dst = base + (int64_t)(m0 + c0) * ld + n;
+                    const int lim = min(p.M - m0, p.n_tile) - c0;
+                    if (split) umma_store_rows<2>(dst, ld, v, lim);
+                    else if (p.accumulate) umma_store_rows<1>(dst, ld, v, lim);
+                    else umma_store_rows<0>(dst, ld, v, lim);
                 }
             }
-            // the accumulator has been read: the issue warp may start the next block of rows
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             __syncwarp();
-            if (lane == 0) mbar_arrive((uint32_t)__cvta_generic_to_shared(&tmem_free_bar));
-            if (split && p.counters) {
-                // K is split across CTAs: the last one to finish this block of rows sums the parts in a fixed order
-                // (without counters the parts are summed by umma_reduce_kernel, launched next)
-                __threadfence();
-                asm volatile("bar.sync 1, %0;" ::"n"(UM_DW * 32) : "memory");
-                if (threadIdx.x == 0) last_flag = atomicAdd(&p.counters[rb], 1) == (int)gridDim.y - 1;
-                asm volatile("bar.sync 1, %0;" ::"n"(UM_DW * 32) : "memory");
-                if (last_flag) {
-                    __threadfence();
-                    const int n0 = rb * UM_ROWS, nrows = min(UM_ROWS, p.N - n0);
-                    const int total = p.M * nrows;
-                    for (int i0 = threadIdx.x; i0 < total; i0 += 4 * UM_DW * 32) {
-                        float sum[4] = {0.0f, 0.0f, 0.0f, 0.0f}, old[4];
-                        float * dst[4];
-#pragma unroll
-                        for (int u = 0; u < 4; u++) {
-                            const int i = min(i0 + u * UM_DW * 32, total - 1);
-                            const int tok = i / nrows, n = n0 + i - tok * nrows;
-                            dst[u] = p.out + (int64_t)tok * p.ldo + n;
-                            old[u] = p.accumulate ? *dst[u] : 0.0f;
-                        }
-                        for (int part = 0; part < (int)gridDim.y; part++) {
-                            float v[4];
-#pragma unroll
-                            for (int u = 0; u < 4; u++) {
-                                const int i = min(i0 + u * UM_DW * 32, total - 1);
-                                const int tok = i / nrows, n = n0 + i - tok * nrows;
-                                v[u] = __ldcg(p.partial + ((size_t)part * p.M + tok) * p.N + n);
-                            }
-#pragma unroll
-                            for (int u = 0; u < 4; u++) sum[u] += v[u];
-                        }
-#pragma unroll
-                        for (int u = 0; u < 4; u++)
-                            if (i0 + u * UM_DW * 32 < total) *dst[u] = old[u] + sum[u];
-                    }
-                    if (threadIdx.x == 0) p.counters[rb] = 0;
-                }
-                asm volatile("bar.sync 1, %0;" ::"n"(UM_DW * 32) : "memory");  // last_flag is reused by the next block
-            }
+            if (lane == 0) mbar_arrive_leader(smem_u32(&acc_empty[acc.at]));
+            acc.next(2);
         }
     }
     if (expired) atomicExch(&g_gemm_wait_expired, 3);
-    // all MMAs have completed (every block's done_bar was waited for) and all epilogue loads are done
+    // every MMA has completed (the epilogue has waited for the last one of each accumulator); nothing of this CTA is touched by
+    // the other one after the barrier
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
-    if (warp == 0)
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(p.tmem_cols) : "memory");
+    cluster_sync_all();
+    if (warp == UM_WARP_MMA)
+        asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(512u) : "memory");
 }
 
 // Sum of the K parts of a split tensor-memory GEMM, in part order: out[tok][n] (+)= sum over parts of
-// partial[part][tok][n]. With many parts and hundreds of activation rows the whole machine sums; the last CTA
-// of a 128-row block doing it alone took longer than the decode the split saved.
+// partial[part][tok][n], by the whole machine (the last CTA of a block doing it alone took longer than the decode the
+// split saves). V = 4 where rows allow 16-byte accesses.
+template <int V>
 __global__ void __launch_bounds__(256) umma_reduce_kernel(float * __restrict__ out, int64_t ldo, const float * __restrict__ partial,
                                                           int parts, int M, int N, int accumulate) {
     pdl_entry();
-    const int n4 = N >> 2;
-    const int64_t total = (int64_t)M * n4;
+    const int nv = N / V;
+    const int64_t total = (int64_t)M * nv;
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
-        const int tok = (int)(i / n4), n = (int)(i - (int64_t)tok * n4) * 4;
-        float4 * dst = reinterpret_cast<float4 *>(out + (int64_t)tok * ldo + n);
-        float4 sum = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        const int tok = (int)(i / nv), n = (int)(i - (int64_t)tok * nv) * V;
+        float * dst = out + (int64_t)tok * ldo + n;
+        float sum[V];
+#pragma unroll
+        for (int e = 0; e < V; e++) sum[e] = 0.0f;
         for (int part = 0; part < parts; part++) {
-            const float4 v = __ldcg(reinterpret_cast<const float4 *>(partial + ((size_t)part * M + tok) * N + n));
-            sum.x += v.x;
-            sum.y += v.y;
-            sum.z += v.z;
-            sum.w += v.w;
+            const float * src = partial + ((size_t)part * M + tok) * N + n;
+            if constexpr (V == 4) {
+                const float4 v = __ldcg(reinterpret_cast<const float4 *>(src));
+                sum[0] += v.x;
+                sum[1] += v.y;
+                sum[2] += v.z;
+                sum[3] += v.w;
+            } else {
+                sum[0] += __ldcg(src);
+            }
         }
-        if (accumulate) {
-            const float4 old = *dst;
-            sum.x = old.x + sum.x;
-            sum.y = old.y + sum.y;
-            sum.z = old.z + sum.z;
-            sum.w = old.w + sum.w;
-        }
-        *dst = sum;
+#pragma unroll
+        for (int e = 0; e < V; e++) dst[e] = accumulate ? dst[e] + sum[e] : sum[e];
     }
 }
 
