@@ -1402,19 +1402,20 @@ static bool umma_enabled() {
 // How a launch of the tensor-memory kernel is cut: m activation rows into n_tiles tiles of n_tile rows, K into kparts.
 struct UmmaPlan {
     int n_tile, n_tiles, kparts;
+    bool halves;
 };
 // K parts: enough pairs of CTAs to fill the machine when the matrix has few blocks of rows, at least two superblocks each.
-// Two parts do not pay for the launch that sums them (9216 x 2560 at 576 rows: 47 us against 39), and without 16-byte
-// stores that sum is four times the loads, so fewer parts pay. (The count does not depend on how the rows are tiled: the
-// sums, and with them the bits of a row's result, do not change with the rows that travel with it, up to 96 rows and
-// beyond where n_out is not a multiple of four.)
+// Two parts do not pay for the launch that sums them (9216 x 2560 at 576 rows: 47 us against 39): one pair then takes both
+// halves of K, in two accumulators that its epilogue adds. Without 16-byte stores the summing launch takes four times the
+// loads, so fewer parts pay. (The count does not depend on how the rows are tiled: the sums, and with them the bits of a
+// row's result, do not change with the rows that travel with it, up to 96 rows and beyond where n_out is a multiple of four.)
 static int umma_kparts(const yuuka_device * dev, int n_out, int n_in, int m) {
     const int n_blocks = (n_out + UM_ROWS - 1) / UM_ROWS, nsb = n_in / 256;
     int ks = dev->sm_count / n_blocks;
     if (ks > nsb / 2) ks = nsb / 2;
-    const int cap = (n_out & 3) == 0 ? 8 : (m <= 96 ? 4 : 1);
+    const int cap = (n_out & 3) == 0 ? 8 : (m <= 96 ? 4 : 2);
     if (ks > cap) ks = cap;
-    return ks <= 2 ? 1 : ks;
+    return ks < 1 ? 1 : ks;
 }
 // The tiling of the rows with the lowest estimate of cycles: rounds of the pairs x (stages of a tile x cycles per stage +
 // a fixed cost for filling and draining the rings). A stage took 634 / 682 / 774 / 890 cycles at 64 / 128 / 192 / 256
@@ -1422,7 +1423,11 @@ static int umma_kparts(const yuuka_device * dev, int n_out, int n_in, int m) {
 constexpr double UMMA_STAGE = 540.0, UMMA_ROW = 1.3, UMMA_TILE = 4000.0;
 static UmmaPlan umma_plan(const yuuka_device * dev, int n_out, int n_in, int m) {
     const int m_blocks = (n_out + 2 * UM_ROWS - 1) / (2 * UM_ROWS), nsb = n_in / 256, pairs = dev->sm_count / 2;
-    UmmaPlan best{0, 0, umma_kparts(dev, n_out, n_in, m)};
+    UmmaPlan best{0, 0, umma_kparts(dev, n_out, n_in, m), false};
+    if (best.kparts == 2) {
+        best.kparts = 1;
+        best.halves = true;
+    }
     double best_cost = 1e30;
     const int t0 = (m + UM_MAX_N - 1) / UM_MAX_N, stages = (nsb + best.kparts - 1) / best.kparts * 4;
     for (int tiles = t0; tiles <= t0 + 4; tiles++) {
@@ -1447,7 +1452,7 @@ void gemm_tiled_scratch_need(const yuuka_device * dev, uint32_t w_dtype, int row
     // enough for this row count and for every smaller one (fewer rows may split K further)
     for (int m : {rows, rows < 96 ? rows : 96}) {
         const int parts = rows >= UMMA_EARLY_ROWS ? umma_kparts(dev, n_out, n_in, m) : 1;
-        if (parts > 1 && (uint64_t)parts * m * n_out > *partial_floats) *partial_floats = (uint64_t)parts * m * n_out;
+        if (parts > 2 && (uint64_t)parts * m * n_out > *partial_floats) *partial_floats = (uint64_t)parts * m * n_out;
     }
     for (int m : {rows < MMA_ROWS ? rows : MMA_ROWS, MMA_ROWS < rows ? rows % MMA_ROWS : 0}) {
         if (m <= 0) continue;
@@ -1628,6 +1633,7 @@ static int launch_umma_dt(const yuuka_device * dev, cudaStream_t s, const TiledG
     p.ldo = a.ldo;
     p.accumulate = (a.flags & YUUKA_GEMM_ACCUMULATE) ? 1 : 0;
     p.kparts = pl.kparts;
+    p.halves = pl.halves ? 1 : 0;
     p.n_tile = pl.n_tile;
     p.n_tiles = pl.n_tiles;
     p.m_blocks = (a.n_out + 2 * UM_ROWS - 1) / (2 * UM_ROWS);

@@ -31,6 +31,7 @@ constexpr int UM_ROWS = 128;     // weight rows per CTA; a pair has 256
 constexpr int UM_KC = 64;        // columns per stage
 constexpr int UM_MAX_N = 256;    // activation rows per tile
 constexpr int UM_MAX_STAGES = 6;
+constexpr int UM_MAX_ACC = 4;  // accumulators of up to 128 columns; two of up to 256
 constexpr int UM_RAW_STAGES = 2; // superblocks of packed weights in shared memory
 constexpr int UM_TILES = 8;      // 16-row tiles per CTA
 constexpr int UM_DW = 16;        // decode warps, two per tile: a half of every record each
@@ -53,6 +54,7 @@ struct UParams {
     int accumulate;
     float * partial;      // [kparts][M][N] when K is split across pairs
     int kparts;
+    int halves;           // kparts == 1: the two halves of K are summed apart, in two accumulators
     int n_tile, n_tiles;  // activation rows per tile (a multiple of 32), tiles
     int m_blocks;         // blocks of 256 weight rows
     uint32_t idesc;
@@ -370,7 +372,7 @@ __global__ void __launch_bounds__(UM_THREADS, 1) gemm_umma_kernel(const UParams 
     __shared__ __align__(8) uint64_t full_bar[UM_MAX_STAGES];   // (even CTA) both CTAs' weights and activations are in the stage
     __shared__ __align__(8) uint64_t x_bar[UM_MAX_STAGES];      // (odd CTA) its activations have landed
     __shared__ __align__(8) uint64_t raw_full[UM_RAW_STAGES], raw_empty[UM_RAW_STAGES];
-    __shared__ __align__(8) uint64_t acc_full[2], acc_empty[2]; // accumulators: finished by the MMAs, read by the epilogue
+    __shared__ __align__(8) uint64_t acc_full[UM_MAX_ACC], acc_empty[UM_MAX_ACC]; // accumulators: finished by the MMAs, read by the epilogue
     __shared__ uint32_t tmem_slot;
     const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;  // (uniform for the compiler too)
     const uint32_t rank = blockIdx.x & 1u;  // clusters are pairs along x
@@ -388,7 +390,7 @@ __global__ void __launch_bounds__(UM_THREADS, 1) gemm_umma_kernel(const UParams 
             mbar_init(smem_u32(&raw_full[s]), 1);
             mbar_init(smem_u32(&raw_empty[s]), UM_DW);
         }
-        for (int s = 0; s < 2; s++) {
+        for (int s = 0; s < UM_MAX_ACC; s++) {
             mbar_init(smem_u32(&acc_full[s]), 1);
             mbar_init(smem_u32(&acc_empty[s]), 2 * UM_EW);
         }
@@ -403,6 +405,7 @@ __global__ void __launch_bounds__(UM_THREADS, 1) gemm_umma_kernel(const UParams 
     cluster_sync_all();  // both CTAs' barriers are set up
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t taddr = tmem_slot, smem_base = smem_u32(smem);
+    const uint32_t acc_cols = p.n_tile <= UM_MAX_N / 2 ? UM_MAX_N / 2 : UM_MAX_N, n_acc = 512u / acc_cols;  // accumulators
     const int n_tiles16 = (p.N + 15) >> 4;
     const size_t rec_row = (size_t)p.nsb * C::REC;
     bool expired = false;
@@ -460,24 +463,33 @@ __global__ void __launch_bounds__(UM_THREADS, 1) gemm_umma_kernel(const UParams 
         const uint32_t step = stage_bytes >> 4;
         for (UmmaWork wk(p); wk.valid(); wk.next()) {
             wait(acc_empty[acc.at], acc.phase ^ 1u);
-            const uint32_t d = taddr + acc.at * (uint32_t)UM_MAX_N;
-            const int chunks = (wk.sb_end(p) - wk.sb_begin(p)) * 4;
+            uint32_t d = taddr + acc.at * acc_cols, keep = 0;
+            const int chunks = (wk.sb_end(p) - wk.sb_begin(p)) * 4, second = p.halves ? (p.nsb >> 1) * 4 : chunks;
             for (int c = 0; c < chunks; c++) {
+                if (c == second) {  // the other half of K goes to an accumulator of its own
+                    if (elect_one()) umma_commit_pair(smem_u32(&acc_full[acc.at]));
+                    __syncwarp();
+                    acc.next(n_acc);
+                    wait(acc_empty[acc.at], acc.phase ^ 1u);
+                    d = taddr + acc.at * acc_cols;
+                    keep = 0;
+                }
                 wait(full_bar[ring.at], ring.phase);
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 const uint64_t da = da0 + (uint64_t)(ring.at * step), db = db0 + (uint64_t)(ring.at * step);
                 if (elect_one()) {
 #pragma unroll
                     for (int j = 0; j < UM_KC / 16; j++)
-                        umma_f16_pair(d, da + (uint64_t)(j * 2), db + (uint64_t)(j * 2), p.idesc, (c > 0 || j > 0) ? 1u : 0u);
+                        umma_f16_pair(d, da + (uint64_t)(j * 2), db + (uint64_t)(j * 2), p.idesc, j > 0 ? 1u : keep);
                     umma_commit_pair(smem_u32(&empty_bar[ring.at]));
                 }
                 __syncwarp();
+                keep = 1;
                 ring.next(p.stages);
             }
             if (elect_one()) umma_commit_pair(smem_u32(&acc_full[acc.at]));
             __syncwarp();
-            acc.next(2);
+            acc.next(n_acc);
         }
     } else if (warp == UM_WARP_MMA) {
         // ---------------- odd CTA: its activations have landed -> the even CTA's barrier ----------------
@@ -530,7 +542,12 @@ __global__ void __launch_bounds__(UM_THREADS, 1) gemm_umma_kernel(const UParams 
         const int quad = warp & 3;
         Ring acc;
         for (UmmaWork wk(p); wk.valid(); wk.next()) {
-            wait(acc_full[acc.at], acc.phase);
+            const uint32_t first = acc.at;
+            wait(acc_full[first], acc.phase);
+            if (p.halves) {
+                acc.next(n_acc);
+                wait(acc_full[acc.at], acc.phase);
+            }
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const int n = (wk.block(p) * 2 + (int)rank) * UM_ROWS + quad * 32 + lane, m0 = wk.n0(p);
             const bool split = p.kparts > 1;
@@ -538,7 +555,14 @@ __global__ void __launch_bounds__(UM_THREADS, 1) gemm_umma_kernel(const UParams 
             const int64_t ld = split ? p.N : p.ldo;
             for (int c0 = 0; c0 < p.n_tile && m0 + c0 < p.M; c0 += 32) {
                 uint32_t v[32];
-                tmem_load32(v, taddr + ((uint32_t)(quad * 32) << 16) + acc.at * (uint32_t)UM_MAX_N + (uint32_t)c0);
+                const uint32_t from = taddr + ((uint32_t)(quad * 32) << 16) + (uint32_t)c0;
+                tmem_load32(v, from + first * acc_cols);
+                if (p.halves) {
+                    uint32_t v2[32];
+                    tmem_load32(v2, from + acc.at * acc_cols);
+#pragma unroll
+                    for (int e = 0; e < 32; e++) v[e] = __float_as_uint(__uint_as_float(v[e]) + __uint_as_float(v2[e]));
+                }
                 if (n < p.N) {
                     float * dst = base + (int64_t)(m0 + c0) * ld + n;
                     const int lim = min(p.M - m0, p.n_tile) - c0;
@@ -549,8 +573,11 @@ __global__ void __launch_bounds__(UM_THREADS, 1) gemm_umma_kernel(const UParams 
             }
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             __syncwarp();
-            if (lane == 0) mbar_arrive_leader(smem_u32(&acc_empty[acc.at]));
-            acc.next(2);
+            if (lane == 0) {
+                mbar_arrive_leader(smem_u32(&acc_empty[first]));
+                if (p.halves) mbar_arrive_leader(smem_u32(&acc_empty[acc.at]));
+            }
+            acc.next(n_acc);
         }
     }
     if (expired) atomicExch(&g_gemm_wait_expired, 3);
