@@ -528,7 +528,7 @@ struct yuuka_session {
     int32_t * d_tables = nullptr;
     std::vector<int> h_pos, h_pos_upper;
     // per step
-    // row metadata of a step, one device block [anc | tokens | parent | depth] filled by one copy from the
+    // row metadata of a step, one device block [anc | tokens | parent | depth | order] filled by one copy from the
     // page-locked mirror h_rows; results [accepted | path | emitted] likewise come back in one copy to h_results
     uint8_t * d_rows = nullptr;
     uint8_t * h_rows = nullptr;
@@ -541,6 +541,7 @@ struct yuuka_session {
     int32_t * d_tokens = nullptr;
     int32_t * d_parent = nullptr;
     int32_t * d_depth = nullptr;
+    int32_t * d_order = nullptr;  // nodes depth first, written for steps with a tree in them
     uint64_t * d_anc = nullptr;
     float *x = nullptr, *xn = nullptr, *qkv_attn = nullptr, *attn_out = nullptr, *gdn_out = nullptr;
     float *gate_up = nullptr, *act = nullptr, *logits = nullptr;
@@ -743,6 +744,7 @@ void run_step(yuuka_session * s, int seq0, int batch, int nodes, uint32_t mode, 
     const int R = batch * nodes, H = c.hidden;
     RowMeta rows{s->d_tokens, s->d_parent, s->d_depth, s->d_anc, s->d_pos0 + seq0, batch, nodes};
     rows.chains = sub > 0 ? 1 : s->st_chains;
+    rows.order = s->d_order;
     if (mapped) rows.seq_map = s->d_seq_map;
     YK_REQUIRE(!mapped || (seq0 == 0 && sub == 0), YUUKA_ERR_INTERNAL, "a mapped step starts at sequence 0 and has no sub-chunks");
     YK_REQUIRE(sub == 0 || (batch == 1 && mode == 3u && nodes <= CHAIN_MAX_SUBS * sub), YUUKA_ERR_INTERNAL,
@@ -1098,10 +1100,33 @@ void sync_and_check(yuuka_session * s) {
     YK_REQUIRE(err == 0, YUUKA_ERR_DEVICE, "a bounded wait inside a kernel expired (code %d); results are invalid", err);
 }
 
-// bytes of the per-step metadata block: ancestor masks, tokens, parents, depths of `cap` rows, the sub-chunk
+// bytes of the per-step metadata block: ancestor masks, tokens, parents, depths and depth-first order of `cap` rows, the sub-chunk
 // positions and acceptances of a wide prompt pass, and the slot -> sequence map
+constexpr size_t ROW_BYTES = 24;
 size_t rows_block_bytes(int cap, int max_batch) {
-    return (size_t)cap * 20 + 2 * CHAIN_MAX_SUBS * sizeof(int32_t) + (size_t)max_batch * sizeof(int32_t);
+    return (size_t)cap * ROW_BYTES + 2 * CHAIN_MAX_SUBS * sizeof(int32_t) + (size_t)max_batch * sizeof(int32_t);
+}
+
+// The nodes of a tree (parents before children in `par`) depth first, children in row order: every node is put in
+// front of its parent's next sibling by threading first-child / next-sibling links.
+void depth_first_order(const int32_t * par, int n, int32_t * order) {
+    int32_t child[64], sibling[64];
+    for (int i = 0; i < n; i++) child[i] = -1;
+    for (int i = n - 1; i > 0; i--) {
+        sibling[i] = child[par[i]];
+        child[par[i]] = i;
+    }
+    sibling[0] = -1;
+    int count = 0;
+    for (int at = 0; at >= 0;) {
+        order[count++] = at;
+        if (child[at] >= 0) {
+            at = child[at];
+            continue;
+        }
+        while (at >= 0 && sibling[at] < 0) at = par[at];
+        if (at >= 0) at = sibling[at];
+    }
 }
 
 // Uploads row metadata of a step: tokens, parents, depths, ancestor masks.
@@ -1118,6 +1143,7 @@ void stage_rows(yuuka_session * s, int seq0, int batch, int nodes, const int32_t
     int32_t * tok = reinterpret_cast<int32_t *>(s->h_rows + (size_t)cap * 8);
     int32_t * par = tok + cap;
     int32_t * dep = par + cap;
+    int32_t * ord = dep + cap;
     s->st_chains = 1;
     for (int b = 0; b < batch; b++) {
         for (int i = 0; i < nodes; i++) {
@@ -1140,11 +1166,12 @@ void stage_rows(yuuka_session * s, int seq0, int batch, int nodes, const int32_t
             dep[r] = i == 0 ? 0 : dep[b * nodes + p] + 1;
             anc[r] = (i == 0 ? 0ull : anc[b * nodes + p]) | (1ull << i);
         }
+        if (parent && sub == 0) depth_first_order(par + b * nodes, nodes, ord + b * nodes);
         const int sq = seq_ids ? seq_ids[b] : seq0 + b;
         YK_REQUIRE(s->h_pos_upper[sq] + nodes <= s->cfg.capacity, YUUKA_ERR_INVALID_ARGUMENT,
                    "token sequence of %d exceeds remaining context %d", nodes, s->cfg.capacity - s->h_pos_upper[sq]);
     }
-    int32_t * pos_sub = reinterpret_cast<int32_t *>(s->h_rows + (size_t)cap * 20);
+    int32_t * pos_sub = reinterpret_cast<int32_t *>(s->h_rows + (size_t)cap * ROW_BYTES);
     int32_t * acc_sub = pos_sub + CHAIN_MAX_SUBS;
     for (int k = 0; k < CHAIN_MAX_SUBS; k++) {
         const int left = sub > 0 ? nodes - k * sub : 0;
@@ -1381,13 +1408,14 @@ yuuka_status yuuka_session_create(yuuka_model * model, const yuuka_session_confi
             s->h_pos_upper.assign(B, 0);
             s->rows_cap = R;
             s->d_rows = dalloc<uint8_t>(rows_block_bytes(R, B), s->owned);
-            s->d_pos_sub = reinterpret_cast<int32_t *>(s->d_rows + (size_t)R * 20);
+            s->d_pos_sub = reinterpret_cast<int32_t *>(s->d_rows + (size_t)R * ROW_BYTES);
             s->d_acc_sub = s->d_pos_sub + CHAIN_MAX_SUBS;
             s->d_seq_map = s->d_acc_sub + CHAIN_MAX_SUBS;
             s->d_anc = reinterpret_cast<uint64_t *>(s->d_rows);
             s->d_tokens = reinterpret_cast<int32_t *>(s->d_rows + (size_t)R * 8);
             s->d_parent = s->d_tokens + R;
             s->d_depth = s->d_parent + R;
+            s->d_order = s->d_depth + R;
             {
                 void * hp = nullptr;
                 const size_t rows_bytes = rows_block_bytes(R, B);

@@ -58,74 +58,116 @@ __device__ __forceinline__ float2 state_update2(float2 s, float2 decay, float2 k
 struct ScanParams {
     GdnArgs a;
     RowMeta rows;
-    int chain;  // front end only: the rows are one chain (row i follows row i - 1), however many there are
+    int chain;       // front end only: the rows are chains (row i follows row i - 1), however many there are
+    int block_rows;  // front end only: rows of a sequence per CTA
 };
 
 // ---------------------------------------------------------------------------
-// Front end, fully parallel over (row, 128-channel unit): depthwise causal conv
-// over the row's ancestors and the stored history + SiLU (forward.go:253-268),
-// L2 norm of the q and k units (forward.go:275-279, 484-493), beta = sigmoid,
+// Front end, parallel over (row, S-channel unit): depthwise causal conv over the row's ancestors and the stored
+// history + SiLU (forward.go:253-268), L2 norm of the q and k units (forward.go:275-279, 484-493), beta = sigmoid,
 // decay = exp(softplus(alpha + dt) * a) (forward.go:245-248).
-// grid (2*groups + rank, nodes, batch), S threads.
-__global__ void gdn_front_kernel(const ScanParams p) {
+// grid (2*groups + rank, row blocks, batch). A warp owns a row of a unit outright, S / 32 channels per lane: every tap of
+// a row is in flight at once, the sums of squares close by shuffles (as many independent chains as channels), nothing
+// meets at a barrier, and a warp goes on to its next row with its weights in registers. It is latency that bounds this
+// kernel: one CTA per (row, unit) spent 39 us on 512 rows of 8192 channels (15 waves of CTAs, each a chain of waits)
+// where its 40 MB take 6.
+// KMAX: taps held in registers (4, or 8 for the longer kernels).
+template <int S, int KMAX>
+__global__ void __launch_bounds__(128) gdn_front_kernel(const ScanParams p) {
     // (releasing the scan from here, so that it could fetch its state while this kernel runs, measured 7 us
     // slower per layer: a dependent grid that starts early and really has to block in griddepcontrol.wait
     // is woken late; only triggers placed at the end of a kernel have paid)
-    pdl_entry();
     const GdnArgs & a = p.a;
-    const int S = a.S, N = p.rows.nodes;
-    const int u = blockIdx.x, node = blockIdx.y, seq = blockIdx.z;
-    const int key_dim = a.groups * S, conv_dim = 2 * key_dim + a.rank * S, K1 = a.kernel - 1;
-    const int r = seq * N + node;
-    __shared__ int par[GDN_MAX_NODES];
-    __shared__ double red[4];
+    constexpr int G = S / 32;
+    const int N = p.rows.nodes, K = a.kernel, K1 = K - 1;
+    const int u = blockIdx.x, seq = blockIdx.z, lane = threadIdx.x & 31;
+    const int key_dim = a.groups * S, conv_dim = 2 * key_dim + a.rank * S;
+    const int c0 = u * S + lane;  // q units, then k units, then v units: exactly the conv row order
+    float w[G][KMAX];
+#pragma unroll
+    for (int i = 0; i < G; i++)
+#pragma unroll
+        for (int t = 0; t < KMAX; t++) w[i][t] = t < K ? a.conv_w[(int64_t)(c0 + 32 * i) * K + t] : 0.0f;
+    int par0 = -1, par1 = -1;  // parents of rows lane and lane + 32
     if (!p.chain) {
-        for (int i = threadIdx.x; i < N; i += blockDim.x) par[i] = p.rows.parent[seq * N + i];
-        __syncthreads();
+        if (lane < N) par0 = p.rows.parent[seq * N + lane];
+        if (lane + 32 < N) par1 = p.rows.parent[seq * N + lane + 32];
     }
-    const int e = threadIdx.x;
-    const int c = u * S + e;  // q units, then k units, then v units: exactly the conv row order
-    float taps[8];
-    {
-        const float * hist = a.conv_state + ((int64_t)seq_of(p.rows, seq) * conv_dim + c) * K1;
+    pdl_entry();
+    const float * proj = a.proj + (int64_t)seq * N * a.ldp;
+    const float * hist = a.conv_state + ((int64_t)seq_of(p.rows, seq) * conv_dim + c0) * K1;
+    const int first = blockIdx.y * p.block_rows, last = min(N, first + p.block_rows);
+    for (int node = first + (int)(threadIdx.x >> 5); node < last; node += (int)(blockDim.x >> 5)) {
+        const int r = seq * N + node;
+        float taps[G][KMAX];
         int cur = node, hidx = K1 - 1;
 #pragma unroll
-        for (int t = 7; t >= 0; t--) {
-            if (t >= a.kernel) { taps[t] = 0.0f; continue; }
-            if (cur >= 0) {
-                taps[t] = a.proj[(int64_t)(seq * N + cur) * a.ldp + c];
-                cur = p.chain ? cur - 1 : par[cur];
-            } else {
-                taps[t] = hist[hidx--];
+        for (int t = KMAX - 1; t >= 0; t--) {
+            if (t < K) {
+                const float * src = cur >= 0 ? proj + (int64_t)cur * a.ldp + c0 : hist + hidx;
+                const int stride = cur >= 0 ? 32 : 32 * K1;
+#pragma unroll
+                for (int i = 0; i < G; i++) taps[i][t] = src[i * stride];
+                if (cur < 0) hidx--;
+                else if (p.chain) cur--;
+                else cur = __shfl_sync(0xffffffffu, cur < 32 ? par0 : par1, cur & 31);
+            }
+        }
+        float v[G];
+#pragma unroll
+        for (int i = 0; i < G; i++) {
+            float sum = 0.0f;
+#pragma unroll
+            for (int t = 0; t < KMAX; t++)
+                if (t < K) sum += w[i][t] * taps[i][t];
+            v[i] = silu_ref(sum);
+        }
+        if (u < 2 * a.groups) {
+            double sq[G];
+#pragma unroll
+            for (int i = 0; i < G; i++) sq[i] = (double)v[i] * (double)v[i];
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+                for (int i = 0; i < G; i++) sq[i] += __shfl_xor_sync(0xffffffffu, sq[i], o);
+            double tot = 0;
+#pragma unroll
+            for (int i = 0; i < G; i++) tot += sq[i];
+            const float scale = (float)(1.0 / sqrt(tot + (double)a.eps));
+            const bool is_q = u < a.groups;
+            const float mul = is_q ? scale * (float)(1.0 / sqrt((double)S)) : scale;
+            float * dst = (is_q ? a.qn + u * S : a.khat + (u - a.groups) * S) + (int64_t)r * key_dim + lane;
+#pragma unroll
+            for (int i = 0; i < G; i++) dst[32 * i] = v[i] * mul;
+        } else {
+            const int h = u - 2 * a.groups;
+            float * dst = a.vconv + (int64_t)r * (a.rank * S) + h * S + lane;
+#pragma unroll
+            for (int i = 0; i < G; i++) dst[32 * i] = v[i];
+            if (lane == 0) {
+                const float * row = a.proj + (int64_t)r * a.ldp;
+                a.beta[(int64_t)r * a.rank + h] = sigmoid_ref(row[conv_dim + a.rank * S + h]);
+                a.decay[(int64_t)r * a.rank + h] = expf(softplus_ref(row[conv_dim + a.rank * S + a.rank + h] + a.dt[h]) * a.a[h]);
             }
         }
     }
-    float sum = 0.0f;
-    const float * w = a.conv_w + (int64_t)c * a.kernel;
-#pragma unroll
-    for (int t = 0; t < 8; t++)
-        if (t < a.kernel) sum += w[t] * taps[t];
-    float v = silu_ref(sum);
-    if (u < 2 * a.groups) {
-        double sq = (double)v * (double)v;
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) sq += __shfl_xor_sync(0xffffffffu, sq, o);
-        if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = sq;
-        __syncthreads();
-        double tot = 0;
-        for (int i = 0; i < (S >> 5); i++) tot += red[i];
-        const float scale = (float)(1.0 / sqrt(tot + (double)a.eps));
-        if (u < a.groups) a.qn[(int64_t)r * key_dim + u * S + e] = v * (scale * (float)(1.0 / sqrt((double)S)));
-        else a.khat[(int64_t)r * key_dim + (u - a.groups) * S + e] = v * (scale * 1.0f);
-    } else {
-        const int h = u - 2 * a.groups;
-        a.vconv[(int64_t)r * (a.rank * S) + h * S + e] = v;
-        if (e == 0) {
-            const float * row = a.proj + (int64_t)r * a.ldp;
-            a.beta[(int64_t)r * a.rank + h] = sigmoid_ref(row[conv_dim + a.rank * S + h]);
-            a.decay[(int64_t)r * a.rank + h] = expf(softplus_ref(row[conv_dim + a.rank * S + a.rank + h] + a.dt[h]) * a.a[h]);
-        }
-    }
+}
+
+// Rows of a unit per CTA of four warps: one row per warp until the launch has a resident wave of warps (24 per SM), then
+// as many as keep it at one wave.
+static void launch_gdn_front(cudaStream_t s, const GdnArgs & a, const RowMeta & rows, bool chain) {
+    YK_REQUIRE(a.kernel >= 2 && a.kernel <= 8, YUUKA_ERR_UNSUPPORTED, "gdn: conv kernel %d is outside 2..8", a.kernel);
+    YK_REQUIRE(a.S == 64 || a.S == 128, YUUKA_ERR_UNSUPPORTED, "gdn: state size %d is not 64 or 128", a.S);
+    ScanParams p{a, rows, chain ? 1 : 0, 0};
+    const int units = 2 * a.groups + a.rank;
+    constexpr int64_t WAVE = 148 * 24;
+    const int64_t per_warp = ((int64_t)units * rows.nodes * rows.batch + WAVE - 1) / WAVE;
+    const int blocks = (int)((rows.nodes + 4 * per_warp - 1) / (4 * per_warp));
+    p.block_rows = (rows.nodes + blocks - 1) / blocks;
+    auto kern = a.S == 128 ? (a.kernel <= 4 ? gdn_front_kernel<128, 4> : gdn_front_kernel<128, 8>)
+                           : (a.kernel <= 4 ? gdn_front_kernel<64, 4> : gdn_front_kernel<64, 8>);
+    launch_k(kern, dim3(units, (rows.nodes + p.block_rows - 1) / p.block_rows, rows.batch), 128, 0, s, p);
+    YK_CUDA(cudaGetLastError());
 }
 
 // ---------------------------------------------------------------------------
@@ -140,32 +182,6 @@ __global__ void gdn_front_kernel(const ScanParams p) {
 // Redoing the front end inside this kernel (every CTA its head's q and k group and its own v
 // columns) to save the launch in between measured 9 us slower per layer: the front end is only
 // cheap when spread over its 576 CTAs.
-// Depth-first (pre-order) numbering of the rows of a tree whose parents precede their children; children in
-// row order. One thread, at most GDN_MAX_NODES rows.
-__device__ __noinline__ void depth_first_order(const int * par, int N, int * order) {
-    unsigned long long seen = 0ull;
-    int cnt = 0, at = -1;
-    while (cnt < N) {
-        int next = -1;
-        for (int c = at + 1; c < N; c++)
-            if (!((seen >> c) & 1ull) && par[c] == at) {
-                next = c;
-                break;
-            }
-        if (next >= 0) {
-            order[cnt++] = next;
-            seen |= 1ull << next;
-            at = next;
-        } else if (at >= 0) {
-            at = par[at];
-        } else {
-            // (unreachable for a valid parent array: rows without a path to the root go last, in row order)
-            for (int c = 0; c < N; c++)
-                if (!((seen >> c) & 1ull)) order[cnt++] = c;
-        }
-    }
-}
-
 // TREE: the rows of a sequence may branch (the host staged parent pointers); they are then walked depth first.
 template <int S, bool TREE>
 __global__ void __launch_bounds__(GDN_WARPS * 32) gdn_scan_kernel(const ScanParams p) {
@@ -197,7 +213,7 @@ __global__ void __launch_bounds__(GDN_WARPS * 32) gdn_scan_kernel(const ScanPara
     float * root_s = reinterpret_cast<float *>(par + N + (N & 1));
     __shared__ double ssq[GDN_MAX_NODES];
     __shared__ float scale_s[GDN_MAX_NODES];
-    __shared__ int order_s[TREE ? GDN_MAX_NODES : 1];
+    __shared__ int order_s[TREE ? GDN_MAX_NODES : 1];  // the rows depth first, worked out by the host when it staged the step
 
     // stored state: the longest fetch (HBM), issued first
     const float * s0 = a.state + ((int64_t)(seq_of(p.rows, seq) * a.rank + h) * S + rq * RPL) * S + col;
@@ -227,28 +243,27 @@ __global__ void __launch_bounds__(GDN_WARPS * 32) gdn_scan_kernel(const ScanPara
         par[node] = p.rows.parent[seq * N + node];
         bet[node] = a.beta[(int64_t)(seq * N + node) * a.rank + h];
         dec[node] = a.decay[(int64_t)(seq * N + node) * a.rank + h];
+        if (TREE) order_s[node] = p.rows.order[seq * N + node];
     }
     __syncthreads();
 
-    // the gate values the last phase needs (up to three per thread: a 9-row step needs 2.25) are fetched
-    // now, so that the end of the kernel does not wait for them
-    constexpr int ZPRE = 3;
-    float zpre[ZPRE];
-#pragma unroll
-    for (int k = 0; k < ZPRE; k++) {
+    // gate values the last phase needs, up to ZPT per thread. The first three (a 9-row step needs 2.25) are fetched now, so
+    // that the end of the kernel does not wait for them; a tree needs the registers
+    constexpr int ZPT = GDN_MAX_NODES * GDN_COLS / (GDN_WARPS * 32), ZPRE = TREE ? 0 : 3;
+    float z[ZPT];
+    auto fetch_z = [&](int k) {
         const int i = threadIdx.x + k * (GDN_WARPS * 32);
         const int node = i / GDN_COLS, c = i - node * GDN_COLS;
-        zpre[k] = i < N * GDN_COLS ? a.z[(int64_t)(seq * N + node) * a.ldz + h * S + cb * GDN_COLS + c] : 0.0f;
-    }
+        z[k] = i < N * GDN_COLS ? a.z[(int64_t)(seq * N + node) * a.ldz + h * S + cb * GDN_COLS + c] : 0.0f;
+    };
+#pragma unroll
+    for (int k = 0; k < ZPRE; k++) fetch_z(k);
 
     // The rows are walked in depth-first order: a row then follows its parent directly unless it is a later
     // sibling, so a branch is replayed from the stored state only when the walk backtracks. In row order
     // (breadth first, as draft trees are numbered) almost every row of a tree switched branches: the 16-node
-    // tree of the batched configuration cost 24 replayed updates on top of its 16, depth first it costs 2.
-    if constexpr (TREE) {
-        if (threadIdx.x == 0) depth_first_order(par, N, order_s);
-        __syncthreads();
-    }
+    // tree of the batched configuration cost 24 replayed updates on top of its 16, depth first it costs 2. (The order is
+    // an input: one thread of every CTA working it out took as long as the recurrence.)
 
     // ---- recurrence (recurrent.go:56-105) ----
     int cur = -1;  // node whose state st currently holds (-1: the stored state)
@@ -259,18 +274,19 @@ __global__ void __launch_bounds__(GDN_WARPS * 32) gdn_scan_kernel(const ScanPara
             // a sibling branch: rebuild the parent's state by replaying the log of its path, from the state after row 0
             // (every row of a step descends from row 0, the pending token; a tree keeps that state in shared memory)
             // or, failing that, from the stored one
-            int path[GDN_MAX_NODES], len = 0;
+            const int stop = TREE && pnode >= 0 ? 0 : -1;  // the row whose state the replay starts from
+            int len = 0;
+            for (int c = pnode; c > stop; c = par[c]) len++;
             if (TREE && pnode >= 0) {
 #pragma unroll
                 for (int i = 0; i < RPL / 2; i++) st[i] = reinterpret_cast<const float2 *>(root_s)[i * (GDN_WARPS * 32) + threadIdx.x];
-                for (int c = pnode; c > 0; c = par[c]) path[len++] = c;
             } else {
 #pragma unroll
                 for (int i = 0; i < RPL / 2; i++) st[i] = make_float2(s0[(int64_t)(2 * i) * S], s0[(int64_t)(2 * i + 1) * S]);
-                for (int c = pnode; c >= 0; c = par[c]) path[len++] = c;
             }
             for (int j = len - 1; j >= 0; j--) {
-                const int c = path[j];
+                int c = pnode;
+                for (int up = 0; up < j; up++) c = par[c];
                 const float dc = dec[c], dv = dd[c * GDN_COLS + cl];
                 const float2 dc2 = make_float2(dc, dc), dv2 = make_float2(dv, dv);
 #pragma unroll
@@ -327,6 +343,10 @@ __global__ void __launch_bounds__(GDN_WARPS * 32) gdn_scan_kernel(const ScanPara
 
     pdl_trigger_late();
     // ---- gated RMSNorm of the head (recurrent.go:39-50), sums of squares exchanged across the cluster ----
+    // (the other gate values are fetched now, into the registers the state has left: the exchanges hide their latency)
+#pragma unroll
+    for (int k = ZPRE; k < ZPT; k++) fetch_z(k);
+    const float norm_w = a.norm[cb * GDN_COLS + (threadIdx.x & (GDN_COLS - 1))];
     __syncthreads();
     for (int node = warp; node < N; node += GDN_WARPS) {
         const double v = (double)o_s[node * GDN_COLS + lane];
@@ -344,23 +364,13 @@ __global__ void __launch_bounds__(GDN_WARPS * 32) gdn_scan_kernel(const ScanPara
     }
     cluster_sync_all();  // scales visible to the CTA; no CTA leaves while another may still read its sums
 #pragma unroll
-    for (int k = 0; k < ZPRE; k++) {
+    for (int k = 0; k < ZPT; k++) {
         const int i = threadIdx.x + k * (GDN_WARPS * 32);
         if (i < N * GDN_COLS) {
-            const int node = i / GDN_COLS, c = i - node * GDN_COLS;
             float t = o_s[i];
-            t *= scale_s[node] * a.norm[cb * GDN_COLS + c];
-            o_s[i] = t * silu_ref(zpre[k]);
+            t *= scale_s[i / GDN_COLS] * norm_w;
+            o_s[i] = t * silu_ref(z[k]);
         }
-    }
-#pragma unroll 8
-    for (int i = threadIdx.x + ZPRE * (GDN_WARPS * 32); i < N * GDN_COLS; i += blockDim.x) {
-        const int node = i / GDN_COLS, c = i - node * GDN_COLS;
-        const int64_t r = seq * N + node;
-        const float zv = a.z[r * a.ldz + h * S + cb * GDN_COLS + c];
-        float t = o_s[i];
-        t *= scale_s[node] * a.norm[cb * GDN_COLS + c];
-        o_s[i] = t * silu_ref(zv);
     }
     __syncthreads();
     for (int gi = threadIdx.x; gi < N * (GDN_COLS >> 4); gi += blockDim.x) {
@@ -379,14 +389,11 @@ __global__ void __launch_bounds__(GDN_WARPS * 32) gdn_scan_kernel(const ScanPara
 
 int launch_gdn_scan(cudaStream_t s, const GdnArgs & a, const RowMeta & rows) {
     YK_REQUIRE(rows.nodes <= GDN_MAX_NODES, YUUKA_ERR_UNSUPPORTED, "gdn: at most %d rows per sequence", GDN_MAX_NODES);
-    YK_REQUIRE(a.kernel >= 2 && a.kernel <= 8, YUUKA_ERR_UNSUPPORTED, "gdn: conv kernel %d is outside 2..8", a.kernel);
-    YK_REQUIRE(a.S == 64 || a.S == 128, YUUKA_ERR_UNSUPPORTED, "gdn: state size %d is not 64 or 128", a.S);
-    ScanParams p{a, rows, 0};
+    YK_REQUIRE(rows.chains || rows.order, YUUKA_ERR_INTERNAL, "gdn: a tree step needs its rows depth first");
+    launch_gdn_front(s, a, rows, rows.chains != 0);
+    ScanParams p{a, rows, 0, 0};
     const int N = rows.nodes;
     dim3 grid(a.S / GDN_COLS, a.rank, rows.batch);
-    dim3 fgrid(2 * a.groups + a.rank, N, rows.batch);
-    launch_k(gdn_front_kernel, fgrid, a.S, 0, s, p);
-    YK_CUDA(cudaGetLastError());
     const size_t smem = sizeof(float) * ((size_t)2 * N * (a.S + 16) + 3 * N * GDN_COLS + 3 * N + (rows.chains ? 0 : (size_t)(a.S / 4) * GDN_WARPS * 32 + 1));
     auto launch = [&](auto kern) {
         YK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
@@ -746,16 +753,11 @@ static size_t gdn_chunk_smem(int N, int S) {
 // The front end alone for one chain of any length (a whole prompt pass of one sequence): conv taps come from the
 // preceding rows of the pass and, for its first kernel - 1 rows, from the stored history.
 void launch_gdn_front_chain(cudaStream_t s, const GdnArgs & a, int seq_slot, int n_rows) {
-    YK_REQUIRE(a.kernel >= 2 && a.kernel <= 8, YUUKA_ERR_UNSUPPORTED, "gdn: conv kernel %d is outside 2..8", a.kernel);
-    YK_REQUIRE(a.S == 64 || a.S == 128, YUUKA_ERR_UNSUPPORTED, "gdn: state size %d is not 64 or 128", a.S);
     (void)seq_slot;
     RowMeta rows{};
     rows.batch = 1;
     rows.nodes = n_rows;
-    ScanParams p{a, rows, 1};
-    dim3 fgrid(2 * a.groups + a.rank, n_rows, 1);
-    launch_k(gdn_front_kernel, fgrid, a.S, 0, s, p);
-    YK_CUDA(cudaGetLastError());
+    launch_gdn_front(s, a, rows, true);
 }
 
 // Chunkwise scan of a chain of at most 64 rows that are all committed, after the front end has run for them; the
@@ -763,7 +765,7 @@ void launch_gdn_front_chain(cudaStream_t s, const GdnArgs & a, int seq_slot, int
 void launch_gdn_chunk(cudaStream_t s, const GdnArgs & a, const RowMeta & rows) {
     YK_REQUIRE(rows.nodes <= GDN_MAX_NODES, YUUKA_ERR_UNSUPPORTED, "gdn: at most %d rows per chunk", GDN_MAX_NODES);
     YK_REQUIRE(a.S == 64 || a.S == 128, YUUKA_ERR_UNSUPPORTED, "gdn: state size %d is not 64 or 128", a.S);
-    ScanParams p{a, rows, 0};
+    ScanParams p{a, rows, 0, 0};
     const int N = rows.nodes;
     dim3 grid(a.S / GDN_COLS, a.rank, rows.batch);
     const size_t smem = gdn_chunk_smem(N, a.S);

@@ -21,6 +21,9 @@ struct RowMeta {
     // set by the host when it staged no parent pointers: every sequence of the step is a chain (row i follows
     // row i - 1), which lets the delta-net scan walk the rows in order without looking for branches
     int chains = 0;
+    // [rows] the nodes of each sequence depth first (parents before children, children in row order), for steps whose
+    // rows may branch (chains == 0); null otherwise
+    const int32_t * order = nullptr;
 };
 #ifdef __CUDACC__
 __device__ __forceinline__ int seq_of(const RowMeta & rows, int slot) { return rows.seq_map ? rows.seq_map[slot] : slot; }
