@@ -105,3 +105,40 @@ def test_strong_decay_stays_finite():
     assert rel_diff(snap_r, snap) <= 2e-3
     gm.close()
     dev.close()
+
+
+@pytest.mark.parametrize("groups,rank,kernel,n_prompt", [
+    (4, 4, 4, 65), (4, 4, 4, 79), (4, 4, 4, 81), (4, 4, 4, 127), (4, 4, 4, 129),  # last chunks around 16-row tiles
+    (1, 8, 8, 144), (2, 12, 2, 97),   # more value heads per key head than are worked on together; the longest and shortest conv
+])
+def test_chunks_at_the_edges_of_their_tiles(groups, rank, kernel, n_prompt):
+    cfg = synth.tiny_config()
+    cfg.update(group_count=groups, time_step_rank=rank, inner_size=rank * 64, conv_kernel=kernel)
+    dev = cuda.Device(0)
+    gm = cuda.Model(dev, cfg, synth.make_model(cfg, "q4_k_m", seed=45, unit_norms=False))
+    prompt = synth.uniform_i32(n_prompt, 0, cfg["vocab"], n_prompt)
+    got_c, snap_c, _ = run_prompt(gm, prompt, 256, True)
+    got_r, snap_r, _ = run_prompt(gm, prompt, 256, False)
+    assert rel_diff(snap_r, snap_c) <= 2e-3, rel_diff(snap_r, snap_c)
+    assert float(np.max(np.abs(got_c - got_r))) <= 5e-3
+    gm.close()
+    dev.close()
+
+
+@pytest.mark.parametrize("hidden,ffn,n_prompt", [(3328, 3328, 48), (256, 3072, 49)])
+def test_wide_pass_whose_rows_exceed_what_a_thread_keeps(hidden, ffn, n_prompt):
+    """Row-wise kernels of wide passes: 3072 columns are one CTA's registers in the norm, one CTA's share of a SwiGLU row."""
+    cfg = synth.tiny_config()
+    cfg.update(hidden=hidden, ffn=ffn, vocab=512)
+    tensors = synth.make_model(cfg, "q4_k_m", seed=46, unit_norms=False)
+    dev = cuda.Device(0)
+    gm = cuda.Model(dev, cfg, tensors)
+    prompt = synth.uniform_i32(n_prompt, 0, cfg["vocab"], 3)
+    st = yo.State(yo.Model(cfg, tensors), 64, yo.KV_F32)
+    want = st.forward(prompt)
+    st.close()
+    got, _, _ = run_prompt(gm, prompt, 64, True)
+    err = float(np.max(np.abs(got - want)))
+    assert err <= 2e-2 * max(1.0, float(np.max(np.abs(want)))) and cosine(got, want) >= 0.9999, (err, cosine(got, want))
+    gm.close()
+    dev.close()

@@ -572,6 +572,10 @@ __global__ void __launch_bounds__(HD / 4 < 32 ? 32 : HD / 4) attention_merge_ker
     o.y = acc.y * inv * sigmoid_ref(gate.y);
     o.z = acc.z * inv * sigmoid_ref(gate.z);
     o.w = acc.w * inv * sigmoid_ref(gate.w);
+    if (prep.hi_only()) {
+        if (has_dims) xprep_store_hi4(prep.xh + (int64_t)r * heads * HD + head * HD + tid * 4, o.x, o.y, o.z, o.w);
+        return;
+    }
     if (has_dims) *reinterpret_cast<float4 *>(out + (int64_t)r * ldo + head * HD + tid * 4) = o;
     if (prep.xh) {
         // gather the 16-dim group in its first lane (four neighbouring threads hold it)

@@ -568,6 +568,9 @@ struct yuuka_session {
     int chain_rows = 0;  // rows per prompt chunk (prefill_logits / forward)
     // L2 prefetch of the next GEMM's weights: matrices in the order a step streams them
     bool prefetch_next = true;
+    bool all_tiled = false;          // every matrix of the layers and the head is in the tiled layout
+    bool hi_step = false;            // this step's matrices read the hi halves of their inputs alone
+    uint8_t * gdn_chunk_scratch = nullptr;  // row-by-row matrices of a prompt pass
     bool gdn_chunked = true;  // prompt sub-chunks through the chunkwise delta-net scan (YUUKA_CUDA_NO_GDN_CHUNK=1: row by row)
     uint64_t prefetch_bytes = 16ull << 20;  // measured: 16 MB ahead 3.09 ms/step, none 3.12, 48 MB 3.13
     std::vector<std::pair<const uint8_t *, uint64_t>> gemm_order;
@@ -695,6 +698,24 @@ void gemm(yuuka_session * s, const Tensor & w, const float * x, int ldx, XPrepOu
     s->launches += launch_gemm_quant(s->model->dev, s->stream.s, a);
 }
 
+// The form a step's producers leave an input in: the hi halves alone where the tensor-memory route is all that reads it.
+XPrepOut step_prep(const yuuka_session * s, XPrepOut p) {
+    if (s->hi_step) {
+        p.xl = nullptr;
+        p.xs16 = nullptr;
+    }
+    return p;
+}
+// The normalised residual rows: the router and the experts of a mixture read more than that.
+XPrepOut step_prep_xn(const yuuka_session * s) { return s->model->cfg.expert_count > 0 ? s->prep_xn : step_prep(s, s->prep_xn); }
+// the prepared rows from row r on
+XPrepOut prep_rows(XPrepOut p, int64_t r, int width) {
+    if (p.xh) p.xh += r * width;
+    if (p.xl) p.xl += r * width;
+    if (p.xs16) p.xs16 += r * (width / 16);
+    return p;
+}
+
 // x += W * in, then xn = rmsnorm(x) * norm_w (skipped when norm_w is null). With up to 32 rows the norm is
 // folded into this GEMM's epilogue and the next GEMM's; otherwise it runs as its own kernel.
 void gemm_residual_norm(yuuka_session * s, const Tensor & w, const float * in, int ld_in, XPrepOut prep_in, int rows,
@@ -711,9 +732,31 @@ void gemm_residual_norm(yuuka_session * s, const Tensor & w, const float * in, i
     gemm(s, w, in, ld_in, prep_in, s->x, H, rows, YUUKA_GEMM_ACCUMULATE);
     if (norm_w) {
         mark(s, YUUKA_OP_RMSNORM);
-        launch_rmsnorm(s->stream.s, s->xn, H, s->x, H, norm_w, H, rows, c.rms_eps, s->prep_xn);
+        launch_rmsnorm(s->stream.s, s->xn, H, s->x, H, norm_w, H, rows, c.rms_eps, step_prep_xn(s));
         s->launches++;
     }
+}
+
+bool matrices_tiled(const yuuka_model & m) {
+    auto all = [](std::initializer_list<const Tensor *> ts) {
+        for (const Tensor * t : ts)
+            if (!t->tiled) return false;
+        return true;
+    };
+    for (int i = 0; i < m.cfg.block_count; i++) {
+        const LayerW & L = m.layers[i];
+        if (m.recurrent(i)) {
+            if (!(L.proj.present() ? all({&L.proj}) : all({&L.qkv, &L.gate, &L.beta, &L.alpha})) || !L.out.tiled) return false;
+        } else {
+            if (!(L.qk.present() ? all({&L.qk}) && (L.qk_has_v || L.v.tiled) : all({&L.q, &L.k, &L.v})) || !L.o.tiled) return false;
+        }
+        if (m.cfg.expert_count > 0) {
+            if (!(L.sh_gate_up.present() ? all({&L.sh_gate_up}) : all({&L.sh_gate, &L.sh_up})) || !L.sh_down.tiled) return false;
+        } else if (!(L.gate_up.present() ? all({&L.gate_up}) : all({&L.ffn_gate, &L.ffn_up})) || !L.ffn_down.tiled) {
+            return false;
+        }
+    }
+    return m.output.tiled;
 }
 
 void reserve_gemm(yuuka_session * s, const Tensor & w, int rows) {
@@ -771,6 +814,8 @@ void run_step(yuuka_session * s, int seq0, int batch, int nodes, uint32_t mode, 
     // with up to 32 rows every norm after the first is folded into the GEMM that finishes the residual rows
     // and the GEMM that reads them
     s->fold_step = s->fold_norm && R <= 32;
+    s->hi_step = s->all_tiled && gemm_tiled_wide(R, (s->cfg.flags & YUUKA_SESSION_EXACT_WIDE) != 0,
+                                                 (s->cfg.flags & YUUKA_SESSION_WIDE_FROM_33) != 0);
     s->norm_point = 0;
     s->xn_raw = false;
     if (s->fold_step) YK_CUDA(cudaMemsetAsync(s->norm_sumsq, 0, sizeof(unsigned long long) * 32 * (size_t)(2 * c.block_count + 2), st));
@@ -791,7 +836,7 @@ void run_step(yuuka_session * s, int seq0, int batch, int nodes, uint32_t mode, 
             s->launches++;
         }
         mark(s, YUUKA_OP_RMSNORM);
-        launch_rmsnorm(st, s->xn, H, s->x, H, m->layers[0].attn_norm, H, R, c.rms_eps, s->prep_xn, sumsq0);
+        launch_rmsnorm(st, s->xn, H, s->x, H, m->layers[0].attn_norm, H, R, c.rms_eps, step_prep_xn(s), sumsq0);
         s->launches++;
     }
     for (int i = 0; i < c.block_count; i++) {
@@ -818,7 +863,7 @@ void run_step(yuuka_session * s, int seq0, int batch, int nodes, uint32_t mode, 
             g.conv_state = LS.conv_state + (int64_t)seq0 * conv_dim * K1;
             g.state = LS.state + (int64_t)seq0 * rank * S * S;
             g.out = s->gdn_out;
-            g.prep = s->prep_gdn;
+            g.prep = step_prep(s, s->prep_gdn);
             g.z = LS.proj + conv_dim;
             g.ldz = np;
             g.norm = L.ssm_norm;
@@ -841,22 +886,15 @@ void run_step(yuuka_session * s, int seq0, int batch, int nodes, uint32_t mode, 
                 // Every row of a prompt pass is committed, so by default the front end runs once for the whole pass,
                 // the chunkwise form of the recurrence writes the state itself, and the conv history moves once.
                 const int key_dim = c.group_count * S;
-                const bool chunked = s->gdn_chunked;
-                if (chunked) {
-                    launch_gdn_front_chain(st, g, seq0, nodes);
-                    s->launches++;
-                }
-                for (int k = 0; k < n_sub; k++) {
+                const bool chunked = s->gdn_chunked && s->gdn_chunk_scratch;
+                if (chunked) s->launches += launch_gdn_chunks(st, g, nodes, s->gdn_chunk_scratch);
+                for (int k = 0; k < n_sub && !chunked; k++) {
                     const int64_t r0 = (int64_t)k * sub;
                     GdnArgs gk = g;
                     gk.proj = g.proj + r0 * np;
                     gk.z = g.z + r0 * np;
                     gk.out = g.out + r0 * inner;
-                    if (g.prep.xh) {
-                        gk.prep.xh = g.prep.xh + r0 * inner;
-                        gk.prep.xl = g.prep.xl + r0 * inner;
-                        gk.prep.xs16 = g.prep.xs16 + r0 * (inner / 16);
-                    }
+                    gk.prep = prep_rows(g.prep, r0, inner);
                     gk.qn = g.qn + r0 * key_dim;
                     gk.vconv = g.vconv + r0 * inner;
                     gk.beta = g.beta + r0 * rank;
@@ -864,11 +902,6 @@ void run_step(yuuka_session * s, int seq0, int batch, int nodes, uint32_t mode, 
                     gk.dlog = g.dlog + r0 * inner;
                     gk.decay = g.decay + r0 * rank;
                     const RowMeta rk = sub_rows(k);
-                    if (chunked) {
-                        launch_gdn_chunk(st, gk, rk);
-                        s->launches++;
-                        continue;
-                    }
                     s->launches += launch_gdn_scan(st, gk, rk);
                     AcceptOut ak{s->d_acc_sub + k, s->acc.path, s->acc.emitted};
                     launch_gdn_commit(st, s->d_gdn_commit + gdn_index, 1, c.group_count, rank, S, c.conv_kernel, conv_dim, seq0, rk,
@@ -934,7 +967,7 @@ void run_step(yuuka_session * s, int seq0, int batch, int nodes, uint32_t mode, 
             mark(s, YUUKA_OP_ATTENTION);
             if (sub == 0) {
                 s->launches += launch_attention(st, s->attn_out, o_dim, qb, nq, c.heads, c.kv_heads, c.head_dim, rows, pool,
-                                                max_total, sc, s->prep_attn);
+                                                max_total, sc, step_prep(s, s->prep_attn));
             } else {
                 // a sub-chunk's K/V rows are in the pool before the next sub-chunk's queries look for them
                 const int half = c.rope_dim / 2;
@@ -943,12 +976,7 @@ void run_step(yuuka_session * s, int seq0, int batch, int nodes, uint32_t mode, 
                     const RowMeta rk = sub_rows(k);
                     launch_attn_prep(st, qb + r0 * nq, nq, kb + r0 * nq, nq, vb + r0 * nq, nq, L.q_norm, L.k_norm, c.heads,
                                      c.kv_heads, c.head_dim, c.rope_dim, s->rope_cs + r0 * half, c.rms_eps, rk, pool);
-                    XPrepOut pk = s->prep_attn;
-                    if (pk.xh) {
-                        pk.xh += r0 * o_dim;
-                        pk.xl += r0 * o_dim;
-                        pk.xs16 += r0 * (o_dim / 16);
-                    }
+                    const XPrepOut pk = prep_rows(step_prep(s, s->prep_attn), r0, o_dim);
                     s->launches += 1 + launch_attention(st, s->attn_out + r0 * o_dim, o_dim, qb + r0 * nq, nq, c.heads, c.kv_heads,
                                                         c.head_dim, rk, pool, max_total, sc, pk);
                 }
@@ -1001,7 +1029,7 @@ void run_step(yuuka_session * s, int seq0, int batch, int nodes, uint32_t mode, 
                 gemm(s, L.sh_up, s->xn, H, s->prep_xn, s->sh_gu + SF, 2 * SF, R, 0);
             }
             mark(s, YUUKA_OP_SILU_MUL);
-            launch_silu_mul(st, s->sh_act, SF, s->sh_gu, s->sh_gu + SF, 2 * SF, SF, R, s->prep_sh_act);
+            launch_silu_mul(st, s->sh_act, SF, s->sh_gu, s->sh_gu + SF, 2 * SF, SF, R, step_prep(s, s->prep_sh_act));
             s->launches++;
             gemm(s, L.sh_down, s->sh_act, SF, s->prep_sh_act, s->sh_y, H, R, 0);
             mark(s, YUUKA_OP_MOE_COMBINE);
@@ -1027,7 +1055,7 @@ void run_step(yuuka_session * s, int seq0, int batch, int nodes, uint32_t mode, 
                 gemm(s, L.ffn_up, s->xn, H, s->prep_xn, s->gate_up + F, 2 * F, R, 0);
             }
             mark(s, YUUKA_OP_SILU_MUL);
-            launch_silu_mul(st, s->act, F, s->gate_up, s->gate_up + (paired ? 16 : F), 2 * F, F, R, s->prep_act, paired ? 32 : 16);
+            launch_silu_mul(st, s->act, F, s->gate_up, s->gate_up + (paired ? 16 : F), 2 * F, F, R, step_prep(s, s->prep_act), paired ? 32 : 16);
             s->launches++;
         }
         gemm_residual_norm(s, L.ffn_down, s->act, F, s->prep_act, R, next_norm);
@@ -1424,6 +1452,7 @@ yuuka_status yuuka_session_create(yuuka_model * model, const yuuka_session_confi
                 s->h_rows = (uint8_t *)hp;
                 s->h_results = reinterpret_cast<int32_t *>(s->h_rows + rows_bytes);
             }
+            s->all_tiled = matrices_tiled(*model);
             const int H = c.hidden;
             s->x = dalloc<float>((size_t)R * H, s->owned);
             s->xn = dalloc<float>((size_t)R * H, s->owned);
@@ -1433,6 +1462,8 @@ yuuka_status yuuka_session_create(yuuka_model * model, const yuuka_session_confi
             s->gdn_qn = dalloc<float>((size_t)R * c.group_count * S, s->owned);
             s->gdn_vconv = dalloc<float>((size_t)R * c.inner_size, s->owned);
             s->gdn_beta = dalloc<float>((size_t)R * rank, s->owned);
+            if (s->gdn_chunked && s->chain_rows > CHAIN_SUB)
+                s->gdn_chunk_scratch = dalloc<uint8_t>(gdn_chunk_scratch_bytes(s->chain_rows, rank), s->owned);
             s->gate_up = dalloc<float>((size_t)R * 2 * c.ffn, s->owned);
             if (c.rope_dim > 0) s->rope_cs = dalloc<float2>((size_t)R * (c.rope_dim / 2), s->owned);
             s->act = dalloc<float>((size_t)R * c.ffn, s->owned);

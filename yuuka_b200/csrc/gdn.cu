@@ -71,18 +71,20 @@ struct ScanParams {
 // meets at a barrier, and a warp goes on to its next row with its weights in registers. It is latency that bounds this
 // kernel: one CTA per (row, unit) spent 39 us on 512 rows of 8192 channels (15 waves of CTAs, each a chain of waits)
 // where its 40 MB take 6.
-// KMAX: taps held in registers (4, or 8 for the longer kernels).
-template <int S, int KMAX>
+// KMAX: taps held in registers (4, or 8 for the longer kernels). SPLIT: a CTA of S / 32 warps per row, 32 channels each
+// (few rows: the chain of a warp is shorter. With a warp per row a 9-row step of 24 such layers took 16 us more).
+template <int S, int KMAX, bool SPLIT>
 __global__ void __launch_bounds__(128) gdn_front_kernel(const ScanParams p) {
     // (releasing the scan from here, so that it could fetch its state while this kernel runs, measured 7 us
     // slower per layer: a dependent grid that starts early and really has to block in griddepcontrol.wait
     // is woken late; only triggers placed at the end of a kernel have paid)
     const GdnArgs & a = p.a;
-    constexpr int G = S / 32;
+    constexpr int G = SPLIT ? 1 : S / 32;
     const int N = p.rows.nodes, K = a.kernel, K1 = K - 1;
-    const int u = blockIdx.x, seq = blockIdx.z, lane = threadIdx.x & 31;
+    const int u = blockIdx.x, seq = blockIdx.z, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int key_dim = a.groups * S, conv_dim = 2 * key_dim + a.rank * S;
-    const int c0 = u * S + lane;  // q units, then k units, then v units: exactly the conv row order
+    const int e0 = (SPLIT ? warp * 32 : 0) + lane;
+    const int c0 = u * S + e0;  // q units, then k units, then v units: exactly the conv row order
     float w[G][KMAX];
 #pragma unroll
     for (int i = 0; i < G; i++)
@@ -97,7 +99,7 @@ __global__ void __launch_bounds__(128) gdn_front_kernel(const ScanParams p) {
     const float * proj = a.proj + (int64_t)seq * N * a.ldp;
     const float * hist = a.conv_state + ((int64_t)seq_of(p.rows, seq) * conv_dim + c0) * K1;
     const int first = blockIdx.y * p.block_rows, last = min(N, first + p.block_rows);
-    for (int node = first + (int)(threadIdx.x >> 5); node < last; node += (int)(blockDim.x >> 5)) {
+    for (int node = first + (SPLIT ? 0 : warp); node < last; node += (SPLIT ? 1 : 4)) {
         const int r = seq * N + node;
         float taps[G][KMAX];
         int cur = node, hidx = K1 - 1;
@@ -131,20 +133,28 @@ __global__ void __launch_bounds__(128) gdn_front_kernel(const ScanParams p) {
 #pragma unroll
                 for (int i = 0; i < G; i++) sq[i] += __shfl_xor_sync(0xffffffffu, sq[i], o);
             double tot = 0;
+            if constexpr (SPLIT) {
+                __shared__ double red[S / 32];  // (one row per CTA)
+                if (lane == 0) red[warp] = sq[0];
+                __syncthreads();
 #pragma unroll
-            for (int i = 0; i < G; i++) tot += sq[i];
+                for (int i = 0; i < S / 32; i++) tot += red[i];
+            } else {
+#pragma unroll
+                for (int i = 0; i < G; i++) tot += sq[i];
+            }
             const float scale = (float)(1.0 / sqrt(tot + (double)a.eps));
             const bool is_q = u < a.groups;
             const float mul = is_q ? scale * (float)(1.0 / sqrt((double)S)) : scale;
-            float * dst = (is_q ? a.qn + u * S : a.khat + (u - a.groups) * S) + (int64_t)r * key_dim + lane;
+            float * dst = (is_q ? a.qn + u * S : a.khat + (u - a.groups) * S) + (int64_t)r * key_dim + e0;
 #pragma unroll
             for (int i = 0; i < G; i++) dst[32 * i] = v[i] * mul;
         } else {
             const int h = u - 2 * a.groups;
-            float * dst = a.vconv + (int64_t)r * (a.rank * S) + h * S + lane;
+            float * dst = a.vconv + (int64_t)r * (a.rank * S) + h * S + e0;
 #pragma unroll
             for (int i = 0; i < G; i++) dst[32 * i] = v[i];
-            if (lane == 0) {
+            if (e0 == 0) {
                 const float * row = a.proj + (int64_t)r * a.ldp;
                 a.beta[(int64_t)r * a.rank + h] = sigmoid_ref(row[conv_dim + a.rank * S + h]);
                 a.decay[(int64_t)r * a.rank + h] = expf(softplus_ref(row[conv_dim + a.rank * S + a.rank + h] + a.dt[h]) * a.a[h]);
@@ -153,21 +163,32 @@ __global__ void __launch_bounds__(128) gdn_front_kernel(const ScanParams p) {
     }
 }
 
-// Rows of a unit per CTA of four warps: one row per warp until the launch has a resident wave of warps (24 per SM), then
-// as many as keep it at one wave.
+// One row per CTA while that is a resident wave of warps or less (24 per SM); beyond that one row per warp, and then as
+// many rows per warp as keep the launch at one wave.
+template <int S>
+static void launch_gdn_front_s(cudaStream_t s, ScanParams & p) {
+    const GdnArgs & a = p.a;
+    const int units = 2 * a.groups + a.rank, N = p.rows.nodes;
+    constexpr int64_t WAVE = 148 * 24;
+    const int64_t unit_rows = (int64_t)units * N * p.rows.batch;
+    if (unit_rows * (S / 32) <= WAVE) {
+        p.block_rows = 1;
+        launch_k(a.kernel <= 4 ? gdn_front_kernel<S, 4, true> : gdn_front_kernel<S, 8, true>, dim3(units, N, p.rows.batch), S, 0, s, p);
+    } else {
+        const int64_t per_warp = (unit_rows + WAVE - 1) / WAVE;
+        const int blocks = (int)((N + 4 * per_warp - 1) / (4 * per_warp));
+        p.block_rows = (N + blocks - 1) / blocks;
+        launch_k(a.kernel <= 4 ? gdn_front_kernel<S, 4, false> : gdn_front_kernel<S, 8, false>,
+                 dim3(units, (N + p.block_rows - 1) / p.block_rows, p.rows.batch), 128, 0, s, p);
+    }
+    YK_CUDA(cudaGetLastError());
+}
 static void launch_gdn_front(cudaStream_t s, const GdnArgs & a, const RowMeta & rows, bool chain) {
     YK_REQUIRE(a.kernel >= 2 && a.kernel <= 8, YUUKA_ERR_UNSUPPORTED, "gdn: conv kernel %d is outside 2..8", a.kernel);
     YK_REQUIRE(a.S == 64 || a.S == 128, YUUKA_ERR_UNSUPPORTED, "gdn: state size %d is not 64 or 128", a.S);
     ScanParams p{a, rows, chain ? 1 : 0, 0};
-    const int units = 2 * a.groups + a.rank;
-    constexpr int64_t WAVE = 148 * 24;
-    const int64_t per_warp = ((int64_t)units * rows.nodes * rows.batch + WAVE - 1) / WAVE;
-    const int blocks = (int)((rows.nodes + 4 * per_warp - 1) / (4 * per_warp));
-    p.block_rows = (rows.nodes + blocks - 1) / blocks;
-    auto kern = a.S == 128 ? (a.kernel <= 4 ? gdn_front_kernel<128, 4> : gdn_front_kernel<128, 8>)
-                           : (a.kernel <= 4 ? gdn_front_kernel<64, 4> : gdn_front_kernel<64, 8>);
-    launch_k(kern, dim3(units, (rows.nodes + p.block_rows - 1) / p.block_rows, rows.batch), 128, 0, s, p);
-    YK_CUDA(cudaGetLastError());
+    if (a.S == 128) launch_gdn_front_s<128>(s, p);
+    else launch_gdn_front_s<64>(s, p);
 }
 
 // ---------------------------------------------------------------------------
@@ -263,7 +284,8 @@ __global__ void __launch_bounds__(GDN_WARPS * 32) gdn_scan_kernel(const ScanPara
     // sibling, so a branch is replayed from the stored state only when the walk backtracks. In row order
     // (breadth first, as draft trees are numbered) almost every row of a tree switched branches: the 16-node
     // tree of the batched configuration cost 24 replayed updates on top of its 16, depth first it costs 2. (The order is
-    // an input: one thread of every CTA working it out took as long as the recurrence.)
+    // an input: one thread of every CTA working it out, its path kept in local memory, cost 56 us of a layer's 239 at
+    // 32 sequences x 17 rows.)
 
     // ---- recurrence (recurrent.go:56-105) ----
     int cur = -1;  // node whose state st currently holds (-1: the stored state)
@@ -347,6 +369,7 @@ __global__ void __launch_bounds__(GDN_WARPS * 32) gdn_scan_kernel(const ScanPara
 #pragma unroll
     for (int k = ZPRE; k < ZPT; k++) fetch_z(k);
     const float norm_w = a.norm[cb * GDN_COLS + (threadIdx.x & (GDN_COLS - 1))];
+    const bool hi_only = a.prep.hi_only();  // the out projection of a wide step reads nothing else
     __syncthreads();
     for (int node = warp; node < N; node += GDN_WARPS) {
         const double v = (double)o_s[node * GDN_COLS + lane];
@@ -369,9 +392,12 @@ __global__ void __launch_bounds__(GDN_WARPS * 32) gdn_scan_kernel(const ScanPara
         if (i < N * GDN_COLS) {
             float t = o_s[i];
             t *= scale_s[i / GDN_COLS] * norm_w;
-            o_s[i] = t * silu_ref(z[k]);
+            t *= silu_ref(z[k]);
+            if (hi_only) a.prep.xh[(int64_t)(seq * N + i / GDN_COLS) * inner + h * S + cb * GDN_COLS + (i & (GDN_COLS - 1))] = __float2half_rn(t);
+            else o_s[i] = t;
         }
     }
+    if (hi_only) return;
     __syncthreads();
     for (int gi = threadIdx.x; gi < N * (GDN_COLS >> 4); gi += blockDim.x) {
         const int node = gi / (GDN_COLS >> 4), part = gi - node * (GDN_COLS >> 4);
@@ -419,10 +445,13 @@ int launch_gdn_scan(cudaStream_t s, const GdnArgs & a, const RowMeta & rows) {
 //   (I + B) D = diag(beta) (V - diag(gam) K S_0),   B[r][s] = beta_r exp(g_r - g_s) (k_r . k_s)  for s < r
 //   o_r = gam_r q_r S_0 + sum_{s <= r} exp(g_r - g_s) (q_r . k_s) d_s
 //   S_C = gam_C S_0 + sum_s exp(g_C - g_s) k_s d_s^T
-// grid (S/32 column blocks, rank, batch), the column blocks of a head one cluster (gated norm as in the scan
-// kernel); a CTA owns 32 columns of the state, of V, D and the outputs, and computes the row-by-row matrices
-// (K K^T, Q K^T: they do not depend on the column) itself. The state is rewritten in place: no delta log, no
-// separate state commit.
+// Three launches take a whole pass. (1) The matrices B and A and the inverses of B's diagonal blocks depend on neither the
+// state nor the column: one CTA per (chunk, key head) makes them for all chunks at once, K K^T and Q K^T shared by the
+// value heads of a key head. (2) One CTA per (head, 32 columns) walks the chunks with its columns of the state in shared
+// memory: K S_0 and Q S_0, the substitution, outputs and state update; the next chunk's q and k arrive meanwhile.
+// (3) The gated norm of all rows, where a head's columns meet again.
+// (One launch per chunk with all of this inside took 22.5 us per 64 rows of 32 heads: a chain of loads, barriers and
+// cluster exchanges, and every column block made B and A again. 512 rows: 180 us then; now 12 + 68 + 9.)
 //
 // Every product is a tensor-core product, mma.sync m16n8k8 on tf32 operands, with both operands split into two
 // tf32 parts (x = hi + lo, three products: lo hi, hi lo, hi hi), which keeps fp32-level accuracy: the two forms
@@ -470,313 +499,388 @@ __device__ __forceinline__ void warp_mma_3x(float (&acc)[NT][4], int ksteps, FA 
     }
 }
 
+__device__ __forceinline__ void cp_async16(void * dst, const void * src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N> __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+
+// What launch (1) leaves for a (chunk, head), pitches chosen for the fragment loads of launch (2) (banks 4 g + t)
+constexpr int GC_ROWS = GDN_MAX_NODES;
+constexpr int GC_NP = GC_ROWS + 4, GC_TP = 20;
+struct ChunkPair {
+    float B[GC_ROWS * GC_NP];  // beta_r w_rs (k_r . k_s), 16 x 16 blocks below the diagonal ones
+    float A[GC_ROWS * GC_NP];  // w_rs (q_r . k_s), blocks up to the diagonal ones
+    float T[GC_ROWS * GC_TP];  // inverses of the 16 x 16 diagonal blocks of I + B
+    float beta[GC_ROWS], gam[GC_ROWS], tail[GC_ROWS];  // beta_r, exp(g_r), exp(g_C - g_r)
+};
+static_assert(sizeof(ChunkPair) % 16 == 0, "copied in 16-byte pieces");
+
+struct ChunkParams {
+    GdnArgs a;
+    int rows;          // of the pass
+    ChunkPair * pairs; // [chunks][rank]
+};
+
+// q and k rows [r0, r0 + n) of one key head -> shared memory, zero rows up to `padded`
 template <int S>
-__global__ void __launch_bounds__(GC_THREADS, 1) gdn_chunk_kernel(const ScanParams p) {
+__device__ __forceinline__ void chunk_fetch_rows(float * dst, const float * src, int key_dim, int n, int padded) {
+    constexpr int KP = S + 4, SQ = S / 4;
+    for (int i = threadIdx.x; i < padded * SQ; i += GC_THREADS) {
+        const int node = i / SQ, e4 = i - node * SQ;
+        if (node < n) cp_async16(dst + node * KP + e4 * 4, src + (int64_t)node * key_dim + e4 * 4);
+        else *reinterpret_cast<float4 *>(dst + node * KP + e4 * 4) = make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+}
+
+// (1) grid (chunks, groups)
+constexpr int GC_HEADS = 4;  // value heads of a key head worked on together
+template <int S>
+__global__ void __launch_bounds__(GC_THREADS, 1) gdn_chunk_pairs_kernel(const ChunkParams p) {
     pdl_entry();
     const GdnArgs & a = p.a;
-    const int cb = blockIdx.x, h = blockIdx.y, seq = blockIdx.z;
-    const int N = p.rows.nodes;
-    const int kh = h % a.groups;
-    const int key_dim = a.groups * S, inner = a.rank * S;
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int g = lane >> 2, t = lane & 3;
+    const int kh = blockIdx.y, r0 = blockIdx.x * GC_ROWS, N = min(GC_ROWS, p.rows - r0);
+    const int key_dim = a.groups * S, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
     constexpr int KP = S + 4;            // pitch of a q / k row: the eight rows an A fragment reads fall on banks 4 g + t
-    constexpr int CP = GC_CP;
     const int MT = (N + 15) >> 4;        // 16-row tiles
     const int NR = MT * 16;              // rows with padding (zero rows)
-    const int NP = NR + 4;               // pitch of the row-by-row matrices (banks 4 g + t again)
-
     extern __shared__ __align__(16) float sm[];
-    float * qn = sm;                     // [NR][KP]
-    float * kn = qn + NR * KP;           // [NR][KP]
-    float * s0 = kn + NR * KP;           // [S][CP]  this CTA's columns of the stored state
-    float * vv = s0 + S * CP;            // [NR][CP] v, later exp(g_C - g_s) d_s
-    float * ks = vv + NR * CP;           // [NR][CP] K S_0, then the right-hand side
-    float * dd = ks + NR * CP;           // [NR][CP] D
-    float * o_s = dd + NR * CP;          // [NR][CP] Q S_0, then the outputs
-    float * Bm = o_s + NR * CP;          // [NR][NP] beta_r w_rs (k_r . k_s), s < r
-    float * Am = Bm + NR * NP;           // [NR][NP] w_rs (q_r . k_s), s <= r
-    float * Tm = Am + NR * NP;           // [NR][20] inverses of the 16 x 16 diagonal blocks of I + B
-    float * lg = Tm + NR * 20;           // [NR] cumulative log decay
-    float * bet = lg + NR;               // [NR]
-    __shared__ double ssq[GDN_MAX_NODES];
-    __shared__ float scale_s[GDN_MAX_NODES];
-
-    // ---- loads, asynchronous: q and k (needed first), then this CTA's block of the state and v; beta, decay ----
-    constexpr int SQ = S / 4;
-    for (int i = tid; i < NR * SQ; i += GC_THREADS) {
-        const int node = i / SQ, e4 = i - node * SQ;
-        if (node < N) {
-            const int64_t at = (int64_t)(seq * N + node) * key_dim + kh * S + e4 * 4;
-            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(qn + node * KP + e4 * 4)),
-                         "l"(a.qn + at) : "memory");
-            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(kn + node * KP + e4 * 4)),
-                         "l"(a.khat + at) : "memory");
-        } else {
-            *reinterpret_cast<float4 *>(qn + node * KP + e4 * 4) = make_float4(0.f, 0.f, 0.f, 0.f);
-            *reinterpret_cast<float4 *>(kn + node * KP + e4 * 4) = make_float4(0.f, 0.f, 0.f, 0.f);
+    float * qn = sm, * kn = qn + NR * KP;
+    __shared__ float lg[GC_HEADS][GC_ROWS], bet[GC_HEADS][GC_ROWS];
+    __shared__ float diag[GC_HEADS][GC_ROWS * 17];  // diagonal blocks of B
+    chunk_fetch_rows<S>(qn, a.qn + (int64_t)r0 * key_dim + kh * S, key_dim, N, NR);
+    chunk_fetch_rows<S>(kn, a.khat + (int64_t)r0 * key_dim + kh * S, key_dim, N, NR);
+    cp_async_commit();
+    cp_async_wait<0>();
+    __syncthreads();
+    // K K^T and Q K^T on the lower triangle: 16 x 16 tiles up to the diagonal one, two per warp at most
+    const int per_mat = MT * (MT + 1) / 2;
+    constexpr int SLOTS = (4 * 5 + GC_WARPS - 1) / GC_WARPS;
+    float acc[SLOTS][2][4];
+    int tile_r[SLOTS], tile_c[SLOTS];
+#pragma unroll
+    for (int slot = 0; slot < SLOTS; slot++) {
+        const int tile = warp + slot * GC_WARPS, mat = tile >= per_mat, rest = tile - mat * per_mat;
+        int mt = 0;
+        while ((mt + 1) * (mt + 2) / 2 <= rest) mt++;
+        tile_r[slot] = mt;
+        tile_c[slot] = rest - mt * (mt + 1) / 2;
+        if (tile >= 2 * per_mat) continue;
+#pragma unroll
+        for (int j = 0; j < 2; j++)
+#pragma unroll
+            for (int e = 0; e < 4; e++) acc[slot][j][e] = 0.0f;
+        const float * arow = (mat ? qn : kn) + (16 * mt) * KP, * brow = kn + (16 * tile_c[slot]) * KP;
+        warp_mma_3x<2>(acc[slot], S / 8, [&](int r, int k) { return arow[r * KP + k]; }, [&](int k, int c) { return brow[c * KP + k]; }, g, t);
+    }
+    for (int h0 = kh; h0 < a.rank; h0 += GC_HEADS * a.groups) {
+        const int heads = min(GC_HEADS, (a.rank - h0 + a.groups - 1) / a.groups);
+        __syncthreads();
+        for (int i = threadIdx.x; i < heads * GC_ROWS; i += GC_THREADS) {
+            const int j = i / GC_ROWS, node = i - j * GC_ROWS;
+            float b = 0.0f, l = 0.0f;
+            if (node < N) {
+                const int64_t at = (int64_t)(r0 + node) * a.rank + h0 + j * a.groups;
+                b = a.beta[at];
+                const float dc = a.decay[at];
+                l = dc > 0.0f ? fmaxf(logf(dc), -100.0f) : -100.0f;  // a decay that underflowed still wipes the state
+            }
+            bet[j][node] = b;
+            lg[j][node] = l;
+        }
+        __syncthreads();
+        if (warp < heads) {
+            // inclusive scan of the (at most 64) log decays: two per lane
+            float s0v = lg[warp][lane], s1v = lg[warp][lane + 32];
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const float u0 = __shfl_up_sync(0xffffffffu, s0v, o), u1 = __shfl_up_sync(0xffffffffu, s1v, o);
+                if (lane >= o) { s0v += u0; s1v += u1; }
+            }
+            const float first = __shfl_sync(0xffffffffu, s0v, 31);
+            lg[warp][lane] = s0v;
+            lg[warp][lane + 32] = first + s1v;
+        }
+        __syncthreads();
+        // decay ratios and beta folded in; entries above the diagonal inside the diagonal tiles are zero
+        for (int j = 0; j < heads; j++) {
+            ChunkPair & out = p.pairs[(int64_t)blockIdx.x * a.rank + h0 + j * a.groups];
+#pragma unroll
+            for (int slot = 0; slot < SLOTS; slot++) {
+                const int tile = warp + slot * GC_WARPS, mat = tile >= per_mat;
+                if (tile >= 2 * per_mat) continue;
+#pragma unroll
+                for (int n = 0; n < 2; n++)
+#pragma unroll
+                    for (int e = 0; e < 4; e++) {
+                        const int rr = g + (e >> 1) * 8, cc = 8 * n + 2 * t + (e & 1);
+                        const int r = 16 * tile_r[slot] + rr, c = 16 * tile_c[slot] + cc;
+                        const float wgt = c <= r ? expf(lg[j][r] - lg[j][c]) : 0.0f;
+                        if (mat) {
+                            out.A[r * GC_NP + c] = wgt * acc[slot][n][e];
+                        } else {
+                            const float v = c < r ? bet[j][r] * wgt * acc[slot][n][e] : 0.0f;
+                            if (tile_r[slot] == tile_c[slot]) diag[j][r * 17 + cc] = v;
+                            else out.B[r * GC_NP + c] = v;
+                        }
+                    }
+            }
+        }
+        __syncthreads();
+        for (int i = threadIdx.x; i < heads * GC_ROWS; i += GC_THREADS) {
+            const int j = i / GC_ROWS, node = i - j * GC_ROWS;
+            ChunkPair & out = p.pairs[(int64_t)blockIdx.x * a.rank + h0 + j * a.groups];
+            out.beta[node] = bet[j][node];
+            out.gam[node] = expf(lg[j][node]);
+            out.tail[node] = node < N ? expf(lg[j][N - 1] - lg[j][node]) : 0.0f;
+        }
+        // half a warp per diagonal block, lane = column s of the inverse T: row r of T is e_r minus the rows before it
+        // weighted by row r of B (forward substitution, as inverseLower of recurrent.go:307-331 does for the
+        // whole chunk). Rows beyond the chunk have B = 0 and stay rows of the identity.
+        if (warp < 2 * heads) {
+            const int j = warp >> 1, b0 = ((warp & 1) * 2 + (lane >> 4)) * 16, sc = lane & 15;
+            if (b0 < N) {
+                float * T = p.pairs[(int64_t)blockIdx.x * a.rank + h0 + j * a.groups].T;
+                float tv[16];
+#pragma unroll
+                for (int r = 0; r < 16; r++) {
+                    float v = r == sc ? 1.0f : 0.0f;
+                    const float * brow = diag[j] + (b0 + r) * 17;
+#pragma unroll
+                    for (int u = 0; u < r; u++) v = fmaf(-brow[u], tv[u], v);
+                    tv[r] = v;
+                    T[(b0 + r) * GC_TP + sc] = v;
+                }
+            }
         }
     }
-    asm volatile("cp.async.commit_group;" ::: "memory");
-    float * state = const_cast<float *>(a.state) + ((int64_t)(seq_of(p.rows, seq) * a.rank + h) * S) * S + cb * GDN_COLS;
+}
+
+// (2) grid (S/32 column blocks, rank)
+template <int S>
+__global__ void __launch_bounds__(GC_THREADS, 1) gdn_chunk_scan_kernel(const ChunkParams p) {
+    pdl_entry();
+    const GdnArgs & a = p.a;
+    const int cb = blockIdx.x, h = blockIdx.y, kh = h % a.groups;
+    const int key_dim = a.groups * S, inner = a.rank * S;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
+    constexpr int KP = S + 4, CP = GC_CP, NP = GC_NP;
+    extern __shared__ __align__(16) float sm[];
+    float * qn = sm;                         // [GC_ROWS][KP]
+    float * kbuf = qn + GC_ROWS * KP;        // two of them: this chunk's keys and the next one's
+    float * s0 = kbuf + 2 * GC_ROWS * KP;    // [S][CP] this CTA's columns of the state
+    float * vv = s0 + S * CP;                // [GC_ROWS][CP] v, later exp(g_C - g_s) d_s
+    float * rhs = vv + GC_ROWS * CP;         // [GC_ROWS][CP] beta (v - gam K S_0)
+    float * dd = rhs + GC_ROWS * CP;         // [GC_ROWS][CP] D
+    ChunkPair & pair = *reinterpret_cast<ChunkPair *>(dd + GC_ROWS * CP);
+    const int chunks = (p.rows + GC_ROWS - 1) / GC_ROWS;
+    const float * qsrc = a.qn + kh * S, * ksrc = a.khat + kh * S, * vsrc = a.vconv + h * S + cb * GDN_COLS;
+    float * state = const_cast<float *>(a.state) + (int64_t)h * S * S + cb * GDN_COLS;
+    float * osrc = a.out + h * S + cb * GDN_COLS;
+
+    auto rows_of = [&](int c) { return min(GC_ROWS, p.rows - c * GC_ROWS); };
+    auto fetch_qk = [&](int c) {
+        const int n = rows_of(c), padded = (n + 15) & ~15;
+        chunk_fetch_rows<S>(qn, qsrc + (int64_t)c * GC_ROWS * key_dim, key_dim, n, padded);
+        chunk_fetch_rows<S>(kbuf + (c & 1) * GC_ROWS * KP, ksrc + (int64_t)c * GC_ROWS * key_dim, key_dim, n, padded);
+        cp_async_commit();
+    };
     for (int i = tid; i < S * (GDN_COLS / 4); i += GC_THREADS) {
         const int row = i / (GDN_COLS / 4), c4 = i - row * (GDN_COLS / 4);
-        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(s0 + row * CP + c4 * 4)),
-                     "l"(state + (int64_t)row * S + c4 * 4) : "memory");
+        cp_async16(s0 + row * CP + c4 * 4, state + (int64_t)row * S + c4 * 4);
     }
-    for (int i = tid; i < NR * (GDN_COLS / 4); i += GC_THREADS) {
-        const int node = i / (GDN_COLS / 4), e4 = i - node * (GDN_COLS / 4);
-        if (node < N)
-            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(vv + node * CP + e4 * 4)),
-                         "l"(a.vconv + (int64_t)(seq * N + node) * inner + h * S + cb * GDN_COLS + e4 * 4) : "memory");
-        else *reinterpret_cast<float4 *>(vv + node * CP + e4 * 4) = make_float4(0.f, 0.f, 0.f, 0.f);
-    }
-    asm volatile("cp.async.commit_group;" ::: "memory");
-    // the gate values and the norm weight the last phase needs (a 64-row chunk: four per thread) are fetched now
-    constexpr int ZPRE = GDN_MAX_NODES * GDN_COLS / GC_THREADS;
-    float zpre[ZPRE];
-#pragma unroll
-    for (int k = 0; k < ZPRE; k++) {
-        const int i = tid + k * GC_THREADS;
-        const int node = i / GDN_COLS, c = i - node * GDN_COLS;
-        zpre[k] = i < N * GDN_COLS ? a.z[(int64_t)(seq * N + node) * a.ldz + h * S + cb * GDN_COLS + c] : 0.0f;
-    }
-    const float norm_w = a.norm[cb * GDN_COLS + (tid & (GDN_COLS - 1))];
-    for (int node = tid; node < NR; node += GC_THREADS) {
-        float b = 0.0f, l = 0.0f;
-        if (node < N) {
-            b = a.beta[(int64_t)(seq * N + node) * a.rank + h];
-            const float dc = a.decay[(int64_t)(seq * N + node) * a.rank + h];
-            l = dc > 0.0f ? fmaxf(logf(dc), -100.0f) : -100.0f;  // a decay that underflowed still wipes the state
+    fetch_qk(0);
+    for (int c = 0; c < chunks; c++) {
+        const int N = rows_of(c), MT = (N + 15) >> 4, NR = MT * 16, r0 = c * GC_ROWS;
+        const float * kn = kbuf + (c & 1) * GC_ROWS * KP;
+        {   // v and the matrices of this chunk: needed after the first products
+            const float4 * src = reinterpret_cast<const float4 *>(p.pairs + (int64_t)c * a.rank + h);
+            for (int i = tid; i < (int)(sizeof(ChunkPair) / 16); i += GC_THREADS) cp_async16(reinterpret_cast<float4 *>(&pair) + i, src + i);
+            for (int i = tid; i < NR * (GDN_COLS / 4); i += GC_THREADS) {
+                const int node = i / (GDN_COLS / 4), e4 = i - node * (GDN_COLS / 4);
+                if (node < N) cp_async16(vv + node * CP + e4 * 4, vsrc + (int64_t)(r0 + node) * inner + e4 * 4);
+                else *reinterpret_cast<float4 *>(vv + node * CP + e4 * 4) = make_float4(0.f, 0.f, 0.f, 0.f);
+            }
+            cp_async_commit();
         }
-        bet[node] = b;
-        o_s[node] = l;  // (scratch until the outputs are written)
-    }
-    asm volatile("cp.async.wait_group 1;" ::: "memory");  // q and k have landed; the state may still be on its way
-    __syncthreads();
-    if (warp == 0) {
-        // inclusive scan of the (at most 64) log decays: two per lane
-        const float l0 = lane < NR ? o_s[lane] : 0.0f, l1 = lane + 32 < NR ? o_s[lane + 32] : 0.0f;
-        float s0v = l0, s1v = l1;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const float u0 = __shfl_up_sync(0xffffffffu, s0v, o), u1 = __shfl_up_sync(0xffffffffu, s1v, o);
-            if (lane >= o) { s0v += u0; s1v += u1; }
+        cp_async_wait<1>();  // q, k (and the state) have landed
+        __syncthreads();
+        // ---- K S_0 (warps 0-7) and Q S_0 (warps 8-15): a warp per 16 rows x 16 columns; Q S_0 stays in registers ----
+        const int nh = warp & 1, mt = (warp >> 1) & 3;
+        const bool is_q = warp >= 8;
+        float acc[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
+        if (mt < MT) {
+            const float * arow = (is_q ? qn : kn) + (16 * mt) * KP, * bcol = s0 + 16 * nh;
+            warp_mma_3x<2>(acc, S / 8, [&](int r, int k) { return arow[r * KP + k]; }, [&](int k, int col) { return bcol[k * CP + col]; }, g, t);
         }
-        const float first = __shfl_sync(0xffffffffu, s0v, 31);
-        if (lane < NR) lg[lane] = s0v;
-        if (lane + 32 < NR) lg[lane + 32] = first + s1v;
-    }
-    __syncthreads();
-
-    // ---- B and A: K K^T and Q K^T on the lower triangle (16 x 16 tiles up to the diagonal one), decay ratios and
-    // beta folded in on the way out; entries above the diagonal inside the diagonal tiles are zero ----
-    {
-        const int per_mat = MT * (MT + 1) / 2;
-        for (int tile = warp; tile < 2 * per_mat; tile += GC_WARPS) {
-            const int mat = tile >= per_mat, rest = tile - mat * per_mat;
-            int mt = 0;
-            while ((mt + 1) * (mt + 2) / 2 <= rest) mt++;
-            const int nt = rest - mt * (mt + 1) / 2;
-            const float * arow = (mat ? qn : kn) + (16 * mt) * KP, * brow = kn + (16 * nt) * KP;
-            float acc[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
-            warp_mma_3x<2>(acc, S / 8, [&](int r, int k) { return arow[r * KP + k]; }, [&](int k, int c) { return brow[c * KP + k]; }, g, t);
+        cp_async_wait<0>();
+        __syncthreads();
+        if (c + 1 < chunks) fetch_qk(c + 1);
+        // ---- right-hand side beta (v - gam K S_0) ----
+        if (!is_q && mt < MT) {
 #pragma unroll
             for (int j = 0; j < 2; j++)
 #pragma unroll
                 for (int e = 0; e < 4; e++) {
-                    const int r = 16 * mt + g + (e >> 1) * 8, c = 16 * nt + 8 * j + 2 * t + (e & 1);
-                    const float wgt = c <= r ? expf(lg[r] - lg[c]) : 0.0f;
-                    if (mat) Am[r * NP + c] = wgt * acc[j][e];
-                    else Bm[r * NP + c] = c < r ? bet[r] * wgt * acc[j][e] : 0.0f;
+                    const int r = 16 * mt + g + (e >> 1) * 8, at = r * CP + 16 * nh + 8 * j + 2 * t + (e & 1);
+                    rhs[at] = pair.beta[r] * (vv[at] - pair.gam[r] * acc[j][e]);
                 }
         }
-    }
-    asm volatile("cp.async.wait_all;" ::: "memory");
-    __syncthreads();
-
-    // ---- K S_0 and Q S_0 for this CTA's columns: a warp per (matrix, 16-row tile, 16-column half) ----
-    for (int task = warp; task < 4 * MT; task += GC_WARPS) {
-        const int nh = task & 1, mt = (task >> 1) % MT, which = task / (2 * MT);
-        const float * arow = (which ? qn : kn) + (16 * mt) * KP, * bcol = s0 + 16 * nh;
-        float acc[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
-        warp_mma_3x<2>(acc, S / 8, [&](int r, int k) { return arow[r * KP + k]; }, [&](int k, int c) { return bcol[k * CP + c]; }, g, t);
-        float * dst = (which ? o_s : ks) + (16 * mt) * CP + 16 * nh;
-#pragma unroll
-        for (int j = 0; j < 2; j++) {
-            *reinterpret_cast<float2 *>(dst + g * CP + 8 * j + 2 * t) = make_float2(acc[j][0], acc[j][1]);
-            *reinterpret_cast<float2 *>(dst + (g + 8) * CP + 8 * j + 2 * t) = make_float2(acc[j][2], acc[j][3]);
-        }
-    }
-    __syncthreads();
-
-    // ---- right-hand side beta (v - gam K S_0); meanwhile two warps invert the 16 x 16 diagonal blocks of I + B ----
-    for (int i = tid; i < NR * GDN_COLS; i += GC_THREADS) {
-        const int r = i / GDN_COLS, c = i - r * GDN_COLS;
-        ks[r * CP + c] = bet[r] * (vv[r * CP + c] - expf(lg[r]) * ks[r * CP + c]);
-    }
-    if (warp >= GC_WARPS - 2) {
-        // half a warp per block, lane = column s of the inverse T: row r of T is e_r minus the rows before it
-        // weighted by row r of B (forward substitution, as inverseLower of recurrent.go:307-331 does for the
-        // whole chunk). Rows beyond the chunk have B = 0 and stay rows of the identity.
-        const int blk = (warp - (GC_WARPS - 2)) * 2 + (lane >> 4), sc = lane & 15, b0 = blk * 16;
-        if (b0 < N) {
-            float tv[16];
-#pragma unroll
-            for (int r = 0; r < 16; r++) {
-                float v = r == sc ? 1.0f : 0.0f;
-                const float * brow = Bm + (b0 + r) * NP + b0;
-#pragma unroll
-                for (int u = 0; u < r; u++) v = fmaf(-brow[u], tv[u], v);
-                tv[r] = v;
-                Tm[(b0 + r) * 20 + sc] = v;
-            }
-        }
-    }
-    __syncthreads();
-    // ---- forward substitution over the blocks: D_b = T_b (rhs_b - B[b][earlier] D[earlier]); a warp per 8 columns ----
-    for (int b0 = 0; b0 < N; b0 += 16) {
-        if (b0 > 0) {
-            if (warp < 4) {
-                float acc[1][4] = {{0.f, 0.f, 0.f, 0.f}};
-                const float * arow = Bm + b0 * NP, * bcol = dd + 8 * warp;
-                warp_mma_3x<1>(acc, b0 / 8, [&](int r, int k) { return arow[r * NP + k]; }, [&](int k, int c) { return bcol[k * CP + c]; }, g, t);
-                float * dst = ks + b0 * CP + 8 * warp + 2 * t;
-                dst[g * CP] -= acc[0][0];
-                dst[g * CP + 1] -= acc[0][1];
-                dst[(g + 8) * CP] -= acc[0][2];
-                dst[(g + 8) * CP + 1] -= acc[0][3];
-            }
-            __syncthreads();
-        }
+        __syncthreads();
+        // ---- forward substitution over the blocks: D_b = T_b (rhs_b - B[b][earlier] D[earlier]); a warp per 8 columns,
+        // which meets no other warp's columns ----
         if (warp < 4) {
-            float acc[1][4] = {{0.f, 0.f, 0.f, 0.f}};
-            const float * arow = Tm + b0 * 20, * bcol = ks + b0 * CP + 8 * warp;
-            warp_mma_3x<1>(acc, 2, [&](int r, int k) { return arow[r * 20 + k]; }, [&](int k, int c) { return bcol[k * CP + c]; }, g, t);
-            float * dst = dd + b0 * CP + 8 * warp + 2 * t;
-            *reinterpret_cast<float2 *>(dst + g * CP) = make_float2(acc[0][0], acc[0][1]);
-            *reinterpret_cast<float2 *>(dst + (g + 8) * CP) = make_float2(acc[0][2], acc[0][3]);
+            for (int b0 = 0; b0 < N; b0 += 16) {
+                float * rh = rhs + b0 * CP + 8 * warp;
+                if (b0 > 0) {
+                    float sub[1][4] = {{0.f, 0.f, 0.f, 0.f}};
+                    const float * arow = pair.B + b0 * NP, * bcol = dd + 8 * warp;
+                    warp_mma_3x<1>(sub, b0 / 8, [&](int r, int k) { return arow[r * NP + k]; }, [&](int k, int col) { return bcol[k * CP + col]; }, g, t);
+                    float * dst = rh + 2 * t;
+                    dst[g * CP] -= sub[0][0];
+                    dst[g * CP + 1] -= sub[0][1];
+                    dst[(g + 8) * CP] -= sub[0][2];
+                    dst[(g + 8) * CP + 1] -= sub[0][3];
+                    __syncwarp();
+                }
+                float d[1][4] = {{0.f, 0.f, 0.f, 0.f}};
+                const float * arow = pair.T + b0 * GC_TP;
+                warp_mma_3x<1>(d, 2, [&](int r, int k) { return arow[r * GC_TP + k]; }, [&](int k, int col) { return rh[k * CP + col]; }, g, t);
+                const int at = b0 * CP + 8 * warp + 2 * t;
+                *reinterpret_cast<float2 *>(dd + at + g * CP) = make_float2(d[0][0], d[0][1]);
+                *reinterpret_cast<float2 *>(dd + at + (g + 8) * CP) = make_float2(d[0][2], d[0][3]);
+                // (v has gone into the right-hand side; its place takes w d)
+                const float w0 = pair.tail[b0 + g], w1 = pair.tail[b0 + g + 8];
+                *reinterpret_cast<float2 *>(vv + at + g * CP) = make_float2(w0 * d[0][0], w0 * d[0][1]);
+                *reinterpret_cast<float2 *>(vv + at + (g + 8) * CP) = make_float2(w1 * d[0][2], w1 * d[0][3]);
+                __syncwarp();
+            }
+        }
+        __syncthreads();
+        // ---- outputs gam_r (Q S_0)_r + sum_{s <= r} A[r][s] d_s (warps 8-15, which hold Q S_0) and the new state
+        // gam_C S_0 + K^T (w d) (warps 0-7: 16 state rows x 32 columns) ----
+        if (is_q) {
+            if (mt < MT) {
+                float o[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
+                const float * arow = pair.A + (16 * mt) * NP, * bcol = dd + 16 * nh;
+                warp_mma_3x<2>(o, 2 * mt + 2, [&](int r, int k) { return arow[r * NP + k]; }, [&](int k, int col) { return bcol[k * CP + col]; }, g, t);
+                const int r = 16 * mt + g;
+                const float g0 = pair.gam[r], g1 = pair.gam[r + 8];
+                float * dst = osrc + (int64_t)(r0 + r) * inner + 16 * nh + 2 * t;
+#pragma unroll
+                for (int j = 0; j < 2; j++) {
+                    if (r < N) *reinterpret_cast<float2 *>(dst + 8 * j) = make_float2(fmaf(g0, acc[j][0], o[j][0]), fmaf(g0, acc[j][1], o[j][1]));
+                    if (r + 8 < N)
+                        *reinterpret_cast<float2 *>(dst + (int64_t)8 * inner + 8 * j) = make_float2(fmaf(g1, acc[j][2], o[j][2]), fmaf(g1, acc[j][3], o[j][3]));
+                }
+            }
+        } else if (warp < S / 16) {
+            const float gam_c = pair.gam[N - 1];
+            float n[4][4];
+#pragma unroll
+            for (int j = 0; j < 4; j++)
+#pragma unroll
+                for (int e = 0; e < 4; e++) n[j][e] = 0.0f;
+            const float * acol = kn + 16 * warp;
+            warp_mma_3x<4>(n, NR / 8, [&](int r, int k) { return acol[k * KP + r]; }, [&](int k, int col) { return vv[k * CP + col]; }, g, t);
+            float * own = s0 + (16 * warp + g) * CP + 2 * t;
+#pragma unroll
+            for (int j = 0; j < 4; j++) {
+                float2 * o0 = reinterpret_cast<float2 *>(own + 8 * j), * o1 = reinterpret_cast<float2 *>(own + 8 * CP + 8 * j);
+                *o0 = make_float2(fmaf(gam_c, o0->x, n[j][0]), fmaf(gam_c, o0->y, n[j][1]));
+                *o1 = make_float2(fmaf(gam_c, o1->x, n[j][2]), fmaf(gam_c, o1->y, n[j][3]));
+            }
         }
         __syncthreads();
     }
-    // vv <- exp(g_C - g_s) d_s for the state update
-    {
-        const float lc = lg[N - 1];
-        for (int i = tid; i < NR * GDN_COLS; i += GC_THREADS) {
-            const int r = i / GDN_COLS, c = i - r * GDN_COLS;
-            vv[r * CP + c] = r < N ? expf(lc - lg[r]) * dd[r * CP + c] : 0.0f;
-        }
-    }
-    __syncthreads();
-
-    // ---- outputs gam_r (Q S_0)_r + sum_{s <= r} A[r][s] d_s (2 MT tasks) and the new state gam_C S_0 + K^T (w d),
-    // written in place (S / 8 tasks): a warp per 16 rows x 16 columns ----
-    {
-        const float gam_c = expf(lg[N - 1]);
-        for (int task = warp; task < 2 * MT + S / 8; task += GC_WARPS) {
-            float acc[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
-            if (task < 2 * MT) {
-                const int nh = task & 1, mt = task >> 1;
-                const float * arow = Am + (16 * mt) * NP, * bcol = dd + 16 * nh;
-                warp_mma_3x<2>(acc, 2 * mt + 2, [&](int r, int k) { return arow[r * NP + k]; }, [&](int k, int c) { return bcol[k * CP + c]; }, g, t);
-                float * dst = o_s + (16 * mt) * CP + 16 * nh;
-                const float g0 = expf(lg[16 * mt + g]), g1 = expf(lg[16 * mt + g + 8]);
-#pragma unroll
-                for (int j = 0; j < 2; j++) {
-                    float2 * lo = reinterpret_cast<float2 *>(dst + g * CP + 8 * j + 2 * t), * hi = reinterpret_cast<float2 *>(dst + (g + 8) * CP + 8 * j + 2 * t);
-                    *lo = make_float2(fmaf(g0, lo->x, acc[j][0]), fmaf(g0, lo->y, acc[j][1]));
-                    *hi = make_float2(fmaf(g1, hi->x, acc[j][2]), fmaf(g1, hi->y, acc[j][3]));
-                }
-            } else {
-                const int e = task - 2 * MT, nh = e & 1, it = e >> 1;  // state rows 16 it .., columns 16 nh ..
-                const float * acol = kn + 16 * it, * bcol = vv + 16 * nh;
-                warp_mma_3x<2>(acc, NR / 8, [&](int r, int k) { return acol[k * KP + r]; }, [&](int k, int c) { return bcol[k * CP + c]; }, g, t);
-                const float * old = s0 + (16 * it) * CP + 16 * nh;
-                float * dst = state + (int64_t)(16 * it) * S + 16 * nh;
-#pragma unroll
-                for (int j = 0; j < 2; j++) {
-                    const float2 o0 = *reinterpret_cast<const float2 *>(old + g * CP + 8 * j + 2 * t);
-                    const float2 o1 = *reinterpret_cast<const float2 *>(old + (g + 8) * CP + 8 * j + 2 * t);
-                    *reinterpret_cast<float2 *>(dst + (int64_t)g * S + 8 * j + 2 * t) = make_float2(fmaf(gam_c, o0.x, acc[j][0]), fmaf(gam_c, o0.y, acc[j][1]));
-                    *reinterpret_cast<float2 *>(dst + (int64_t)(g + 8) * S + 8 * j + 2 * t) = make_float2(fmaf(gam_c, o1.x, acc[j][2]), fmaf(gam_c, o1.y, acc[j][3]));
-                }
-            }
-        }
-    }
-    __syncthreads();
-
     pdl_trigger_late();
-    // ---- gated RMSNorm of the head (recurrent.go:39-50), sums of squares exchanged across the cluster ----
-    for (int node = warp; node < N; node += GC_WARPS) {
-        const double v = (double)o_s[node * CP + lane];
-        double sq = v * v;
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) sq += __shfl_xor_sync(0xffffffffu, sq, o);
-        if (lane == 0) ssq[node] = sq;
+    for (int i = tid; i < S * (GDN_COLS / 4); i += GC_THREADS) {
+        const int row = i / (GDN_COLS / 4), c4 = i - row * (GDN_COLS / 4);
+        *reinterpret_cast<float4 *>(state + (int64_t)row * S + c4 * 4) = *reinterpret_cast<const float4 *>(s0 + row * CP + c4 * 4);
     }
-    cluster_sync_all();
-    for (int node = tid; node < N; node += GC_THREADS) {
-        double tot = 0;
-        for (unsigned r = 0; r < gridDim.x; r++) tot += ld_cluster_f64(ssq + node, r);  // the cluster spans gridDim.x
-        const float mean = (float)(tot / (double)S);
-        scale_s[node] = (float)(1.0 / sqrt((double)(mean + a.eps)));
-    }
-    cluster_sync_all();  // scales visible to the CTA; no CTA leaves while another may still read its sums
+}
+
+// (3) gated RMSNorm (recurrent.go:39-50) of every (row, head): a warp each, S / 32 columns per lane, the sums of squares
+// in the scan kernel's order. Reads the outputs from a.out and leaves them there and prepared, or, where the out
+// projection reads nothing but their fp16 form, only that.
+template <int S>
+__global__ void __launch_bounds__(256) gdn_gated_norm_kernel(const GdnArgs a, int rows) {
+    pdl_entry();
+    constexpr int G = S / 32;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, inner = a.rank * S;
+    const int64_t item = (int64_t)blockIdx.x * 8 + warp;
+    __shared__ __align__(16) float stage[8][S];
+    if (item >= (int64_t)rows * a.rank) return;
+    const int r = (int)(item / a.rank), h = (int)(item - (int64_t)r * a.rank);
+    const int64_t at = (int64_t)r * inner + h * S + lane;
+    float o[G], z[G], w[G];
+    double sq[G];
 #pragma unroll
-    for (int k = 0; k < ZPRE; k++) {
-        const int i = tid + k * GC_THREADS;
-        if (i < N * GDN_COLS) {
-            const int node = i / GDN_COLS, c = i - node * GDN_COLS;
-            o_s[node * CP + c] = o_s[node * CP + c] * (scale_s[node] * norm_w) * silu_ref(zpre[k]);
+    for (int i = 0; i < G; i++) {
+        o[i] = a.out[at + 32 * i];
+        z[i] = a.z[(int64_t)r * a.ldz + h * S + lane + 32 * i];
+        w[i] = a.norm[lane + 32 * i];
+    }
+#pragma unroll
+    for (int i = 0; i < G; i++) sq[i] = (double)o[i] * (double)o[i];
+#pragma unroll
+    for (int k = 16; k > 0; k >>= 1)
+#pragma unroll
+        for (int i = 0; i < G; i++) sq[i] += __shfl_xor_sync(0xffffffffu, sq[i], k);
+    double tot = 0;
+#pragma unroll
+    for (int i = 0; i < G; i++) tot += sq[i];
+    const float mean = (float)(tot / (double)S);
+    const float scale = (float)(1.0 / sqrt((double)(mean + a.eps)));
+    const bool hi_only = a.prep.hi_only();
+#pragma unroll
+    for (int i = 0; i < G; i++) {
+        const float v = o[i] * (scale * w[i]) * silu_ref(z[i]);
+        if (hi_only) {
+            a.prep.xh[at + 32 * i] = __float2half_rn(v);
+        } else {
+            a.out[at + 32 * i] = v;
+            stage[warp][lane + 32 * i] = v;
         }
     }
-    __syncthreads();
-    for (int gi = tid; gi < N * (GDN_COLS >> 4); gi += GC_THREADS) {
-        const int node = gi / (GDN_COLS >> 4), part = gi - node * (GDN_COLS >> 4);
-        const int64_t r = seq * N + node;
-        const int c0 = h * S + cb * GDN_COLS + part * 16;
+    if (hi_only || !a.prep.xh) return;
+    __syncwarp();
+    if (lane < S / 16) {
         float g16[16];
 #pragma unroll
-        for (int i = 0; i < 16; i++) g16[i] = o_s[node * CP + part * 16 + i];
-        float4 * dst = reinterpret_cast<float4 *>(a.out + r * inner + c0);
-#pragma unroll
-        for (int i = 0; i < 4; i++) dst[i] = make_float4(g16[4 * i], g16[4 * i + 1], g16[4 * i + 2], g16[4 * i + 3]);
-        if (a.prep.xh) xprep_store16(a.prep.xh + r * inner + c0, a.prep.xl + r * inner + c0, a.prep.xs16 + r * (inner >> 4) + (c0 >> 4), g16);
+        for (int i = 0; i < 16; i++) g16[i] = stage[warp][lane * 16 + i];
+        const int64_t c0 = (int64_t)r * inner + h * S + lane * 16;
+        xprep_store16(a.prep.xh + c0, a.prep.xl + c0, a.prep.xs16 + (c0 >> 4), g16);
     }
 }
 
-static size_t gdn_chunk_smem(int N, int S) {
-    const size_t nr = (size_t)((N + 15) & ~15);
-    return sizeof(float) * (2 * nr * (S + 4) + (size_t)S * GC_CP + 4 * nr * GC_CP + 2 * nr * (nr + 4) + nr * 20 + 2 * nr);
-}
+size_t gdn_chunk_scratch_bytes(int rows, int rank) { return (size_t)((rows + GC_ROWS - 1) / GC_ROWS) * rank * sizeof(ChunkPair); }
 
-// The front end alone for one chain of any length (a whole prompt pass of one sequence): conv taps come from the
-// preceding rows of the pass and, for its first kernel - 1 rows, from the stored history.
-void launch_gdn_front_chain(cudaStream_t s, const GdnArgs & a, int seq_slot, int n_rows) {
-    (void)seq_slot;
+// One chain of any length whose rows are all committed (a prompt pass of one sequence): the front end for the whole pass
+// (conv taps come from the preceding rows and, for the first kernel - 1 rows, from the stored history), then the chunkwise
+// scan; the state is rewritten in place (the conv history still moves with launch_gdn_commit(..., conv_only)).
+template <int S>
+static void launch_gdn_chunks_s(cudaStream_t s, const ChunkParams & p) {
+    const GdnArgs & a = p.a;
+    constexpr size_t ROW = sizeof(float) * GC_ROWS * (S + 4);
+    const size_t pairs_smem = 2 * ROW;
+    const size_t scan_smem = 3 * ROW + sizeof(float) * (S + 3 * GC_ROWS) * GC_CP + sizeof(ChunkPair);
+    YK_CUDA(cudaFuncSetAttribute(gdn_chunk_pairs_kernel<S>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pairs_smem));
+    YK_CUDA(cudaFuncSetAttribute(gdn_chunk_scan_kernel<S>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)scan_smem));
+    launch_k(gdn_chunk_pairs_kernel<S>, dim3((p.rows + GC_ROWS - 1) / GC_ROWS, a.groups), GC_THREADS, pairs_smem, s, p);
+    launch_k(gdn_chunk_scan_kernel<S>, dim3(S / GDN_COLS, a.rank), GC_THREADS, scan_smem, s, p);
+    launch_k(gdn_gated_norm_kernel<S>, (int)(((int64_t)p.rows * a.rank + 7) / 8), 256, 0, s, a, p.rows);
+    YK_CUDA(cudaGetLastError());
+}
+int launch_gdn_chunks(cudaStream_t s, const GdnArgs & a, int n_rows, void * scratch) {
     RowMeta rows{};
     rows.batch = 1;
     rows.nodes = n_rows;
     launch_gdn_front(s, a, rows, true);
-}
-
-// Chunkwise scan of a chain of at most 64 rows that are all committed, after the front end has run for them; the
-// state is rewritten in place (the conv history still moves with launch_gdn_commit(..., conv_only)).
-void launch_gdn_chunk(cudaStream_t s, const GdnArgs & a, const RowMeta & rows) {
-    YK_REQUIRE(rows.nodes <= GDN_MAX_NODES, YUUKA_ERR_UNSUPPORTED, "gdn: at most %d rows per chunk", GDN_MAX_NODES);
-    YK_REQUIRE(a.S == 64 || a.S == 128, YUUKA_ERR_UNSUPPORTED, "gdn: state size %d is not 64 or 128", a.S);
-    ScanParams p{a, rows, 0, 0};
-    const int N = rows.nodes;
-    dim3 grid(a.S / GDN_COLS, a.rank, rows.batch);
-    const size_t smem = gdn_chunk_smem(N, a.S);
-    if (a.S == 128) {
-        YK_CUDA(cudaFuncSetAttribute(gdn_chunk_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        launch_k_cluster(gdn_chunk_kernel<128>, grid, GC_THREADS, smem, s, grid.x, p);
-    } else {
-        YK_CUDA(cudaFuncSetAttribute(gdn_chunk_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        launch_k_cluster(gdn_chunk_kernel<64>, grid, GC_THREADS, smem, s, grid.x, p);
-    }
-    YK_CUDA(cudaGetLastError());
+    const ChunkParams p{a, n_rows, static_cast<ChunkPair *>(scratch)};
+    if (a.S == 128) launch_gdn_chunks_s<128>(s, p);
+    else launch_gdn_chunks_s<64>(s, p);
+    return 4;
 }
 
 // ---------------------------------------------------------------------------

@@ -286,7 +286,12 @@ __global__ void xprep_kernel(__half * __restrict__ xh, __half * __restrict__ xl,
         float v[16];
         load8(x + (int64_t)m * ldx + gq * 16, *reinterpret_cast<float(*)[8]>(v));
         load8(x + (int64_t)m * ldx + gq * 16 + 8, *reinterpret_cast<float(*)[8]>(v + 8));
-        xprep_store16(xh + (int64_t)m * K + gq * 16, xl + (int64_t)m * K + gq * 16, xs16 + (int64_t)m * groups + gq, v);
+        if (xl) {
+            xprep_store16(xh + (int64_t)m * K + gq * 16, xl + (int64_t)m * K + gq * 16, xs16 + (int64_t)m * groups + gq, v);
+        } else {
+#pragma unroll
+            for (int j = 0; j < 16; j += 4) xprep_store_hi4(xh + (int64_t)m * K + gq * 16 + j, v[j], v[j + 1], v[j + 2], v[j + 3]);
+        }
     }
 }
 
@@ -1399,6 +1404,10 @@ static bool umma_enabled() {
     return on;
 }
 
+bool gemm_tiled_wide(int rows, bool exact_only, bool wide_from_33) {
+    return rows >= (wide_from_33 ? UMMA_EARLY_ROWS : UMMA_MIN_ROWS) && umma_enabled() && !exact_only;
+}
+
 // How a launch of the tensor-memory kernel is cut: m activation rows into n_tiles tiles of n_tile rows, K into kparts.
 struct UmmaPlan {
     int n_tile, n_tiles, kparts;
@@ -1669,21 +1678,22 @@ template <int DT>
 static int launch_mma_dt(const yuuka_device * dev, cudaStream_t s, const TiledGemmArgs & a) {
     int launches = 0;
     XPrepOut xp = a.xprep;
+    const bool wide = gemm_tiled_wide(a.rows, a.exact_only, a.wide_from_33);
     if (!xp.xh) {
         // activations arrive as f32 / bf16: convert once into the scratch
         YK_REQUIRE(a.x && a.scratch && a.scratch->xh && a.scratch->xl && a.scratch->xh_elems >= (uint64_t)a.rows * a.n_in,
                    YUUKA_ERR_INTERNAL, "gemm: no prepared activations and no scratch to prepare them in");
+        __half * xl = wide ? nullptr : a.scratch->xl;  // (the wide route reads the hi halves alone)
         if (a.x_dtype == YUUKA_DTYPE_F32)
-            launch_xprep<float>(s, a.scratch->xh, a.scratch->xl, a.scratch->xs16, (const float *)a.x, a.ldx, a.n_in, a.rows);
+            launch_xprep<float>(s, a.scratch->xh, xl, a.scratch->xs16, (const float *)a.x, a.ldx, a.n_in, a.rows);
         else
-            launch_xprep<__nv_bfloat16>(s, a.scratch->xh, a.scratch->xl, a.scratch->xs16, (const __nv_bfloat16 *)a.x, a.ldx, a.n_in, a.rows);
+            launch_xprep<__nv_bfloat16>(s, a.scratch->xh, xl, a.scratch->xs16, (const __nv_bfloat16 *)a.x, a.ldx, a.n_in, a.rows);
         xp.xh = a.scratch->xh;
-        xp.xl = a.scratch->xl;
+        xp.xl = xl;
         xp.xs16 = a.scratch->xs16;
         launches++;
     }
-    if (a.rows >= (a.wide_from_33 ? UMMA_EARLY_ROWS : UMMA_MIN_ROWS) && umma_enabled() && !a.exact_only)
-        return launches + launch_umma_dt<DT>(dev, s, a, xp.xh);
+    if (wide) return launches + launch_umma_dt<DT>(dev, s, a, xp.xh);
     YK_REQUIRE(xp.xl && xp.xs16, YUUKA_ERR_INTERNAL, "gemm: the prepared activations lack their lo halves or sums");
     for (int m0 = 0; m0 < a.rows; m0 += MMA_ROWS) {
         const int m = a.rows - m0 < MMA_ROWS ? a.rows - m0 : MMA_ROWS;

@@ -101,6 +101,8 @@ struct TiledGemmArgs {
 };
 
 int launch_gemm_tiled(const yuuka_device * dev, cudaStream_t stream, const TiledGemmArgs & a);
+// whether a launch of so many rows takes the tensor-memory route, which reads the hi halves of the activations alone
+bool gemm_tiled_wide(int rows, bool exact_only, bool wide_from_33);
 // Scratch the launch above needs for this shape (0 partial floats when K is not split across CTAs).
 void gemm_tiled_scratch_need(const yuuka_device * dev, uint32_t w_dtype, int rows, int n_out, int n_in,
                              uint64_t * partial_floats, int * counters);

@@ -6,7 +6,8 @@
 // product per activation row), so the fp16 operand type costs no accuracy; the tensor-memory kernel of
 // wide passes reads xh alone. The sums feed the one extra MMA per superblock that applies the "- min"
 // term of Q4_K / Q5_K. Row-wise producer kernels (RMSNorm, SwiGLU product, gated norms, attention merge)
-// emit this form directly.
+// emit this form directly. xl == nullptr asks them for xh alone (and for no f32 result): a step whose every reader
+// is the tensor-memory kernel.
 #pragma once
 
 #include <cuda_fp16.h>
@@ -16,6 +17,7 @@
 namespace yk {
 
 struct XPrepOut {
+    __host__ __device__ bool hi_only() const { return xh && !xl; }
     __half * xh = nullptr;     // [rows][cols]
     __half * xl = nullptr;     // [rows][cols]
     __half2 * xs16 = nullptr;  // [rows][cols / 16]
@@ -46,6 +48,12 @@ __device__ __forceinline__ void xprep_store16(__half * dst_hi, __half * dst_lo, 
     const __half hi = __float2half_rn(s);
     const __half lo = __float2half_rn(s - __half2float(hi));
     *sum = __halves2half2(hi, lo);
+}
+
+// The hi halves alone of four consecutive values starting at a multiple of 4.
+__device__ __forceinline__ void xprep_store_hi4(__half * dst, float a, float b, float c, float d) {
+    const __half2 lo = __floats2half2_rn(a, b), hi = __floats2half2_rn(c, d);
+    *reinterpret_cast<uint2 *>(dst) = make_uint2(*reinterpret_cast<const uint32_t *>(&lo), *reinterpret_cast<const uint32_t *>(&hi));
 }
 
 // Both halves of one value.
