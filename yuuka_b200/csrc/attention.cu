@@ -10,6 +10,7 @@
 
 #include <cfloat>
 #include <cstdlib>
+#include <type_traits>
 
 #include "layers.cuh"
 #include "quant.cuh"
@@ -63,13 +64,14 @@ __global__ void __launch_bounds__(ATT_WARPS * 32) attention_partial_kernel(const
     const int seq = blockIdx.z;
     const int kvh = blockIdx.y % p.kv_heads, qt = blockIdx.y / p.kv_heads;
     const int split = blockIdx.x;
-    const int G = p.heads / p.kv_heads, N = p.rows.nodes;
+    const int G = p.heads / p.kv_heads, N = p.rows.nodes, live = rows_of_seq(p.rows, seq);
     const int sq = seq_of(p.rows, seq);
     const int pos0 = p.rows.pos0[sq];
-    const int total = pos0 + N;
+    const int total = pos0 + live;
     const int k_begin = split * p.key_split;
     const int k_end = min(total, k_begin + p.key_split);
-    const int nq = min(ATT_QT, G * N - qt * ATT_QT);
+    const int nq = min(ATT_QT, G * live - qt * ATT_QT);
+    if (k_begin >= k_end || nq <= 0) return;  // (the merge knows how many ranges hold keys)
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const float scale = (float)(1.0 / sqrt((double)HD));
 
@@ -192,29 +194,30 @@ __global__ void __launch_bounds__(ATT_WARPS * 32) attention_partial_kernel(const
 
 // ---------------------------------------------------------------------------
 // Tensor-core form of the partial kernel (mma.sync m16n8k16, fp16 operands, fp32 accumulate).
-// A CTA of twelve warps covers up to 48 query rows (three blocks of 16) of one KV head and one key
-// range; warp (rb, dq) owns row block rb and a quarter dq of the head dimension. The warps of a row
-// block build the 16 x 32 score tile together, each over its quarter of the head dimension (queries
-// as an fp16 hi + lo pair, so scores keep fp32-level accuracy; keys are exact when the pool stores
-// F16 rows, otherwise they are split the same way), add the four partial tiles in one order, hence
-// hold the same softmax statistics, and each multiplies the probabilities (fp16) with its own
-// 16 x 32 x HD/4 slice of V, fetched with ldmatrix.trans.
+// A CTA covers RB blocks of 16 query rows of one KV head and one key range, two warps per block: each owns half of the
+// head dimension, its queries in registers as fp16 hi + lo pairs (so scores keep fp32-level accuracy; keys are exact
+// when the pool stores F16 rows, otherwise they are split the same way). The two build the 16 x 32 score tile together,
+// each over its two quarters of the head dimension, exchange the sums of the quarters and add the four in one order,
+// hence hold the same softmax statistics, and each multiplies the probabilities (fp16) with its half of V.
+// K and V of an F16 pool arrive by cp.async, one or two tiles ahead.
+// What bounds it: a warp's chain of loads, products and exchange from tile to tile. The form before had four warps per
+// block, the queries in shared memory and the next tile in registers: 137 registers in twelve warps, one CTA per SM.
+// 32 sequences x 17 rows at contexts of 256 to 3072 (head 256): 356 -> 231 us with the merge.
 constexpr int AM_KT = 32;
-// Query rows per CTA: 16 per row block of four warps; three row blocks (a 9-row tree of four query heads per KV head
-// fits), four when a sequence has more than 48 query rows per KV head (64 cover a 16-row tree in one pass over the keys).
-constexpr int AM_RB_SMALL = 3, AM_RB_LARGE = 4;
+constexpr int AM_RB_MAX = 5;
 
-// Row blocks per CTA for q_rows query rows of one KV head: whichever of the two sizes walks the keys with fewer
-// row blocks in all (tiles x blocks per tile; the larger on a tie). 64 rows: one tile of four blocks; 68 rows (a
-// 17-row tree of four query heads): two tiles of three blocks rather than two of four.
+// Row blocks per CTA for q_rows query rows of one KV head: as many as there are when one CTA can hold them; beyond that
+// the size of four or five that walks the keys with fewer row blocks in all.
 static int attention_row_blocks(int q_rows) {
-    const int small = (q_rows + 16 * AM_RB_SMALL - 1) / (16 * AM_RB_SMALL) * AM_RB_SMALL;
-    const int large = (q_rows + 16 * AM_RB_LARGE - 1) / (16 * AM_RB_LARGE) * AM_RB_LARGE;
-    return small < large ? AM_RB_SMALL : AM_RB_LARGE;
+    const int blocks = (q_rows + 15) / 16;
+    if (blocks <= AM_RB_MAX) return blocks;
+    return (blocks + 4) / 5 * 5 < (blocks + 3) / 4 * 4 ? 5 : 4;
 }
+// The key ranges are cut for tiles of three or four row blocks, whichever needs fewer: the cut decides the order of the
+// sums, so it does not follow the row blocks a CTA happens to hold.
 int attention_query_tiles(int q_rows) {
-    const int per = 16 * attention_row_blocks(q_rows);
-    return (q_rows + per - 1) / per;
+    const int t3 = (q_rows + 47) / 48, t4 = (q_rows + 63) / 64;
+    return t3 * 3 < t4 * 4 ? t3 : t4;
 }
 
 __device__ __forceinline__ void mma16816h(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
@@ -233,63 +236,106 @@ __device__ __forceinline__ __half split_half(float v, __half & lo) {
     return hi;
 }
 
+__device__ __forceinline__ void ldmatrix4(uint32_t (&r)[4], const __half * p) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                 : "r"((uint32_t)__cvta_generic_to_shared(p)));
+}
+__device__ __forceinline__ void ldmatrix4_trans(uint32_t (&r)[4], const __half * p) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                 : "r"((uint32_t)__cvta_generic_to_shared(p)));
+}
+
+// Shared memory: stages of [K | K's low halves (KSPLIT) | V] tiles, then the exchange buffers
+constexpr int AM_SX = 48 * 32;  // floats per row block
+constexpr int attention_stages(bool ksplit, int rb) { return ksplit ? 1 : (rb <= 3 ? 2 : 3); }  // (up to three blocks: two CTAs per SM)
+constexpr size_t attention_stage_halves(int hd, bool ksplit) { return (size_t)(ksplit ? 3 : 2) * AM_KT * (hd + 8); }
+
 template <int HD, bool KSPLIT, int RB>
-__global__ void __launch_bounds__(RB * 128) attention_mma_kernel(const AttnParams p) {
-    pdl_entry();
-    constexpr int AM_ROWS = 16 * RB, AM_WARPS = 4 * RB;
+__global__ void __launch_bounds__(RB * 64, RB <= 3 ? 2 : 1) attention_mma_kernel(const AttnParams p) {
+    constexpr int AM_ROWS = 16 * RB, THREADS = RB * 64;
     constexpr int STR = HD + 8;   // halves per shared-memory row: 16 bytes of padding spread the banks
-    constexpr int DW = HD / 4;    // head dimensions per warp
+    constexpr int DW = HD / 2;    // head dimensions per warp
     constexpr int NT_O = DW / 8;  // 8-column output tiles per warp
+    constexpr int KQ = HD / 64;   // 16-dimension steps of a quarter of the head
+    constexpr int STAGES = attention_stages(KSPLIT, RB);
     extern __shared__ __align__(16) uint8_t smraw[];
-    __half * qhi = reinterpret_cast<__half *>(smraw);
-    __half * qlo = qhi + AM_ROWS * STR;
-    __half * ks = qlo + AM_ROWS * STR;
-    __half * kl = ks + AM_KT * STR;  // low parts of K (KSPLIT only)
-    __half * vs = KSPLIT ? kl + AM_KT * STR : kl;
-    float * sx = reinterpret_cast<float *>(vs + AM_KT * STR);  // [AM_WARPS][16][32] partial scores, see below
+    __half * stage0 = reinterpret_cast<__half *>(smraw);
+    constexpr size_t STAGE = attention_stage_halves(HD, KSPLIT);
+    constexpr int V_AT = (KSPLIT ? 2 : 1) * AM_KT * STR;
+    pdl_entry();
 
     const int seq = blockIdx.z;
     const int kvh = blockIdx.y % p.kv_heads, qt = blockIdx.y / p.kv_heads;
     const int split = blockIdx.x;
-    const int G = p.heads / p.kv_heads, N = p.rows.nodes;
+    const int G = p.heads / p.kv_heads, N = p.rows.nodes, live = rows_of_seq(p.rows, seq);
     const int sq = seq_of(p.rows, seq);
     const int pos0 = p.rows.pos0[sq];
-    const int total = pos0 + N;
+    const int total = pos0 + live;
     const int k_begin = split * p.key_split;
     const int k_end = min(total, k_begin + p.key_split);
-    const int nq = min(AM_ROWS, G * N - qt * AM_ROWS);
+    const int nq = min(AM_ROWS, G * live - qt * AM_ROWS);
+    if (k_begin >= k_end || nq <= 0) return;  // (the merge knows how many ranges hold keys)
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int g = lane >> 2, t = lane & 3;
-    const int rb = warp >> 2, dq = warp & 3;
+    const int rb = warp >> 1, hw = warp & 1;  // row block; half of the head dimension
     const float scale = (float)(1.0 / sqrt((double)HD));
 
-    // queries of this tile as fp16 hi / lo; rows beyond nq are zero
-    for (int i = threadIdx.x; i < AM_ROWS * (HD / 4); i += AM_WARPS * 32) {
-        const int qi = i / (HD / 4), c = i - qi * (HD / 4);
-        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (qi < nq) {
-            const int gq = qt * AM_ROWS + qi, node = gq / G, head = kvh * G + gq % G;
-            v = reinterpret_cast<const float4 *>(p.q + (int64_t)(seq * N + node) * p.ldq + (int64_t)head * 2 * HD)[c];
+    // (block sizes are powers of two in practice: a shift and a mask instead of two integer divisions per piece)
+    const int bsz = p.pool.block_size, bshift = (bsz & (bsz - 1)) == 0 ? __ffs(bsz) - 1 : -1;
+    const int32_t * table = p.pool.tables + (int64_t)sq * p.pool.table_stride;
+    auto row_offset = [&](int pos) {
+        const int bi = bshift >= 0 ? pos >> bshift : pos / bsz, within = bshift >= 0 ? pos & (bsz - 1) : pos - bi * bsz;
+        return ((int64_t)__ldg(table + bi) * bsz + within) * p.pool.row_bytes;
+    };
+    constexpr int PIECES = AM_KT * (HD / 8);  // 16-byte pieces (eight fp16 values) of a K or V tile
+    auto fetch = [&](int tile) {  // F16 pool: cp.async, zeros beyond the range
+        __half * st = stage0 + (size_t)(tile % STAGES) * STAGE;
+        const int k0 = k_begin + tile * AM_KT;
+#pragma unroll 4
+        for (int i = threadIdx.x; i < PIECES; i += THREADS) {
+            const int j = i / (HD / 8), c8 = i - j * (HD / 8), pos = k0 + j;
+            const bool in = pos < k_end;
+            const size_t off = in ? row_offset(pos) + (size_t)(kvh * HD + c8 * 8) * 2 : 0;
+            const uint32_t dst = (uint32_t)__cvta_generic_to_shared(st + j * STR + c8 * 8);
+            const int bytes = in ? 16 : 0;
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(p.pool.k + off), "r"(bytes) : "memory");
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst + V_AT * 2), "l"(p.pool.v + off), "r"(bytes) : "memory");
         }
-        __half l0, l1, l2, l3;
-        const __half h0 = split_half(v.x, l0), h1 = split_half(v.y, l1), h2 = split_half(v.z, l2), h3 = split_half(v.w, l3);
-        __half2 * dh = reinterpret_cast<__half2 *>(qhi + qi * STR + c * 4);
-        __half2 * dl = reinterpret_cast<__half2 *>(qlo + qi * STR + c * 4);
-        dh[0] = __halves2half2(h0, h1);
-        dh[1] = __halves2half2(h2, h3);
-        dl[0] = __halves2half2(l0, l1);
-        dl[1] = __halves2half2(l2, l3);
+    };
+    const int tiles = (k_end - k_begin + AM_KT - 1) / AM_KT;
+    if constexpr (!KSPLIT) {
+#pragma unroll
+        for (int s = 0; s < STAGES - 1; s++) {
+            if (s < tiles) fetch(s);
+            asm volatile("cp.async.commit_group;" ::: "memory");
+        }
     }
 
-    // the two query rows this lane holds in the accumulator layout: local rows rb*16 + g and + 8
+    // the two query rows of this lane (local rows rb * 16 + g and + 8): fragments of this warp's half of the head
+    // dimension, zeros beyond nq; the rows' ancestor masks
+    uint32_t qh[2 * KQ][4], ql[2 * KQ][4];
     uint64_t mask[2];
     int row_ok[2];
 #pragma unroll
     for (int h = 0; h < 2; h++) {
         const int qi = rb * 16 + g + 8 * h;
         row_ok[h] = qi < nq;
-        const int node = row_ok[h] ? (qt * AM_ROWS + qi) / G : 0;
+        const int gq = qt * AM_ROWS + (row_ok[h] ? qi : 0), node = gq / G, head = kvh * G + gq - node * G;
         mask[h] = row_ok[h] ? p.rows.anc_mask[seq * N + node] : 0ull;
+        const float * src = p.q + (int64_t)(seq * N + node) * p.ldq + (int64_t)head * 2 * HD + hw * DW + 2 * t;
+#pragma unroll
+        for (int kk = 0; kk < 2 * KQ; kk++)
+#pragma unroll
+            for (int e = 0; e < 2; e++) {
+                const float2 v = row_ok[h] ? *reinterpret_cast<const float2 *>(src + 16 * kk + 8 * e) : make_float2(0.f, 0.f);
+                __half lx, ly;
+                const __half hx = split_half(v.x, lx), hy = split_half(v.y, ly);
+                const __half2 hi = __halves2half2(hx, hy), lo = __halves2half2(lx, ly);
+                qh[kk][h + 2 * e] = *reinterpret_cast<const uint32_t *>(&hi);
+                ql[kk][h + 2 * e] = *reinterpret_cast<const uint32_t *>(&lo);
+            }
     }
     float m[2] = {-INFINITY, -INFINITY}, l[2] = {0.0f, 0.0f};
     float o[NT_O][4];
@@ -297,53 +343,24 @@ __global__ void __launch_bounds__(RB * 128) attention_mma_kernel(const AttnParam
     for (int nt = 0; nt < NT_O; nt++)
 #pragma unroll
         for (int c = 0; c < 4; c++) o[nt][c] = 0.0f;
+    float4 * sx = reinterpret_cast<float4 *>(reinterpret_cast<float *>(stage0 + STAGES * STAGE) + rb * AM_SX) + lane;
 
-    // F16 pool: the 16-byte pieces of the next key tile are fetched into registers while this one is multiplied
-    constexpr int PIECES = AM_KT * (HD / 8);
-    constexpr int PER = (PIECES + AM_WARPS * 32 - 1) / (AM_WARPS * 32);
-    uint4 nk[PER], nv[PER];
-    // (block sizes are powers of two in practice: a shift and a mask instead of two integer divisions per piece)
-    const int bsz = p.pool.block_size, bshift = (bsz & (bsz - 1)) == 0 ? __ffs(bsz) - 1 : -1;
-    auto fetch = [&](int k0) {
-#pragma unroll
-        for (int u = 0; u < PER; u++) {
-            const int i = threadIdx.x + u * AM_WARPS * 32;
-            const int j = i / (HD / 8), c8 = i - j * (HD / 8);
-            const int pos = k0 + j;
-            nk[u] = make_uint4(0, 0, 0, 0);
-            nv[u] = nk[u];
-            if (i < PIECES && pos < k_end) {
-                const int bi = bshift >= 0 ? pos >> bshift : pos / bsz, within = bshift >= 0 ? pos & (bsz - 1) : pos - bi * bsz;
-                const int block = p.pool.tables[(int64_t)sq * p.pool.table_stride + bi];
-                const int64_t off = ((int64_t)block * bsz + within) * p.pool.row_bytes;
-                nk[u] = *reinterpret_cast<const uint4 *>(p.pool.k + off + (size_t)(kvh * HD + c8 * 8) * 2);
-                nv[u] = *reinterpret_cast<const uint4 *>(p.pool.v + off + (size_t)(kvh * HD + c8 * 8) * 2);
-            }
-        }
-    };
-    if (!KSPLIT && k_begin < k_end) fetch(k_begin);
-
-    for (int k0 = k_begin; k0 < k_end; k0 += AM_KT) {
-        __syncthreads();  // the previous tile has been consumed (and, first time, the queries are in place)
-        if (!KSPLIT) {
-#pragma unroll
-            for (int u = 0; u < PER; u++) {
-                const int i = threadIdx.x + u * AM_WARPS * 32;
-                const int j = i / (HD / 8), c8 = i - j * (HD / 8);
-                if (i < PIECES) {
-                    *reinterpret_cast<uint4 *>(ks + j * STR + c8 * 8) = nk[u];
-                    *reinterpret_cast<uint4 *>(vs + j * STR + c8 * 8) = nv[u];
-                }
-            }
-            if (k0 + AM_KT < k_end) fetch(k0 + AM_KT);
+    for (int tile = 0; tile < tiles; tile++) {
+        const int k0 = k_begin + tile * AM_KT;
+        const __half * ks = stage0 + (size_t)(tile % STAGES) * STAGE;
+        if constexpr (!KSPLIT) {
+            asm volatile("cp.async.wait_group %0;" ::"n"(STAGES - 2) : "memory");
+            __syncthreads();  // the tile has landed, and the previous one has been consumed
+            if (tile + STAGES - 1 < tiles) fetch(tile + STAGES - 1);
+            asm volatile("cp.async.commit_group;" ::: "memory");
         } else {
-            for (int i = threadIdx.x; i < PIECES; i += AM_WARPS * 32) {
+            __syncthreads();
+            for (int i = threadIdx.x; i < PIECES; i += THREADS) {
                 const int j = i / (HD / 8), c8 = i - j * (HD / 8);
                 const int pos = k0 + j;
                 uint4 kh4 = make_uint4(0, 0, 0, 0), kl4 = kh4, vh4 = kh4;
                 if (pos < k_end) {
-                    const int block = p.pool.tables[(int64_t)sq * p.pool.table_stride + pos / p.pool.block_size];
-                    const int64_t off = ((int64_t)block * p.pool.block_size + pos % p.pool.block_size) * p.pool.row_bytes;
+                    const int64_t off = row_offset(pos);
                     float kw[8], vw[8];
                     kv_decode8(p.pool.k + off, p.pool.format, kvh * (HD / 8) + c8, kw);
                     kv_decode8(p.pool.v + off, p.pool.format, kvh * (HD / 8) + c8, vw);
@@ -357,67 +374,79 @@ __global__ void __launch_bounds__(RB * 128) attention_mma_kernel(const AttnParam
                     kl4 = *reinterpret_cast<const uint4 *>(ll);
                     vh4 = *reinterpret_cast<const uint4 *>(vv);
                 }
-                *reinterpret_cast<uint4 *>(ks + j * STR + c8 * 8) = kh4;
-                *reinterpret_cast<uint4 *>(kl + j * STR + c8 * 8) = kl4;
-                *reinterpret_cast<uint4 *>(vs + j * STR + c8 * 8) = vh4;
+                __half * at = stage0 + j * STR + c8 * 8;
+                *reinterpret_cast<uint4 *>(at) = kh4;
+                *reinterpret_cast<uint4 *>(at + AM_KT * STR) = kl4;
+                *reinterpret_cast<uint4 *>(at + V_AT) = vh4;
+            }
+            __syncthreads();
+        }
+        if (rb * 16 >= nq) continue;  // (both warps of the block)
+
+        // scores of the block's 16 rows against the 32 keys: this warp's two quarters of the head dimension
+        float s[2][4][4];
+#pragma unroll
+        for (int q = 0; q < 2; q++)
+#pragma unroll
+            for (int nt = 0; nt < 4; nt++)
+#pragma unroll
+                for (int c = 0; c < 4; c++) s[q][nt][c] = 0.0f;
+        const __half * krow = ks + (8 * (lane >> 4) + (lane & 7)) * STR + hw * DW + 8 * ((lane >> 3) & 1);
+#pragma unroll
+        for (int kk = 0; kk < 2 * KQ; kk++) {
+            const int q = kk / KQ;
+#pragma unroll
+            for (int n2 = 0; n2 < 2; n2++) {
+                uint32_t b[4];
+                ldmatrix4(b, krow + 16 * n2 * STR + 16 * kk);
+                mma16816h(s[q][2 * n2], qh[kk], b[0], b[1]);
+                mma16816h(s[q][2 * n2 + 1], qh[kk], b[2], b[3]);
+                mma16816h(s[q][2 * n2], ql[kk], b[0], b[1]);
+                mma16816h(s[q][2 * n2 + 1], ql[kk], b[2], b[3]);
+                if constexpr (KSPLIT) {
+                    uint32_t bl[4];
+                    ldmatrix4(bl, krow + AM_KT * STR + 16 * n2 * STR + 16 * kk);
+                    mma16816h(s[q][2 * n2], qh[kk], bl[0], bl[1]);
+                    mma16816h(s[q][2 * n2 + 1], qh[kk], bl[2], bl[3]);
+                }
             }
         }
-        __syncthreads();
-
-        // scores of this warp's 16 rows against the 32 keys
-        float s[4][4];
-#pragma unroll
-        for (int nt = 0; nt < 4; nt++)
-#pragma unroll
-            for (int c = 0; c < 4; c++) s[nt][c] = 0.0f;
-        const __half * qh_row = qhi + (rb * 16 + g) * STR + 2 * t;
-        const __half * ql_row = qlo + (rb * 16 + g) * STR + 2 * t;
-        // the four warps of a row block share the head dimensions of the score product: each multiplies its
-        // quarter, the partial tiles meet in shared memory and every warp adds them in the same order (each
-        // warp redoing the whole product kept the tensor pipe busy four times as long)
-        constexpr int KQ = HD / 16 / 4;
-#pragma unroll
-        for (int kq = 0; kq < KQ; kq++) {
-            const int kk = dq * KQ + kq;
-            uint32_t ah[4], al[4];
-            ah[0] = *reinterpret_cast<const uint32_t *>(qh_row + 16 * kk);
-            ah[1] = *reinterpret_cast<const uint32_t *>(qh_row + 8 * STR + 16 * kk);
-            ah[2] = *reinterpret_cast<const uint32_t *>(qh_row + 16 * kk + 8);
-            ah[3] = *reinterpret_cast<const uint32_t *>(qh_row + 8 * STR + 16 * kk + 8);
-            al[0] = *reinterpret_cast<const uint32_t *>(ql_row + 16 * kk);
-            al[1] = *reinterpret_cast<const uint32_t *>(ql_row + 8 * STR + 16 * kk);
-            al[2] = *reinterpret_cast<const uint32_t *>(ql_row + 16 * kk + 8);
-            al[3] = *reinterpret_cast<const uint32_t *>(ql_row + 8 * STR + 16 * kk + 8);
+        // the four quarters meet, always as ((q0 + q1) + q2) + q3
+        if (hw == 0) {
 #pragma unroll
             for (int nt = 0; nt < 4; nt++) {
-                const __half * kr = ks + (8 * nt + g) * STR + 16 * kk + 2 * t;
-                const uint32_t b0 = *reinterpret_cast<const uint32_t *>(kr), b1 = *reinterpret_cast<const uint32_t *>(kr + 8);
-                mma16816h(s[nt], ah, b0, b1);
-                mma16816h(s[nt], al, b0, b1);
-                if (KSPLIT) {
-                    const __half * lr = kl + (8 * nt + g) * STR + 16 * kk + 2 * t;
-                    mma16816h(s[nt], ah, *reinterpret_cast<const uint32_t *>(lr), *reinterpret_cast<const uint32_t *>(lr + 8));
-                }
+#pragma unroll
+                for (int c = 0; c < 4; c++) s[0][nt][c] = s[0][nt][c] + s[1][nt][c];
+                sx[nt * 32] = make_float4(s[0][nt][0], s[0][nt][1], s[0][nt][2], s[0][nt][3]);
+            }
+        } else {
+#pragma unroll
+            for (int nt = 0; nt < 4; nt++) {
+                sx[(4 + nt) * 32] = make_float4(s[0][nt][0], s[0][nt][1], s[0][nt][2], s[0][nt][3]);
+                sx[(8 + nt) * 32] = make_float4(s[1][nt][0], s[1][nt][1], s[1][nt][2], s[1][nt][3]);
             }
         }
-        {
-            float * mine = sx + warp * 512;
+        asm volatile("bar.sync %0, 64;" ::"r"(rb + 1) : "memory");
+        float sc[4][4];
 #pragma unroll
-            for (int nt = 0; nt < 4; nt++)
-#pragma unroll
-                for (int c = 0; c < 4; c++) mine[(nt * 4 + c) * 32 + lane] = s[nt][c];
-            asm volatile("bar.sync %0, 128;" ::"r"(rb + 1) : "memory");
-            const float * blk = sx + rb * 4 * 512;
-#pragma unroll
-            for (int nt = 0; nt < 4; nt++)
-#pragma unroll
-                for (int c = 0; c < 4; c++) {
-                    const int at = (nt * 4 + c) * 32 + lane;
-                    s[nt][c] = ((blk[at] + blk[512 + at]) + blk[1024 + at]) + blk[1536 + at];
-                }
+        for (int nt = 0; nt < 4; nt++) {
+            if (hw == 0) {
+                const float4 q2 = sx[(4 + nt) * 32], q3 = sx[(8 + nt) * 32];
+                sc[nt][0] = (s[0][nt][0] + q2.x) + q3.x;
+                sc[nt][1] = (s[0][nt][1] + q2.y) + q3.y;
+                sc[nt][2] = (s[0][nt][2] + q2.z) + q3.z;
+                sc[nt][3] = (s[0][nt][3] + q2.w) + q3.w;
+            } else {
+                const float4 q01 = sx[nt * 32];
+                sc[nt][0] = (q01.x + s[0][nt][0]) + s[1][nt][0];
+                sc[nt][1] = (q01.y + s[0][nt][1]) + s[1][nt][1];
+                sc[nt][2] = (q01.z + s[0][nt][2]) + s[1][nt][2];
+                sc[nt][3] = (q01.w + s[0][nt][3]) + s[1][nt][3];
+            }
         }
-        // mask, online softmax; s[nt][0,1] -> row g, keys 8 nt + 2 t + {0,1}; s[nt][2,3] -> row g + 8
+        // mask, online softmax; sc[nt][0,1] -> row g, keys 8 nt + 2 t + {0,1}; sc[nt][2,3] -> row g + 8
         uint32_t pa[2][4];  // probabilities as A fragments of the two 16-key steps
+        float corr[2];
         // a tile that lies entirely in the committed context is visible to every row: no mask, no range test
         const bool plain_tile = k0 + AM_KT <= min(pos0, k_end);
 #pragma unroll
@@ -429,7 +458,7 @@ __global__ void __launch_bounds__(RB * 128) attention_mma_kernel(const AttnParam
                 for (int nt = 0; nt < 4; nt++)
 #pragma unroll
                     for (int e = 0; e < 2; e++) {
-                        sv[nt][e] = row_ok[h] ? s[nt][2 * h + e] * scale : -INFINITY;
+                        sv[nt][e] = row_ok[h] ? sc[nt][2 * h + e] * scale : -INFINITY;
                         mx = fmaxf(mx, sv[nt][e]);
                     }
             } else {
@@ -439,16 +468,16 @@ __global__ void __launch_bounds__(RB * 128) attention_mma_kernel(const AttnParam
                     for (int e = 0; e < 2; e++) {
                         const int pos = k0 + 8 * nt + 2 * t + e;
                         const bool vis = pos < k_end && row_ok[h] && (pos < pos0 || ((mask[h] >> (pos - pos0)) & 1ull));
-                        sv[nt][e] = vis ? s[nt][2 * h + e] * scale : -INFINITY;
+                        sv[nt][e] = vis ? sc[nt][2 * h + e] * scale : -INFINITY;
                         mx = fmaxf(mx, sv[nt][e]);
                     }
             }
             mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
             mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
             const float m_new = fmaxf(m[h], mx);
-            float corr = 1.0f, sum = 0.0f;
+            float sum = 0.0f;
             float pr[4][2];
-            if (m_new != -INFINITY) corr = __expf(m[h] - m_new);
+            corr[h] = m_new != -INFINITY ? __expf(m[h] - m_new) : 1.0f;
 #pragma unroll
             for (int nt = 0; nt < 4; nt++)
 #pragma unroll
@@ -460,31 +489,34 @@ __global__ void __launch_bounds__(RB * 128) attention_mma_kernel(const AttnParam
                 }
             sum += __shfl_xor_sync(0xffffffffu, sum, 1);
             sum += __shfl_xor_sync(0xffffffffu, sum, 2);
-            l[h] = l[h] * corr + sum;
+            l[h] = l[h] * corr[h] + sum;
             m[h] = m_new;
-#pragma unroll
-            for (int nt = 0; nt < NT_O; nt++) {
-                o[nt][2 * h] *= corr;
-                o[nt][2 * h + 1] *= corr;
-            }
             // A fragment registers: [0] row g / [1] row g+8 for keys 2t..; [2], [3] the same rows, keys 2t+8..
             pa[0][h] = pack_h2(pr[0][0], pr[0][1]);
             pa[0][2 + h] = pack_h2(pr[1][0], pr[1][1]);
             pa[1][h] = pack_h2(pr[2][0], pr[2][1]);
             pa[1][2 + h] = pack_h2(pr[3][0], pr[3][1]);
         }
-        // O += P V on this warp's DW dimensions
-#pragma unroll
-        for (int kk = 0; kk < 2; kk++) {
-            const __half * vrow = vs + (16 * kk + (lane & 15)) * STR + dq * DW;
+        if (__any_sync(0xffffffffu, corr[0] != 1.0f || corr[1] != 1.0f)) {  // (a maximum moved)
 #pragma unroll
             for (int nt = 0; nt < NT_O; nt++) {
-                uint32_t b0, b1;
-                const uint32_t addr = (uint32_t)__cvta_generic_to_shared(vrow + 8 * nt);
-                asm volatile("ldmatrix.sync.aligned.m8n8.x2.trans.shared.b16 {%0, %1}, [%2];" : "=r"(b0), "=r"(b1) : "r"(addr));
-                mma16816h(o[nt], pa[kk], b0, b1);
+                o[nt][0] *= corr[0];
+                o[nt][1] *= corr[0];
+                o[nt][2] *= corr[1];
+                o[nt][3] *= corr[1];
             }
         }
+        // O += P V on this warp's half of the head dimension
+        const __half * vrow = ks + V_AT + (lane & 15) * STR + hw * DW + 8 * (lane >> 4);
+#pragma unroll
+        for (int kk = 0; kk < 2; kk++)
+#pragma unroll
+            for (int nt = 0; nt < NT_O; nt += 2) {
+                uint32_t b[4];
+                ldmatrix4_trans(b, vrow + 16 * kk * STR + 8 * nt);
+                mma16816h(o[nt], pa[kk], b[0], b[1]);
+                mma16816h(o[nt + 1], pa[kk], b[2], b[3]);
+            }
     }
 
 #pragma unroll
@@ -495,9 +527,9 @@ __global__ void __launch_bounds__(RB * 128) attention_mma_kernel(const AttnParam
 #pragma unroll
         for (int nt = 0; nt < NT_O; nt++) {
             float2 v = make_float2(o[nt][2 * h], o[nt][2 * h + 1]);
-            *reinterpret_cast<float2 *>(dst + dq * DW + 8 * nt + 2 * t) = v;
+            *reinterpret_cast<float2 *>(dst + hw * DW + 8 * nt + 2 * t) = v;
         }
-        if (dq == 0 && t == 0) {
+        if (hw == 0 && t == 0) {
             dst[HD] = m[h];
             dst[HD + 1] = l[h];
         }
@@ -514,14 +546,16 @@ constexpr int MERGE_MAX_SPLITS = 1024;
 
 template <int HD>
 __global__ void __launch_bounds__(HD / 4 < 32 ? 32 : HD / 4) attention_merge_kernel(float * __restrict__ out, int ldo, const float * __restrict__ partial,
-                                                                 const float * __restrict__ q, int ldq, int heads, int splits,
-                                                                 XPrepOut prep) {
+                                                                 const float * __restrict__ q, int ldq, int heads, int all_splits,
+                                                                 int key_split, const RowMeta rows, XPrepOut prep) {
     pdl_entry();
     __shared__ float w_s[MERGE_MAX_SPLITS], l_s[MERGE_MAX_SPLITS];
     __shared__ float inv_l;
     const int r = blockIdx.x / heads, head = blockIdx.x - r * heads;
     const int tid = threadIdx.x;
-    const float * base = partial + ((int64_t)r * heads + head) * splits * (HD + 2);
+    // the key ranges that hold keys of the row's sequence; the others have written nothing
+    const int seq = r / rows.nodes, splits = (rows.pos0[seq_of(rows, seq)] + rows_of_seq(rows, seq) + key_split - 1) / key_split;
+    const float * base = partial + ((int64_t)r * heads + head) * all_splits * (HD + 2);
     constexpr int THREADS = HD / 4 < 32 ? 32 : HD / 4;  // whole warps; threads beyond HD / 4 only help with the statistics
     const bool has_dims = tid < HD / 4;
     // the split's running maximum and sum, all splits in flight at once (one lane summing them straight from
@@ -615,16 +649,24 @@ static int launch_attention_hd(cudaStream_t s, float * out, int ldo, const float
     static const bool use_mma = [] { const char * e = getenv("YUUKA_CUDA_ATTN_FP32"); return !(e && e[0] == '1'); }();
     if (use_mma) {
         // tensor-core partials; keys are taken as they are from an F16 pool and split into hi + lo otherwise
-        const bool ksplit = pool.format != YUUKA_KV_F16;
-        const int qtiles = attention_query_tiles(G * rows.nodes);
-        const int rb = attention_row_blocks(G * rows.nodes);
-        const size_t smem = sizeof(__half) * (size_t)(HD + 8) * (2 * 16 * rb + (ksplit ? 3 : 2) * AM_KT) +
-                            sizeof(float) * 4 * rb * 512;
-        auto kern = rb == AM_RB_LARGE ? (ksplit ? attention_mma_kernel<HD, true, AM_RB_LARGE> : attention_mma_kernel<HD, false, AM_RB_LARGE>)
-                                      : (ksplit ? attention_mma_kernel<HD, true, AM_RB_SMALL> : attention_mma_kernel<HD, false, AM_RB_SMALL>);
-        YK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        dim3 grid(sc.splits, kv_heads * qtiles, rows.batch);
-        launch_k(kern, grid, rb * 128, smem, s, p);
+        const int rb = attention_row_blocks(G * rows.nodes), qtiles = (G * rows.nodes + 16 * rb - 1) / (16 * rb);
+        auto launch = [&](auto ksplit) {
+            constexpr bool KS = decltype(ksplit)::value;
+            auto with = [&](auto kern) {
+                const size_t smem = sizeof(__half) * attention_stages(KS, rb) * attention_stage_halves(HD, KS) + sizeof(float) * AM_SX * rb;
+                YK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+                launch_k(kern, dim3(sc.splits, kv_heads * qtiles, rows.batch), rb * 64, smem, s, p);
+            };
+            switch (rb) {
+            case 1: with(attention_mma_kernel<HD, KS, 1>); break;
+            case 2: with(attention_mma_kernel<HD, KS, 2>); break;
+            case 3: with(attention_mma_kernel<HD, KS, 3>); break;
+            case 4: with(attention_mma_kernel<HD, KS, 4>); break;
+            default: with(attention_mma_kernel<HD, KS, 5>); break;
+            }
+        };
+        if (pool.format != YUUKA_KV_F16) launch(std::true_type());
+        else launch(std::false_type());
         YK_CUDA(cudaGetLastError());
     } else {
         const int qtiles = (G * rows.nodes + ATT_QT - 1) / ATT_QT;
@@ -637,8 +679,8 @@ static int launch_attention_hd(cudaStream_t s, float * out, int ldo, const float
     }
     YK_REQUIRE(sc.splits <= MERGE_MAX_SPLITS, YUUKA_ERR_UNSUPPORTED, "attention: %d key splits exceed the merge kernel's %d",
                sc.splits, MERGE_MAX_SPLITS);
-    launch_k(attention_merge_kernel<HD>, rows.batch * rows.nodes * heads, HD / 4 < 32 ? 32 : HD / 4, 0, s, out, ldo, sc.partial, q, ldq, heads,
-             sc.splits, prep);
+    launch_k(attention_merge_kernel<HD>, rows_of_step(rows) * heads, HD / 4 < 32 ? 32 : HD / 4, 0, s, out, ldo, sc.partial, q, ldq, heads,
+             sc.splits, sc.key_split, rows, prep);
     YK_CUDA(cudaGetLastError());
     return 2;
 }

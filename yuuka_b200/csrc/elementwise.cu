@@ -289,33 +289,42 @@ struct PrepParams {
     float * k; int ldk;
     const float * v; int ldv;
     const float * q_norm; const float * k_norm;
-    int heads, kv_heads, hd, rope_dim;
+    int heads, kv_heads, rope_dim;
     const float2 * rope_cs;  // [rows][rope_dim / 2] (cos, sin), see rope_table_kernel
     float eps;
     RowMeta rows;
     KvPool pool;
 };
 
-// rmsNormInPlace (forward.go:472-482) on hd values handled by one warp, then
-// RoPE over the first rope_dim dims (forward.go:495-514) with the row's
-// (cos, sin) table.
-__device__ void norm_rope_head(float * x, const float * w, int hd, int rope_dim, const float2 * cs, float eps) {
+// rmsNormInPlace (forward.go:472-482) on the HD values of one head, HD / 32 per lane of a warp (lane + 32 k), then
+// RoPE over the first rope_dim dims (forward.go:495-514) with the row's (cos, sin) table. The pairs of the rotation meet in
+// shared memory (`sm`, HD floats of the warp's own).
+template <int HD>
+__device__ __forceinline__ void norm_rope_head(float (&x)[HD / 32], const float * w, int rope_dim, const float2 * cs, float eps, float * sm) {
     const int lane = threadIdx.x & 31;
     double sum = 0;
-    for (int i = lane; i < hd; i += 32) sum += (double)x[i] * (double)x[i];
+#pragma unroll
+    for (int k = 0; k < HD / 32; k++) sum += (double)x[k] * (double)x[k];
     sum = warp_sum_d(sum);
-    float mean = (float)(sum / (double)hd);
-    float scale = (float)(1.0 / sqrt((double)(mean + eps)));
-    for (int i = lane; i < hd; i += 32) x[i] *= scale * w[i];
+    const float mean = (float)(sum / (double)HD);
+    const float scale = (float)(1.0 / sqrt((double)(mean + eps)));
+#pragma unroll
+    for (int k = 0; k < HD / 32; k++) {
+        x[k] *= scale * w[lane + 32 * k];
+        sm[lane + 32 * k] = x[k];
+    }
     __syncwarp();
     const int half = rope_dim / 2;
     for (int i = lane; i < half; i += 32) {
         const float c = cs[i].x, s = cs[i].y;
-        float x0 = x[i], x1 = x[i + half];
-        x[i] = x0 * c - x1 * s;
-        x[i + half] = x0 * s + x1 * c;
+        float x0 = sm[i], x1 = sm[i + half];
+        sm[i] = x0 * c - x1 * s;
+        sm[i + half] = x0 * s + x1 * c;
     }
     __syncwarp();
+#pragma unroll
+    for (int k = 0; k < HD / 32; k++)
+        if (32 * k < rope_dim) x[k] = sm[lane + 32 * k];
 }
 
 __device__ __forceinline__ int64_t kv_row_offset(const KvPool & pool, int seq, int slot) {
@@ -338,24 +347,27 @@ __global__ void rope_table_kernel(float2 * __restrict__ cs, RowMeta rows, int ro
 }
 
 void launch_rope_table(cudaStream_t s, float2 * cs, const RowMeta & rows, int rope_dim, double rope_base) {
-    launch_k(rope_table_kernel, rows.batch * rows.nodes, 64, 0, s, cs, rows, rope_dim, rope_base);
+    launch_k(rope_table_kernel, rows_of_step(rows), 64, 0, s, cs, rows, rope_dim, rope_base);
     YK_CUDA(cudaGetLastError());
 }
 
-// KVFormat.EncodeRow (model/qwen35/kv_format.go:75-131) for the n values of one head (n a multiple of
-// 32), by one warp; dst is the row in the pool, first the head's first element. Q8_0 blocks are 32
-// values, so a head's blocks are its own.
-__device__ void kv_encode_head(uint8_t * row, int format, const float * src, int first, int n) {
+// KVFormat.EncodeRow (model/qwen35/kv_format.go:75-131) for the HD values of one head (lane + 32 k), by one warp; dst is
+// the row in the pool, first the head's first element. Q8_0 blocks are 32 values, so a head's blocks are its own.
+template <int HD>
+__device__ __forceinline__ void kv_encode_head(uint8_t * row, int format, const float (&x)[HD / 32], int first) {
     const int lane = threadIdx.x & 31;
     if (format == YUUKA_KV_F32) {
-        float * d = reinterpret_cast<float *>(row) + first;
-        for (int i = lane; i < n; i += 32) d[i] = src[i];
+        float * d = reinterpret_cast<float *>(row) + first + lane;
+#pragma unroll
+        for (int k = 0; k < HD / 32; k++) d[32 * k] = x[k];
     } else if (format == YUUKA_KV_F16) {
-        uint16_t * d = reinterpret_cast<uint16_t *>(row) + first;
-        for (int i = lane; i < n; i += 32) d[i] = f32_to_f16_ref(src[i]);
+        uint16_t * d = reinterpret_cast<uint16_t *>(row) + first + lane;
+#pragma unroll
+        for (int k = 0; k < HD / 32; k++) d[32 * k] = f32_to_f16_ref(x[k]);
     } else {
-        for (int blk = 0; blk < n / 32; blk++) {
-            const float v = src[blk * 32 + lane];
+#pragma unroll
+        for (int blk = 0; blk < HD / 32; blk++) {
+            const float v = x[blk];
             float amax = fabsf(v);
 #pragma unroll
             for (int o = 16; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
@@ -370,39 +382,45 @@ __device__ void kv_encode_head(uint8_t * row, int format, const float * src, int
 }
 
 // grid (rows, ceil((heads + 2 kv_heads) / 4)), one warp per unit of work: a query head (norm + RoPE in
-// place), a key head (norm + RoPE, then its slice of the pool row) or a value head (its slice of the pool row).
+// place), a key head (norm + RoPE, into its slice of the pool row) or a value head (its slice of the pool row). A head stays
+// in the warp's registers from load to store.
+template <int HD>
 __global__ void __launch_bounds__(128) attn_prep_kernel(const PrepParams p) {
     pdl_entry();
+    __shared__ float stage[4][HD];
     const int r = blockIdx.x;
     const int seq = r / p.rows.nodes, node = r - seq * p.rows.nodes;
     const int sq = seq_of(p.rows, seq);
-    const int unit = blockIdx.y * (blockDim.x >> 5) + (threadIdx.x >> 5);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, unit = blockIdx.y * 4 + warp;
     if (unit >= p.heads + 2 * p.kv_heads) return;
     const float2 * cs = p.rope_cs + (int64_t)r * (p.rope_dim / 2);
-    // every row is stored at slot pos0 + node; the commit moves accepted rows of
-    // a tree to their final positions
-    if (unit < p.heads) {
-        norm_rope_head(p.q + (int64_t)r * p.ldq + (int64_t)unit * 2 * p.hd, p.q_norm, p.hd, p.rope_dim, cs, p.eps);
-    } else if (unit < p.heads + p.kv_heads) {
-        const int h = unit - p.heads;
-        float * k = p.k + (int64_t)r * p.ldk + (int64_t)h * p.hd;
-        norm_rope_head(k, p.k_norm, p.hd, p.rope_dim, cs, p.eps);
-        const int64_t off = kv_row_offset(p.pool, sq, p.rows.pos0[sq] + node);
-        kv_encode_head(p.pool.k + off, p.pool.format, k, h * p.hd, p.hd);
+    const bool is_q = unit < p.heads, is_k = !is_q && unit < p.heads + p.kv_heads;
+    const int h = is_q ? unit : (is_k ? unit - p.heads : unit - p.heads - p.kv_heads);
+    const float * src = is_q ? p.q + (int64_t)r * p.ldq + (int64_t)h * 2 * HD
+                             : (is_k ? p.k + (int64_t)r * p.ldk + (int64_t)h * HD : p.v + (int64_t)r * p.ldv + (int64_t)h * HD);
+    float x[HD / 32];
+#pragma unroll
+    for (int k = 0; k < HD / 32; k++) x[k] = src[lane + 32 * k];
+    if (is_q || is_k) norm_rope_head<HD>(x, is_q ? p.q_norm : p.k_norm, p.rope_dim, cs, p.eps, stage[warp]);
+    if (is_q) {
+        float * dst = p.q + (int64_t)r * p.ldq + (int64_t)h * 2 * HD;
+#pragma unroll
+        for (int k = 0; k < HD / 32; k++) dst[lane + 32 * k] = x[k];
     } else {
-        const int h = unit - p.heads - p.kv_heads;
+        // every row is stored at slot pos0 + node; the commit moves accepted rows of a tree to their final positions
         const int64_t off = kv_row_offset(p.pool, sq, p.rows.pos0[sq] + node);
-        kv_encode_head(p.pool.v + off, p.pool.format, p.v + (int64_t)r * p.ldv + (int64_t)h * p.hd, h * p.hd, p.hd);
+        kv_encode_head<HD>((is_k ? p.pool.k : p.pool.v) + off, p.pool.format, x, h * HD);
     }
 }
 
 void launch_attn_prep(cudaStream_t s, float * q, int ldq, float * k, int ldk, const float * v, int ldv,
                       const float * q_norm, const float * k_norm, int heads, int kv_heads, int head_dim, int rope_dim,
                       const float2 * rope_cs, float eps, const RowMeta & rows, const KvPool & pool) {
-    YK_REQUIRE(head_dim % 32 == 0 && rope_cs, YUUKA_ERR_UNSUPPORTED, "attn_prep: head width %d is not a multiple of 32", head_dim);
-    PrepParams p{q, ldq, k, ldk, v, ldv, q_norm, k_norm, heads, kv_heads, head_dim, rope_dim, rope_cs, eps, rows, pool};
-    dim3 grid(rows.batch * rows.nodes, (heads + 2 * kv_heads + 3) / 4);
-    launch_k(attn_prep_kernel, grid, 128, 0, s, p);
+    YK_REQUIRE((head_dim == 64 || head_dim == 128 || head_dim == 256) && rope_cs, YUUKA_ERR_UNSUPPORTED,
+               "attn_prep: head_dim %d is not 64, 128 or 256", head_dim);
+    PrepParams p{q, ldq, k, ldk, v, ldv, q_norm, k_norm, heads, kv_heads, rope_dim, rope_cs, eps, rows, pool};
+    dim3 grid(rows_of_step(rows), (heads + 2 * kv_heads + 3) / 4);
+    launch_k(head_dim == 64 ? attn_prep_kernel<64> : (head_dim == 128 ? attn_prep_kernel<128> : attn_prep_kernel<256>), grid, 128, 0, s, p);
     YK_CUDA(cudaGetLastError());
 }
 

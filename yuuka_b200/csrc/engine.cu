@@ -767,10 +767,23 @@ enum LogitRows { LOGITS_NONE, LOGITS_LAST, LOGITS_ALL };
 
 // Prompt tokens run through the step kernels in chains of up to this many rows (the row masks are 64 bits
 // wide); from 48 rows on the GEMMs take the tensor-memory route.
+// Key ranges of a step's attention. About one CTA per SM at capacity (measured at a 1500-token context: 3.11 ms per step,
+// against 3.16 with two or four per SM: fewer partials for the merge kernel outweigh the shorter key ranges). Many sequences
+// of different lengths: key ranges of at most 512 keys, so that the CTAs of a long context spread over the machine instead
+// of one of them walking it alone (ranges beyond a sequence's end exit at once).
+int attention_splits(const yuuka_session * s, int batch, int nodes, int max_total) {
+    const yuuka_model_config & c = s->model->cfg;
+    const int sms = s->model->dev->sm_count, base = c.kv_heads * attention_query_tiles(c.heads / c.kv_heads * nodes) * batch;
+    int splits = (sms + base - 1) / base;
+    if (base >= sms && splits < (max_total + 511) / 512) splits = (max_total + 511) / 512;
+    const int most = (max_total + 31) / 32;
+    if (splits > most) splits = most;
+    return splits < 1 ? 1 : splits;
+}
+
 // A prompt runs in passes of up to CHAIN_ROWS rows: the GEMMs and row-wise kernels take the whole pass (the
-// tensor-memory GEMM route decodes a weight tile once for up to 512 rows), the sequential mixers (delta-net
-// scan + state commit, attention front end + attention) walk it in sub-chunks of CHAIN_SUB rows, the limit
-// of their per-step row bookkeeping (64-bit ancestor masks).
+// tensor-memory GEMM route decodes a weight tile once for up to 512 rows), the mixers work on it in sub-chunks of
+// CHAIN_SUB rows, the limit of their per-step row bookkeeping (64-bit ancestor masks).
 constexpr int CHAIN_ROWS = 512;
 constexpr int CHAIN_SUB = 64;
 constexpr int CHAIN_MAX_SUBS = CHAIN_ROWS / CHAIN_SUB;
@@ -830,8 +843,9 @@ void run_step(yuuka_session * s, int seq0, int batch, int nodes, uint32_t mode, 
         launch_embedding(st, s->x, H, m->embedding.ptr, m->embedding.dtype, H, c.vocab, s->d_tokens, R);
         s->launches++;
         if (s->rope_cs) {
-            // (a wide pass: every sub-chunk counts positions from its own start; rows past the end are scratch)
+            // (a wide pass: every sub-chunk counts positions from its own start)
             RowMeta rr = sub > 0 ? RowMeta{s->d_tokens, s->d_parent, s->d_depth, s->d_anc, s->d_pos_sub, n_sub, sub} : rows;
+            if (sub > 0) rr.limit = R;
             launch_rope_table(st, s->rope_cs, rr, c.rope_dim, c.rope_freq_base);
             s->launches++;
         }
@@ -940,47 +954,30 @@ void run_step(yuuka_session * s, int seq0, int batch, int nodes, uint32_t mode, 
             pool.row_bytes = s->kv_row_bytes;
             pool.tables = s->d_tables + (int64_t)seq0 * s->table_stride;
             pool.table_stride = s->table_stride;
-            mark(s, YUUKA_OP_ATTN_PREP);
-            if (sub == 0) {
-                launch_attn_prep(st, qb, nq, kb, nq, vb, nq, L.q_norm, L.k_norm, c.heads, c.kv_heads, c.head_dim, c.rope_dim,
-                                 s->rope_cs, c.rms_eps, rows, pool);
-                s->launches++;
+            // The sub-chunks of a wide pass go as sequences over one block table: each has its own first position, so a row
+            // sees what it would see if they ran one after another (512 rows: three launches instead of 24).
+            RowMeta ra = rows;
+            if (sub > 0) {
+                ra.pos0 = s->d_pos_sub;
+                ra.batch = n_sub;
+                ra.nodes = sub;
+                ra.limit = R;
+                pool.table_stride = 0;
             }
+            mark(s, YUUKA_OP_ATTN_PREP);
+            launch_attn_prep(st, qb, nq, kb, nq, vb, nq, L.q_norm, L.k_norm, c.heads, c.kv_heads, c.head_dim, c.rope_dim,
+                             s->rope_cs, c.rms_eps, ra, pool);
+            s->launches++;
             AttnScratch sc;
-            const int G = c.heads / c.kv_heads;
-            const int qtiles = attention_query_tiles(G * (sub > 0 ? sub : nodes));
-            const int base = c.kv_heads * qtiles * batch;
-            // about one CTA per SM at capacity (measured at a 1500-token context: 3.11 ms per step, against 3.16 with
-            // two or four per SM: fewer partials for the merge kernel outweigh the shorter key ranges)
-            int splits = (m->dev->sm_count + base - 1) / base;
-            // many sequences of different lengths: key ranges of at most 512 keys, so that the CTAs of a long context
-            // spread over the machine instead of one of them walking it alone (ranges beyond a sequence's end exit at once)
-            if (base >= m->dev->sm_count && splits < (max_total + 511) / 512) splits = (max_total + 511) / 512;
-            int max_splits = (max_total + 31) / 32;
-            if (splits > max_splits) splits = max_splits;
-            if (splits < 1) splits = 1;
+            const int splits = attention_splits(s, sub > 0 ? 1 : batch, sub > 0 ? sub : nodes, max_total);
             sc.key_split = (((max_total + splits - 1) / splits + 31) / 32) * 32;
             sc.splits = (max_total + sc.key_split - 1) / sc.key_split;
             sc.partial = s->attn_partial;
-            YK_REQUIRE(attention_scratch_floats(sub > 0 ? sub : R, c.heads, c.head_dim, sc.splits) <= s->attn_partial_floats,
+            YK_REQUIRE(attention_scratch_floats(R, c.heads, c.head_dim, sc.splits) <= s->attn_partial_floats,
                        YUUKA_ERR_INTERNAL, "attention scratch is too small");
             mark(s, YUUKA_OP_ATTENTION);
-            if (sub == 0) {
-                s->launches += launch_attention(st, s->attn_out, o_dim, qb, nq, c.heads, c.kv_heads, c.head_dim, rows, pool,
-                                                max_total, sc, step_prep(s, s->prep_attn));
-            } else {
-                // a sub-chunk's K/V rows are in the pool before the next sub-chunk's queries look for them
-                const int half = c.rope_dim / 2;
-                for (int k = 0; k < n_sub; k++) {
-                    const int64_t r0 = (int64_t)k * sub;
-                    const RowMeta rk = sub_rows(k);
-                    launch_attn_prep(st, qb + r0 * nq, nq, kb + r0 * nq, nq, vb + r0 * nq, nq, L.q_norm, L.k_norm, c.heads,
-                                     c.kv_heads, c.head_dim, c.rope_dim, s->rope_cs + r0 * half, c.rms_eps, rk, pool);
-                    const XPrepOut pk = prep_rows(step_prep(s, s->prep_attn), r0, o_dim);
-                    s->launches += 1 + launch_attention(st, s->attn_out + r0 * o_dim, o_dim, qb + r0 * nq, nq, c.heads, c.kv_heads,
-                                                        c.head_dim, rk, pool, max_total, sc, pk);
-                }
-            }
+            s->launches += launch_attention(st, s->attn_out, o_dim, qb, nq, c.heads, c.kv_heads, c.head_dim, ra, pool, max_total, sc,
+                                            step_prep(s, s->prep_attn));
             gemm_residual_norm(s, L.o, s->attn_out, o_dim, s->prep_attn, R, L.post_norm);
         }
         if (c.expert_count > 0) {
@@ -1524,8 +1521,10 @@ yuuka_status yuuka_session_create(yuuka_model * model, const yuuka_session_confi
                     if (splits < by_length) splits = by_length;
                     return (size_t)bx * nx * c.heads * splits * (size_t)(c.head_dim + 2);
                 };
-                const size_t a = need(B, N), b = need(1, s->chain_rows);
-                s->attn_partial_floats = a > b ? a : b;
+                s->attn_partial_floats = std::max(need(B, N), need(1, std::min(s->chain_rows, CHAIN_SUB)));
+                if (s->chain_rows > CHAIN_SUB)  // a wide prompt pass: all its rows at once
+                    s->attn_partial_floats = std::max(s->attn_partial_floats,
+                                                      attention_scratch_floats(s->chain_rows, c.heads, c.head_dim, attention_splits(s, 1, CHAIN_SUB, sc.capacity)));
             }
             s->attn_partial = dalloc<float>(s->attn_partial_floats, s->owned, false);
             // split-K scratch for every matrix shape of the step and of a prompt pass: the register-fed route

@@ -24,8 +24,15 @@ struct RowMeta {
     // [rows] the nodes of each sequence depth first (parents before children, children in row order), for steps whose
     // rows may branch (chains == 0); null otherwise
     const int32_t * order = nullptr;
+    // rows of the step where the last sequence has fewer than `nodes` (the sub-chunks of a wide prompt pass seen as
+    // sequences); 0: batch * nodes
+    int limit = 0;
 };
+inline int rows_of_step(const RowMeta & rows) { return rows.limit ? rows.limit : rows.batch * rows.nodes; }
 #ifdef __CUDACC__
+__device__ __forceinline__ int rows_of_seq(const RowMeta & rows, int slot) {
+    return rows.limit ? min(rows.nodes, rows.limit - slot * rows.nodes) : rows.nodes;
+}
 __device__ __forceinline__ int seq_of(const RowMeta & rows, int slot) { return rows.seq_map ? rows.seq_map[slot] : slot; }
 #endif
 
