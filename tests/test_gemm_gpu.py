@@ -173,3 +173,21 @@ def test_rejections(dev):
         cuda.gemm_quant(stream, b, b, b, 256, 8, 1, 99)
     b.free()
     stream.destroy()
+
+
+@pytest.mark.parametrize("dtype", [synth.Q4_K, synth.Q6_K, synth.Q8_0, synth.Q5_K])
+@pytest.mark.parametrize("n_out,n_in,rows", [
+    (24, 256, 17),                                                   # fewer weight rows than a CTA takes, one superblock
+    (520, 2560, 24), (520, 2560, 25), (520, 2560, 33), (520, 2560, 37), (520, 2560, 41),   # every count of product tiles
+    (2560, 4096, 36), (2560, 9216, 47), (2560, 9216, 32),            # ranges of K on different CTAs
+    (19000, 512, 40),                                                # more work than CTAs
+])
+def test_rows_beyond_one_pass_equal_passes_of_sixteen(dev, dtype, n_out, n_in, rows):
+    """17 to 47 rows decode the weights once; the sums are those of 16-row passes, to the last bit."""
+    w = synth.normal_quant(n_out, n_in, dtype, 0.02, 400 + dtype)
+    x = synth.normal_f32(rows * n_in, 1.0, 29 + rows).reshape(rows, n_in)
+    base = synth.normal_f32(rows * n_out, 1.0, 30).reshape(rows, n_out)
+    want = np.concatenate([run_gemm(dev, w, dtype, n_out, n_in, x[m:m + 16], cuda.PATH_MMA, accumulate=base[m:m + 16])
+                           for m in range(0, rows, 16)])
+    got = run_gemm(dev, w, dtype, n_out, n_in, x, cuda.PATH_MMA, accumulate=base)
+    assert np.array_equal(got, want), float(np.abs(got - want).max())

@@ -20,6 +20,7 @@
 // own fp32 decode (tensor/quant.go:105-125,261-285), CUDA-core FMAs.
 #include <cuda.h>
 
+#include <algorithm>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
@@ -391,16 +392,27 @@ __device__ __forceinline__ void header_k4_exact(const uint4 & hdr, int lane, uin
     if (hf == 0) reinterpret_cast<float2 *>(tab + X::D_OFF)[r] = make_float2(f16_bits_to_f32(hdr.x), -f16_bits_to_f32(hdr.x >> 16));
 }
 
+// Where a warp finds its activation fragments of one superblock: q16(j, k) the 16 bytes of sub-block k of product tile j
+// (q8(j, k, h): 8 bytes of 16-element group h of it, for types that read them apart), sum(j, i) the (hi, lo) sum of
+// 16-element group i. XResident: every row's columns lie in shared memory (gemm_tiled_mma_kernel).
+template <int NT> struct XResident {
+    const uint8_t * row[NT];
+    const uint8_t * sums[NT];
+    int sbl;  // superblock within the columns held
+    __device__ uint4 q16(int j, int k) const { return *reinterpret_cast<const uint4 *>(row[j] + (sbl * 256 + 32 * k) * 2); }
+    __device__ uint2 q8(int j, int k, int h) const { return *reinterpret_cast<const uint2 *>(row[j] + (sbl * 256 + 32 * k + 16 * h) * 2); }
+    __device__ uint32_t sum(int j, int i) const { return reinterpret_cast<const uint32_t *>(sums[j])[sbl * 16 + i]; }
+};
+
 // One MMA adding  sum_s16 A[row][s16] * xsum[tok][s16]  for eight 16-element groups base..base+7.
 // a_* are the (value, value) pairs for groups base+t and base+t+4 of rows g and g+8. A column that stands for
 // the lo half of an activation row takes no part (the sums already hold hi + lo).
-template <int NT>
+template <int NT, class XA>
 __device__ __forceinline__ void sum_mma(uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, int t, int s16_base,
-                                        const uint8_t * const (&xsrow)[NT], bool lo_col, float (&acc)[NT][4]) {
+                                        const XA & x, bool lo_col, float (&acc)[NT][4]) {
 #pragma unroll
     for (int j = 0; j < NT; j++) {
-        const uint32_t * xs = reinterpret_cast<const uint32_t *>(xsrow[j]) + s16_base;
-        const uint32_t b0 = lo_col ? 0u : xs[t], b1 = lo_col ? 0u : xs[t + 4];
+        const uint32_t b0 = lo_col ? 0u : x.sum(j, s16_base + t), b1 = lo_col ? 0u : x.sum(j, s16_base + t + 4);
         mma16816(acc[j], a0, a1, a2, a3, b0, b1);
     }
 }
@@ -426,8 +438,8 @@ __device__ __forceinline__ void fold_rows(float (&acc)[NT][4], const float (&q)[
 }
 
 // - dmin * sum_sub m[sub] * sum(x[sub]) of one Q4_K / Q5_K superblock
-template <typename X, int NT>
-__device__ __forceinline__ void min_part(const uint8_t * tab, int g, int t, int sbl, const uint8_t * const (&xsrow)[NT], bool lo_col,
+template <typename X, int NT, class XA>
+__device__ __forceinline__ void min_part(const uint8_t * tab, int g, int t, const XA & x, bool lo_col,
                                          float (&acc)[NT][4], float ndmin_g, float ndmin_h) {
     float mq[NT][4];
 #pragma unroll
@@ -439,7 +451,7 @@ __device__ __forceinline__ void min_part(const uint8_t * tab, int g, int t, int 
 #pragma unroll
     for (int half = 0; half < 2; half++) {
         const int k0 = 4 * half + (t >> 1);  // 16-element group 8 half + t belongs to sub-block 4 half + t / 2
-        sum_mma<NT>(mg[k0], mh[k0], mg[k0 + 2], mh[k0 + 2], t, sbl * 16 + 8 * half, xsrow, lo_col, mq);
+        sum_mma<NT>(mg[k0], mh[k0], mg[k0 + 2], mh[k0 + 2], t, 8 * half, x, lo_col, mq);
     }
     fold_rows<NT>(acc, mq, ndmin_g, ndmin_h);
 }
@@ -450,12 +462,12 @@ template <int NT> struct XMma<YUUKA_DTYPE_Q4_K, NT> {
     using C = Codec<YUUKA_DTYPE_Q4_K>;
     using X = XTab<YUUKA_DTYPE_Q4_K>;
     __device__ static void header(const typename C::Regs & r, int lane, uint8_t * tab) { header_k4_exact<X>(r.hdr, lane, tab); }
-    __device__ static void run(const typename C::Regs & r, int lane, const uint8_t * tab, const uint8_t * const (&xrow)[NT],
-                               const uint8_t * const (&xsrow)[NT], bool lo_col, int sbl, float (&acc)[NT][4],
-                               const DecodeConsts & kc) {
+    template <class XA>
+    __device__ static void run(const typename C::Regs & r, int lane, const uint8_t * tab, const XA & x, bool lo_col,
+                               float (&acc)[NT][4], const DecodeConsts & kc) {
         const int g = lane >> 2, t = lane & 3;
         const float2 dg = reinterpret_cast<const float2 *>(tab + X::D_OFF)[g], dh = reinterpret_cast<const float2 *>(tab + X::D_OFF)[g + 8];
-        min_part<X, NT>(tab, g, t, sbl, xsrow, lo_col, acc, dg.y, dh.y);
+        min_part<X, NT>(tab, g, t, x, lo_col, acc, dg.y, dh.y);
         float q[NT][4];
 #pragma unroll
         for (int j = 0; j < NT; j++)
@@ -486,7 +498,7 @@ template <int NT> struct XMma<YUUKA_DTYPE_Q4_K, NT> {
                     const int k = 2 * j + n;
 #pragma unroll
                     for (int jt = 0; jt < NT; jt++) {
-                        const uint4 b = *reinterpret_cast<const uint4 *>(xrow[jt] + (sbl * 256 + 32 * k) * 2);
+                        const uint4 b = x.q16(jt, k);
                         mma16816(q[jt], a[0][0], a[0][1], a[0][2], a[0][3], b.x, b.y);
                         mma16816(q[jt], a[1][0], a[1][1], a[1][2], a[1][3], b.z, b.w);
                     }
@@ -518,9 +530,9 @@ template <int NT> struct XMma<YUUKA_DTYPE_Q5_K, NT> {
         a[2] = h2_fma(and_or(vg >> 8, mask, hibit<K, tgt, true>(hg, bit, kc.magic)), s_g, c_g);
         a[3] = h2_fma(and_or(vh >> 8, mask, hibit<K, tgt, true>(hh, bit, kc.magic)), s_h, c_h);
     }
-    template <int K>
-    __device__ static void subblock(const typename C::Regs & r, const uint8_t * tg, const uint8_t * th,
-                                    const uint8_t * const (&xrow)[NT], int sbl, float (&q)[NT][4], const DecodeConsts & kc) {
+    template <int K, class XA>
+    __device__ static void subblock(const typename C::Regs & r, const uint8_t * tg, const uint8_t * th, const XA & x,
+                                    float (&q)[NT][4], const DecodeConsts & kc) {
         constexpr int j = K >> 1, n = K & 1, jj = j >> 1, jl = j & 1;
         const uint32_t qg[4] = {r.q[jj].x, r.q[jj].y, r.q[jj].z, r.q[jj].w};
         const uint32_t qh[4] = {r.q[2 + jj].x, r.q[2 + jj].y, r.q[2 + jj].z, r.q[2 + jj].w};
@@ -533,27 +545,27 @@ template <int NT> struct XMma<YUUKA_DTYPE_Q5_K, NT> {
             sub<K>(qg[2 * jl + h], qh[2 * jl + h], hg[h], hh[h], s_g, c_g, s_h, c_h, a[h], kc);
 #pragma unroll
         for (int jt = 0; jt < NT; jt++) {
-            const uint4 b = *reinterpret_cast<const uint4 *>(xrow[jt] + (sbl * 256 + 32 * K) * 2);
+            const uint4 b = x.q16(jt, K);
             mma16816(q[jt], a[0][0], a[0][1], a[0][2], a[0][3], b.x, b.y);
             mma16816(q[jt], a[1][0], a[1][1], a[1][2], a[1][3], b.z, b.w);
         }
     }
-    __device__ static void run(const typename C::Regs & r, int lane, const uint8_t * tab, const uint8_t * const (&xrow)[NT],
-                               const uint8_t * const (&xsrow)[NT], bool lo_col, int sbl, float (&acc)[NT][4],
-                               const DecodeConsts & kc) {
+    template <class XA>
+    __device__ static void run(const typename C::Regs & r, int lane, const uint8_t * tab, const XA & x, bool lo_col,
+                               float (&acc)[NT][4], const DecodeConsts & kc) {
         const int g = lane >> 2, t = lane & 3;
         const float2 dg = reinterpret_cast<const float2 *>(tab + X::D_OFF)[g], dh = reinterpret_cast<const float2 *>(tab + X::D_OFF)[g + 8];
-        min_part<X, NT>(tab, g, t, sbl, xsrow, lo_col, acc, dg.y, dh.y);
+        min_part<X, NT>(tab, g, t, x, lo_col, acc, dg.y, dh.y);
         float q[NT][4];
 #pragma unroll
         for (int j = 0; j < NT; j++)
 #pragma unroll
             for (int c = 0; c < 4; c++) q[j][c] = 0.0f;
         const uint8_t * tg = tab + g * X::SCL_STRIDE, * th = tab + (g + 8) * X::SCL_STRIDE;
-        subblock<0>(r, tg, th, xrow, sbl, q, kc); subblock<1>(r, tg, th, xrow, sbl, q, kc);
-        subblock<2>(r, tg, th, xrow, sbl, q, kc); subblock<3>(r, tg, th, xrow, sbl, q, kc);
-        subblock<4>(r, tg, th, xrow, sbl, q, kc); subblock<5>(r, tg, th, xrow, sbl, q, kc);
-        subblock<6>(r, tg, th, xrow, sbl, q, kc); subblock<7>(r, tg, th, xrow, sbl, q, kc);
+        subblock<0>(r, tg, th, x, q, kc); subblock<1>(r, tg, th, x, q, kc);
+        subblock<2>(r, tg, th, x, q, kc); subblock<3>(r, tg, th, x, q, kc);
+        subblock<4>(r, tg, th, x, q, kc); subblock<5>(r, tg, th, x, q, kc);
+        subblock<6>(r, tg, th, x, q, kc); subblock<7>(r, tg, th, x, q, kc);
         fold_rows<NT>(acc, q, dg.x, dh.x);
     }
 };
@@ -572,10 +584,9 @@ template <int NT> struct XMma<YUUKA_DTYPE_Q6_K, NT> {
         ds[1] = make_float4(d * (float)(int8_t)(wb & 0xff), d * (float)(int8_t)((wb >> 8) & 0xff), d * (float)(int8_t)((wb >> 16) & 0xff),
                             d * (float)(int8_t)(wb >> 24));
     }
-    __device__ static void run(const typename C::Regs & r, int lane, const uint8_t * tab, const uint8_t * const (&xrow)[NT],
-                               const uint8_t * const (&xsrow)[NT], bool lo_col, int sbl, float (&acc)[NT][4],
-                               const DecodeConsts & kc) {
-        (void)xsrow;
+    template <class XA>
+    __device__ static void run(const typename C::Regs & r, int lane, const uint8_t * tab, const XA & x, bool lo_col,
+                               float (&acc)[NT][4], const DecodeConsts & kc) {
         (void)lo_col;
         const int g = lane >> 2;
         const float4 * dsg = reinterpret_cast<const float4 *>(tab + g * X::DS_STRIDE);
@@ -613,7 +624,7 @@ template <int NT> struct XMma<YUUKA_DTYPE_Q6_K, NT> {
                         const float s_g = sgv[gi], s_h = shv[gi];
 #pragma unroll
                         for (int jt = 0; jt < NT; jt++) {
-                            const uint2 b = *reinterpret_cast<const uint2 *>(xrow[jt] + (sbl * 256 + 32 * k + 16 * h) * 2);
+                            const uint2 b = x.q8(jt, k, h);
                             float tmp[4];
                             mma16816_zero(tmp, a[h][0], a[h][1], a[h][2], a[h][3], b.x, b.y);
                             fma2(acc[jt][0], acc[jt][1], s_g, tmp[0], tmp[1]);
@@ -637,10 +648,9 @@ template <int NT> struct XMma<YUUKA_DTYPE_Q8_0, NT> {
         float4 * ds = reinterpret_cast<float4 *>(tab + row * X::DS_STRIDE) + hf;
         ds[0] = make_float4(f16_bits_to_f32(da), f16_bits_to_f32(da >> 16), f16_bits_to_f32(db), f16_bits_to_f32(db >> 16));
     }
-    __device__ static void run(const typename C::Regs & r, int lane, const uint8_t * tab, const uint8_t * const (&xrow)[NT],
-                               const uint8_t * const (&xsrow)[NT], bool lo_col, int sbl, float (&acc)[NT][4],
-                               const DecodeConsts & kc) {
-        (void)xsrow;
+    template <class XA>
+    __device__ static void run(const typename C::Regs & r, int lane, const uint8_t * tab, const XA & x, bool lo_col,
+                               float (&acc)[NT][4], const DecodeConsts & kc) {
         (void)lo_col;
         (void)kc;
         const int g = lane >> 2;
@@ -667,7 +677,7 @@ template <int NT> struct XMma<YUUKA_DTYPE_Q8_0, NT> {
                 }
 #pragma unroll
                 for (int jt = 0; jt < NT; jt++) {
-                    const uint4 b = *reinterpret_cast<const uint4 *>(xrow[jt] + (sbl * 256 + 32 * k) * 2);
+                    const uint4 b = x.q16(jt, k);
                     float tmp[4];
                     mma16816_zero(tmp, a[0][0], a[0][1], a[0][2], a[0][3], b.x, b.y);
                     mma16816(tmp, a[1][0], a[1][1], a[1][2], a[1][3], b.z, b.w);
@@ -902,13 +912,12 @@ __global__ void __launch_bounds__(MW * 32, 1) gemm_tiled_mma_kernel(const TParam
     uint8_t * tab = tabs + warp * X::TAB;
     // column 8j + g of the product: activation row (8j + g) / 2, hi half if g is even
     const bool lo_col = (g & 1) != 0;
-    const uint8_t * xrow[NT];
-    const uint8_t * xsrow[NT];
+    XResident<NT> xa;
 #pragma unroll
     for (int j = 0; j < NT; j++) {
         const int col = min(8 * j + g, 2 * Mrows - 1);
-        xrow[j] = xs + (size_t)col * xstride + t * X::XT_BYTES;
-        xsrow[j] = xsum + (size_t)(col >> 1) * xsum_stride;
+        xa.row[j] = xs + (size_t)col * xstride + t * X::XT_BYTES;
+        xa.sums[j] = xsum + (size_t)(col >> 1) * xsum_stride;
     }
 
     const DecodeConsts kc = p.kc;
@@ -939,7 +948,8 @@ __global__ void __launch_bounds__(MW * 32, 1) gemm_tiled_mma_kernel(const TParam
             }
             MM::header(cur, lane, tab);
             __syncwarp();
-            MM::run(cur, lane, tab, xrow, xsrow, lo_col, sb - c0, acc, kc);
+            xa.sbl = sb - c0;
+            MM::run(cur, lane, tab, xa, lo_col, acc, kc);
             __syncwarp();
             cur = nxt;
         }
@@ -1150,6 +1160,266 @@ __global__ void __launch_bounds__(MW * 32, 1) gemm_tiled_mma_kernel(const TParam
         const uint32_t step = gridDim.x * gridDim.y * (MW * 32);
         for (uint32_t line = first; line < p.next_lines; line += step) prefetch_l2(p.next_w + (size_t)line * 128);
     }
+}
+
+// ===========================================================================
+// Register-fed kernel for more activation rows than one launch of the kernel above holds (17 to 48): every weight record is
+// decoded once and multiplied with all of them.
+//
+// A CTA has up to eight warps, a 16-row tile each, that walk the superblocks of K together (a ninth warp for the copies would
+// leave a thread 168 registers instead of 255); the first one also has the superblocks' activations of all rows brought two
+// ahead by TMA (hi and lo halves in boxes of 64 columns, swizzled, and the sums). The columns of a row need not fit shared memory, so K is not cut for that; where a matrix has few tiles, ranges of
+// K go to different CTAs. What bounds it: 32 products per four activation rows, superblock and tile, 2.1 cycles each, 310
+// cycles per record at 36 rows, of which the two warps of a scheduler reach some 40 % between decode, reads and folds.
+// In a step of 36 rows (three passes of sixteen before): 12352 x 2560 Q4_K 52 -> 35 us, 2560 x 4096 Q4_K 38 -> 23,
+// 18432 x 2560 Q4_K 53 -> 35, 2560 x 9216 Q6_K 66 -> 37; of 47 rows 62 -> 45, 45 -> 27, 62 -> 48, 72 -> 46.
+//
+// The sums of a row are those of the kernel above to the last bit. That kernel cuts K for its own rows: into chunks across
+// CTAs, and those into parts across warps (TPlan); a row's parts are added in order, then its chunks. Here one accumulator
+// runs over a part and is added up at the part's end, 16-row passes and the rest of the rows each at the ends of their own cut.
+constexpr int RW_WARPS = 8, RW_MAX_ROWS = 48, RW_MAX_STAGES = 4, RW_MAX_SPLITS = 8;
+
+// Where K is cut for the rows of a pass: bit sb of `parts` / `chunks`: a part / chunk ends after superblock sb.
+struct RowCut {
+    uint64_t parts, chunks;
+};
+struct RParams {
+    DecodeConsts kc;
+    const uint8_t * w;
+    int N, nsb, M;
+    float * out;
+    int64_t ldo;
+    int accumulate;
+    int tg;              // warps (tiles) of a CTA that work
+    int groups, splits;  // work items: groups of tg tiles x ranges of K
+    int split_at[RW_MAX_SPLITS + 1];
+    RowCut cut[2];       // [0]: rows below first_rest, [1]: the rest
+    int first_rest;      // a multiple of 16
+    float * partial;     // splits > 1: [part][M][N]
+    int stages;
+    const uint8_t * next_w;  // see TParams
+    uint32_t next_lines;
+};
+
+// Activations of one superblock: four column blocks of hi rows, four of lo rows, the sums. The lo box starts four rows
+// before row 0 (zeros), so that a row's hi and lo pieces, which one phase of a warp's reads takes together, differ in the
+// swizzle and with that in their banks.
+template <int DT, int NT> struct RowStage {
+    static constexpr int HI_ROWS = 4 * NT, LO_ROWS = 4 * NT + 4;
+    static constexpr int BLOCK = (LO_ROWS + 7) / 8 * 1024;  // bytes of a 64-column block
+    static constexpr int SUMS_AT = 8 * BLOCK, SUM_BYTES = XTab<DT>::SUMS ? HI_ROWS * 64 : 0;
+    static constexpr int BYTES = (SUMS_AT + SUM_BYTES + 1023) / 1024 * 1024;
+    static constexpr uint32_t TX = 4u * (HI_ROWS + LO_ROWS) * 128u + SUM_BYTES;  // what the copies of a superblock write
+};
+
+// Lane (g, t) of a warp reads column g of a product tile: row pi(g / 2) of the tile's four, hi half if g is even. pi swaps
+// rows 1 and 2: the two rows that a phase of 8-byte reads takes together are then two apart, and so are their banks.
+__device__ __forceinline__ int row_pi(int u) { return ((u & 1) << 1) | (u >> 1); }
+template <int DT, int NT> struct XStaged {
+    using R = RowStage<DT, NT>;
+    static constexpr bool WIDE = XTab<DT>::XT_BYTES == 16;
+    // 16-byte piece c of a row of tile j lies at c ^ (row mod 8), bit 2 of which is j's parity (the opposite in lo rows): the
+    // lane's address for even and for odd k ^ j, and (8-byte pieces) for either half of a sub-block
+    uint32_t even, odd, flip_h, sums_at;
+    const uint8_t * stage;
+    __device__ void init(int g, int t) {
+        const int u = row_pi(g >> 1), lo = g & 1;
+        const int at = (lo ? 4 * R::BLOCK + 512 : 0) + u * 128;
+        const int piece = WIDE ? (t ^ u) * 16 : ((t >> 1) ^ u) * 16 + (t & 1) * 8;
+        even = at + piece + (lo ? 64 : 0);
+        odd = at + piece + (lo ? 0 : 64);
+        flip_h = (piece & 32) ? (uint32_t)-32 : 32u;
+        sums_at = R::SUMS_AT + u * 64;
+    }
+    __device__ const uint8_t * at(int j, int k) const { return stage + (((k ^ j) & 1) ? odd : even) + j * 512 + (k >> 1) * R::BLOCK; }
+    __device__ uint4 q16(int j, int k) const { return *reinterpret_cast<const uint4 *>(at(j, k)); }
+    __device__ uint2 q8(int j, int k, int h) const { return *reinterpret_cast<const uint2 *>(at(j, k) + (int)(h ? flip_h : 0u)); }
+    __device__ uint32_t sum(int j, int i) const { return *reinterpret_cast<const uint32_t *>(stage + sums_at + j * 256 + i * 4); }
+};
+
+template <int DT, int NT>
+__global__ void __launch_bounds__(RW_WARPS * 32, 1)
+    gemm_tiled_rows_kernel(const RParams p, const __grid_constant__ CUtensorMap hi_map, const __grid_constant__ CUtensorMap lo_map,
+                           const __grid_constant__ CUtensorMap sum_map) {
+    using C = Codec<DT>;
+    using X = XTab<DT>;
+    using R = RowStage<DT, NT>;
+    extern __shared__ __align__(128) uint8_t smem_raw[];
+    uint8_t * smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);  // the swizzled blocks need 1024-byte alignment
+    __shared__ __align__(8) uint64_t full_bar[RW_MAX_STAGES], empty_bar[RW_MAX_STAGES];
+    const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < p.stages; s++) {
+            mbar_init(smem_u32(&full_bar[s]), 1);
+            mbar_init(smem_u32(&empty_bar[s]), p.tg);
+        }
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    __syncthreads();
+    pdl_trigger();
+    const int items = p.groups * p.splits;
+    bool expired = false;
+    auto wait = [&](const uint64_t & bar, uint32_t parity) {
+        if (!expired && !mbar_wait(smem_u32(&bar), parity)) expired = true;
+    };
+    // (warp 0) the copies of the next superblock in the order of work, once the warps have read what its stage held
+    Ring fill;
+    int fill_item = blockIdx.x, fill_sb = fill_item < items ? p.split_at[fill_item / p.groups] : 0;
+    auto fetch = [&] {
+        if (fill_item >= items) return;
+        wait(empty_bar[fill.at], fill.phase ^ 1u);
+        if (lane == 0) {
+            const uint32_t bar = smem_u32(&full_bar[fill.at]), st = smem_u32(smem) + fill.at * (uint32_t)R::BYTES;
+            mbar_expect(bar, R::TX);
+            auto load = [&](uint32_t dst, const CUtensorMap & map, int col, int row) {
+                asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
+                             :
+                             : "r"(dst), "l"(&map), "r"(col), "r"(row), "r"(bar)
+                             : "memory");
+            };
+#pragma unroll
+            for (int b = 0; b < 4; b++) {
+                load(st + b * R::BLOCK, hi_map, fill_sb * 256 + b * 64, 0);
+                load(st + (4 + b) * R::BLOCK, lo_map, fill_sb * 256 + b * 64, -4);
+            }
+            if (X::SUMS) load(st + R::SUMS_AT, sum_map, fill_sb * 16, 0);
+        }
+        __syncwarp();
+        fill.next(p.stages);
+        if (++fill_sb == p.split_at[fill_item / p.groups + 1]) {
+            fill_item += gridDim.x;
+            if (fill_item < items) fill_sb = p.split_at[fill_item / p.groups];
+        }
+    };
+    {
+        Ring ring;
+        const int g = lane >> 2, t = lane & 3;
+        const int n_tiles = (p.N + 15) >> 4;
+        const size_t rec_row = (size_t)p.nsb * C::REC;
+        uint8_t * tab = smem + (size_t)p.stages * R::BYTES + warp * X::TAB;
+        const bool lo_col = (g & 1) != 0;
+        const DecodeConsts kc = p.kc;
+        XStaged<DT, NT> xa;
+        xa.init(g, t);
+        typename C::Regs cur, nxt;
+        auto record = [&](int item) {
+            const int split = item / p.groups, rt = min((item - split * p.groups) * p.tg + warp, n_tiles - 1);
+            return p.w + rt * rec_row + (size_t)p.split_at[split] * C::REC;
+        };
+        if ((int)blockIdx.x < items) C::load(record(blockIdx.x), lane, cur);
+        pdl_wait();
+        if (warp == 0)
+            for (int s = 0; s < p.stages - 2; s++) fetch();
+        for (int item = blockIdx.x; item < items; item += gridDim.x) {
+            const int split = item / p.groups, sb0 = p.split_at[split], sb1 = p.split_at[split + 1];
+            const int rt = (item - split * p.groups) * p.tg + warp;
+            const uint8_t * rec = record(item);
+            float acc[NT][4], chunk[NT][2], total[NT][2];
+#pragma unroll
+            for (int j = 0; j < NT; j++) {
+#pragma unroll
+                for (int c = 0; c < 4; c++) acc[j][c] = 0.0f;
+                chunk[j][0] = chunk[j][1] = total[j][0] = total[j][1] = 0.0f;
+            }
+            const int n_g = rt * 16 + g, n_h = n_g + 8;
+            const bool ok_g = n_g < p.N, ok_h = n_h < p.N;
+            for (int sb = sb0; sb < sb1; sb++) {
+                rec += C::REC;
+                if (sb + 1 < sb1) C::load(rec, lane, nxt);
+                else if (item + (int)gridDim.x < items) C::load(record(item + gridDim.x), lane, nxt);
+                if (warp == 0) fetch();  // (into the stage of the superblock before the last)
+                XMma<DT, NT>::header(cur, lane, tab);
+                __syncwarp();
+                wait(full_bar[ring.at], ring.phase);
+                xa.stage = smem + (size_t)ring.at * R::BYTES;
+                XMma<DT, NT>::run(cur, lane, tab, xa, lo_col, acc, kc);
+                __syncwarp();
+                if (lane == 0) mbar_arrive(smem_u32(&empty_bar[ring.at]));
+                ring.next(p.stages);
+                cur = nxt;
+#pragma unroll
+                for (int rest = 0; rest < 2; rest++) {
+                    const uint64_t below = (1ull << sb) - 1;
+                    const RowCut cut = p.cut[rest];
+                    if (!((cut.parts >> sb) & 1)) continue;
+                    const bool first = __clzll(cut.parts & below) == __clzll(cut.chunks & below);  // of its chunk
+                    const bool last = (cut.chunks >> sb) & 1, many = (cut.chunks & (cut.chunks - 1)) != 0;
+                    float * part = p.splits > 1 ? p.partial + (size_t)__popcll(cut.parts & below) * p.M * p.N : nullptr;
+#pragma unroll
+                    for (int j = 0; j < NT; j++) {
+                        if ((4 * j >= p.first_rest) != (rest != 0)) continue;
+                        const float v0 = acc[j][0] + acc[j][1], v1 = acc[j][2] + acc[j][3];
+                        acc[j][0] = acc[j][1] = acc[j][2] = acc[j][3] = 0.0f;
+                        if (part) {
+                            const int tok = 4 * j + row_pi(t);
+                            if (tok < p.M) {
+                                if (ok_g) __stcg(part + (int64_t)tok * p.N + n_g, v0);
+                                if (ok_h) __stcg(part + (int64_t)tok * p.N + n_h, v1);
+                            }
+                        } else {
+                            chunk[j][0] = first ? v0 : chunk[j][0] + v0;
+                            chunk[j][1] = first ? v1 : chunk[j][1] + v1;
+                            if (last) {
+                                total[j][0] = many ? total[j][0] + chunk[j][0] : chunk[j][0];
+                                total[j][1] = many ? total[j][1] + chunk[j][1] : chunk[j][1];
+                            }
+                        }
+                    }
+                }
+            }
+            if (p.splits == 1) {
+#pragma unroll
+                for (int j = 0; j < NT; j++) {
+                    const int tok = 4 * j + row_pi(t);
+                    if (tok >= p.M) continue;
+                    float * dst = p.out + (int64_t)tok * p.ldo;
+                    if (ok_g) dst[n_g] = p.accumulate ? dst[n_g] + total[j][0] : total[j][0];
+                    if (ok_h) dst[n_h] = p.accumulate ? dst[n_h] + total[j][1] : total[j][1];
+                }
+            }
+        }
+    }
+    if (expired) atomicExch(&g_gemm_wait_expired, 4);
+    pdl_trigger_late();
+    if (p.next_w)
+        for (uint32_t line = blockIdx.x * blockDim.x + threadIdx.x; line < p.next_lines; line += gridDim.x * blockDim.x)
+            prefetch_l2(p.next_w + (size_t)line * 128);
+}
+
+// Sum of the parts of a launch whose K ranges went to different CTAs: parts within a chunk, then chunks, in order.
+__global__ void __launch_bounds__(256) rows_reduce_kernel(float * __restrict__ out, int64_t ldo, const float * __restrict__ partial,
+                                                          int M, int N, int first_rest, const RowCut cut0, const RowCut cut1, int accumulate) {
+    pdl_entry();
+    const int tok = blockIdx.y, n = blockIdx.x * 256 + threadIdx.x;
+    if (n >= N) return;
+    const RowCut cut = tok >= first_rest ? cut1 : cut0;
+    const bool many = (cut.chunks & (cut.chunks - 1)) != 0;
+    const float * src = partial + (size_t)tok * N + n;
+    float * dst = out + (int64_t)tok * ldo + n;
+    const float old = accumulate ? *dst : 0.0f;
+    float total = 0.0f, chunk = 0.0f;
+    bool first = true;
+    for (uint64_t left = cut.parts; left;) {
+        // four parts in flight
+        float v[4];
+        uint64_t ahead = left;
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+            v[u] = ahead ? __ldcg(src + (size_t)u * M * N) : 0.0f;
+            ahead &= ahead - 1;
+        }
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+            if (!left) break;
+            const uint64_t bit = left & (~left + 1);
+            left &= left - 1;
+            chunk = first ? v[u] : chunk + v[u];
+            first = (cut.chunks & bit) != 0;
+            if (first) total = many ? total + chunk : chunk;
+        }
+        src += (size_t)4 * M * N;
+    }
+    *dst = accumulate ? old + total : total;
 }
 
 // ===========================================================================
@@ -1453,6 +1723,61 @@ static UmmaPlan umma_plan(const yuuka_device * dev, int n_out, int n_in, int m) 
     return best;
 }
 
+// Where plan_tiled cuts K for passes of m rows.
+static RowCut row_cut(const yuuka_device * dev, uint32_t dtype, int m, int n_out, int n_in) {
+    TPlan pl;
+    plan_tiled(dev, dtype, m, n_out, n_in, pl);
+    const int nsb = n_in / 256;
+    RowCut cut{0, 0};
+    for (int c0 = 0; c0 < nsb; c0 += pl.nsb_chunk) {
+        const int cnt = nsb - c0 < pl.nsb_chunk ? nsb - c0 : pl.nsb_chunk;
+        for (int k = 1; k <= pl.KS; k++)
+            if (cnt * k / pl.KS > 0) cut.parts |= 1ull << (c0 + cnt * k / pl.KS - 1);
+        cut.chunks |= 1ull << (c0 + cnt - 1);
+    }
+    return cut;
+}
+
+// How 17 to 48 rows are cut into work for gemm_tiled_rows_kernel: tg tiles per CTA and ranges of K that end where parts of
+// all rows end. The cost is in records per SM (a record takes as long however many warps share the SM's tensor pipe): rounds
+// x (tiles x records + 2 for the start and the stores of an item), and 10 for the launch that adds the ranges up.
+static void plan_rows(const yuuka_device * dev, uint32_t dtype, int m, int n_out, int n_in, RParams & p) {
+    const int nsb = n_in / 256, n_tiles = (n_out + 15) / 16;
+    p.first_rest = m / 16 * 16;
+    p.cut[0] = row_cut(dev, dtype, 16, n_out, n_in);
+    p.cut[1] = m > p.first_rest ? row_cut(dev, dtype, m - p.first_rest, n_out, n_in) : p.cut[0];
+    const uint64_t ends = p.cut[0].parts & p.cut[1].parts;
+    double best = 1e30;
+    for (int splits = 1; splits <= RW_MAX_SPLITS && splits <= nsb; splits++) {
+        int at[RW_MAX_SPLITS + 1], n = 0, longest = 0;
+        at[0] = 0;
+        for (int sb = 0; sb < nsb; sb++)
+            if (sb + 1 == nsb || (((ends >> sb) & 1) && (sb + 1) * splits >= (n + 1) * nsb && n + 1 < splits)) {
+                at[++n] = sb + 1;
+                if (at[n] - at[n - 1] > longest) longest = at[n] - at[n - 1];
+            }
+        if (n != splits) continue;
+        for (int tg = 4; tg <= RW_WARPS; tg++) {
+            const int groups = (n_tiles + tg - 1) / tg, rounds = (groups * splits + dev->sm_count - 1) / dev->sm_count;
+            const double cost = rounds * (tg * longest + 2.0) + (splits > 1 ? 10.0 : 0.0);
+            if (cost >= best) continue;
+            best = cost;
+            p.tg = tg;
+            p.groups = groups;
+            p.splits = splits;
+            memcpy(p.split_at, at, sizeof(at));
+        }
+    }
+}
+static uint64_t rows_partial_floats(const RParams & p, int m, int n_out) {
+    if (p.splits == 1) return 0;
+    const int parts = std::max(__builtin_popcountll(p.cut[0].parts), __builtin_popcountll(p.cut[1].parts));
+    return (uint64_t)parts * m * n_out;
+}
+// From 17 rows, where passes of sixteen would begin to decode the weights more than once; K of at most 64 superblocks (the
+// masks of RowCut). (Launches that fold a norm or SwiGLU into their epilogue, steps of up to 32 rows, stay with the passes.)
+static bool rows_route(int m, int n_in) { return m > MMA_ROWS && n_in <= 64 * 256; }
+
 void gemm_tiled_scratch_need(const yuuka_device * dev, uint32_t w_dtype, int rows, int n_out, int n_in,
                              uint64_t * partial_floats, int * counters) {
     *partial_floats = 0;
@@ -1463,6 +1788,14 @@ void gemm_tiled_scratch_need(const yuuka_device * dev, uint32_t w_dtype, int row
         const int parts = rows >= UMMA_EARLY_ROWS ? umma_kparts(dev, n_out, n_in, m) : 1;
         if (parts > 2 && (uint64_t)parts * m * n_out > *partial_floats) *partial_floats = (uint64_t)parts * m * n_out;
     }
+    for (int m : {rows, RW_MAX_ROWS, 40, 32, 24})
+        if (m <= rows && m <= RW_MAX_ROWS && rows_route(m, n_in)) {
+            for (int mm = m; mm > MMA_ROWS && mm > m - 16; mm--) {
+                RParams p{};
+                plan_rows(dev, w_dtype, mm, n_out, n_in, p);
+                *partial_floats = std::max(*partial_floats, rows_partial_floats(p, mm, n_out));
+            }
+        }
     for (int m : {rows < MMA_ROWS ? rows : MMA_ROWS, MMA_ROWS < rows ? rows % MMA_ROWS : 0}) {
         if (m <= 0) continue;
         for (bool paired : {false, true}) {
@@ -1674,6 +2007,76 @@ static int launch_umma_dt(const yuuka_device * dev, cudaStream_t s, const TiledG
     return 2;
 }
 
+// [m][k / 16] pairs of sums: boxes of one superblock (16 pairs) x box_rows
+static void make_sum_map(CUtensorMap * map, const __half2 * sums, int m, int k, int box_rows) {
+    TensorMapEncodeFn enc = tensor_map_encoder();
+    YK_REQUIRE(enc, YUUKA_ERR_DEVICE, "gemm: the driver has no tensor-map encoder");
+    const cuuint64_t gdim[2] = {(cuuint64_t)k / 16, (cuuint64_t)m};
+    const cuuint64_t gstride[1] = {(cuuint64_t)k / 4};
+    const cuuint32_t box[2] = {16, (cuuint32_t)box_rows};
+    const cuuint32_t estr[2] = {1, 1};
+    YK_REQUIRE(enc(map, CU_TENSOR_MAP_DATA_TYPE_INT32, 2, (void *)sums, gdim, gstride, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                   CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS,
+               YUUKA_ERR_INTERNAL, "gemm: the tensor map of the activations' sums could not be encoded");
+}
+
+template <int DT, int NT>
+static void launch_rows_inst(const yuuka_device * dev, cudaStream_t s, RParams & p, const XPrepOut & xp, int m0) {
+    using R = RowStage<DT, NT>;
+    const int K = p.nsb * 256;
+    alignas(64) CUtensorMap hi, lo, sums;
+    make_x_map(&hi, xp.xh + (int64_t)m0 * K, p.M, K, R::HI_ROWS);
+    make_x_map(&lo, xp.xl + (int64_t)m0 * K, p.M, K, R::LO_ROWS);
+    if (XTab<DT>::SUMS) make_sum_map(&sums, xp.xs16 + (int64_t)m0 * (K / 16), p.M, K, R::HI_ROWS);
+    else sums = hi;
+    const size_t fixed = (size_t)RW_WARPS * XTab<DT>::TAB + 1024;
+    p.stages = RW_MAX_STAGES;
+    while (fixed + (size_t)p.stages * R::BYTES + 1024 > dev->prop.sharedMemPerBlockOptin && p.stages > 3) p.stages--;
+    const size_t smem = fixed + (size_t)p.stages * R::BYTES;
+    YK_REQUIRE(smem + 1024 <= dev->prop.sharedMemPerBlockOptin, YUUKA_ERR_INTERNAL, "gemm: stage buffers do not fit shared memory");
+    YK_CUDA(cudaFuncSetAttribute(gemm_tiled_rows_kernel<DT, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    const int items = p.groups * p.splits;
+    launch_k(gemm_tiled_rows_kernel<DT, NT>, items < dev->sm_count ? items : dev->sm_count, p.tg * 32, smem, s, p, hi, lo, sums);
+    YK_CUDA(cudaGetLastError());
+}
+
+template <int DT>
+static int launch_rows_dt(const yuuka_device * dev, cudaStream_t s, const TiledGemmArgs & a, const XPrepOut & xp, int m0, int m) {
+    RParams p{};
+    p.kc = decode_consts(DT);
+    p.w = a.w;
+    p.N = a.n_out;
+    p.nsb = a.n_in / 256;
+    p.M = m;
+    p.out = a.out + (int64_t)m0 * a.ldo;
+    p.ldo = a.ldo;
+    p.accumulate = (a.flags & YUUKA_GEMM_ACCUMULATE) ? 1 : 0;
+    plan_rows(dev, DT, m, a.n_out, a.n_in, p);
+    if (p.splits > 1) {
+        YK_REQUIRE(a.scratch && a.scratch->partial_floats >= rows_partial_floats(p, m, a.n_out), YUUKA_ERR_INTERNAL,
+                   "gemm: split-K scratch is too small");
+        p.partial = a.scratch->partial;
+    }
+    if (a.next_w) {
+        p.next_w = a.next_w;
+        p.next_lines = (uint32_t)(a.next_bytes / 128);
+    }
+    switch ((m + 3) / 4) {  // product tiles, four rows each
+    case 5:
+    case 6: launch_rows_inst<DT, 6>(dev, s, p, xp, m0); break;
+    case 7:
+    case 8: launch_rows_inst<DT, 8>(dev, s, p, xp, m0); break;
+    case 9: launch_rows_inst<DT, 9>(dev, s, p, xp, m0); break;
+    case 10: launch_rows_inst<DT, 10>(dev, s, p, xp, m0); break;
+    default: launch_rows_inst<DT, 12>(dev, s, p, xp, m0); break;
+    }
+    if (p.splits == 1) return 1;
+    launch_k(rows_reduce_kernel, dim3((a.n_out + 255) / 256, m), 256, 0, s, p.out, p.ldo, (const float *)p.partial, m, a.n_out, p.first_rest,
+             p.cut[0], p.cut[1], p.accumulate);
+    YK_CUDA(cudaGetLastError());
+    return 2;
+}
+
 template <int DT>
 static int launch_mma_dt(const yuuka_device * dev, cudaStream_t s, const TiledGemmArgs & a) {
     int launches = 0;
@@ -1695,8 +2098,15 @@ static int launch_mma_dt(const yuuka_device * dev, cudaStream_t s, const TiledGe
     }
     if (wide) return launches + launch_umma_dt<DT>(dev, s, a, xp.xh);
     YK_REQUIRE(xp.xl && xp.xs16, YUUKA_ERR_INTERNAL, "gemm: the prepared activations lack their lo halves or sums");
-    for (int m0 = 0; m0 < a.rows; m0 += MMA_ROWS) {
-        const int m = a.rows - m0 < MMA_ROWS ? a.rows - m0 : MMA_ROWS;
+    const bool folded = a.norm.produce_w || a.norm.consume_now || a.swiglu.xh;
+    int m = 0;
+    for (int m0 = 0; m0 < a.rows; m0 += m) {
+        m = a.rows - m0 < RW_MAX_ROWS ? a.rows - m0 : RW_MAX_ROWS;
+        if (rows_route(m, a.n_in) && !folded && !(a.flags & YUUKA_GEMM_TEST_DROP_COPIES)) {
+            launches += launch_rows_dt<DT>(dev, s, a, xp, m0, m);
+            continue;
+        }
+        m = m < MMA_ROWS ? m : MMA_ROWS;
         TPlan pl;
         plan_tiled(dev, a.w_dtype, m, a.n_out, a.n_in, pl, a.swiglu.xh != nullptr);
         YK_REQUIRE(pl.smem + 4096 <= dev->prop.sharedMemPerBlockOptin, YUUKA_ERR_UNSUPPORTED,
@@ -1798,6 +2208,11 @@ static void preload_dt() {
     cudaFuncAttributes fa;
     YK_CUDA(cudaFuncGetAttributes(&fa, gemm_tiled_mma_kernel<DT, 1, false, false>));
     YK_CUDA(cudaFuncGetAttributes(&fa, gemm_tiled_mma_kernel<DT, 2, false, false>));
+    YK_CUDA(cudaFuncGetAttributes(&fa, gemm_tiled_rows_kernel<DT, 6>));
+    YK_CUDA(cudaFuncGetAttributes(&fa, gemm_tiled_rows_kernel<DT, 8>));
+    YK_CUDA(cudaFuncGetAttributes(&fa, gemm_tiled_rows_kernel<DT, 9>));
+    YK_CUDA(cudaFuncGetAttributes(&fa, gemm_tiled_rows_kernel<DT, 10>));
+    YK_CUDA(cudaFuncGetAttributes(&fa, gemm_tiled_rows_kernel<DT, 12>));
     YK_CUDA(cudaFuncGetAttributes(&fa, gemm_tiled_mma_kernel<DT, 3, false, false>));
     YK_CUDA(cudaFuncGetAttributes(&fa, gemm_tiled_mma_kernel<DT, 4, false, false>));
     YK_CUDA(cudaFuncGetAttributes(&fa, gemm_tiled_fp32_kernel<DT, float>));
@@ -1812,6 +2227,7 @@ void gemm_tiled_preload_kernels() {
     preload_dt<YUUKA_DTYPE_Q8_0>();
     YK_CUDA(cudaFuncGetAttributes(&fa, xprep_kernel<float>));
     YK_CUDA(cudaFuncGetAttributes(&fa, xprep_kernel<__nv_bfloat16>));
+    YK_CUDA(cudaFuncGetAttributes(&fa, rows_reduce_kernel));
     YK_CUDA(cudaFuncGetAttributes(&fa, umma_reduce_kernel<4>));
     YK_CUDA(cudaFuncGetAttributes(&fa, umma_reduce_kernel<1>));
     tensor_map_encoder();  // the driver entry point look-up happens once, here
