@@ -662,3 +662,26 @@ def test_an_expired_device_wait_is_reported_once_and_the_path_keeps_working(tiny
         b.free()
     stream.destroy()
     sess.close(); st.close()
+
+
+@pytest.mark.parametrize("B,N,hidden,ffn", [(3, 11, 256, 768), (1, 47, 256, 3328), (4, 10, 3328, 768)])
+def test_steps_of_33_to_47_rows_with_folded_tails(B, N, hidden, ffn):
+    """SwiGLU in the gate|up GEMM and the norm in the launch that adds up the parts of K, at rows that fill no product tile
+    and widths beyond what one CTA's registers hold (3072)."""
+    cfg = synth.tiny_config()
+    cfg.update(hidden=hidden, ffn=ffn, vocab=512)
+    tensors = synth.make_model(cfg, "q4_k_m", seed=48, unit_norms=False)
+    dev = cuda.Device(0)
+    gm, om = cuda.Model(dev, cfg, tensors), yo.Model(cfg, tensors)
+    sess = cuda.Session(gm, max_batch=B, max_nodes=N, capacity=96, kv_format=cuda.KV_F32)
+    toks = synth.uniform_i32(B * N, 0, cfg["vocab"], 12).reshape(B, N)
+    res = sess.verify(toks, want_logits=True)
+    for b in range(B):
+        st = yo.State(om, 96, yo.KV_F32)
+        _, _, want = st.verify_chain(int(toks[b, 0]), toks[b, 1:], want_logits=True)
+        st.close()
+        err = float(np.max(np.abs(res.logits[b] - want)))
+        assert err <= 5e-4 * max(1.0, float(np.max(np.abs(want)))), err
+    sess.close()
+    gm.close()
+    dev.close()

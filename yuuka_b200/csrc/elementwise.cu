@@ -167,50 +167,134 @@ __global__ void rmsnorm_kernel(float * __restrict__ dst, int ldd, const float * 
     rmsnorm_row(dst + (int64_t)r * ldd, src + (int64_t)r * lds, weight, cols, eps, prep, sumsq_out, r, red);
 }
 
-// Wide steps: the fp16 form alone. The row's values stay in registers between the sum and the product (the general
-// kernel reads them twice and has 16 columns per thread in the second pass, 160 of its 256 threads on 2560 columns);
-// the sum runs in the same order. 512 rows of 2560 columns: 11.8 -> 5.3 us.
-constexpr int RMS_KEEP = 12;
-__global__ void __launch_bounds__(256) rmsnorm_hi_kernel(__half * __restrict__ dst, const float * __restrict__ src, int lds,
-                                                         const float * __restrict__ weight, int cols, float eps) {
+// RMSNorm of a row by a CTA, after adding the row's parts of a split GEMM where there are some. A thread keeps its columns
+// (tid + 256 k) in registers from the parts to the product: one pass over the row instead of two, or of four with a summing
+// launch ahead, and the sum of squares runs in rmsnorm_row's order. HI: the fp16 form alone (wide steps); otherwise f32 rows
+// and the whole prepared form, whose 16-column groups meet in shared memory. (PARTS: apart because it takes 120 registers
+// and the norm alone 48.)
+// It is bound by the latency of a row's chain (loads, f64 sum, barriers): every load of a thread is in flight at once.
+// 512 rows of 2560 columns, HI: norm alone 11.8 -> 5.3 us.
+constexpr int RN_KEEP = 12, RN_SPAN = RN_KEEP * 256;
+template <bool HI, bool PARTS>
+__global__ void __launch_bounds__(256) rows_norm_kernel(float * __restrict__ x, int64_t ldx, const RowParts parts, int rows, int cols,
+                                                        int accumulate, const RowNorm norm) {
     __shared__ double red[32];
-    float v[RMS_KEEP], w[RMS_KEEP];
+    __shared__ __align__(16) float stage[HI ? 4 : RN_SPAN];
+    float w[RN_KEEP], v[RN_KEEP];
 #pragma unroll
-    for (int k = 0; k < RMS_KEEP; k++) {
+    for (int k = 0; k < RN_KEEP; k++) {
         const int i = threadIdx.x + k * 256;
-        w[k] = i < cols ? weight[i] : 0.0f;
+        w[k] = i < cols ? norm.w[i] : 0.0f;
     }
     pdl_entry();
-    const float * x = src + (int64_t)blockIdx.x * lds;
-    dst += (int64_t)blockIdx.x * cols;
+    const int r = blockIdx.x;
+    float * row = x + r * ldx;
+    const RowCut cut = parts.cut[r >= parts.first_rest ? 1 : 0];
+    const bool many = (cut.chunks & (cut.chunks - 1)) != 0;
     double sum = 0;
+    for (int c0 = 0; c0 < cols; c0 += RN_SPAN) {
+        if (PARTS && !accumulate) {
 #pragma unroll
-    for (int k = 0; k < RMS_KEEP; k++) {
-        const int i = threadIdx.x + k * 256;
-        v[k] = i < cols ? x[i] : 0.0f;
+            for (int k = 0; k < RN_KEEP; k++) v[k] = 0.0f;
+        } else {
+#pragma unroll
+            for (int k = 0; k < RN_KEEP; k++) {
+                const int i = c0 + threadIdx.x + k * 256;
+                v[k] = i < cols ? row[i] : 0.0f;
+            }
+        }
+        if constexpr (PARTS) {
+            const float * src = parts.partial + (int64_t)r * cols + c0 + threadIdx.x;
+            float chunk[RN_KEEP], total[RN_KEEP];
+#pragma unroll
+            for (int k = 0; k < RN_KEEP; k++) chunk[k] = total[k] = 0.0f;
+            bool first = true;
+            for (uint64_t left = cut.parts; left;) {
+                constexpr int AHEAD = 4;  // parts in flight
+                float ld[AHEAD][RN_KEEP];
+                uint64_t ahead = left;
+#pragma unroll
+                for (int u = 0; u < AHEAD; u++) {
+#pragma unroll
+                    for (int k = 0; k < RN_KEEP; k++)
+                        ld[u][k] = ahead && c0 + threadIdx.x + k * 256 < cols ? __ldcg(src + (int64_t)u * rows * cols + k * 256) : 0.0f;
+                    ahead &= ahead - 1;
+                }
+#pragma unroll
+                for (int u = 0; u < AHEAD; u++) {
+                    if (!left) break;
+                    const uint64_t bit = left & (~left + 1);
+                    left &= left - 1;
+#pragma unroll
+                    for (int k = 0; k < RN_KEEP; k++) chunk[k] = first ? ld[u][k] : chunk[k] + ld[u][k];
+                    first = (cut.chunks & bit) != 0;
+                    if (first) {
+#pragma unroll
+                        for (int k = 0; k < RN_KEEP; k++) total[k] = many ? total[k] + chunk[k] : chunk[k];
+                    }
+                }
+                src += (int64_t)AHEAD * rows * cols;
+            }
+#pragma unroll
+            for (int k = 0; k < RN_KEEP; k++) {
+                const int i = c0 + threadIdx.x + k * 256;
+                v[k] = accumulate ? v[k] + total[k] : total[k];
+                if (i < cols) row[i] = v[k];
+            }
+        }
+#pragma unroll
+        for (int k = 0; k < RN_KEEP; k++)
+            if (c0 + threadIdx.x + k * 256 < cols) sum += (double)v[k] * (double)v[k];
     }
-#pragma unroll
-    for (int k = 0; k < RMS_KEEP; k++)
-        if (threadIdx.x + k * 256 < cols) sum += (double)v[k] * (double)v[k];
-    for (int i = threadIdx.x + RMS_KEEP * 256; i < cols; i += 256) sum += (double)x[i] * (double)x[i];
     sum = block_sum_d(sum, red);
     const float mean = (float)(sum / (double)cols);
-    const float scale = (float)(1.0 / sqrt((double)(mean + eps)));
+    const float scale = (float)(1.0 / sqrt((double)(mean + norm.eps)));
+    const bool one = cols <= RN_SPAN;  // the row is still in registers (otherwise each thread reads its own columns again)
+    for (int c0 = 0; c0 < cols; c0 += RN_SPAN) {
 #pragma unroll
-    for (int k = 0; k < RMS_KEEP; k++) {
-        const int i = threadIdx.x + k * 256;
-        if (i < cols) dst[i] = __float2half_rn(v[k] * scale * w[k]);
+        for (int k = 0; k < RN_KEEP; k++) {
+            const int i = c0 + threadIdx.x + k * 256;
+            if (i >= cols) continue;
+            if (!one) {
+                v[k] = row[i];
+                w[k] = norm.w[i];
+            }
+            const float o = v[k] * scale * w[k];
+            if constexpr (HI) {
+                norm.prep.xh[(int64_t)r * cols + i] = __float2half_rn(o);
+            } else {
+                norm.xn[(int64_t)r * norm.ldxn + i] = o;
+                stage[i - c0] = o;
+            }
+        }
+        if constexpr (!HI) {
+            if (!norm.prep.xh) continue;
+            __syncthreads();
+            for (int gq = threadIdx.x; gq < (min(RN_SPAN, cols - c0) >> 4); gq += 256) {
+                float g16[16];
+                load16(stage + gq * 16, g16);
+                const int64_t at = (int64_t)r * cols + c0 + gq * 16;
+                xprep_store16(norm.prep.xh + at, norm.prep.xl + at, norm.prep.xs16 + (at >> 4), g16);
+            }
+            __syncthreads();
+        }
     }
-    for (int i = threadIdx.x + RMS_KEEP * 256; i < cols; i += 256) dst[i] = __float2half_rn(x[i] * scale * weight[i]);
+}
+
+void launch_rows_norm(cudaStream_t s, float * out, int64_t ldo, const RowParts & parts, int rows, int cols, bool accumulate, const RowNorm & norm) {
+    YK_REQUIRE(!norm.prep.xh || (cols & 15) == 0, YUUKA_ERR_UNSUPPORTED, "rmsnorm: prepared output needs a width that is a multiple of 16");
+    auto kern = norm.prep.hi_only() ? (parts.partial ? rows_norm_kernel<true, true> : rows_norm_kernel<true, false>)
+                                    : (parts.partial ? rows_norm_kernel<false, true> : rows_norm_kernel<false, false>);
+    launch_k(kern, rows, 256, 0, s, out, ldo, parts, rows, cols, accumulate ? 1 : 0, norm);
+    YK_CUDA(cudaGetLastError());
 }
 
 void launch_rmsnorm(cudaStream_t s, float * dst, int ldd, const float * src, int lds, const float * weight, int cols,
                     int rows, float eps, XPrepOut prep, unsigned long long * sumsq_out) {
     YK_REQUIRE(!prep.xh || ((cols & 15) == 0 && (ldd & 3) == 0), YUUKA_ERR_UNSUPPORTED,
                "rmsnorm: prepared output needs a width that is a multiple of 16");
-    if (prep.hi_only() && !sumsq_out) {
-        launch_k(rmsnorm_hi_kernel, rows, 256, 0, s, prep.xh, src, lds, weight, cols, eps);
-        YK_CUDA(cudaGetLastError());
+    if (!sumsq_out) {
+        launch_rows_norm(s, const_cast<float *>(src), lds, RowParts(), rows, cols, true, RowNorm{weight, eps, dst, ldd, prep});  // (src is only read)
         return;
     }
     launch_k(rmsnorm_kernel, rows, 256, 0, s, dst, ldd, src, lds, weight, cols, eps, prep, sumsq_out);

@@ -4,9 +4,11 @@
 // verify step: k+1 (or tree) rows through every layer, on-device acceptance,
 // KV / recurrent-state commit.
 #include <algorithm>
+#include <array>
 #include <cstdlib>
 #include <cstring>
 #include <map>
+#include <set>
 #include <string>
 #include <vector>
 
@@ -569,6 +571,7 @@ struct yuuka_session {
     // L2 prefetch of the next GEMM's weights: matrices in the order a step streams them
     bool prefetch_next = true;
     bool all_tiled = false;          // every matrix of the layers and the head is in the tiled layout
+    std::set<std::array<int, 4>> reserved;  // (rows, dtype, n_out, n_in) whose GEMM scratch is there
     bool hi_step = false;            // this step's matrices read the hi halves of their inputs alone
     uint8_t * gdn_chunk_scratch = nullptr;  // row-by-row matrices of a prompt pass
     bool gdn_chunked = true;  // prompt sub-chunks through the chunkwise delta-net scan (YUUKA_CUDA_NO_GDN_CHUNK=1: row by row)
@@ -626,7 +629,7 @@ void mark(yuuka_session * s, uint32_t code) {
 }
 
 void gemm(yuuka_session * s, const Tensor & w, const float * x, int ldx, XPrepOut prep, float * out, int ldo, int rows,
-          uint32_t flags, const float * produce_norm_w = nullptr, const XPrepOut * swiglu = nullptr) {
+          uint32_t flags, const float * produce_norm_w = nullptr, const XPrepOut * swiglu = nullptr, const RowNorm * row_norm = nullptr) {
     mark(s, w.rows > 65536 ? YUUKA_OP_LM_HEAD : YUUKA_OP_GEMM);
     if (w.tiled) {
         TiledGemmArgs t;
@@ -648,6 +651,7 @@ void gemm(yuuka_session * s, const Tensor & w, const float * x, int ldx, XPrepOu
         t.wide_from_33 = (s->cfg.flags & YUUKA_SESSION_WIDE_FROM_33) != 0;
         if (s->cfg.flags & YUUKA_SESSION_TEST_DROP_COPIES) t.flags |= YUUKA_GEMM_TEST_DROP_COPIES;
         if (swiglu) t.swiglu = *swiglu;
+        t.row_norm = row_norm;
         if (s->fold_step) {
             const yuuka_model_config & mc = s->model->cfg;
             t.norm.eps = mc.rms_eps;
@@ -729,6 +733,11 @@ void gemm_residual_norm(yuuka_session * s, const Tensor & w, const float * in, i
         s->xn_raw = true;
         return;
     }
+    if (norm_w && w.tiled) {
+        const RowNorm norm{norm_w, c.rms_eps, s->xn, H, step_prep_xn(s)};
+        gemm(s, w, in, ld_in, prep_in, s->x, H, rows, YUUKA_GEMM_ACCUMULATE, nullptr, nullptr, &norm);
+        return;
+    }
     gemm(s, w, in, ld_in, prep_in, s->x, H, rows, YUUKA_GEMM_ACCUMULATE);
     if (norm_w) {
         mark(s, YUUKA_OP_RMSNORM);
@@ -760,7 +769,8 @@ bool matrices_tiled(const yuuka_model & m) {
 }
 
 void reserve_gemm(yuuka_session * s, const Tensor & w, int rows) {
-    if (w.present()) gemm_scratch_reserve(s->model->dev, s->gemm, w.dtype, rows, (int)w.rows, (int)w.cols);
+    if (w.present() && s->reserved.insert({rows, (int)w.dtype, (int)w.rows, (int)w.cols}).second)
+        gemm_scratch_reserve(s->model->dev, s->gemm, w.dtype, rows, (int)w.rows, (int)w.cols);
 }
 
 enum LogitRows { LOGITS_NONE, LOGITS_LAST, LOGITS_ALL };
@@ -1040,7 +1050,9 @@ void run_step(yuuka_session * s, int seq0, int batch, int nodes, uint32_t mode, 
             continue;
         }
         // forwardFFN (model/qwen35/forward.go:295-315); its input norm came with the mixer's output GEMM
-        if (L.gate_up.present() && L.gate_up.paired && L.gate_up.tiled && L.ffn_down.tiled && s->fold_swiglu && R <= 32) {
+        const bool fold_rows = gemm_tiled_rows_swiglu(R, H, (s->cfg.flags & YUUKA_SESSION_EXACT_WIDE) != 0,
+                                                      (s->cfg.flags & YUUKA_SESSION_WIDE_FROM_33) != 0);
+        if (L.gate_up.present() && L.gate_up.paired && L.gate_up.tiled && L.ffn_down.tiled && s->fold_swiglu && (R <= 32 || fold_rows)) {
             // silu(gate) * up leaves the GEMM's epilogue in the form the down projection reads
             gemm(s, L.gate_up, s->xn, H, s->prep_xn, s->gate_up, 2 * F, R, 0, nullptr, &s->prep_act);
         } else {

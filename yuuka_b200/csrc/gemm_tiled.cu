@@ -1166,9 +1166,10 @@ __global__ void __launch_bounds__(MW * 32, 1) gemm_tiled_mma_kernel(const TParam
 // Register-fed kernel for more activation rows than one launch of the kernel above holds (17 to 48): every weight record is
 // decoded once and multiplied with all of them.
 //
-// A CTA has up to eight warps, a 16-row tile each, that walk the superblocks of K together (a ninth warp for the copies would
-// leave a thread 168 registers instead of 255); the first one also has the superblocks' activations of all rows brought two
-// ahead by TMA (hi and lo halves in boxes of 64 columns, swizzled, and the sums). The columns of a row need not fit shared memory, so K is not cut for that; where a matrix has few tiles, ranges of
+// A CTA has up to eight warps, a 16-row tile each, that walk the superblocks of K together (a ninth warp for the copies
+// would leave a thread 168 registers instead of 255); the first one also has the superblocks' activations of all rows
+// brought two ahead by TMA (hi and lo halves in boxes of 64 columns, swizzled, and the sums). The columns of a row need
+// not fit shared memory, so K is not cut for that; where a matrix has few tiles, ranges of
 // K go to different CTAs. What bounds it: 32 products per four activation rows, superblock and tile, 2.1 cycles each, 310
 // cycles per record at 36 rows, of which the two warps of a scheduler reach some 40 % between decode, reads and folds.
 // In a step of 36 rows (three passes of sixteen before): 12352 x 2560 Q4_K 52 -> 35 us, 2560 x 4096 Q4_K 38 -> 23,
@@ -1179,10 +1180,6 @@ __global__ void __launch_bounds__(MW * 32, 1) gemm_tiled_mma_kernel(const TParam
 // runs over a part and is added up at the part's end, 16-row passes and the rest of the rows each at the ends of their own cut.
 constexpr int RW_WARPS = 8, RW_MAX_ROWS = 48, RW_MAX_STAGES = 4, RW_MAX_SPLITS = 8;
 
-// Where K is cut for the rows of a pass: bit sb of `parts` / `chunks`: a part / chunk ends after superblock sb.
-struct RowCut {
-    uint64_t parts, chunks;
-};
 struct RParams {
     DecodeConsts kc;
     const uint8_t * w;
@@ -1196,6 +1193,7 @@ struct RParams {
     RowCut cut[2];       // [0]: rows below first_rest, [1]: the rest
     int first_rest;      // a multiple of 16
     float * partial;     // splits > 1: [part][M][N]
+    XPrepOut swiglu;     // see TParams::sw_xh; splits == 1
     int stages;
     const uint8_t * next_w;  // see TParams
     uint32_t next_lines;
@@ -1367,7 +1365,48 @@ __global__ void __launch_bounds__(RW_WARPS * 32, 1)
                     }
                 }
             }
-            if (p.splits == 1) {
+            if (p.swiglu.xh) {
+                // gate tile 2i and up tile 2i + 1 are neighbouring warps'. The up sums go over through shared memory, the products
+                // come back through it row by row: a lane prepares all sixteen columns of a row.
+                float * ex = reinterpret_cast<float *>(smem + (size_t)p.stages * R::BYTES + RW_WARPS * X::TAB) + (warp >> 1) * (NT * 64);
+                if (warp & 1) {
+#pragma unroll
+                    for (int j = 0; j < NT; j++) {
+                        ex[(2 * j) * 32 + lane] = total[j][0];
+                        ex[(2 * j + 1) * 32 + lane] = total[j][1];
+                    }
+                }
+                asm volatile("bar.sync %0, 64;" ::"r"((warp >> 1) + 1) : "memory");
+                if (!(warp & 1)) {
+#pragma unroll
+                    for (int j = 0; j < NT; j++) {
+                        total[j][0] = swiglu(total[j][0], ex[(2 * j) * 32 + lane]);
+                        total[j][1] = swiglu(total[j][1], ex[(2 * j + 1) * 32 + lane]);
+                    }
+                    __syncwarp();
+#pragma unroll
+                    for (int j = 0; j < NT; j++) {
+                        ex[(4 * j + row_pi(t)) * 16 + g] = total[j][0];
+                        ex[(4 * j + row_pi(t)) * 16 + g + 8] = total[j][1];
+                    }
+                    __syncwarp();
+                    if (rt < n_tiles)
+                        for (int tok = lane; tok < p.M; tok += 32) {
+                            float v[16];
+#pragma unroll
+                            for (int i = 0; i < 4; i++) {
+                                const float4 q = reinterpret_cast<const float4 *>(ex + tok * 16)[i];
+                                v[4 * i] = q.x;
+                                v[4 * i + 1] = q.y;
+                                v[4 * i + 2] = q.z;
+                                v[4 * i + 3] = q.w;
+                            }
+                            const int64_t at = (int64_t)tok * (p.N >> 1) + (rt >> 1) * 16;
+                            xprep_store16(p.swiglu.xh + at, p.swiglu.xl + at, p.swiglu.xs16 + (at >> 4), v);
+                        }
+                }
+                asm volatile("bar.sync %0, 64;" ::"r"((warp >> 1) + 1) : "memory");
+            } else if (p.splits == 1) {
 #pragma unroll
                 for (int j = 0; j < NT; j++) {
                     const int tok = 4 * j + row_pi(t);
@@ -1728,7 +1767,7 @@ static RowCut row_cut(const yuuka_device * dev, uint32_t dtype, int m, int n_out
     TPlan pl;
     plan_tiled(dev, dtype, m, n_out, n_in, pl);
     const int nsb = n_in / 256;
-    RowCut cut{0, 0};
+    RowCut cut;
     for (int c0 = 0; c0 < nsb; c0 += pl.nsb_chunk) {
         const int cnt = nsb - c0 < pl.nsb_chunk ? nsb - c0 : pl.nsb_chunk;
         for (int k = 1; k <= pl.KS; k++)
@@ -1740,15 +1779,16 @@ static RowCut row_cut(const yuuka_device * dev, uint32_t dtype, int m, int n_out
 
 // How 17 to 48 rows are cut into work for gemm_tiled_rows_kernel: tg tiles per CTA and ranges of K that end where parts of
 // all rows end. The cost is in records per SM (a record takes as long however many warps share the SM's tensor pipe): rounds
-// x (tiles x records + 2 for the start and the stores of an item), and 10 for the launch that adds the ranges up.
-static void plan_rows(const yuuka_device * dev, uint32_t dtype, int m, int n_out, int n_in, RParams & p) {
+// x (tiles x records + 2 for the start and the stores of an item), and 10 for the launch that adds the ranges up. paired: tiles
+// 2i and 2i + 1 share a CTA, all of K (SwiGLU epilogue).
+static void plan_rows(const yuuka_device * dev, uint32_t dtype, int m, int n_out, int n_in, RParams & p, bool paired) {
     const int nsb = n_in / 256, n_tiles = (n_out + 15) / 16;
     p.first_rest = m / 16 * 16;
     p.cut[0] = row_cut(dev, dtype, 16, n_out, n_in);
     p.cut[1] = m > p.first_rest ? row_cut(dev, dtype, m - p.first_rest, n_out, n_in) : p.cut[0];
     const uint64_t ends = p.cut[0].parts & p.cut[1].parts;
     double best = 1e30;
-    for (int splits = 1; splits <= RW_MAX_SPLITS && splits <= nsb; splits++) {
+    for (int splits = 1; splits <= (paired ? 1 : RW_MAX_SPLITS) && splits <= nsb; splits++) {
         int at[RW_MAX_SPLITS + 1], n = 0, longest = 0;
         at[0] = 0;
         for (int sb = 0; sb < nsb; sb++)
@@ -1757,7 +1797,7 @@ static void plan_rows(const yuuka_device * dev, uint32_t dtype, int m, int n_out
                 if (at[n] - at[n - 1] > longest) longest = at[n] - at[n - 1];
             }
         if (n != splits) continue;
-        for (int tg = 4; tg <= RW_WARPS; tg++) {
+        for (int tg = 4; tg <= RW_WARPS; tg += paired ? 2 : 1) {
             const int groups = (n_tiles + tg - 1) / tg, rounds = (groups * splits + dev->sm_count - 1) / dev->sm_count;
             const double cost = rounds * (tg * longest + 2.0) + (splits > 1 ? 10.0 : 0.0);
             if (cost >= best) continue;
@@ -1777,6 +1817,9 @@ static uint64_t rows_partial_floats(const RParams & p, int m, int n_out) {
 // From 17 rows, where passes of sixteen would begin to decode the weights more than once; K of at most 64 superblocks (the
 // masks of RowCut). (Launches that fold a norm or SwiGLU into their epilogue, steps of up to 32 rows, stay with the passes.)
 static bool rows_route(int m, int n_in) { return m > MMA_ROWS && n_in <= 64 * 256; }
+bool gemm_tiled_rows_swiglu(int rows, int n_in, bool exact_only, bool wide_from_33) {
+    return rows > 32 && rows <= RW_MAX_ROWS && rows_route(rows, n_in) && !gemm_tiled_wide(rows, exact_only, wide_from_33);
+}
 
 void gemm_tiled_scratch_need(const yuuka_device * dev, uint32_t w_dtype, int rows, int n_out, int n_in,
                              uint64_t * partial_floats, int * counters) {
@@ -1788,14 +1831,12 @@ void gemm_tiled_scratch_need(const yuuka_device * dev, uint32_t w_dtype, int row
         const int parts = rows >= UMMA_EARLY_ROWS ? umma_kparts(dev, n_out, n_in, m) : 1;
         if (parts > 2 && (uint64_t)parts * m * n_out > *partial_floats) *partial_floats = (uint64_t)parts * m * n_out;
     }
-    for (int m : {rows, RW_MAX_ROWS, 40, 32, 24})
-        if (m <= rows && m <= RW_MAX_ROWS && rows_route(m, n_in)) {
-            for (int mm = m; mm > MMA_ROWS && mm > m - 16; mm--) {
-                RParams p{};
-                plan_rows(dev, w_dtype, mm, n_out, n_in, p);
-                *partial_floats = std::max(*partial_floats, rows_partial_floats(p, mm, n_out));
-            }
-        }
+    // 17 to 48 rows: at most as many parts as the passes of any of these rows have
+    if (rows_route(rows, n_in)) {
+        int parts = 0;
+        for (int m = 1; m <= MMA_ROWS; m++) parts = std::max(parts, __builtin_popcountll(row_cut(dev, w_dtype, m, n_out, n_in).parts));
+        if (parts > 1) *partial_floats = std::max(*partial_floats, (uint64_t)parts * (rows < RW_MAX_ROWS ? rows : RW_MAX_ROWS) * n_out);
+    }
     for (int m : {rows < MMA_ROWS ? rows : MMA_ROWS, MMA_ROWS < rows ? rows % MMA_ROWS : 0}) {
         if (m <= 0) continue;
         for (bool paired : {false, true}) {
@@ -1961,6 +2002,11 @@ static void make_x_map(CUtensorMap * map, const __half * xh, int m, int k, int b
                YUUKA_ERR_INTERNAL, "umma gemm: the tensor map of the activations could not be encoded");
 }
 
+// Whether the launch that adds up the parts of K takes the rows' norm along: one CTA per row, two per SM, so while the rows
+// are one wave. (2560 columns, 36 rows: 4 x 9-row step 5.5 -> 5.3 ms; 512 rows of seven parts: 14 us against 7 to 11 + 5 in
+// two launches, of which the first uses the whole machine evenly.)
+static bool fuse_row_norm(const yuuka_device * dev, const TiledGemmArgs & a) { return a.row_norm && a.rows <= 2 * dev->sm_count; }
+
 template <int DT>
 static int launch_umma_dt(const yuuka_device * dev, cudaStream_t s, const TiledGemmArgs & a, const __half * xh) {
     using S = UmmaStage<DT>;
@@ -1999,6 +2045,13 @@ static int launch_umma_dt(const yuuka_device * dev, cudaStream_t s, const TiledG
     launch_k_cluster(gemm_umma_kernel<DT>, dim3(2 * (items < pairs ? items : pairs)), UM_THREADS, smem, s, 2, p, xmap);
     YK_CUDA(cudaGetLastError());
     if (pl.kparts == 1) return 1;
+    if (fuse_row_norm(dev, a)) {
+        RowParts parts;
+        parts.partial = p.partial;
+        parts.cut[0].parts = parts.cut[0].chunks = parts.cut[1].parts = parts.cut[1].chunks = (1ull << pl.kparts) - 1;
+        launch_rows_norm(s, a.out, a.ldo, parts, a.rows, a.n_out, p.accumulate != 0, *a.row_norm);
+        return 2;
+    }
     const bool vec = (a.n_out & 3) == 0 && (a.ldo & 3) == 0 && ((uintptr_t)a.out & 15) == 0;
     const int64_t want = ((int64_t)a.rows * (a.n_out / (vec ? 4 : 1)) + 255) / 256, most = (int64_t)dev->sm_count * 8;
     launch_k(vec ? umma_reduce_kernel<4> : umma_reduce_kernel<1>, (int)(want < most ? want : most), 256, 0, s, p.out, p.ldo,
@@ -2029,7 +2082,7 @@ static void launch_rows_inst(const yuuka_device * dev, cudaStream_t s, RParams &
     make_x_map(&lo, xp.xl + (int64_t)m0 * K, p.M, K, R::LO_ROWS);
     if (XTab<DT>::SUMS) make_sum_map(&sums, xp.xs16 + (int64_t)m0 * (K / 16), p.M, K, R::HI_ROWS);
     else sums = hi;
-    const size_t fixed = (size_t)RW_WARPS * XTab<DT>::TAB + 1024;
+    const size_t fixed = (size_t)RW_WARPS * XTab<DT>::TAB + (p.swiglu.xh ? (size_t)RW_WARPS / 2 * NT * 256 : 0) + 1024;
     p.stages = RW_MAX_STAGES;
     while (fixed + (size_t)p.stages * R::BYTES + 1024 > dev->prop.sharedMemPerBlockOptin && p.stages > 3) p.stages--;
     const size_t smem = fixed + (size_t)p.stages * R::BYTES;
@@ -2051,11 +2104,15 @@ static int launch_rows_dt(const yuuka_device * dev, cudaStream_t s, const TiledG
     p.out = a.out + (int64_t)m0 * a.ldo;
     p.ldo = a.ldo;
     p.accumulate = (a.flags & YUUKA_GEMM_ACCUMULATE) ? 1 : 0;
-    plan_rows(dev, DT, m, a.n_out, a.n_in, p);
+    plan_rows(dev, DT, m, a.n_out, a.n_in, p, a.swiglu.xh != nullptr);
     if (p.splits > 1) {
         YK_REQUIRE(a.scratch && a.scratch->partial_floats >= rows_partial_floats(p, m, a.n_out), YUUKA_ERR_INTERNAL,
                    "gemm: split-K scratch is too small");
         p.partial = a.scratch->partial;
+    }
+    if (a.swiglu.xh) {
+        const int64_t half = a.n_out / 2;
+        p.swiglu = XPrepOut{a.swiglu.xh + m0 * half, a.swiglu.xl + m0 * half, a.swiglu.xs16 + m0 * (half / 16)};
     }
     if (a.next_w) {
         p.next_w = a.next_w;
@@ -2071,6 +2128,10 @@ static int launch_rows_dt(const yuuka_device * dev, cudaStream_t s, const TiledG
     default: launch_rows_inst<DT, 12>(dev, s, p, xp, m0); break;
     }
     if (p.splits == 1) return 1;
+    if (m == a.rows && fuse_row_norm(dev, a)) {
+        launch_rows_norm(s, p.out, p.ldo, RowParts{p.partial, {p.cut[0], p.cut[1]}, p.first_rest}, m, a.n_out, p.accumulate != 0, *a.row_norm);
+        return 2;
+    }
     launch_k(rows_reduce_kernel, dim3((a.n_out + 255) / 256, m), 256, 0, s, p.out, p.ldo, (const float *)p.partial, m, a.n_out, p.first_rest,
              p.cut[0], p.cut[1], p.accumulate);
     YK_CUDA(cudaGetLastError());
@@ -2080,6 +2141,12 @@ static int launch_rows_dt(const yuuka_device * dev, cudaStream_t s, const TiledG
 template <int DT>
 static int launch_mma_dt(const yuuka_device * dev, cudaStream_t s, const TiledGemmArgs & a) {
     int launches = 0;
+    // the norm of the finished rows, where no launch above has taken it along
+    auto norm = [&](bool taken) {
+        if (!a.row_norm || taken) return 0;
+        launch_rows_norm(s, a.out, a.ldo, RowParts(), a.rows, a.n_out, true, *a.row_norm);
+        return 1;
+    };
     XPrepOut xp = a.xprep;
     const bool wide = gemm_tiled_wide(a.rows, a.exact_only, a.wide_from_33);
     if (!xp.xh) {
@@ -2096,14 +2163,20 @@ static int launch_mma_dt(const yuuka_device * dev, cudaStream_t s, const TiledGe
         xp.xs16 = a.scratch->xs16;
         launches++;
     }
-    if (wide) return launches + launch_umma_dt<DT>(dev, s, a, xp.xh);
+    if (wide) {
+        const int n = launch_umma_dt<DT>(dev, s, a, xp.xh);
+        return launches + n + norm(n > 1 && fuse_row_norm(dev, a));
+    }
     YK_REQUIRE(xp.xl && xp.xs16, YUUKA_ERR_INTERNAL, "gemm: the prepared activations lack their lo halves or sums");
-    const bool folded = a.norm.produce_w || a.norm.consume_now || a.swiglu.xh;
+    const bool folded = a.norm.produce_w || a.norm.consume_now || (a.swiglu.xh && a.rows <= 32);
     int m = 0;
+    bool normed = false;
     for (int m0 = 0; m0 < a.rows; m0 += m) {
         m = a.rows - m0 < RW_MAX_ROWS ? a.rows - m0 : RW_MAX_ROWS;
         if (rows_route(m, a.n_in) && !folded && !(a.flags & YUUKA_GEMM_TEST_DROP_COPIES)) {
-            launches += launch_rows_dt<DT>(dev, s, a, xp, m0, m);
+            const int n = launch_rows_dt<DT>(dev, s, a, xp, m0, m);
+            normed = n > 1 && m == a.rows && fuse_row_norm(dev, a);
+            launches += n;
             continue;
         }
         m = m < MMA_ROWS ? m : MMA_ROWS;
@@ -2123,7 +2196,7 @@ static int launch_mma_dt(const yuuka_device * dev, cudaStream_t s, const TiledGe
         }
         launches++;
     }
-    return launches;
+    return launches + norm(normed);
 }
 
 template <int DT, typename XT>
@@ -2159,7 +2232,7 @@ static int launch_fp32_dt(const yuuka_device * dev, cudaStream_t s, const TiledG
 template <int DT>
 static int launch_tiled_dt(const yuuka_device * dev, cudaStream_t s, const TiledGemmArgs & a, bool mma) {
     if (mma) return launch_mma_dt<DT>(dev, s, a);
-    YK_REQUIRE(a.x, YUUKA_ERR_INVALID_ARGUMENT, "gemm fp32 route: needs the f32 / bf16 activations");
+    YK_REQUIRE(a.x && !a.row_norm, YUUKA_ERR_INVALID_ARGUMENT, "gemm fp32 route: needs the f32 / bf16 activations, and folds no norm");
     return a.x_dtype == YUUKA_DTYPE_F32 ? launch_fp32_dt<DT, float>(dev, s, a) : launch_fp32_dt<DT, __nv_bfloat16>(dev, s, a);
 }
 
@@ -2171,7 +2244,9 @@ int launch_gemm_tiled(const yuuka_device * dev, cudaStream_t stream, const Tiled
                    YUUKA_ERR_INVALID_ARGUMENT, "gemm: the SwiGLU epilogue needs gate and up tiles in pairs and a plain output");
         YK_REQUIRE(!a.norm.consume_now || a.norm.cols > 0, YUUKA_ERR_INVALID_ARGUMENT, "gemm: the folded RMSNorm needs the row width");
     }
-    if (a.norm.produce_w || a.norm.consume_now || a.swiglu.xh) {
+    if (a.swiglu.xh && !a.norm.consume_now && gemm_tiled_rows_swiglu(a.rows, a.n_in, a.exact_only, a.wide_from_33)) {
+        YK_REQUIRE(a.swiglu.xl, YUUKA_ERR_INTERNAL, "gemm: the SwiGLU epilogue writes both halves");
+    } else if (a.norm.produce_w || a.norm.consume_now || a.swiglu.xh) {
         const uint32_t route = a.path == YUUKA_GEMM_PATH_AUTO ? YUUKA_GEMM_PATH_MMA : a.path;
         YK_REQUIRE(route == YUUKA_GEMM_PATH_MMA && a.rows <= 32 && (a.rows < UMMA_MIN_ROWS || !umma_enabled()) &&
                        (!a.swiglu.xh || a.swiglu.xl) && (!a.norm.produce_w || a.norm.produce_prep.xl),

@@ -94,8 +94,11 @@ struct TiledGemmArgs {
     GemmScratch * scratch = nullptr;  // needed when the plan splits K across CTAs
     NormFuse norm;
     // Set: `w` holds ffn_gate and ffn_up interleaved by 16-row tile and the launch writes silu(gate) * up in
-    // prepared form, [rows][n_out / 2], instead of `out` (register-fed mma route, up to 32 rows).
+    // prepared form, [rows][n_out / 2], instead of `out` (register-fed mma routes, up to 48 rows).
     XPrepOut swiglu;
+    // Set: xn = rmsnorm(out) follows, in the launch that adds up the parts of K where there is one. (The caller launches the
+    // norm itself with the folded form, `norm`.)
+    const RowNorm * row_norm = nullptr;
     const uint8_t * next_w = nullptr;  // optional L2 prefetch hint: the next matrix to be streamed (mma route)
     uint64_t next_bytes = 0;
 };
@@ -103,6 +106,8 @@ struct TiledGemmArgs {
 int launch_gemm_tiled(const yuuka_device * dev, cudaStream_t stream, const TiledGemmArgs & a);
 // whether a launch of so many rows takes the tensor-memory route, which reads the hi halves of the activations alone
 bool gemm_tiled_wide(int rows, bool exact_only, bool wide_from_33);
+// whether a launch of more rows than the folded epilogues of the step take (32) can still fold SwiGLU into its own
+bool gemm_tiled_rows_swiglu(int rows, int n_in, bool exact_only, bool wide_from_33);
 // Scratch the launch above needs for this shape (0 partial floats when K is not split across CTAs).
 void gemm_tiled_scratch_need(const yuuka_device * dev, uint32_t w_dtype, int rows, int n_out, int n_in,
                              uint64_t * partial_floats, int * counters);

@@ -11,6 +11,7 @@
 #pragma once
 
 #include <cuda_fp16.h>
+#include <cuda_runtime.h>
 
 #include <cstdint>
 
@@ -22,6 +23,29 @@ struct XPrepOut {
     __half * xl = nullptr;     // [rows][cols]
     __half2 * xs16 = nullptr;  // [rows][cols / 16]
 };
+
+// Where K is cut for a row: bit sb of `parts` / `chunks`: a part / chunk of the sum ends after superblock sb.
+struct RowCut {
+    uint64_t parts = 0, chunks = 0;
+};
+// Sums of a GEMM whose K ranges went to different CTAs, [part][rows][cols]: the value of an element is its parts added in
+// order within a chunk, then its chunks in order. Rows from first_rest on have a cut of their own.
+struct RowParts {
+    const float * partial = nullptr;
+    RowCut cut[2];
+    int first_rest = 0;
+};
+// RMSNorm of the rows a GEMM has just finished: xn = rmsnorm(out) * w, and its prepared form.
+struct RowNorm {
+    const float * w = nullptr;
+    float eps = 0.0f;
+    float * xn = nullptr;
+    int ldxn = 0;
+    XPrepOut prep;
+};
+
+// out (+)= the sums in `parts`, xn = rmsnorm(out): one CTA per row (cols: of out, of the parts and of xn)
+void launch_rows_norm(cudaStream_t s, float * out, int64_t ldo, const RowParts & parts, int rows, int cols, bool accumulate, const RowNorm & norm);
 
 // dst_* and v cover 16 consecutive elements starting at a multiple of 16
 __device__ __forceinline__ void xprep_store16(__half * dst_hi, __half * dst_lo, __half2 * sum, const float (&v)[16]) {
