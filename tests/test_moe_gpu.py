@@ -95,3 +95,27 @@ def test_batched_tree_rows_spread_over_experts(moe):
         assert err <= LOGIT_TOL and cosine(res.logits[b], log_o) >= 0.9999, (b, err)
         states[b].close()
     sess.close()
+
+
+@pytest.mark.parametrize("experts,used,hidden,n", [
+    (8, 2, 256, 300),     # more pairs than a group of every warp takes
+    (256, 3, 256, 33),    # as many experts as eight logits per lane hold
+    (257, 4, 512, 9), (8, 8, 256, 17),   # one more; every expert of every row
+])
+def test_routing_at_the_edges_of_its_layout(experts, used, hidden, n):
+    cfg = synth.tiny_moe_config()
+    cfg.update(expert_count=experts, expert_used=used, hidden=hidden, vocab=512)
+    tensors = synth.make_model(cfg, "q4_k_m", seed=49, unit_norms=False)
+    dev = cuda.Device(0)
+    gm, om = cuda.Model(dev, cfg, tensors), yo.Model(cfg, tensors)
+    sess = cuda.Session(gm, max_batch=1, max_nodes=1, capacity=320, kv_format=cuda.KV_F32)
+    prompt = synth.uniform_i32(n, 0, cfg["vocab"], 5)
+    st = yo.State(om, 320, yo.KV_F32)
+    want, got = st.forward(prompt), sess.forward(prompt)
+    st.close()
+    # (wide passes round the activations to fp16, and a near tie of the router may then fall the other way)
+    cos = float(np.dot(got, want) / (np.linalg.norm(got) * np.linalg.norm(want)))
+    assert cos >= (0.99999 if n < 48 else 0.99), cos
+    sess.close()
+    gm.close()
+    dev.close()

@@ -281,6 +281,7 @@ void launch_tile_weights(cudaStream_t s, uint8_t * dst, const uint8_t * src, uin
 template <typename XT>
 __global__ void xprep_kernel(__half * __restrict__ xh, __half * __restrict__ xl, __half2 * __restrict__ xs16, const XT * __restrict__ x, int64_t ldx,
                              int K, int M) {
+    pdl_entry();  // (the GEMM that follows sets itself up and asks for its weights meanwhile)
     const int groups = K >> 4;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < M * groups; i += gridDim.x * blockDim.x) {
         const int m = i / groups, gq = i - m * groups;
@@ -299,7 +300,7 @@ __global__ void xprep_kernel(__half * __restrict__ xh, __half * __restrict__ xl,
 template <typename XT>
 static void launch_xprep(cudaStream_t s, __half * xh, __half * xl, __half2 * xs16, const XT * x, int64_t ldx, int K, int M) {
     const int total = M * (K / 16);
-    xprep_kernel<XT><<<(total + 127) / 128, 128, 0, s>>>(xh, xl, xs16, x, ldx, K, M);
+    launch_k(xprep_kernel<XT>, (total + 127) / 128, 128, 0, s, xh, xl, xs16, x, ldx, K, M);
     YK_CUDA(cudaGetLastError());
 }
 
