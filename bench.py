@@ -391,7 +391,7 @@ def run_c2(args, rank: int, local_rank: int, world: int) -> None:
             "e2e": {"value": emitted_all / t_e2e, "unit": UNIT, "ms_per_step": t_e2e / args.steps * 1e3,
                     # one copy in: ancestor masks, tokens, parents, depths, the slot's sequence; one copy out:
                     # accepted count, path, emitted tokens, plus the two device error words
-                    "h2d_bytes_per_step": rows * (8 + 4 + 4 + 4) + 4, "d2h_bytes_per_step": 4 + 2 * rows * 4 + 8},
+                    "h2d_bytes_per_step": rows * (8 + 4 + 4 + 4 + 4) + 4, "d2h_bytes_per_step": 4 + 2 * rows * 4 + 8},
             "gpu_launches": launches * args.steps,
             "clocks": clocks,
             "roofline": {"bound": "hbm", "kernel": "gemm_tiled_mma_kernel (every quantized GEMM launch of a step, LM head included)",
@@ -609,9 +609,9 @@ def run_c3(args, rank: int, local_rank: int, world: int) -> None:
                            "l2": "no flush needed: a step streams gigabytes of weights, KV rows and state"},
                 "accepted_per_step": accepted_total / args.steps, "emitted_per_step": emitted_total / args.steps,
                 "e2e": {"value": tot.emitted / tot.wall_s, "unit": UNIT, "ms_per_step": tot.wall_s / args.steps * 1e3,
-                        "h2d_bytes_per_step": R * 20 + B * 4 + R * 8, "d2h_bytes_per_step": B * 4 + 2 * R * 4 + 8},
+                        "h2d_bytes_per_step": R * 24 + B * 4 + R * 8, "d2h_bytes_per_step": B * 4 + 2 * R * 4 + 8},
                 "gpu_launches": launches * args.steps, "clocks": clocks,
-                "roofline": {"bound": "tensor", "kernel": "gemm_umma_ws_kernel (every quantized GEMM of a step; 512 rows per launch)",
+                "roofline": {"bound": "tensor", "kernel": "gemm_umma_kernel (every quantized GEMM of a step)",
                              "achieved": flops / (ms * 1e-3) / 1e12, "peak": peaks["bf16_tflops_sustained"], "unit": "TFLOP/s",
                              "frac": flops / (ms * 1e-3) / 1e12 / peaks["bf16_tflops_sustained"], "peak_source": peaks["source"],
                              "note": "whole-step time in the denominator: attention, the recurrent scan and acceptance are inside it",

@@ -286,13 +286,11 @@ typedef struct yuuka_session_config {
 /* Steps and prompt passes of 48 rows or more normally take the tensor-memory GEMM route, which rounds
  * the decoded weights and the activations to fp16 (about 1e-3 relative per product; logits of a deep
  * model then sit around 1e-2 of the fp32 CPU path, and a qwen35moe router may pick another expert at a
- * near-tie). With this flag such passes run as 16-row passes of the register-fed route instead, which
- * multiplies exact integer weights with two-half activations (fp32-level results, weights streamed once
- * per 16 rows). */
+ * near-tie). With this flag such passes run as passes of at most 48 rows on the register-fed route instead,
+ * which multiplies exact integer weights with two-half activations (fp32-level results). */
 #define YUUKA_SESSION_EXACT_WIDE 0x1u
-/* The other way round: steps of 33..47 rows, which by default run as three exact 16-row passes, also take the
- * tensor-memory route (one pass over the weights: a 36-row step of the 4B model 8.1 -> 4.7 ms) at that route's
- * fp16-rounded precision. For hosts that batch a handful of sequences per step and prefer the speed. */
+/* The other way round: steps of 33..47 rows, which by default run on the exact route, also take the tensor-memory
+ * route, at its fp16-rounded precision. For hosts that batch a handful of sequences per step and prefer the speed. */
 #define YUUKA_SESSION_WIDE_FROM_33 0x2u
 /* Test hook: every GEMM of the session's steps carries YUUKA_GEMM_TEST_DROP_COPIES. */
 #define YUUKA_SESSION_TEST_DROP_COPIES 0x80000000u
@@ -380,7 +378,7 @@ YUUKA_API yuuka_status yuuka_verify_step(yuuka_session * s, const yuuka_verify_b
 /* The acceptance stage on its own, over f32 logits [batch, nodes, vocab] that are already on the device: the
  * greedy walk (argmaxLogit first-maximum rule, engine/speculative.go:263-271, along the tree) or the rejection-
  * sampling walk, with the arguments' meaning as in yuuka_verify_batch (tokens, parent, uniforms on the host;
- * draft_probs on the device). Row metadata and scratch are allocated for the call. begin / end (optional) are
+ * draft_probs on the device). The scratch stays with the stream (at most 16 MiB). begin / end (optional) are
  * recorded around the acceptance kernels. Synchronous. */
 YUUKA_API yuuka_status yuuka_accept_tree(yuuka_stream * stream, const yuuka_buffer * logits, int32_t batch, int32_t nodes,
                                          int32_t vocab, const int32_t * tokens, const int32_t * parent, uint32_t mode,
