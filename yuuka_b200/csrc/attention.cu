@@ -9,6 +9,7 @@
 #include <cuda_fp16.h>
 
 #include <cfloat>
+#include <algorithm>
 #include <cstdlib>
 #include <type_traits>
 
@@ -355,6 +356,7 @@ __global__ void __launch_bounds__(RB * 64, RB <= 3 ? 2 : 1) attention_mma_kernel
             asm volatile("cp.async.commit_group;" ::: "memory");
         } else {
             __syncthreads();
+#pragma unroll 2
             for (int i = threadIdx.x; i < PIECES; i += THREADS) {
                 const int j = i / (HD / 8), c8 = i - j * (HD / 8);
                 const int pos = k0 + j;
@@ -649,7 +651,11 @@ static int launch_attention_hd(cudaStream_t s, float * out, int ldo, const float
     static const bool use_mma = [] { const char * e = getenv("YUUKA_CUDA_ATTN_FP32"); return !(e && e[0] == '1'); }();
     if (use_mma) {
         // tensor-core partials; keys are taken as they are from an F16 pool and split into hi + lo otherwise
-        const int rb = attention_row_blocks(G * rows.nodes), qtiles = (G * rows.nodes + 16 * rb - 1) / (16 * rb);
+        // (F32 and Q8_0 rows are converted on the way in: the ten warps of the largest CTA do that where one holds all rows.
+        // With the two warps of a one-row step alone it took 33 us more per layer over 2500 Q8_0 rows)
+        const bool convert = pool.format != YUUKA_KV_F16;
+        const int blocks = attention_row_blocks(G * rows.nodes), rb = convert && G * rows.nodes <= 16 * AM_RB_MAX ? AM_RB_MAX : blocks;
+        const int qtiles = (G * rows.nodes + 16 * rb - 1) / (16 * rb);
         auto launch = [&](auto ksplit) {
             constexpr bool KS = decltype(ksplit)::value;
             auto with = [&](auto kern) {
@@ -665,7 +671,7 @@ static int launch_attention_hd(cudaStream_t s, float * out, int ldo, const float
             default: with(attention_mma_kernel<HD, KS, 5>); break;
             }
         };
-        if (pool.format != YUUKA_KV_F16) launch(std::true_type());
+        if (convert) launch(std::true_type());
         else launch(std::false_type());
         YK_CUDA(cudaGetLastError());
     } else {

@@ -777,12 +777,12 @@ __device__ __forceinline__ __half2 prep_sum(float gs) {
 // Register-fed kernel: one CTA of MW warps per SM, at most MMA_ROWS activation rows per launch. Row m of
 // the activations occupies two columns of the tensor-core product, 2m (hi half) and 2m + 1 (lo half), which
 // land in the same lane's accumulator pair and are added before anything else happens to them.
-// GROUPED: blockIdx.z walks a device-built list of row segments, each bound to one expert's matrix
+// GROUPED: blockIdx.z walks a device-built list of row segments (sg: this CTA's), each bound to one expert's matrix
 // (qwen35moe expert FFNs). A segment's rows are contiguous in the prepared-activation and output
 // arrays unless row_index redirects the activation rows.
 // FOLD: the RMSNorm on either side of this GEMM is folded into its epilogue (TParams::nf_* / cs_*).
 template <int DT, int NT, bool GROUPED, bool FOLD>
-__global__ void __launch_bounds__(MW * 32, 1) gemm_tiled_mma_kernel(const TParams p) {
+__device__ __forceinline__ void tiled_mma_body(const TParams & p, const GemmSegment & sg) {
     using C = Codec<DT>;
     using X = XTab<DT>;
     using MM = XMma<DT, NT>;
@@ -800,11 +800,6 @@ __global__ void __launch_bounds__(MW * 32, 1) gemm_tiled_mma_kernel(const TParam
     int Mrows = p.M;
     const int32_t * row_index = nullptr;
     if constexpr (GROUPED) {
-        // the segment list is written by the kernel before this one: nothing can start ahead of the wait
-        pdl_trigger();
-        pdl_wait();
-        const GemmSegment sg = p.segments[blockIdx.z];
-        if (sg.count <= 0) return;  // the whole CTA: unused slot of the segment list
         wbase += (size_t)sg.expert * p.expert_stride;
         Mrows = sg.count;
         outp += (int64_t)sg.row0 * p.ldo;
@@ -1091,7 +1086,7 @@ __global__ void __launch_bounds__(MW * 32, 1) gemm_tiled_mma_kernel(const TParam
                 if (FOLD && p.sw_xh) {
                     // gate and up columns of the group, 16 by 16 (nrows is a multiple of 32: row tiles come in pairs)
                     const int half_rows = nrows >> 1, half_n = p.N >> 1, live_n = Mrows * half_rows;
-                    for (int i = threadIdx.x; i < ((live_n + 31) & ~31); i += MW * 32) {
+                    for (int i = threadIdx.x; i < ((live_n + 31) & ~31); i += blockDim.x) {
                         const bool live = i < live_n;
                         const int tok = live ? i / half_rows : 0, cl = live ? i - tok * half_rows : 0;
                         const int n = row0 + (cl >> 4) * 32 + (cl & 15);
@@ -1115,7 +1110,7 @@ __global__ void __launch_bounds__(MW * 32, 1) gemm_tiled_mma_kernel(const TParam
                         }
                     }
                 } else
-                for (int i = threadIdx.x; i < padded; i += MW * 32) {
+                for (int i = threadIdx.x; i < padded; i += blockDim.x) {
                     const bool live = i < Mrows * nrows;
                     const int tok = live ? i / nrows : 0, n = row0 + (live ? i - tok * nrows : 0);
                     float s = 0.0f;
@@ -1157,10 +1152,27 @@ __global__ void __launch_bounds__(MW * 32, 1) gemm_tiled_mma_kernel(const TParam
 
     pdl_trigger_late();
     if (p.next_w) {
-        const uint32_t first = ((blockIdx.y * gridDim.x + blockIdx.x) * (MW * 32) + threadIdx.x);
-        const uint32_t step = gridDim.x * gridDim.y * (MW * 32);
+        const uint32_t first = ((blockIdx.y * gridDim.x + blockIdx.x) * blockDim.x + threadIdx.x);
+        const uint32_t step = gridDim.x * gridDim.y * blockDim.x;
         for (uint32_t line = first; line < p.next_lines; line += step) prefetch_l2(p.next_w + (size_t)line * 128);
     }
+}
+
+template <int DT, int NT, bool FOLD>
+__global__ void __launch_bounds__(MW * 32, 1) gemm_tiled_mma_kernel(const TParams p) {
+    tiled_mma_body<DT, NT, false, FOLD>(p, GemmSegment{});
+}
+// One CTA (or a few) per segment. The segments of a routed step hold five rows on average: up to four take one product tile
+// and the others two (moe 32 x 5 rows, 256 experts).
+template <int DT>
+__global__ void __launch_bounds__(MW * 32, 1) gemm_tiled_grouped_kernel(const TParams p) {
+    // the segment list is written by the kernel before this one: nothing can start ahead of the wait
+    pdl_trigger();
+    pdl_wait();
+    const GemmSegment sg = p.segments[blockIdx.z];
+    if (sg.count <= 0) return;  // the whole CTA: unused slot of the segment list
+    if (sg.count <= GEMM_SEGMENT_ROWS / 2) tiled_mma_body<DT, GEMM_SEGMENT_ROWS / 8, true, false>(p, sg);
+    else tiled_mma_body<DT, GEMM_SEGMENT_ROWS / 4, true, false>(p, sg);
 }
 
 // ===========================================================================
@@ -1693,9 +1705,16 @@ static void plan_tiled(const yuuka_device * dev, uint32_t dtype, int m, int n_ou
     }
     pl.KS = ks;
     pl.TG = MW / ks;
-    pl.n_groups = (n_tiles + pl.TG - 1) / pl.TG;
     pl.nsb_chunk = (nsb + kchunks - 1) / kchunks;
     pl.kchunks = (nsb + pl.nsb_chunk - 1) / pl.nsb_chunk;
+    // one wave with SMs to spare: fewer tiles (warps) per CTA on more of them, at least four warps: 772 tiles in two parts
+    // of K are 129 CTAs of twelve warps instead of 97 of sixteen (a 9-row step 2.75 -> 2.66 ms, one of the 256-column model
+    // 203 -> 171 us)
+    const int spread = (n_tiles * pl.kchunks + slots - 1) / slots, fewest = (4 + ks - 1) / ks;
+    int tg = spread > fewest ? spread : fewest;
+    if (paired) tg = (tg + 1) & ~1;
+    if (tg < pl.TG && (n_tiles + tg - 1) / tg * pl.kchunks <= slots) pl.TG = tg;
+    pl.n_groups = (n_tiles + pl.TG - 1) / pl.TG;
     pl.smem = mma_smem(dtype, m, pl.nsb_chunk, ks, paired);
     int per = slots / pl.kchunks;
     if (per < 1) per = 1;
@@ -1855,7 +1874,7 @@ void gemm_tiled_scratch_need(const yuuka_device * dev, uint32_t w_dtype, int row
 template <int DT, int NT>
 static void launch_mma_inst(cudaStream_t s, const TiledGemmArgs & a, const XPrepOut & xp, int m0, int m, const TPlan & pl) {
     const bool fold = a.norm.produce_w || a.norm.consume_now || a.swiglu.xh;
-    auto kern = fold ? gemm_tiled_mma_kernel<DT, NT, false, true> : gemm_tiled_mma_kernel<DT, NT, false, false>;
+    auto kern = fold ? gemm_tiled_mma_kernel<DT, NT, true> : gemm_tiled_mma_kernel<DT, NT, false>;
     YK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pl.smem));
     TParams p{};
     p.kc = decode_consts(DT);
@@ -1904,14 +1923,13 @@ static void launch_mma_inst(cudaStream_t s, const TiledGemmArgs & a, const XPrep
         p.next_lines = (uint32_t)(a.next_bytes / 128);
     }
     dim3 grid(pl.grid_x, pl.kchunks);
-    launch_k(kern, grid, MW * 32, pl.smem, s, p);
+    launch_k(kern, grid, pl.TG * pl.KS * 32, pl.smem, s, p);
     YK_CUDA(cudaGetLastError());
 }
 
 template <int DT>
 static void launch_grouped_dt(const yuuka_device * dev, cudaStream_t s, const GroupedGemmArgs & a) {
     const int nsb = a.n_in / 256, n_tiles = (a.n_out + 15) / 16;
-    constexpr int NT = (2 * GEMM_SEGMENT_ROWS + 7) / 8;
     TPlan pl;
     pl.KS = 1;
     pl.TG = MW;
@@ -1927,7 +1945,7 @@ static void launch_grouped_dt(const yuuka_device * dev, cudaStream_t s, const Gr
     pl.grid_x = (pl.n_groups + per - 1) / per;
     YK_REQUIRE(pl.smem + 4096 <= dev->prop.sharedMemPerBlockOptin, YUUKA_ERR_UNSUPPORTED,
                "grouped gemm: %d columns of activations do not fit shared memory", a.n_in);
-    auto kern = gemm_tiled_mma_kernel<DT, NT, true, false>;
+    auto kern = gemm_tiled_grouped_kernel<DT>;
     YK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pl.smem));
     TParams p{};
     p.kc = decode_consts(DT);
@@ -2282,15 +2300,15 @@ int launch_gemm_tiled(const yuuka_device * dev, cudaStream_t stream, const Tiled
 template <int DT>
 static void preload_dt() {
     cudaFuncAttributes fa;
-    YK_CUDA(cudaFuncGetAttributes(&fa, gemm_tiled_mma_kernel<DT, 1, false, false>));
-    YK_CUDA(cudaFuncGetAttributes(&fa, gemm_tiled_mma_kernel<DT, 2, false, false>));
+    YK_CUDA(cudaFuncGetAttributes(&fa, gemm_tiled_mma_kernel<DT, 1, false>));
+    YK_CUDA(cudaFuncGetAttributes(&fa, gemm_tiled_mma_kernel<DT, 2, false>));
     YK_CUDA(cudaFuncGetAttributes(&fa, gemm_tiled_rows_kernel<DT, 6>));
     YK_CUDA(cudaFuncGetAttributes(&fa, gemm_tiled_rows_kernel<DT, 8>));
     YK_CUDA(cudaFuncGetAttributes(&fa, gemm_tiled_rows_kernel<DT, 9>));
     YK_CUDA(cudaFuncGetAttributes(&fa, gemm_tiled_rows_kernel<DT, 10>));
     YK_CUDA(cudaFuncGetAttributes(&fa, gemm_tiled_rows_kernel<DT, 12>));
-    YK_CUDA(cudaFuncGetAttributes(&fa, gemm_tiled_mma_kernel<DT, 3, false, false>));
-    YK_CUDA(cudaFuncGetAttributes(&fa, gemm_tiled_mma_kernel<DT, 4, false, false>));
+    YK_CUDA(cudaFuncGetAttributes(&fa, gemm_tiled_mma_kernel<DT, 3, false>));
+    YK_CUDA(cudaFuncGetAttributes(&fa, gemm_tiled_mma_kernel<DT, 4, false>));
     YK_CUDA(cudaFuncGetAttributes(&fa, gemm_tiled_fp32_kernel<DT, float>));
     YK_CUDA(cudaFuncGetAttributes(&fa, gemm_tiled_fp32_kernel<DT, __nv_bfloat16>));
     YK_CUDA(cudaFuncGetAttributes(&fa, gemm_umma_kernel<DT>));
