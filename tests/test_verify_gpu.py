@@ -685,3 +685,17 @@ def test_steps_of_33_to_47_rows_with_folded_tails(B, N, hidden, ffn):
     sess.close()
     gm.close()
     dev.close()
+
+
+@pytest.mark.parametrize("n,kv", [(65, cuda.KV_F16), (155, cuda.KV_Q8_0)])
+def test_prompt_that_fills_a_session_shorter_than_its_chunks(tiny, n, kv):
+    """A pass of 65 rows is two chunks of 64 as far as row bookkeeping goes; the session's tables hold 65."""
+    cfg, gm, om = tiny
+    prompt = synth.uniform_i32(n, 0, cfg["vocab"], 70 + n)
+    st = yo.State(om, n, {cuda.KV_F16: yo.KV_F16, cuda.KV_Q8_0: yo.KV_Q8_0}[kv])
+    want = st.forward(prompt)
+    st.close()
+    sess = cuda.Session(gm, max_batch=1, max_nodes=4, capacity=n, kv_format=kv)
+    got = sess.forward(prompt)
+    sess.close()
+    assert float(np.max(np.abs(got - want))) <= LOGIT_TOL

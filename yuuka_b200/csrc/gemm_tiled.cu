@@ -1835,10 +1835,14 @@ static uint64_t rows_partial_floats(const RParams & p, int m, int n_out) {
     return (uint64_t)parts * m * n_out;
 }
 // From 17 rows, where passes of sixteen would begin to decode the weights more than once; K of at most 64 superblocks (the
-// masks of RowCut). (Launches that fold a norm or SwiGLU into their epilogue, steps of up to 32 rows, stay with the passes.)
-static bool rows_route(int m, int n_in) { return m > MMA_ROWS && n_in <= 64 * 256; }
+// masks of RowCut). Up to 24 rows a matrix of under 1024 records has too little to decode for that to matter: 700 x 2048
+// takes 15.7 us in two passes and 17.5 here at 17 rows, 16.9 and 17.6 at 24. (Launches that fold a norm or SwiGLU into their
+// epilogue, steps of up to 32 rows, stay with the passes.)
+static bool rows_route(int m, int n_out, int n_in) {
+    return m > MMA_ROWS && n_in <= 64 * 256 && (m > 24 || (int64_t)((n_out + 15) / 16) * (n_in / 256) >= 1024);
+}
 bool gemm_tiled_rows_swiglu(int rows, int n_in, bool exact_only, bool wide_from_33) {
-    return rows > 32 && rows <= RW_MAX_ROWS && rows_route(rows, n_in) && !gemm_tiled_wide(rows, exact_only, wide_from_33);
+    return rows > 32 && rows <= RW_MAX_ROWS && rows_route(rows, 16, n_in) && !gemm_tiled_wide(rows, exact_only, wide_from_33);
 }
 
 void gemm_tiled_scratch_need(const yuuka_device * dev, uint32_t w_dtype, int rows, int n_out, int n_in,
@@ -1852,7 +1856,7 @@ void gemm_tiled_scratch_need(const yuuka_device * dev, uint32_t w_dtype, int row
         if (parts > 2 && (uint64_t)parts * m * n_out > *partial_floats) *partial_floats = (uint64_t)parts * m * n_out;
     }
     // 17 to 48 rows: at most as many parts as the passes of any of these rows have
-    if (rows_route(rows, n_in)) {
+    if (rows > MMA_ROWS && n_in <= 64 * 256) {
         int parts = 0;
         for (int m = 1; m <= MMA_ROWS; m++) parts = std::max(parts, __builtin_popcountll(row_cut(dev, w_dtype, m, n_out, n_in).parts));
         if (parts > 1) *partial_floats = std::max(*partial_floats, (uint64_t)parts * (rows < RW_MAX_ROWS ? rows : RW_MAX_ROWS) * n_out);
@@ -2192,7 +2196,7 @@ static int launch_mma_dt(const yuuka_device * dev, cudaStream_t s, const TiledGe
     bool normed = false;
     for (int m0 = 0; m0 < a.rows; m0 += m) {
         m = a.rows - m0 < RW_MAX_ROWS ? a.rows - m0 : RW_MAX_ROWS;
-        if (rows_route(m, a.n_in) && !folded && !(a.flags & YUUKA_GEMM_TEST_DROP_COPIES)) {
+        if (rows_route(m, a.n_out, a.n_in) && !folded && !(a.flags & YUUKA_GEMM_TEST_DROP_COPIES)) {
             const int n = launch_rows_dt<DT>(dev, s, a, xp, m0, m);
             normed = n > 1 && m == a.rows && fuse_row_norm(dev, a);
             launches += n;
