@@ -30,8 +30,10 @@ def tiled_weights(dev, stream, dtype, n_out, n_in, seed):
 
 
 # (dtype, n_out, n_in, rows, path): split-K across CTAs, no split, fp32 route, rows > 32, and from 48 rows on
-# the tensor-memory route: 2560 outputs split K seven ways with the parts summed by a second kernel, 9216
-# outputs split it two ways with the sum inside the kernel; both keep their partial sums in the fixed array
+# the tensor-memory route: 2560 outputs split K seven ways with the parts, in the fixed array, summed by a second
+# kernel; 9216 outputs leave both halves of K to one pair of CTAs. Then calls that need little or nothing of the
+# array although other row counts of the same matrix would fill it, and two whose partial sums fit only in part:
+# 16384 columns go without ranges of K on different CTAs, 740 rows by 512.
 SHAPES = [
     (synth.Q6_K, 2560, 9216, 9, cuda.PATH_MMA),
     (synth.Q4_K, 2560, 2560, 9, cuda.PATH_MMA),
@@ -40,6 +42,10 @@ SHAPES = [
     (synth.Q5_K, 520, 4096, 40, cuda.PATH_MMA),
     (synth.Q4_K, 2560, 2560, 64, cuda.PATH_MMA),
     (synth.Q6_K, 9216, 2560, 64, cuda.PATH_MMA),
+    (synth.Q4_K, 18432, 2560, 256, cuda.PATH_MMA),
+    (synth.Q6_K, 2560, 9216, 64, cuda.PATH_MMA),
+    (synth.Q4_K, 2560, 16384, 30, cuda.PATH_AUTO),
+    (synth.Q4_K, 24, 2560, 740, cuda.PATH_AUTO),
 ]
 
 

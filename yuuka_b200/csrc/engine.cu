@@ -770,7 +770,7 @@ bool matrices_tiled(const yuuka_model & m) {
 
 void reserve_gemm(yuuka_session * s, const Tensor & w, int rows) {
     if (w.present() && s->reserved.insert({rows, (int)w.dtype, (int)w.rows, (int)w.cols}).second)
-        gemm_scratch_reserve(s->model->dev, s->gemm, w.dtype, rows, (int)w.rows, (int)w.cols);
+        gemm_scratch_reserve(s->model->dev, s->gemm, w.dtype, rows, (int)w.rows, (int)w.cols, true);
 }
 
 enum LogitRows { LOGITS_NONE, LOGITS_LAST, LOGITS_ALL };
@@ -1539,20 +1539,12 @@ yuuka_status yuuka_session_create(yuuka_model * model, const yuuka_session_confi
                                                       attention_scratch_floats(s->chain_rows, c.heads, c.head_dim, attention_splits(s, 1, CHAIN_SUB, sc.capacity)));
             }
             s->attn_partial = dalloc<float>(s->attn_partial_floats, s->owned, false);
-            // split-K scratch for every matrix shape of the step and of a prompt pass: the register-fed route
-            // (up to 32 rows per launch), one row, and the tensor-memory route at the widest pass a launch
-            // takes (gemm_tiled_scratch_need covers every row count up to the one it is given)
-            for (int rows : {R < 32 ? R : 32, 1, R}) {
-                for (const LayerW & L : model->layers) {
-                    for (const Tensor * t : {&L.q, &L.k, &L.v, &L.o, &L.qkv, &L.gate, &L.beta, &L.alpha, &L.out, &L.ffn_gate,
-                                             &L.ffn_up, &L.ffn_down, &L.proj, &L.qk, &L.gate_up, &L.sh_gate, &L.sh_up,
-                                             &L.sh_down, &L.sh_gate_up})
-                        reserve_gemm(s, *t, rows);
-                }
-                reserve_gemm(s, model->output, rows);
-            }
-            for (int r = 1; r < R && r < 32; r++) reserve_gemm(s, model->layers[0].ffn_down, r);
-            for (int r = 1; r < R && r < 32; r++) reserve_gemm(s, model->layers[0].sh_down, r);
+            // scratch for every matrix shape of a step or prompt pass, whatever its rows and route
+            for (const LayerW & L : model->layers)
+                for (const Tensor * t : {&L.q, &L.k, &L.v, &L.o, &L.qkv, &L.gate, &L.beta, &L.alpha, &L.out, &L.ffn_gate, &L.ffn_up,
+                                         &L.ffn_down, &L.proj, &L.qk, &L.gate_up, &L.sh_gate, &L.sh_up, &L.sh_down, &L.sh_gate_up})
+                    reserve_gemm(s, *t, R);
+            reserve_gemm(s, model->output, R);
         } catch (...) {
             yuuka_session_destroy(s);
             throw;

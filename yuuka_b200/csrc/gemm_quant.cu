@@ -138,11 +138,11 @@ uint32_t gemm_auto_path(uint32_t w_dtype, int rows, int n_in) {
     return YUUKA_GEMM_PATH_MMA;
 }
 
-void gemm_scratch_reserve(const yuuka_device * dev, GemmScratch & s, uint32_t w_dtype, int rows, int n_out, int n_in) {
+void gemm_scratch_reserve(const yuuka_device * dev, GemmScratch & s, uint32_t w_dtype, int rows, int n_out, int n_in, bool up_to) {
     set_device(dev);
-    uint64_t want = 0;
-    int tiles = 0;
-    gemm_tiled_scratch_need(dev, w_dtype, rows, n_out, n_in, &want, &tiles);
+    const TiledScratchNeed need = (up_to ? gemm_tiled_scratch_bound : gemm_tiled_scratch_need)(dev, w_dtype, rows, n_out, n_in);
+    const uint64_t want = need.wanted;
+    const int tiles = need.counters;
     if (want > s.partial_floats) {
         if (s.partial) cudaFree(s.partial);
         s.partial = nullptr;

@@ -40,8 +40,8 @@ int launch_gemm_quant(const yuuka_device * dev, cudaStream_t stream, const GemmA
 // Which route AUTO takes for this shape.
 uint32_t gemm_auto_path(uint32_t w_dtype, int rows, int n_in);
 
-// Grows (never shrinks) a scratch so it fits a launch of this shape.
-void gemm_scratch_reserve(const yuuka_device * dev, GemmScratch & s, uint32_t w_dtype, int rows, int n_out, int n_in);
+// Grows (never shrinks) a scratch so it fits a launch of this shape (up_to: of up to so many rows, with any options).
+void gemm_scratch_reserve(const yuuka_device * dev, GemmScratch & s, uint32_t w_dtype, int rows, int n_out, int n_in, bool up_to = false);
 void gemm_scratch_free(GemmScratch & s);
 
 // Sticky device-side error word: set when a bounded wait inside a kernel gave

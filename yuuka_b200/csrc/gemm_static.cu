@@ -84,12 +84,11 @@ extern "C" yuuka_status yuuka_gemm_quant_static(yuuka_stream * stream, yuuka_buf
         YK_REQUIRE(dev->index >= 0 && dev->index < 16, YUUKA_ERR_UNSUPPORTED, "gemm_quant_static: device index out of range");
 
         // carve the fixed array: counters | xh | xl | xs16 | split-K partial sums
-        uint64_t partial_floats = 0;
-        int counters = 0;
-        gemm_tiled_scratch_need(dev, w_dtype, (int)rows, (int)n_out, (int)n_in, &partial_floats, &counters);
+        const TiledScratchNeed sums = gemm_tiled_scratch_need(dev, w_dtype, (int)rows, (int)n_out, (int)n_in);
+        const int counters = sums.counters;
         const uint64_t xh_bytes = align256(rows * n_in * sizeof(__half));
         const uint64_t xs_bytes = align256(rows * n_in / 16 * sizeof(__half2) + 16);
-        const uint64_t need = STATIC_COUNTER_BYTES + 2 * xh_bytes + xs_bytes + align256(partial_floats * sizeof(float));
+        const uint64_t need = STATIC_COUNTER_BYTES + 2 * xh_bytes + xs_bytes + align256(sums.floats * sizeof(float));
         YK_REQUIRE((uint64_t)counters * sizeof(int) <= STATIC_COUNTER_BYTES && need <= YUUKA_GEMM_STATIC_SCRATCH_BYTES,
                    YUUKA_ERR_UNSUPPORTED,
                    "gemm_quant_static: rows=%llu n_out=%llu n_in=%llu needs %llu bytes of scratch (%d counters), the fixed "

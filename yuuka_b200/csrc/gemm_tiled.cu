@@ -1724,6 +1724,7 @@ static void plan_tiled(const yuuka_device * dev, uint32_t dtype, int m, int n_ou
 // Rows from which the tensor-memory route takes over from 16-row passes of the register-fed kernel.
 constexpr int UMMA_MIN_ROWS = 48;
 constexpr int UMMA_EARLY_ROWS = 33;  // on request: where three passes of the register-fed route would begin
+constexpr int UMMA_PART_ROWS = 512;  // a launch whose parts of K do not all fit the scratch goes by so many rows
 
 static bool umma_enabled() {
     static const bool on = [] {
@@ -1800,15 +1801,18 @@ static RowCut row_cut(const yuuka_device * dev, uint32_t dtype, int m, int n_out
 // How 17 to 48 rows are cut into work for gemm_tiled_rows_kernel: tg tiles per CTA and ranges of K that end where parts of
 // all rows end. The cost is in records per SM (a record takes as long however many warps share the SM's tensor pipe): rounds
 // x (tiles x records + 2 for the start and the stores of an item), and 10 for the launch that adds the ranges up. paired: tiles
-// 2i and 2i + 1 share a CTA, all of K (SwiGLU epilogue).
-static void plan_rows(const yuuka_device * dev, uint32_t dtype, int m, int n_out, int n_in, RParams & p, bool paired) {
+// 2i and 2i + 1 share a CTA, all of K (SwiGLU epilogue). partial_floats: room for the parts of several ranges; without enough
+// of it K stays whole, with the same sums.
+static void plan_rows(const yuuka_device * dev, uint32_t dtype, int m, int n_out, int n_in, RParams & p, bool paired, uint64_t partial_floats) {
     const int nsb = n_in / 256, n_tiles = (n_out + 15) / 16;
     p.first_rest = m / 16 * 16;
     p.cut[0] = row_cut(dev, dtype, 16, n_out, n_in);
     p.cut[1] = m > p.first_rest ? row_cut(dev, dtype, m - p.first_rest, n_out, n_in) : p.cut[0];
     const uint64_t ends = p.cut[0].parts & p.cut[1].parts;
+    const int parts = std::max(__builtin_popcountll(p.cut[0].parts), __builtin_popcountll(p.cut[1].parts));
+    const int most = paired || (uint64_t)parts * m * n_out > partial_floats ? 1 : RW_MAX_SPLITS;
     double best = 1e30;
-    for (int splits = 1; splits <= (paired ? 1 : RW_MAX_SPLITS) && splits <= nsb; splits++) {
+    for (int splits = 1; splits <= most && splits <= nsb; splits++) {
         int at[RW_MAX_SPLITS + 1], n = 0, longest = 0;
         at[0] = 0;
         for (int sb = 0; sb < nsb; sb++)
@@ -1845,34 +1849,58 @@ bool gemm_tiled_rows_swiglu(int rows, int n_in, bool exact_only, bool wide_from_
     return rows > 32 && rows <= RW_MAX_ROWS && rows_route(rows, 16, n_in) && !gemm_tiled_wide(rows, exact_only, wide_from_33);
 }
 
-void gemm_tiled_scratch_need(const yuuka_device * dev, uint32_t w_dtype, int rows, int n_out, int n_in,
-                             uint64_t * partial_floats, int * counters) {
-    *partial_floats = 0;
-    *counters = 0;
-    if (!tiled_supported(w_dtype, n_in)) return;
-    // enough for this row count and for every smaller one (fewer rows may split K further)
-    for (int m : {rows, rows < 96 ? rows : 96}) {
-        const int parts = rows >= UMMA_EARLY_ROWS ? umma_kparts(dev, n_out, n_in, m) : 1;
-        if (parts > 2 && (uint64_t)parts * m * n_out > *partial_floats) *partial_floats = (uint64_t)parts * m * n_out;
-    }
-    // 17 to 48 rows: at most as many parts as the passes of any of these rows have
-    if (rows > MMA_ROWS && n_in <= 64 * 256) {
-        int parts = 0;
-        for (int m = 1; m <= MMA_ROWS; m++) parts = std::max(parts, __builtin_popcountll(row_cut(dev, w_dtype, m, n_out, n_in).parts));
-        if (parts > 1) *partial_floats = std::max(*partial_floats, (uint64_t)parts * (rows < RW_MAX_ROWS ? rows : RW_MAX_ROWS) * n_out);
-    }
-    for (int m : {rows < MMA_ROWS ? rows : MMA_ROWS, MMA_ROWS < rows ? rows % MMA_ROWS : 0}) {
-        if (m <= 0) continue;
-        for (bool paired : {false, true}) {
-            TPlan pl;
-            plan_tiled(dev, w_dtype, m, n_out, n_in, pl, paired);
-            if (pl.kchunks > 1) {
-                uint64_t need = (uint64_t)pl.kchunks * m * n_out;
-                if (need > *partial_floats) *partial_floats = need;
-                if (pl.n_groups > *counters) *counters = pl.n_groups;
-            }
+// What passes of m rows (at most MMA_ROWS) leave in the scratch where their plan cuts K across CTAs.
+static void add_pass_need(const yuuka_device * dev, uint32_t dtype, int m, int n_out, int n_in, bool paired, TiledScratchNeed & need) {
+    TPlan pl;
+    plan_tiled(dev, dtype, m, n_out, n_in, pl, paired);
+    if (pl.kchunks == 1) return;
+    need.floats = std::max(need.floats, (uint64_t)pl.kchunks * m * n_out);
+    need.counters = std::max(need.counters, pl.n_groups);
+}
+
+TiledScratchNeed gemm_tiled_scratch_need(const yuuka_device * dev, uint32_t w_dtype, int rows, int n_out, int n_in) {
+    TiledScratchNeed need;
+    if (!tiled_supported(w_dtype, n_in)) return need;
+    if (gemm_tiled_wide(rows, false, false)) {
+        const int parts = umma_plan(dev, n_out, n_in, rows).kparts;
+        if (parts > 1) {
+            need.floats = (uint64_t)parts * std::min(rows, UMMA_PART_ROWS) * n_out;
+            need.wanted = (uint64_t)parts * rows * n_out;
         }
+        return need;
     }
+    // passes of sixteen, which a launch of more rows falls back to, and their rest (48 is a multiple of sixteen)
+    add_pass_need(dev, w_dtype, std::min(rows, MMA_ROWS), n_out, n_in, false, need);
+    if (rows > MMA_ROWS && rows % MMA_ROWS) add_pass_need(dev, w_dtype, rows % MMA_ROWS, n_out, n_in, false, need);
+    need.wanted = need.floats;
+    for (int m0 = 0; m0 < rows; m0 += RW_MAX_ROWS) {
+        const int m = std::min(rows - m0, RW_MAX_ROWS);
+        if (!rows_route(m, n_out, n_in) || (m0 > 0 && m == RW_MAX_ROWS)) continue;
+        RParams p{};
+        plan_rows(dev, w_dtype, m, n_out, n_in, p, false, UINT64_MAX);
+        need.wanted = std::max(need.wanted, rows_partial_floats(p, m, n_out));
+    }
+    return need;
+}
+
+TiledScratchNeed gemm_tiled_scratch_bound(const yuuka_device * dev, uint32_t w_dtype, int rows, int n_out, int n_in) {
+    TiledScratchNeed need;
+    if (!tiled_supported(w_dtype, n_in)) return need;
+    if (rows >= UMMA_EARLY_ROWS)
+        for (int m : {rows, std::min(rows, 96)}) {  // (fewer rows may split K further: umma_kparts)
+            const int parts = umma_kparts(dev, n_out, n_in, m);
+            if (parts > 2) need.floats = std::max(need.floats, (uint64_t)parts * m * n_out);
+        }
+    for (int m = 1; m <= std::min(rows, MMA_ROWS); m++)
+        for (bool paired : {false, true}) add_pass_need(dev, w_dtype, m, n_out, n_in, paired, need);
+    for (int m = MMA_ROWS + 1; m <= std::min(rows, RW_MAX_ROWS); m++) {
+        if (!rows_route(m, n_out, n_in)) continue;
+        RParams p{};
+        plan_rows(dev, w_dtype, m, n_out, n_in, p, false, UINT64_MAX);
+        need.floats = std::max(need.floats, rows_partial_floats(p, m, n_out));
+    }
+    need.wanted = need.floats;
+    return need;
 }
 
 template <int DT, int NT>
@@ -2030,6 +2058,10 @@ static void make_x_map(CUtensorMap * map, const __half * xh, int m, int k, int b
 // two launches, of which the first uses the whole machine evenly.)
 static bool fuse_row_norm(const yuuka_device * dev, const TiledGemmArgs & a) { return a.row_norm && a.rows <= 2 * dev->sm_count; }
 
+static bool umma_parts_fit(const TiledGemmArgs & a, int kparts) {
+    return a.scratch && a.scratch->partial_floats >= (uint64_t)kparts * a.rows * a.n_out;
+}
+
 template <int DT>
 static int launch_umma_dt(const yuuka_device * dev, cudaStream_t s, const TiledGemmArgs & a, const __half * xh) {
     using S = UmmaStage<DT>;
@@ -2051,8 +2083,7 @@ static int launch_umma_dt(const yuuka_device * dev, cudaStream_t s, const TiledG
     // instruction descriptor: D f32, A and B f16, both K-major, N = activation rows of the tile, M = 256 (the pair)
     p.idesc = (1u << 4) | ((uint32_t)(pl.n_tile >> 3) << 17) | ((uint32_t)(2 * UM_ROWS >> 4) << 24);
     if (pl.kparts > 1) {
-        YK_REQUIRE(a.scratch && a.scratch->partial_floats >= (uint64_t)pl.kparts * a.rows * a.n_out, YUUKA_ERR_INTERNAL,
-                   "umma gemm: split-K scratch is too small");
+        YK_REQUIRE(umma_parts_fit(a, pl.kparts), YUUKA_ERR_INTERNAL, "umma gemm: split-K scratch is too small");
         p.partial = a.scratch->partial;
     }
     alignas(64) CUtensorMap xmap;
@@ -2127,12 +2158,8 @@ static int launch_rows_dt(const yuuka_device * dev, cudaStream_t s, const TiledG
     p.out = a.out + (int64_t)m0 * a.ldo;
     p.ldo = a.ldo;
     p.accumulate = (a.flags & YUUKA_GEMM_ACCUMULATE) ? 1 : 0;
-    plan_rows(dev, DT, m, a.n_out, a.n_in, p, a.swiglu.xh != nullptr);
-    if (p.splits > 1) {
-        YK_REQUIRE(a.scratch && a.scratch->partial_floats >= rows_partial_floats(p, m, a.n_out), YUUKA_ERR_INTERNAL,
-                   "gemm: split-K scratch is too small");
-        p.partial = a.scratch->partial;
-    }
+    plan_rows(dev, DT, m, a.n_out, a.n_in, p, a.swiglu.xh != nullptr, a.scratch ? a.scratch->partial_floats : 0);
+    if (p.splits > 1) p.partial = a.scratch->partial;
     if (a.swiglu.xh) {
         const int64_t half = a.n_out / 2;
         p.swiglu = XPrepOut{a.swiglu.xh + m0 * half, a.swiglu.xl + m0 * half, a.swiglu.xs16 + m0 * (half / 16)};
@@ -2187,6 +2214,18 @@ static int launch_mma_dt(const yuuka_device * dev, cudaStream_t s, const TiledGe
         launches++;
     }
     if (wide) {
+        const int parts = umma_plan(dev, a.n_out, a.n_in, a.rows).kparts;
+        if (a.rows > UMMA_PART_ROWS && parts > 1 && !umma_parts_fit(a, parts)) {
+            // (the fixed scratch of yuuka_gemm_quant_static, nearly filled by the activations)
+            for (int m0 = 0; m0 < a.rows; m0 += UMMA_PART_ROWS) {
+                TiledGemmArgs b = a;
+                b.rows = std::min(a.rows - m0, UMMA_PART_ROWS);
+                b.out += (int64_t)m0 * a.ldo;
+                b.row_norm = nullptr;
+                launches += launch_umma_dt<DT>(dev, s, b, xp.xh + (int64_t)m0 * a.n_in);
+            }
+            return launches + norm(false);
+        }
         const int n = launch_umma_dt<DT>(dev, s, a, xp.xh);
         return launches + n + norm(n > 1 && fuse_row_norm(dev, a));
     }

@@ -108,9 +108,15 @@ int launch_gemm_tiled(const yuuka_device * dev, cudaStream_t stream, const Tiled
 bool gemm_tiled_wide(int rows, bool exact_only, bool wide_from_33);
 // whether a launch of more rows than the folded epilogues of the step take (32) can still fold SwiGLU into its own
 bool gemm_tiled_rows_swiglu(int rows, int n_in, bool exact_only, bool wide_from_33);
-// Scratch the launch above needs for this shape (0 partial floats when K is not split across CTAs).
-void gemm_tiled_scratch_need(const yuuka_device * dev, uint32_t w_dtype, int rows, int n_out, int n_in,
-                             uint64_t * partial_floats, int * counters);
+// Scratch for partial sums of launch_gemm_tiled. floats, counters: without them the launch is refused; wanted: what its plan
+// uses where there is as much (17 to 47 rows; with less, K stays whole). `need`: of a launch of these rows with default
+// options; `bound`: enough for every launch of at most so many rows, with any options.
+struct TiledScratchNeed {
+    uint64_t floats = 0, wanted = 0;
+    int counters = 0;
+};
+TiledScratchNeed gemm_tiled_scratch_need(const yuuka_device * dev, uint32_t w_dtype, int rows, int n_out, int n_in);
+TiledScratchNeed gemm_tiled_scratch_bound(const yuuka_device * dev, uint32_t w_dtype, int rows, int n_out, int n_in);
 
 // Makes the driver load the code of every kernel launch_gemm_tiled can launch (the current device).
 void gemm_tiled_preload_kernels();
