@@ -62,6 +62,8 @@ def test_umma_route_accumulates(dev):
     (1001, 1536, 97),    # K split with rows that 16-byte stores do not divide
     (1000, 2560, 289),   # K split, two tiles of rows
     (2560, 768, 513),
+    (96000, 256, 48),    # more tiles per pair than there are accumulators
+    (9216, 1024, 577),   # the two halves of K in accumulators that a tile before has used
 ])
 @pytest.mark.parametrize("dtype", [synth.Q4_K, synth.Q6_K])
 def test_umma_route_at_the_edges_of_its_tiles(dev, n_out, n_in, rows, dtype):

@@ -20,7 +20,8 @@
 //
 // Roles of a CTA's warps: sixteen decode warps (two per 16-row tile), four epilogue warps, one warp that copies packed
 // weights (one bulk copy per record, a superblock of all eight tiles per stage, ahead of everything else), one that copies
-// activations, one that issues the MMAs (even CTA) or passes on that the activations have landed (odd CTA).
+// activations, one that issues the MMAs (even CTA) or passes on, stage by stage, what the odd CTA's other warps have arrived
+// for.
 // Every mbarrier wait is bounded; on expiry the device error word is set, the kernel carries on (results are then
 // garbage), frees its tensor memory and returns.
 #pragma once
@@ -275,13 +276,32 @@ __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
 __device__ __forceinline__ void mbar_expect(uint32_t bar, uint32_t bytes) {
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
 }
-// One arrival on the barrier at this offset in the even CTA of the pair, from a thread of either CTA. Release at CTA scope
-// only: what the barrier announces are this CTA's own shared memory and tensor memory, which its own tensor core
-// reads, and a release at cluster scope stalls for some 900 cycles.
-__device__ __forceinline__ void mbar_arrive_leader(uint32_t bar) {
-    uint32_t remote;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(bar), "r"(0u));
-    asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(remote) : "memory");
+// From the odd CTA: UM_NOTE bytes into the even CTA's `note`, counted by the barrier at this offset there. The count is a
+// release at cluster scope (PTX ISA, st.async: "the complete-tx operation on the mbarrier has .release semantics at the
+// .cluster scope"), so whoever waits for it with an acquire at that scope sees what this thread has seen. An arrival would
+// order nothing between the CTAs at its default scope, and at cluster scope its release takes some 1500 cycles: with one
+// thread passing on the stages 9216 x 2560 took 68 us at 576 rows, with two in turn 45, with four 39, and so 34.6 (34.4 with
+// arrivals at CTA scope straight from the decode warps).
+constexpr uint32_t UM_NOTE = 4;
+__device__ __forceinline__ void note_leader(uint32_t note, uint32_t bar) {
+    uint32_t remote_note, remote_bar;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote_note) : "r"(note), "r"(0u));
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote_bar) : "r"(bar), "r"(0u));
+    asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.b32 [%0], %1, [%2];" ::"r"(remote_note), "r"(1u), "r"(remote_bar)
+                 : "memory");
+}
+// (Only this wait needs the wider scope. What the odd CTA waits for from the even one are completions of asynchronous
+// operations, tcgen05.commit, which the waiter of the barrier sees by the rules of those.)
+__device__ __forceinline__ bool mbar_wait_cluster(uint32_t bar, uint32_t parity) {
+    uint32_t ok = 0;
+    for (uint32_t i = 0; i < (1u << 22) && !ok; i++) {
+        asm volatile(
+            "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+            : "=r"(ok)
+            : "r"(bar), "r"(parity)
+            : "memory");
+    }
+    return ok != 0;
 }
 // completion of this thread's MMAs so far -> one arrival on the barrier at this offset in both CTAs of the pair
 __device__ __forceinline__ void umma_commit_pair(uint32_t bar) {
@@ -369,11 +389,10 @@ __global__ void __launch_bounds__(UM_THREADS, 1) gemm_umma_kernel(const UParams 
     extern __shared__ __align__(128) uint8_t smem_raw[];
     uint8_t * smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);  // the swizzled stages need 1024-byte alignment
     __shared__ __align__(8) uint64_t empty_bar[UM_MAX_STAGES];  // the tensor pipe has read the stage
-    __shared__ __align__(8) uint64_t full_bar[UM_MAX_STAGES];   // (even CTA) both CTAs' weights and activations are in the stage
-    __shared__ __align__(8) uint64_t x_bar[UM_MAX_STAGES];      // (odd CTA) its activations have landed
+    __shared__ __align__(8) uint64_t full_bar[UM_MAX_STAGES];   // this CTA's weights and activations are in the stage (even CTA: both CTAs')
     __shared__ __align__(8) uint64_t raw_full[UM_RAW_STAGES], raw_empty[UM_RAW_STAGES];
     __shared__ __align__(8) uint64_t acc_full[UM_MAX_ACC], acc_empty[UM_MAX_ACC]; // accumulators: finished by the MMAs, read by the epilogue
-    __shared__ uint32_t tmem_slot;
+    __shared__ uint32_t tmem_slot, odd_note[UM_MAX_STAGES];  // (the notes' contents are not read)
     const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;  // (uniform for the compiler too)
     const uint32_t rank = blockIdx.x & 1u;  // clusters are pairs along x
     const uint32_t half_n = (uint32_t)p.n_tile >> 1, b_bytes = half_n * 128u, stage_bytes = UM_A_BYTES + b_bytes;
@@ -383,8 +402,7 @@ __global__ void __launch_bounds__(UM_THREADS, 1) gemm_umma_kernel(const UParams 
     if (threadIdx.x == 0) {
         for (int s = 0; s < UM_MAX_STAGES; s++) {
             mbar_init(smem_u32(&empty_bar[s]), 1);
-            mbar_init(smem_u32(&full_bar[s]), 2 * UM_TILES + 2);
-            mbar_init(smem_u32(&x_bar[s]), 1);
+            mbar_init(smem_u32(&full_bar[s]), UM_TILES + 1);
         }
         for (int s = 0; s < UM_RAW_STAGES; s++) {
             mbar_init(smem_u32(&raw_full[s]), 1);
@@ -392,7 +410,7 @@ __global__ void __launch_bounds__(UM_THREADS, 1) gemm_umma_kernel(const UParams 
         }
         for (int s = 0; s < UM_MAX_ACC; s++) {
             mbar_init(smem_u32(&acc_full[s]), 1);
-            mbar_init(smem_u32(&acc_empty[s]), 2 * UM_EW);
+            mbar_init(smem_u32(&acc_empty[s]), UM_EW);
         }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -443,9 +461,9 @@ __global__ void __launch_bounds__(UM_THREADS, 1) gemm_umma_kernel(const UParams 
             const int row = wk.n0(p) + (int)(rank * half_n), sb1 = wk.sb_end(p);
             for (int col = wk.sb_begin(p) * 256; col < sb1 * 256; col += UM_KC) {
                 wait(empty_bar[ring.at], ring.phase ^ 1u);
-                const uint32_t bar = smem_u32(rank == 0 ? &full_bar[ring.at] : &x_bar[ring.at]);
+                const uint32_t bar = smem_u32(&full_bar[ring.at]);
                 if (lane == 0) {
-                    mbar_expect(bar, b_bytes);
+                    mbar_expect(bar, b_bytes + (rank == 0 ? UM_NOTE : 0u));
                     asm volatile(
                         "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
                         :
@@ -474,7 +492,7 @@ __global__ void __launch_bounds__(UM_THREADS, 1) gemm_umma_kernel(const UParams 
                     d = taddr + acc.at * acc_cols;
                     keep = 0;
                 }
-                wait(full_bar[ring.at], ring.phase);
+                if (!expired && !mbar_wait_cluster(smem_u32(&full_bar[ring.at]), ring.phase)) expired = true;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 const uint64_t da = da0 + (uint64_t)(ring.at * step), db = db0 + (uint64_t)(ring.at * step);
                 if (elect_one()) {
@@ -492,13 +510,18 @@ __global__ void __launch_bounds__(UM_THREADS, 1) gemm_umma_kernel(const UParams 
             acc.next(n_acc);
         }
     } else if (warp == UM_WARP_MMA) {
-        // ---------------- odd CTA: its activations have landed -> the even CTA's barrier ----------------
-        Ring ring;
+        // ---------------- odd CTA: its part of a stage is there (and, at the start of an accumulator, its epilogue has
+        // read what the accumulator held) -> the even CTA's barrier ----------------
+        Ring ring, acc;
         for (UmmaWork wk(p); wk.valid(); wk.next()) {
-            const int chunks = (wk.sb_end(p) - wk.sb_begin(p)) * 4;
+            const int chunks = (wk.sb_end(p) - wk.sb_begin(p)) * 4, second = p.halves ? (p.nsb >> 1) * 4 : chunks;
             for (int c = 0; c < chunks; c++) {
-                wait(x_bar[ring.at], ring.phase);
-                if (lane == 0) mbar_arrive_leader(smem_u32(&full_bar[ring.at]));
+                if (c == 0 || c == second) {
+                    wait(acc_empty[acc.at], acc.phase ^ 1u);
+                    acc.next(n_acc);
+                }
+                wait(full_bar[ring.at], ring.phase);
+                if (lane == 0) note_leader(smem_u32(&odd_note[ring.at]), smem_u32(&full_bar[ring.at]));
                 __syncwarp();
                 ring.next(p.stages);
             }
@@ -527,7 +550,7 @@ __global__ void __launch_bounds__(UM_THREADS, 1) gemm_umma_kernel(const UParams 
                     r.template store<decltype(c)::value>(lane, tab, kc, smem + (size_t)ring.at * stage_bytes + tile * 16 * 128);
                     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
                     __syncwarp();
-                    if (lane == 0) mbar_arrive_leader(smem_u32(&full_bar[ring.at]));
+                    if (lane == 0) mbar_arrive(smem_u32(&full_bar[ring.at]));
                     ring.next(p.stages);
                 };
                 chunk(std::integral_constant<int, 0>());
@@ -574,8 +597,8 @@ __global__ void __launch_bounds__(UM_THREADS, 1) gemm_umma_kernel(const UParams 
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             __syncwarp();
             if (lane == 0) {
-                mbar_arrive_leader(smem_u32(&acc_empty[first]));
-                if (p.halves) mbar_arrive_leader(smem_u32(&acc_empty[acc.at]));
+                mbar_arrive(smem_u32(&acc_empty[first]));
+                if (p.halves) mbar_arrive(smem_u32(&acc_empty[acc.at]));
             }
             acc.next(n_acc);
         }
