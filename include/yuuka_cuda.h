@@ -143,9 +143,9 @@ YUUKA_API yuuka_status yuuka_buffer_copy(yuuka_stream * stream, yuuka_buffer * d
  * the mma route and by the fast fp32 route; GGUF-layout weights take a slower
  * generic kernel). */
 #define YUUKA_GEMM_TILED 0x2u
-/* bit 31, test hook: the register-fed kernel never issues the copies of its activations and its wait for them
- * gives up after a short limit, so that the expiry path (device error word, YUUKA_ERR_DEVICE at the next
- * session fetch) can be exercised with nothing in flight. The outputs of such a launch are garbage. */
+/* bit 31, test hook: the mma kernels never issue copies of their activations (the tensor-memory kernel: half of
+ * them) and give up waiting after a short limit, so that the expiry path (device error word, YUUKA_ERR_DEVICE at
+ * the next session fetch) can be exercised with nothing in flight. The outputs of such a launch are garbage. */
 #define YUUKA_GEMM_TEST_DROP_COPIES 0x80000000u
 YUUKA_API yuuka_status yuuka_gemm_quant(yuuka_stream * stream,
                                         yuuka_buffer * out, uint64_t out_offset,

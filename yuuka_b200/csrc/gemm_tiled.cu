@@ -894,7 +894,7 @@ __device__ __forceinline__ void tiled_mma_body(const TParams & p, const GemmSegm
         // bounded wait for the copies; on expiry the error word is set and the results are garbage
         const uint32_t bar = (uint32_t)__cvta_generic_to_shared(&xbar);
         uint32_t ok = 0;
-        const uint32_t limit = p.drop_copies ? (1u << 8) : (1u << 22);
+        const uint32_t limit = p.drop_copies ? WAIT_LIMIT_TEST : WAIT_LIMIT;
         for (uint32_t i = 0; i < limit && !ok; i++) {
             asm volatile(
                 "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], 0;\n\tselp.u32 %0, 1, 0, p;\n\t}"
@@ -1210,6 +1210,7 @@ struct RParams {
     int stages;
     const uint8_t * next_w;  // see TParams
     uint32_t next_lines;
+    int drop_copies;
 };
 
 // Activations of one superblock: four column blocks of hi rows, four of lo rows, the sums. The lo box starts four rows
@@ -1269,16 +1270,20 @@ __global__ void __launch_bounds__(RW_WARPS * 32, 1)
     __syncthreads();
     pdl_trigger();
     const int items = p.groups * p.splits;
+    // (bounded waits: on expiry the device error word is set and the kernel carries on without waiting or copying; the copies
+    // issued before have had the whole of that wait to land)
+    const uint32_t limit = p.drop_copies ? WAIT_LIMIT_TEST : WAIT_LIMIT;
     bool expired = false;
     auto wait = [&](const uint64_t & bar, uint32_t parity) {
-        if (!expired && !mbar_wait(smem_u32(&bar), parity)) expired = true;
+        if (!expired) expired = __any_sync(0xffffffffu, !mbar_wait(smem_u32(&bar), parity, limit));  // (by whole warps)
     };
     // (warp 0) the copies of the next superblock in the order of work, once the warps have read what its stage held
     Ring fill;
     int fill_item = blockIdx.x, fill_sb = fill_item < items ? p.split_at[fill_item / p.groups] : 0;
     auto fetch = [&] {
-        if (fill_item >= items) return;
+        if (fill_item >= items || p.drop_copies) return;
         wait(empty_bar[fill.at], fill.phase ^ 1u);
+        if (expired) return;
         if (lane == 0) {
             const uint32_t bar = smem_u32(&full_bar[fill.at]), st = smem_u32(smem) + fill.at * (uint32_t)R::BYTES;
             mbar_expect(bar, R::TX);
@@ -2075,6 +2080,7 @@ static int launch_umma_dt(const yuuka_device * dev, cudaStream_t s, const TiledG
     p.out = a.out;
     p.ldo = a.ldo;
     p.accumulate = (a.flags & YUUKA_GEMM_ACCUMULATE) ? 1 : 0;
+    p.drop_copies = (a.flags & YUUKA_GEMM_TEST_DROP_COPIES) ? 1 : 0;
     p.kparts = pl.kparts;
     p.halves = pl.halves ? 1 : 0;
     p.n_tile = pl.n_tile;
@@ -2158,6 +2164,7 @@ static int launch_rows_dt(const yuuka_device * dev, cudaStream_t s, const TiledG
     p.out = a.out + (int64_t)m0 * a.ldo;
     p.ldo = a.ldo;
     p.accumulate = (a.flags & YUUKA_GEMM_ACCUMULATE) ? 1 : 0;
+    p.drop_copies = (a.flags & YUUKA_GEMM_TEST_DROP_COPIES) ? 1 : 0;
     plan_rows(dev, DT, m, a.n_out, a.n_in, p, a.swiglu.xh != nullptr, a.scratch ? a.scratch->partial_floats : 0);
     if (p.splits > 1) p.partial = a.scratch->partial;
     if (a.swiglu.xh) {
@@ -2235,7 +2242,7 @@ static int launch_mma_dt(const yuuka_device * dev, cudaStream_t s, const TiledGe
     bool normed = false;
     for (int m0 = 0; m0 < a.rows; m0 += m) {
         m = a.rows - m0 < RW_MAX_ROWS ? a.rows - m0 : RW_MAX_ROWS;
-        if (rows_route(m, a.n_out, a.n_in) && !folded && !(a.flags & YUUKA_GEMM_TEST_DROP_COPIES)) {
+        if (rows_route(m, a.n_out, a.n_in) && !folded) {
             const int n = launch_rows_dt<DT>(dev, s, a, xp, m0, m);
             normed = n > 1 && m == a.rows && fuse_row_norm(dev, a);
             launches += n;

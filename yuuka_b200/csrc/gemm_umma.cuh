@@ -22,8 +22,9 @@
 // weights (one bulk copy per record, a superblock of all eight tiles per stage, ahead of everything else), one that copies
 // activations, one that issues the MMAs (even CTA) or passes on, stage by stage, what the odd CTA's other warps have arrived
 // for.
-// Every mbarrier wait is bounded; on expiry the device error word is set, the kernel carries on (results are then
-// garbage), frees its tensor memory and returns.
+// Every mbarrier wait is bounded. A warp whose wait runs out leaves its loop: it issues no copy and no MMA after that, and
+// those it issued before have had the whole of that wait to finish. The others run out of what it owes them and follow; the
+// kernel sets the device error word, frees its tensor memory and returns (results are garbage).
 #pragma once
 
 namespace yk {
@@ -60,6 +61,7 @@ struct UParams {
     int m_blocks;         // blocks of 256 weight rows
     uint32_t idesc;
     uint32_t stages;      // ring depth
+    int drop_copies;      // test hook: the even CTA's activations are never copied
 };
 
 // Both operands: K-major, 128-byte swizzle: rows of 64 halves (128 bytes), eight rows per 1024-byte atom, as a tensor-map
@@ -256,9 +258,10 @@ template <> struct HalfRecord<YUUKA_DTYPE_Q8_0> {
 };
 
 __device__ __forceinline__ uint32_t smem_u32(const void * p) { return (uint32_t)__cvta_generic_to_shared(p); }
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
+constexpr uint32_t WAIT_LIMIT = 1u << 22, WAIT_LIMIT_TEST = 1u << 8;  // polls of some 4 us each: 17 s; with the test hook 1 ms
+__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, uint32_t limit) {
     uint32_t ok = 0;
-    for (uint32_t i = 0; i < (1u << 22) && !ok; i++) {
+    for (uint32_t i = 0; i < limit && !ok; i++) {
         asm volatile(
             "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
             : "=r"(ok)
@@ -292,9 +295,9 @@ __device__ __forceinline__ void note_leader(uint32_t note, uint32_t bar) {
 }
 // (Only this wait needs the wider scope. What the odd CTA waits for from the even one are completions of asynchronous
 // operations, tcgen05.commit, which the waiter of the barrier sees by the rules of those.)
-__device__ __forceinline__ bool mbar_wait_cluster(uint32_t bar, uint32_t parity) {
+__device__ __forceinline__ bool mbar_wait_cluster(uint32_t bar, uint32_t parity, uint32_t limit) {
     uint32_t ok = 0;
-    for (uint32_t i = 0; i < (1u << 22) && !ok; i++) {
+    for (uint32_t i = 0; i < limit && !ok; i++) {
         asm volatile(
             "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
             : "=r"(ok)
@@ -426,9 +429,12 @@ __global__ void __launch_bounds__(UM_THREADS, 1) gemm_umma_kernel(const UParams 
     const uint32_t acc_cols = p.n_tile <= UM_MAX_N / 2 ? UM_MAX_N / 2 : UM_MAX_N, n_acc = 512u / acc_cols;  // accumulators
     const int n_tiles16 = (p.N + 15) >> 4;
     const size_t rec_row = (size_t)p.nsb * C::REC;
+    const uint32_t limit = p.drop_copies ? WAIT_LIMIT_TEST : WAIT_LIMIT;
     bool expired = false;
+    // (by whole warps, whose lanes agree on the outcome)
     auto wait = [&](const uint64_t & bar, uint32_t parity) {
-        if (!expired && !mbar_wait(smem_u32(&bar), parity)) expired = true;
+        expired = __any_sync(0xffffffffu, !mbar_wait(smem_u32(&bar), parity, limit));
+        return !expired;
     };
 
     pdl_trigger();
@@ -437,11 +443,11 @@ __global__ void __launch_bounds__(UM_THREADS, 1) gemm_umma_kernel(const UParams 
     if (warp == UM_WARP_RAW) {
         // ---------------- packed weights: they do not depend on the previous kernel ----------------
         Ring ring;
-        for (UmmaWork wk(p); wk.valid(); wk.next()) {
+        for (UmmaWork wk(p); wk.valid() && !expired; wk.next()) {
             const int rt = min((wk.block(p) * 2 + (int)rank) * UM_TILES + (lane & (UM_TILES - 1)), n_tiles16 - 1), sb1 = wk.sb_end(p);
             const uint8_t * src = p.w + rt * rec_row;
             for (int sb = wk.sb_begin(p); sb < sb1; sb++) {
-                wait(raw_empty[ring.at], ring.phase ^ 1u);
+                if (!wait(raw_empty[ring.at], ring.phase ^ 1u)) break;
                 const uint32_t bar = smem_u32(&raw_full[ring.at]);
                 if (lane == 0) mbar_expect(bar, S::RAW_BYTES);
                 __syncwarp();
@@ -457,12 +463,12 @@ __global__ void __launch_bounds__(UM_THREADS, 1) gemm_umma_kernel(const UParams 
         // ---------------- activations: this CTA's half of the tile's rows ----------------
         pdl_wait();
         Ring ring;
-        for (UmmaWork wk(p); wk.valid(); wk.next()) {
+        for (UmmaWork wk(p); wk.valid() && !expired; wk.next()) {
             const int row = wk.n0(p) + (int)(rank * half_n), sb1 = wk.sb_end(p);
             for (int col = wk.sb_begin(p) * 256; col < sb1 * 256; col += UM_KC) {
-                wait(empty_bar[ring.at], ring.phase ^ 1u);
+                if (!wait(empty_bar[ring.at], ring.phase ^ 1u)) break;
                 const uint32_t bar = smem_u32(&full_bar[ring.at]);
-                if (lane == 0) {
+                if (lane == 0 && !(p.drop_copies && rank == 0)) {
                     mbar_expect(bar, b_bytes + (rank == 0 ? UM_NOTE : 0u));
                     asm volatile(
                         "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
@@ -479,8 +485,8 @@ __global__ void __launch_bounds__(UM_THREADS, 1) gemm_umma_kernel(const UParams 
         Ring ring, acc;
         const uint64_t da0 = umma_desc_sw128(smem_base), db0 = umma_desc_sw128(smem_base + UM_A_BYTES);
         const uint32_t step = stage_bytes >> 4;
-        for (UmmaWork wk(p); wk.valid(); wk.next()) {
-            wait(acc_empty[acc.at], acc.phase ^ 1u);
+        for (UmmaWork wk(p); wk.valid() && !expired; wk.next()) {
+            if (!wait(acc_empty[acc.at], acc.phase ^ 1u)) break;
             uint32_t d = taddr + acc.at * acc_cols, keep = 0;
             const int chunks = (wk.sb_end(p) - wk.sb_begin(p)) * 4, second = p.halves ? (p.nsb >> 1) * 4 : chunks;
             for (int c = 0; c < chunks; c++) {
@@ -488,11 +494,12 @@ __global__ void __launch_bounds__(UM_THREADS, 1) gemm_umma_kernel(const UParams 
                     if (elect_one()) umma_commit_pair(smem_u32(&acc_full[acc.at]));
                     __syncwarp();
                     acc.next(n_acc);
-                    wait(acc_empty[acc.at], acc.phase ^ 1u);
+                    if (!wait(acc_empty[acc.at], acc.phase ^ 1u)) break;
                     d = taddr + acc.at * acc_cols;
                     keep = 0;
                 }
-                if (!expired && !mbar_wait_cluster(smem_u32(&full_bar[ring.at]), ring.phase)) expired = true;
+                expired = __any_sync(0xffffffffu, !mbar_wait_cluster(smem_u32(&full_bar[ring.at]), ring.phase, limit));
+                if (expired) break;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 const uint64_t da = da0 + (uint64_t)(ring.at * step), db = db0 + (uint64_t)(ring.at * step);
                 if (elect_one()) {
@@ -505,6 +512,7 @@ __global__ void __launch_bounds__(UM_THREADS, 1) gemm_umma_kernel(const UParams 
                 keep = 1;
                 ring.next(p.stages);
             }
+            if (expired) break;
             if (elect_one()) umma_commit_pair(smem_u32(&acc_full[acc.at]));
             __syncwarp();
             acc.next(n_acc);
@@ -513,14 +521,14 @@ __global__ void __launch_bounds__(UM_THREADS, 1) gemm_umma_kernel(const UParams 
         // ---------------- odd CTA: its part of a stage is there (and, at the start of an accumulator, its epilogue has
         // read what the accumulator held) -> the even CTA's barrier ----------------
         Ring ring, acc;
-        for (UmmaWork wk(p); wk.valid(); wk.next()) {
+        for (UmmaWork wk(p); wk.valid() && !expired; wk.next()) {
             const int chunks = (wk.sb_end(p) - wk.sb_begin(p)) * 4, second = p.halves ? (p.nsb >> 1) * 4 : chunks;
             for (int c = 0; c < chunks; c++) {
                 if (c == 0 || c == second) {
-                    wait(acc_empty[acc.at], acc.phase ^ 1u);
+                    if (!wait(acc_empty[acc.at], acc.phase ^ 1u)) break;
                     acc.next(n_acc);
                 }
-                wait(full_bar[ring.at], ring.phase);
+                if (!wait(full_bar[ring.at], ring.phase)) break;
                 if (lane == 0) note_leader(smem_u32(&odd_note[ring.at]), smem_u32(&full_bar[ring.at]));
                 __syncwarp();
                 ring.next(p.stages);
@@ -536,17 +544,17 @@ __global__ void __launch_bounds__(UM_THREADS, 1) gemm_umma_kernel(const UParams 
             ring.next(p.stages);
             ring.next(p.stages);
         }
-        for (UmmaWork wk(p); wk.valid(); wk.next()) {
+        for (UmmaWork wk(p); wk.valid() && !expired; wk.next()) {
             for (int n = wk.sb_end(p) - wk.sb_begin(p); n > 0; n--) {
                 HalfRecord<DT> r;
-                wait(raw_full[rr.at], rr.phase);
+                if (!wait(raw_full[rr.at], rr.phase)) break;
                 r.fetch(raw + (size_t)rr.at * S::RAW_BYTES + tile * C::REC, lane, half);
                 r.header(lane, half, tab);
                 __syncwarp();  // the table is complete, and every lane has its part of the record
                 if (lane == 0) mbar_arrive(smem_u32(&raw_empty[rr.at]));
                 rr.next(UM_RAW_STAGES);
                 auto chunk = [&](auto c) {
-                    wait(empty_bar[ring.at], ring.phase ^ 1u);
+                    if (expired || !wait(empty_bar[ring.at], ring.phase ^ 1u)) return;
                     r.template store<decltype(c)::value>(lane, tab, kc, smem + (size_t)ring.at * stage_bytes + tile * 16 * 128);
                     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
                     __syncwarp();
@@ -555,6 +563,7 @@ __global__ void __launch_bounds__(UM_THREADS, 1) gemm_umma_kernel(const UParams 
                 };
                 chunk(std::integral_constant<int, 0>());
                 chunk(std::integral_constant<int, 1>());
+                if (expired) break;
                 ring.next(p.stages);
                 ring.next(p.stages);
             }
@@ -564,12 +573,12 @@ __global__ void __launch_bounds__(UM_THREADS, 1) gemm_umma_kernel(const UParams 
         pdl_wait();
         const int quad = warp & 3;
         Ring acc;
-        for (UmmaWork wk(p); wk.valid(); wk.next()) {
+        for (UmmaWork wk(p); wk.valid() && !expired; wk.next()) {
             const uint32_t first = acc.at;
-            wait(acc_full[first], acc.phase);
+            if (!wait(acc_full[first], acc.phase)) break;
             if (p.halves) {
                 acc.next(n_acc);
-                wait(acc_full[acc.at], acc.phase);
+                if (!wait(acc_full[acc.at], acc.phase)) break;
             }
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const int n = (wk.block(p) * 2 + (int)rank) * UM_ROWS + quad * 32 + lane, m0 = wk.n0(p);
