@@ -1357,7 +1357,8 @@ int yo_verify_tree_greedy(const yo_model *m, yo_state *s, const int32_t *tokens,
  * ACCEPT_RULE, at node cur (start: root 0), with children in node order:
  *   mx   = max_i L[cur][i]
  *   e_i  = exp_det((L[cur][i] - mx) * (1/T))              (fp32, yo_exp_det)
- *   w_i  = (uint64) (e_i * 2^40)                           (truncation)
+ *   w_i  = (uint64) (e_i * 2^40)                           (truncation; 2^63 where e_i is a NaN, as at a
+ *                                                            logit of +infinity or where 1/T overflows)
  *   r = w, R = sum_i w_i
  *   for child c (token x, draft distribution Q[c][.], uniform u = U[2c]):
  *     accept iff (double)(u * Q[c][x]) * (double)R <= (double) r_x
@@ -1368,7 +1369,9 @@ int yo_verify_tree_greedy(const yo_model *m, yo_state *s, const int32_t *tokens,
  *     emit the smallest j with sum_{i<=j} r_i > t, stop.
  */
 
+/* polynomial and two-part ln 2: expf of the Cephes library */
 float yo_exp_det(float x) {
+    if (x != x) return x;
     if (x < -87.0f) return 0.0f;
     if (x > 88.0f) x = 88.0f;
     float n = rintf(x * 1.44269504f);
@@ -1403,7 +1406,7 @@ int yo_accept_rejection_tree(const float *logits, const float *Q, int V, const i
         uint64_t Z = 0;
         for (int i = 0; i < V; i++) {
             float e = yo_exp_det((L[i] - mx) * inv_t);
-            w[i] = (uint64_t)(e * 1099511627776.0f);
+            w[i] = e != e ? 1ull << 63 : (uint64_t)(e * 1099511627776.0f);
             Z += w[i];
         }
         memcpy(r, w, sizeof(uint64_t) * (size_t)V);

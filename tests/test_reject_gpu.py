@@ -222,3 +222,36 @@ def test_rejection_walk_at_the_vocabulary_sizes_where_the_launch_changes(B, V):
     lb.free(); qb.free()
     stream.destroy()
     dev.close()
+
+
+@pytest.mark.parametrize("V", [1000, 4099, 65536, 262147])
+@pytest.mark.parametrize("T", [0.8, 1e-39])   # 1 / 1e-39 overflows: only the maximum keeps weight
+def test_infinite_logits_take_all_the_weight(V, T):
+    """A chain whose first row has +infinity at the drafted token (accepted) and whose second has it at another one
+    (the draft is rejected, that token emitted); masked tokens at -infinity and at the lowest float."""
+    N, B = 4, 2
+    rng = np.random.default_rng(V)
+    logits = rng.standard_normal((B, N, V), dtype=np.float32)
+    logits[:, :, rng.choice(V, V // 3, replace=False)] = -np.inf
+    logits[1][:, rng.choice(V, V // 3, replace=False)] = np.finfo(np.float32).min
+    q = np.zeros((B, N, V), np.float32)
+    tokens = np.zeros((B, N), np.int32)
+    for b in range(B):
+        hot = rng.choice(V, 2, replace=False)
+        logits[b, 0, hot[0]] = logits[b, 1, hot[1]] = np.inf
+        tokens[b, 1:] = hot[0]
+        q[b, :, hot[0]] = 0.9
+    uniforms = np.full((B, N, 2), 0.5, np.float32)
+    parent = np.arange(-1, N - 1, dtype=np.int32)
+    dev = cuda.Device(0)
+    stream = dev.stream()
+    lb, qb = dev.upload(logits), dev.upload(q)
+    acc, em, path = cuda.accept_tree(stream, lb, tokens, V, mode=cuda.ACCEPT_REJECTION, temperature=T, draft_probs=qb,
+                                     uniforms=uniforms)
+    for b in range(B):
+        a, p_o, e_o = yo.accept_rejection_tree(logits[b], q[b], tokens[b], parent, T, uniforms[b])
+        assert a == 1 and e_o.tolist() == [int(tokens[b, 1]), int(np.argmax(logits[b, 1]))]
+        assert int(acc[b]) == a and path[b, :a].tolist() == p_o.tolist() and em[b, :a + 1].tolist() == e_o.tolist()
+    lb.free(); qb.free()
+    stream.destroy()
+    dev.close()

@@ -180,13 +180,20 @@ __device__ __forceinline__ unsigned long long add_p(unsigned long long a, unsign
     asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
     return d;
 }
+__device__ __forceinline__ float max_nan(float a, float b) {
+    float d;
+    asm("max.NaN.f32 %0, %1, %2;" : "=f"(d) : "f"(a), "f"(b));
+    return d;
+}
 // Weights of two logits: w = (uint64)(exp_det((L - mx) / T) * 2^40) with
 //   exp_det(x): n = rint(x * 1.44269504), r = x - n ln 2 in two parts, a degree-5 polynomial, times 2^n; 0 below -87.
-// rint is an addition and subtraction of 1.5 * 2^23 (|x log2 e| < 2^22), whose low bits are n; 2^n * 2^40 is one
-// exact multiplication; x is clamped at -87, where the weight is 0 as well (anything below 2^-40 is).
+// (the polynomial and the parts of ln 2 are those of expf in the Cephes library). rint is an addition and subtraction of
+// 1.5 * 2^23 (|x log2 e| < 2^22), whose low bits are n; 2^n * 2^40 is one exact multiplication; x is clamped at -87, where
+// the weight is 0 as well (anything below 2^-40 is). A logit of +infinity, or a 1 / T that overflows, makes x a NaN at the
+// maximum: it passes the clamp and converts to 2^63, so that such a token takes all the weight.
 __device__ __forceinline__ void target_weights2(float l0, float l1, float mx, float inv_t, unsigned long long & w0, unsigned long long & w1) {
     const float2 xs = unpack2(mul_p(add_p(pack2(l0, l1), pack2(-mx, -mx)), pack2(inv_t, inv_t)));
-    const unsigned long long x = pack2(fmaxf(xs.x, -87.0f), fmaxf(xs.y, -87.0f));
+    const unsigned long long x = pack2(max_nan(xs.x, -87.0f), max_nan(xs.y, -87.0f));
     const unsigned long long shifted = add_p(mul_p(x, pack2(1.44269504f, 1.44269504f)), pack2(12582912.0f, 12582912.0f));
     const unsigned long long n = add_p(shifted, pack2(-12582912.0f, -12582912.0f));
     unsigned long long r = fma_p(n, pack2(-0.693359375f, -0.693359375f), x);
