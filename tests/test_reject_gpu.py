@@ -255,3 +255,64 @@ def test_infinite_logits_take_all_the_weight(V, T):
     lb.free(); qb.free()
     stream.destroy()
     dev.close()
+
+
+@pytest.mark.parametrize("B,N,V", [(1, 64, 4099), (2, 20, 65538), (3, 33, 32768), (9, 18, 248320)])
+def test_nodes_with_many_children(B, N, V):
+    """Most drafts are children of the root, the others of its last child; the walk stores its weights from a second
+    rejection on. Some draft rows take everything away, after which the target's own weights count again (sequence 0);
+    in the others the best token keeps its weight, so that the last child is reached and accepted."""
+    T = 0.9
+    rng = np.random.default_rng(N)
+    parent = np.zeros(N, np.int32)
+    parent[0], parent[N - 6:] = -1, N - 7
+    seqs = min(B, 3)
+    logits = (3.0 * rng.standard_normal((seqs, N, V), dtype=np.float32)).astype(np.float32)
+    q, tokens = np.zeros((seqs, N, V), np.float32), np.zeros((seqs, N), np.int32)
+    for b in range(seqs):
+        p = softmax32(logits[b, :1] / T)[0], softmax32(logits[b, N - 7:N - 6] / T)[0]
+        for c in range(1, N):
+            q[b, c] = p[c >= N - 6] * np.float32(2.0 if (b + c) % 11 == 5 else rng.uniform(0.02, 0.3))
+            tokens[b, c] = rng.integers(0, V)
+            if c != N - 7: q[b, c, tokens[b, c]] = 0.5  # (much against the target's weight: rejected)
+        tokens[b, N - 7] = best = int(np.argmax(logits[b, 0]))
+        q[b, N - 7, best] = 1e-6
+        if b: q[b, 1:N - 7, best] = 0.0
+    uniforms = np.minimum(rng.random((B, N, 2), dtype=np.float32) * 0.1 + 0.89, np.float32(0.99999994))
+    tile = [b % seqs for b in range(B)]
+    dev = cuda.Device(0)
+    stream = dev.stream()
+    lb, qb = dev.upload(logits[tile]), dev.upload(q[tile])
+    acc, em, path = cuda.accept_tree(stream, lb, tokens[tile], V, parent=np.tile(parent, (B, 1)), mode=cuda.ACCEPT_REJECTION,
+                                     temperature=T, draft_probs=qb, uniforms=uniforms)
+    deep = 0
+    for b in range(B):
+        a, p_o, e_o = yo.accept_rejection_tree(logits[tile[b]], q[tile[b]], tokens[tile[b]], parent, T, uniforms[b])
+        assert int(acc[b]) == a and path[b, :a].tolist() == p_o.tolist() and em[b, :a + 1].tolist() == e_o.tolist(), b
+        deep += a > 0
+    assert deep > 0 or B == 1
+    lb.free(); qb.free()
+    stream.destroy()
+    dev.close()
+
+
+def test_session_step_with_many_children(tiny):
+    cfg, gm, dev = tiny
+    V, N, B = cfg["vocab"], 18, 2
+    rng = np.random.default_rng(8)
+    parent = np.zeros(N, np.int32)
+    parent[0] = -1
+    sess = cuda.Session(gm, max_batch=B, max_nodes=N, capacity=64, kv_format=cuda.KV_F32)
+    tokens = rng.integers(0, V, (B, N)).astype(np.int32)
+    logits = sess.verify(tokens, parent=parent, mode=cuda.ACCEPT_NONE, want_logits=True).logits
+    q = np.repeat(softmax32(logits[:, :1] / 0.8) * np.float32(0.2), N, 1)
+    np.put_along_axis(q, tokens[:, :, None].astype(np.int64), np.float32(0.6), 2)
+    uniforms = np.full((B, N, 2), 0.97, np.float32)
+    qbuf = dev.upload(q)
+    res = sess.verify(tokens, parent=parent, mode=cuda.ACCEPT_REJECTION, temperature=0.8, draft_probs=qbuf, uniforms=uniforms)
+    for b in range(B):
+        a, p_o, e_o = yo.accept_rejection_tree(logits[b], q[b], tokens[b], parent, 0.8, uniforms[b])
+        assert int(res.accepted[b]) == a and res.path[b, :a].tolist() == p_o.tolist()
+        assert res.emitted[b, :a + 1].tolist() == e_o.tolist()
+    qbuf.free()
+    sess.close()

@@ -6,6 +6,7 @@
 // cur the wanted token is argmax(logits[cur]); the lowest-numbered child of
 // cur that carries it is accepted and becomes cur; otherwise the wanted token
 // is emitted as the correction and the walk ends.
+#include <algorithm>
 #include <cstring>
 #include <mutex>
 #include <vector>
@@ -216,11 +217,13 @@ constexpr int REJ_THREADS = 512;
 constexpr int REJ_WARPS = REJ_THREADS / 32;
 constexpr int REJ_MAX_CLUSTER = 8;   // CTAs that share one sequence's vocabulary
 constexpr int REJ_MAX_NODES = 64;
+constexpr int REJ_KEEP = 2;       // rejected drafts of a node whose rows a pass reads again; at this many the weights are stored
 
 struct RejectParams {
     const float * logits;   // [batch][nodes][vocab]
     const float * q;        // [batch][nodes][vocab]
     const float * u;        // [batch][nodes][2]
+    unsigned long long * r; // [batch][vocab], for trees with many siblings (see REJ_STORE_SIBLINGS), else null
     int vocab;
     float inv_t;
     RowMeta rows;
@@ -248,16 +251,19 @@ __device__ __forceinline__ unsigned long long take_away(unsigned long long r, fl
 // contiguous run of `run` tokens. All CTAs of a cluster walk the tree together: the deciding quantities (the
 // maximum, R, r[x], the uniforms) are the same everywhere, so they take the same turns; rank 0 writes the path.
 //
-// The residual weights are never stored. They are elementwise functions of a row of logits and of the draft rows
-// rejected at the node so far, so each pass recomputes them from those rows, which the first pass has left in L2:
+// The residual weights are not stored as long as a node has few children. They are elementwise functions of a row of
+// logits and of the draft rows rejected at the node so far, so each pass recomputes them from those rows, which the first pass has left in L2:
 // 4 bytes read per token and pass, where keeping them moved 16. What bounds the walk is then latency (two
 // passes, two exchanges a node, each behind the one before), so the grid is chosen for one wave of all sequences
 // (rejection_cluster), with two CTAs to an SM to overlap one's exchanges with another's passes.
 // 64 sequences x 9 rows x 248,320 tokens at T = 0.7 (1.6 accepted a sequence): 361 -> 181 us, one sequence 39 us; all
 // eight drafts accepted 262 us, of which 9 x 64 MB of logits are 90 us at the measured copy rate.
+// Each pass after a rejection reads one draft row more, so a node with many children stores the weights from the second
+// rejection on and each pass reads them and one draft row. One sequence, all drafts children of the root and rejected:
+// eight drafts 224 -> 127 us, sixteen 634 -> 225, 63 7167 -> 963; with four 93 either way, so those go without the scratch.
 // Sums and maxima cross the cluster by stores into every CTA's slots and one hardware barrier; slots alternate
 // between two sets (a CTA can only be one exchange ahead of the slowest).
-template <int CL, bool VEC>
+template <int CL, bool VEC, bool STORE>
 __global__ void __launch_bounds__(REJ_THREADS, 2) rejection_walk_kernel(const RejectParams p, int slice, int run) {
     pdl_entry();
     __shared__ unsigned long long red[REJ_WARPS];
@@ -272,6 +278,7 @@ __global__ void __launch_bounds__(REJ_THREADS, 2) rejection_walk_kernel(const Re
     const int32_t * parent = p.rows.parent + (int64_t)seq * N;
     const float * U = p.u + (int64_t)seq * N * 2;
     const float * Q = p.q + (int64_t)seq * N * V;
+    unsigned long long * r = STORE ? p.r + (int64_t)seq * V : nullptr;
     int32_t * path = p.out.path + (int64_t)seq * N;
     int32_t * emitted = p.out.emitted + (int64_t)seq * N;
     if constexpr (CL > 1) cluster_sync_all();  // every CTA of the cluster has started before another stores into it
@@ -314,11 +321,17 @@ __global__ void __launch_bounds__(REJ_THREADS, 2) rejection_walk_kernel(const Re
 #pragma unroll
         for (int c = 0; c < CL; c++) mx = fmaxf(mx, __uint_as_float((uint32_t)slots[turn ^ 1][c]));
         int n_rej = 0;
+        bool stored = false;  // r holds the weights, and the list of rejected rows those that r does not know of yet
         // weights of tokens i .. i + 3, zero from `end` on
         auto weights_at4 = [&](int i, int end, unsigned long long (&w)[4]) {
-            const float4 l = load4<VEC>(L, i, end, -INFINITY);
-            target_weights2(l.x, l.y, mx, p.inv_t, w[0], w[1]);
-            target_weights2(l.z, l.w, mx, p.inv_t, w[2], w[3]);
+            if (STORE && stored) {
+#pragma unroll
+                for (int e = 0; e < 4; e++) w[e] = i + e < end ? __ldcg(r + i + e) : 0ull;
+            } else {
+                const float4 l = load4<VEC>(L, i, end, -INFINITY);
+                target_weights2(l.x, l.y, mx, p.inv_t, w[0], w[1]);
+                target_weights2(l.z, l.w, mx, p.inv_t, w[2], w[3]);
+            }
             for (int j = 0; j < n_rej; j++) {
                 const float4 q = load4<VEC>(Q + (int64_t)rejected[j] * V, i, end, 0.0f);
                 const double Rj = rejected_R[j];
@@ -331,6 +344,27 @@ __global__ void __launch_bounds__(REJ_THREADS, 2) rejection_walk_kernel(const Re
         // sum of the weights of this warp's run
         auto run_sum = [&]() {
             unsigned long long sum = 0;
+            if (STORE && stored) {  // and one row since
+                const float * q = Q + (int64_t)rejected[0] * V;
+                const double R0 = rejected_R[0];
+                for (int i0 = s0 + lane; i0 < s1; i0 += 8 * 32) {
+                    unsigned long long w[8];
+                    float d[8];
+#pragma unroll
+                    for (int u = 0; u < 8; u++) {
+                        const int i = i0 + u * 32;
+                        w[u] = i < s1 ? __ldcg(r + i) : 0ull;
+                        d[u] = i < s1 ? q[i] : 0.0f;
+                    }
+#pragma unroll
+                    for (int u = 0; u < 8; u++) {
+                        w[u] = take_away(w[u], d[u], R0);
+                        sum += w[u];
+                        if (i0 + u * 32 < s1) __stcg(r + i0 + u * 32, w[u]);
+                    }
+                }
+                return sum;
+            }
             if (n_rej == 0) {
                 for (int i0 = s0 + lane * 4; i0 < s1; i0 += 4 * 128) {
                     float4 l[4];
@@ -371,12 +405,18 @@ __global__ void __launch_bounds__(REJ_THREADS, 2) rejection_walk_kernel(const Re
                 unsigned long long w[4];
                 weights_at4(i0, s1, w);
                 sum += (w[0] + w[1]) + (w[2] + w[3]);
+                if (STORE) {
+#pragma unroll
+                    for (int e = 0; e < 4; e++)
+                        if (i0 + e < s1) __stcg(r + i0 + e, w[e]);
+                }
             }
             return sum;
         };
         auto weight_at = [&](int x) {
             unsigned long long w, unused;
-            target_weights2(L[x], mx, mx, p.inv_t, w, unused);
+            if (STORE && stored) w = __ldcg(r + x);  // (another CTA's, perhaps: an exchange lies between)
+            else target_weights2(L[x], mx, mx, p.inv_t, w, unused);
             for (int j = 0; j < n_rej; j++) w = take_away(w, Q[(int64_t)rejected[j] * V + x], rejected_R[j]);
             return w;
         };
@@ -404,7 +444,8 @@ __global__ void __launch_bounds__(REJ_THREADS, 2) rejection_walk_kernel(const Re
                 next = c;
                 break;
             }
-            __syncthreads();  // the list may still be in use
+            if (STORE && CL > 1 && stored) cluster_sync_all();  // every CTA has read r[x], which its owner is about to replace
+            else __syncthreads();                      // the list may still be in use
             if (tid == 0) {
                 rejected[n_rej] = c;
                 rejected_R[n_rej] = (double)R;
@@ -413,7 +454,12 @@ __global__ void __launch_bounds__(REJ_THREADS, 2) rejection_walk_kernel(const Re
             __syncthreads();
             exchange(run_sum(), false);
             R = total();
+            if (STORE && n_rej >= (stored ? 1 : REJ_KEEP)) {
+                stored = true;
+                n_rej = 0;
+            }
             if (R == 0) {  // nothing is left: the target's own weights again
+                stored = false;
                 n_rej = 0;
                 exchange(run_sum(), false);
                 R = total();
@@ -491,16 +537,26 @@ template <int CL>
 static void launch_rejection(cudaStream_t s, const RejectParams & p) {
     const int slice = ((p.vocab + CL - 1) / CL + 3) & ~3, run = ((slice + REJ_WARPS - 1) / REJ_WARPS + 3) & ~3;
     const bool vec = (p.vocab & 3) == 0 && (((uintptr_t)p.logits | (uintptr_t)p.q) & 15) == 0;
-    auto kern = vec ? rejection_walk_kernel<CL, true> : rejection_walk_kernel<CL, false>;
+    auto kern = p.r ? (vec ? rejection_walk_kernel<CL, true, true> : rejection_walk_kernel<CL, false, true>)
+                    : (vec ? rejection_walk_kernel<CL, true, false> : rejection_walk_kernel<CL, false, false>);
     if (CL > 1) launch_k_cluster(kern, dim3(p.rows.batch * CL), REJ_THREADS, 0, s, CL, p, slice, run);
     else launch_k(kern, p.rows.batch, REJ_THREADS, 0, s, p, slice, run);
 }
 
-int launch_accept_rejection(cudaStream_t s, const float * logits, const float * draft_probs, const float * uniforms, int vocab,
-                            float temperature, const RowMeta & rows, const AcceptOut & out) {
+int rejection_siblings(const int32_t * parent, int batch, int nodes) {
+    int most = 1;
+    for (int b = 0; parent && b < batch; b++) {
+        int children[REJ_MAX_NODES] = {};
+        for (int i = 1; i < nodes; i++) most = std::max(most, ++children[parent[b * nodes + i]]);
+    }
+    return most;
+}
+
+int launch_accept_rejection(cudaStream_t s, const float * logits, const float * draft_probs, const float * uniforms, unsigned long long * residual,
+                            int vocab, float temperature, const RowMeta & rows, const AcceptOut & out) {
     YK_REQUIRE(temperature > 0.0f, YUUKA_ERR_INVALID_ARGUMENT, "rejection sampling needs a temperature above zero");
     YK_REQUIRE(rows.nodes <= REJ_MAX_NODES, YUUKA_ERR_UNSUPPORTED, "rejection sampling: at most %d rows per sequence", REJ_MAX_NODES);
-    RejectParams p{logits, draft_probs, uniforms, vocab, 1.0f / temperature, rows, out};
+    RejectParams p{logits, draft_probs, uniforms, residual, vocab, 1.0f / temperature, rows, out};
     switch (rejection_cluster(rows.batch, vocab)) {
     case 8: launch_rejection<8>(s, p); break;
     case 4: launch_rejection<4>(s, p); break;
@@ -574,11 +630,14 @@ extern "C" yuuka_status yuuka_accept_tree(yuuka_stream * stream, const yuuka_buf
         const int chunks = argmax_chunks(vocab);
         const bool reject = mode == YUUKA_ACCEPT_REJECTION;
         // inputs, filled by one copy: anc | uniforms | tokens | parent | depth; results, read by one copy: accepted |
-        // path | emitted; then scratch: argmax val, idx
+        // path | emitted; then scratch: argmax val, idx or the residual weights
         const size_t o_anc = 0, o_uni = o_anc + R * 8, o_tok = o_uni + (reject ? R * 8 : 0), o_par = o_tok + R * 4, o_dep = o_par + R * 4,
                      o_acc = o_dep + R * 4, o_path = o_acc + (size_t)batch * 4, o_em = o_path + R * 4, staged = o_em + R * 4,
-                     o_val = (staged + 255) / 256 * 256, o_idx = o_val + (reject ? 0 : R * chunks * 4),
-                     total = o_idx + (reject ? 0 : R * chunks * 4);
+                     o_val = (staged + 255) / 256 * 256, o_idx = o_val + (reject ? 0 : R * chunks * 4), weights = (size_t)batch * vocab * 8;
+        // (weights beyond what the stream's scratch keeps cost an allocation, about what 16 rejected siblings cost without them)
+        const int siblings = reject ? rejection_siblings(parent, batch, nodes) : 0;
+        const bool stores = siblings >= REJ_STORE_SIBLINGS && (o_val + weights <= StreamScratch::KEEP || siblings > 16);
+        const size_t total = o_idx + (reject ? (stores ? weights : 0) : R * chunks * 4);
         std::lock_guard<std::mutex> lock(stream->scratch.mutex);
         StreamScratchUse use(stream->scratch, total, staged);
         uint8_t * d = use.device, * h = use.host;
@@ -598,7 +657,7 @@ extern "C" yuuka_status yuuka_accept_tree(yuuka_stream * stream, const yuuka_buf
             launch_accept_greedy(st, (const float *)logits->ptr, vocab, rows, sc, out);
         } else {
             launch_accept_rejection(st, (const float *)logits->ptr, (const float *)draft_probs->ptr, (const float *)(d + o_uni),
-                                    vocab, temperature, rows, out);
+                                    stores ? (unsigned long long *)(d + o_val) : nullptr, vocab, temperature, rows, out);
         }
         if (end) YK_CUDA(cudaEventRecord(end->e, st));
         YK_CUDA(cudaMemcpyAsync(h + o_acc, d + o_acc, staged - o_acc, cudaMemcpyDeviceToHost, st));

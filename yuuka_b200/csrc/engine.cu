@@ -598,6 +598,8 @@ struct yuuka_session {
     float st_temperature = 0.0f;
     const float * st_draft_probs = nullptr;   // device, rejection mode
     float * d_uniforms = nullptr;             // [max_batch * max_nodes * 2]
+    unsigned long long * reject_residual = nullptr;  // [max_batch][vocab], allocated by the first rejection step that stores weights
+    bool st_stores = false;
     bool staged = false, launched = false;
     uint32_t launches = 0;
     // captured steps, keyed by (seq0, batch, nodes, chains, mode), least recently used first; at most
@@ -1086,8 +1088,8 @@ void run_step(yuuka_session * s, int seq0, int batch, int nodes, uint32_t mode, 
     if (mode == YUUKA_ACCEPT_GREEDY) {
         s->launches += launch_accept_greedy(st, s->logits, c.vocab, rows, s->argmax, s->acc);
     } else if (mode == YUUKA_ACCEPT_REJECTION) {
-        s->launches += launch_accept_rejection(st, s->logits, s->st_draft_probs, s->d_uniforms, c.vocab, s->st_temperature,
-                                               rows, s->acc);
+        s->launches += launch_accept_rejection(st, s->logits, s->st_draft_probs, s->d_uniforms, s->st_stores ? s->reject_residual : nullptr,
+                                               c.vocab, s->st_temperature, rows, s->acc);
     } else {
         launch_accept_all(st, rows, s->acc);  // forced commit of a chain
         s->launches++;
@@ -1733,6 +1735,9 @@ yuuka_status yuuka_verify_stage(yuuka_session * s, const yuuka_verify_batch * b)
         s->st_seqs.resize((size_t)b->batch);
         for (int i = 0; i < b->batch; i++) s->st_seqs[(size_t)i] = b->seq_ids ? b->seq_ids[i] : i;
         if (b->mode == YUUKA_ACCEPT_REJECTION) {
+            s->st_stores = rejection_siblings(b->parent, b->batch, b->nodes) >= REJ_STORE_SIBLINGS;
+            if (s->st_stores && !s->reject_residual)
+                s->reject_residual = dalloc<unsigned long long>((size_t)s->cfg.max_batch * s->model->cfg.vocab, s->owned, false);
             for (int i = 0; i < b->batch * b->nodes * 2; i++)
                 YK_REQUIRE(b->uniforms[i] >= 0.0f && b->uniforms[i] < 1.0f, YUUKA_ERR_INVALID_ARGUMENT,
                            "verify: uniform draw %d is outside [0, 1)", i);

@@ -132,8 +132,12 @@ int launch_accept_greedy(cudaStream_t s, const float * logits, int vocab, const 
                          const ArgmaxScratch & scratch, const AcceptOut & out);
 // Rejection-sampling walk (rule in accept.cu).
 // draft_probs [batch][nodes][vocab] and uniforms [batch][nodes][2] are device arrays.
-int launch_accept_rejection(cudaStream_t s, const float * logits, const float * draft_probs, const float * uniforms, int vocab,
-                            float temperature, const RowMeta & rows, const AcceptOut & out);
+// residual: scratch of batch * vocab 64-bit words for trees of which a node has many children (rejection_siblings, the most
+// that a node has), or null: from REJ_STORE_SIBLINGS on the walk is faster with it (see the kernel).
+constexpr int REJ_STORE_SIBLINGS = 5;
+int rejection_siblings(const int32_t * parent, int batch, int nodes);
+int launch_accept_rejection(cudaStream_t s, const float * logits, const float * draft_probs, const float * uniforms, unsigned long long * residual,
+                            int vocab, float temperature, const RowMeta & rows, const AcceptOut & out);
 // Accept every row of a chain (prefill / forced commit): accepted = nodes-1.
 void launch_accept_all(cudaStream_t s, const RowMeta & rows, const AcceptOut & out);
 int argmax_chunks(int vocab);
