@@ -734,3 +734,30 @@ def test_an_expired_wait_in_each_gemm_kernel_leaves_the_device_usable(tiny, n):
         b.free()
     stream.destroy()
     sess.close()
+
+
+@pytest.mark.parametrize("kv", [cuda.KV_F16, cuda.KV_F32, cuda.KV_Q8_0])
+@pytest.mark.parametrize("nodes,head_dim", [(16, 64), (17, 64), (20, 256), (21, 128), (33, 256), (40, 64)])
+def test_steps_at_the_edges_of_the_query_rows_a_cta_holds(kv, nodes, head_dim):
+    """Four query heads per KV head: 64 and 80 query rows are one CTA's, more are two's, and the key ranges are cut for
+    as many as there are; contexts end within a tile of keys."""
+    cfg = synth.tiny_config()
+    cfg.update(heads=8, kv_heads=2, head_dim=head_dim, rope_dim=32, vocab=512)
+    tensors = synth.make_model(cfg, "q8_0", seed=50 + nodes, unit_norms=False)
+    dev = cuda.Device(0)
+    gm, om = cuda.Model(dev, cfg, tensors), yo.Model(cfg, tensors)
+    sess = cuda.Session(gm, max_batch=1, max_nodes=nodes, capacity=320, kv_format=kv)
+    prompt = synth.uniform_i32(203, 0, cfg["vocab"], 51)
+    rows = synth.uniform_i32(nodes, 0, cfg["vocab"], 52)
+    sess.set_flags(cuda.SESSION_EXACT_WIDE)
+    sess.forward(prompt, want_logits=False)
+    got = sess.verify([rows], mode=cuda.ACCEPT_NONE, want_logits=True).logits[0]
+    st = yo.State(om, 320, {cuda.KV_F16: yo.KV_F16, cuda.KV_F32: yo.KV_F32, cuda.KV_Q8_0: yo.KV_Q8_0}[kv])
+    st.forward(prompt)
+    _, _, want = st.verify_chain(int(rows[0]), rows[1:], want_logits=True)
+    st.close()
+    err = float(np.max(np.abs(got - want)))
+    assert err <= LOGIT_TOL, err
+    sess.close()
+    gm.close()
+    dev.close()

@@ -52,6 +52,24 @@ __device__ __forceinline__ void kv_decode8(const uint8_t * row, int format, int 
     }
 }
 
+// The same of an F32 or a Q8_0 row (blocks of 34 bytes: two at a time).
+template <bool F32> __device__ __forceinline__ void kv_read8(const uint8_t * row, int e8, float (&w)[8]) {
+    if constexpr (F32) {
+        const float4 * p = reinterpret_cast<const float4 *>(row + e8 * 32);
+        const float4 a = __ldg(p), b = __ldg(p + 1);
+        w[0] = a.x; w[1] = a.y; w[2] = a.z; w[3] = a.w; w[4] = b.x; w[5] = b.y; w[6] = b.z; w[7] = b.w;
+    } else {
+        const uint16_t * blk = reinterpret_cast<const uint16_t *>(row + (e8 >> 2) * 34);
+        const float d = __half2float(__ushort_as_half(__ldg(blk)));
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            const uint32_t q = __ldg(blk + 1 + (e8 & 3) * 4 + i);
+            w[2 * i] = d * (float)(int8_t)(q & 0xffu);
+            w[2 * i + 1] = d * (float)(int8_t)(q >> 8);
+        }
+    }
+}
+
 template <int HD>
 __global__ void __launch_bounds__(ATT_WARPS * 32) attention_partial_kernel(const AttnParams p) {
     pdl_entry();
@@ -214,8 +232,11 @@ static int attention_row_blocks(int q_rows) {
     if (blocks <= AM_RB_MAX) return blocks;
     return (blocks + 4) / 5 * 5 < (blocks + 3) / 4 * 4 ? 5 : 4;
 }
-// The key ranges are cut for tiles of three or four row blocks, whichever needs fewer: the cut decides the order of the
-// sums, so it does not follow the row blocks a CTA happens to hold.
+int attention_query_ctas(int q_rows) {
+    const int per = 16 * attention_row_blocks(q_rows);
+    return (q_rows + per - 1) / per;
+}
+// The key ranges of many sequences are cut for tiles of three or four row blocks, whichever needs fewer.
 int attention_query_tiles(int q_rows) {
     const int t3 = (q_rows + 47) / 48, t4 = (q_rows + 63) / 64;
     return t3 * 3 < t4 * 4 ? t3 : t4;
@@ -261,6 +282,7 @@ __global__ void __launch_bounds__(RB * 64, RB <= 3 ? 2 : 1) attention_mma_kernel
     constexpr int NT_O = DW / 8;  // 8-column output tiles per warp
     constexpr int KQ = HD / 64;   // 16-dimension steps of a quarter of the head
     constexpr int STAGES = attention_stages(KSPLIT, RB);
+    constexpr int CONVERT = RB == 4 ? 4 : 2;  // (five row blocks leave a thread 168 registers instead of 255)
     extern __shared__ __align__(16) uint8_t smraw[];
     __half * stage0 = reinterpret_cast<__half *>(smraw);
     constexpr size_t STAGE = attention_stage_halves(HD, KSPLIT);
@@ -303,6 +325,37 @@ __global__ void __launch_bounds__(RB * 64, RB <= 3 ? 2 : 1) attention_mma_kernel
             const int bytes = in ? 16 : 0;
             asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(p.pool.k + off), "r"(bytes) : "memory");
             asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst + V_AT * 2), "l"(p.pool.v + off), "r"(bytes) : "memory");
+        }
+    };
+    // F32 or Q8_0 pool: by way of registers, the loads of CONVERT pieces in flight at once. (One after the other, each behind
+    // the stores of the one before, a 9-row step over 16,000 F32 rows took 755 us in four layers instead of 644.)
+    auto convert = [&](int tile, auto f32) {
+        const int k0 = k_begin + tile * AM_KT;
+        for (int i0 = threadIdx.x; i0 < PIECES; i0 += CONVERT * THREADS) {
+            float kw[CONVERT][8], vw[CONVERT][8];
+#pragma unroll
+            for (int u = 0; u < CONVERT; u++) {
+                const int i = min(i0 + u * THREADS, PIECES - 1), j = i / (HD / 8), e8 = kvh * (HD / 8) + i - j * (HD / 8);
+                const int64_t off = row_offset(min(k0 + j, k_end - 1));
+                kv_read8<decltype(f32)::value>(p.pool.k + off, e8, kw[u]);
+                kv_read8<decltype(f32)::value>(p.pool.v + off, e8, vw[u]);
+            }
+#pragma unroll
+            for (int u = 0; u < CONVERT; u++) {
+                const int i = i0 + u * THREADS, j = i / (HD / 8), c8 = i - j * (HD / 8);
+                if (i >= PIECES) continue;
+                const bool in = k0 + j < k_end;
+                __half hh[8], ll[8], vv[8];
+#pragma unroll
+                for (int e = 0; e < 8; e++) {
+                    hh[e] = split_half(in ? kw[u][e] : 0.0f, ll[e]);
+                    vv[e] = __float2half_rn(in ? vw[u][e] : 0.0f);
+                }
+                __half * at = stage0 + j * STR + c8 * 8;
+                *reinterpret_cast<uint4 *>(at) = *reinterpret_cast<const uint4 *>(hh);
+                *reinterpret_cast<uint4 *>(at + AM_KT * STR) = *reinterpret_cast<const uint4 *>(ll);
+                *reinterpret_cast<uint4 *>(at + V_AT) = *reinterpret_cast<const uint4 *>(vv);
+            }
         }
     };
     const int tiles = (k_end - k_begin + AM_KT - 1) / AM_KT;
@@ -356,31 +409,8 @@ __global__ void __launch_bounds__(RB * 64, RB <= 3 ? 2 : 1) attention_mma_kernel
             asm volatile("cp.async.commit_group;" ::: "memory");
         } else {
             __syncthreads();
-#pragma unroll 2
-            for (int i = threadIdx.x; i < PIECES; i += THREADS) {
-                const int j = i / (HD / 8), c8 = i - j * (HD / 8);
-                const int pos = k0 + j;
-                uint4 kh4 = make_uint4(0, 0, 0, 0), kl4 = kh4, vh4 = kh4;
-                if (pos < k_end) {
-                    const int64_t off = row_offset(pos);
-                    float kw[8], vw[8];
-                    kv_decode8(p.pool.k + off, p.pool.format, kvh * (HD / 8) + c8, kw);
-                    kv_decode8(p.pool.v + off, p.pool.format, kvh * (HD / 8) + c8, vw);
-                    __half hh[8], ll[8], vv[8];
-#pragma unroll
-                    for (int e = 0; e < 8; e++) {
-                        hh[e] = split_half(kw[e], ll[e]);
-                        vv[e] = __float2half_rn(vw[e]);
-                    }
-                    kh4 = *reinterpret_cast<const uint4 *>(hh);
-                    kl4 = *reinterpret_cast<const uint4 *>(ll);
-                    vh4 = *reinterpret_cast<const uint4 *>(vv);
-                }
-                __half * at = stage0 + j * STR + c8 * 8;
-                *reinterpret_cast<uint4 *>(at) = kh4;
-                *reinterpret_cast<uint4 *>(at + AM_KT * STR) = kl4;
-                *reinterpret_cast<uint4 *>(at + V_AT) = vh4;
-            }
+            if (p.pool.format == YUUKA_KV_F32) convert(tile, std::true_type());
+            else convert(tile, std::false_type());
             __syncthreads();
         }
         if (rb * 16 >= nq) continue;  // (both warps of the block)
@@ -651,10 +681,11 @@ static int launch_attention_hd(cudaStream_t s, float * out, int ldo, const float
     static const bool use_mma = [] { const char * e = getenv("YUUKA_CUDA_ATTN_FP32"); return !(e && e[0] == '1'); }();
     if (use_mma) {
         // tensor-core partials; keys are taken as they are from an F16 pool and split into hi + lo otherwise
-        // (F32 and Q8_0 rows are converted on the way in: the ten warps of the largest CTA do that where one holds all rows.
-        // With the two warps of a one-row step alone it took 33 us more per layer over 2500 Q8_0 rows)
+        // (F32 and Q8_0 rows are converted on the way in: by eight warps at least, which have a tile's loads in flight all at
+        // once. With the ten of a CTA of five row blocks a one-row step over 16,000 Q8_0 rows took 643 us in four layers, with
+        // eight 545)
         const bool convert = pool.format != YUUKA_KV_F16;
-        const int blocks = attention_row_blocks(G * rows.nodes), rb = convert && G * rows.nodes <= 16 * AM_RB_MAX ? AM_RB_MAX : blocks;
+        const int blocks = attention_row_blocks(G * rows.nodes), rb = convert ? std::max(blocks, 4) : blocks;
         const int qtiles = (G * rows.nodes + 16 * rb - 1) / (16 * rb);
         auto launch = [&](auto ksplit) {
             constexpr bool KS = decltype(ksplit)::value;
@@ -663,12 +694,12 @@ static int launch_attention_hd(cudaStream_t s, float * out, int ldo, const float
                 YK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
                 launch_k(kern, dim3(sc.splits, kv_heads * qtiles, rows.batch), rb * 64, smem, s, p);
             };
-            switch (rb) {
-            case 1: with(attention_mma_kernel<HD, KS, 1>); break;
-            case 2: with(attention_mma_kernel<HD, KS, 2>); break;
-            case 3: with(attention_mma_kernel<HD, KS, 3>); break;
-            case 4: with(attention_mma_kernel<HD, KS, 4>); break;
-            default: with(attention_mma_kernel<HD, KS, 5>); break;
+            if (rb == 5) with(attention_mma_kernel<HD, KS, 5>);
+            else if (rb == 4) with(attention_mma_kernel<HD, KS, 4>);
+            else if constexpr (!KS) {
+                if (rb == 3) with(attention_mma_kernel<HD, KS, 3>);
+                else if (rb == 2) with(attention_mma_kernel<HD, KS, 2>);
+                else with(attention_mma_kernel<HD, KS, 1>);
             }
         };
         if (convert) launch(std::true_type());

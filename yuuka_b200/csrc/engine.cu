@@ -785,8 +785,11 @@ enum LogitRows { LOGITS_NONE, LOGITS_LAST, LOGITS_ALL };
 // of one of them walking it alone (ranges beyond a sequence's end exit at once).
 int attention_splits(const yuuka_session * s, int batch, int nodes, int max_total) {
     const yuuka_model_config & c = s->model->cfg;
-    const int sms = s->model->dev->sm_count, base = c.kv_heads * attention_query_tiles(c.heads / c.kv_heads * nodes) * batch;
+    const int q_rows = c.heads / c.kv_heads * nodes, ctas = c.kv_heads * attention_query_ctas(q_rows) * batch;
+    const int sms = s->model->dev->sm_count, base = c.kv_heads * attention_query_tiles(q_rows) * batch;
     int splits = (sms + base - 1) / base;
+    // (where a CTA holds more rows than that cut assumes, an SM of its own each: 17 rows of four heads take 37 ranges, not 19)
+    if (base < sms && ctas < base) splits = sms / ctas;
     if (base >= sms && splits < (max_total + 511) / 512) splits = (max_total + 511) / 512;
     const int most = (max_total + 31) / 32;
     if (splits > most) splits = most;
