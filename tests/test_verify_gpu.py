@@ -701,24 +701,30 @@ def test_prompt_that_fills_a_session_shorter_than_its_chunks(tiny, n, kv):
     assert float(np.max(np.abs(got - want))) <= LOGIT_TOL
 
 
-@pytest.mark.parametrize("n", [4, 30, 48, 300])
-def test_an_expired_wait_in_each_gemm_kernel_leaves_the_device_usable(tiny, n):
-    """Passes of sixteen rows, 17 to 47 rows, tensor memory with one and with several tiles of rows: without their
-    activations the kernels give up, a step reports it, and the same product and step then give the same bits again."""
+@pytest.mark.parametrize("dtype,n_out,n_in,n,code", [
+    (synth.Q8_0, 700, 2048, 4, 1),                                    # passes of sixteen rows
+    (synth.Q8_0, 700, 2048, 30, 4), (synth.Q4_K, 24, 256, 17, 4),     # 17 to 47 rows, small matrices too
+    (synth.Q6_K, 9216, 2560, 20, 4), (synth.Q8_0, 9216, 2560, 20, 1), (synth.Q4_K, 9216, 2560, 28, 1), (synth.Q4_K, 9216, 2560, 29, 4),
+    (synth.Q8_0, 6144, 4096, 20, 4), (synth.Q5_K, 256, 9216, 20, 1), (synth.Q5_K, 256, 9216, 21, 4),
+    (synth.Q4_K, 512, 16640, 20, 1),                                  # more superblocks than the cuts have bits
+    (synth.Q8_0, 700, 2048, 48, 3), (synth.Q8_0, 700, 2048, 300, 3),  # tensor memory, one and several tiles of rows
+])
+def test_an_expired_wait_in_each_gemm_kernel_leaves_the_device_usable(tiny, dtype, n_out, n_in, n, code):
+    """Without their activations the kernels give up, a step reports it with the code of the kernel that the route has
+    taken, and the same product and step then give the same bits again."""
     cfg, gm, om = tiny
     rows = synth.uniform_i32(5, 0, cfg["vocab"], 902).tolist()
     sess = cuda.Session(gm, max_batch=1, max_nodes=5, capacity=64, kv_format=cuda.KV_F32)
     good = sess.verify([rows], mode=cuda.ACCEPT_NONE, want_logits=True).logits[0].copy()
     stream = gm.dev.stream()
-    n_out, n_in = 700, 2048
-    raw = gm.dev.upload(synth.normal_quant(n_out, n_in, synth.Q8_0, 0.02, 3))
-    wb = gm.dev.alloc(cuda.tiled_bytes(synth.Q8_0, n_out, n_in) + 256)
-    cuda.tile_weights(stream, wb, raw, synth.Q8_0, n_out, n_in)
+    raw = gm.dev.upload(synth.normal_quant(n_out, n_in, dtype, 0.02, 3))
+    wb = gm.dev.alloc(cuda.tiled_bytes(dtype, n_out, n_in) + 256)
+    cuda.tile_weights(stream, wb, raw, dtype, n_out, n_in)
     xb = gm.dev.upload(synth.normal_f32(n * n_in, 1.0, 4))
     ob = gm.dev.alloc(n * n_out * 4)
 
     def product(flags=0):
-        cuda.gemm_quant(stream, ob, xb, wb, n_in, n_out, n, synth.Q8_0, cuda.F32, cuda.PATH_MMA, flags=cuda.GEMM_TILED | flags)
+        cuda.gemm_quant(stream, ob, xb, wb, n_in, n_out, n, dtype, cuda.F32, cuda.PATH_MMA, flags=cuda.GEMM_TILED | flags)
         stream.synchronize()
         return ob.read(np.uint32, n * n_out)
 
@@ -726,7 +732,7 @@ def test_an_expired_wait_in_each_gemm_kernel_leaves_the_device_usable(tiny, n):
     product(cuda.GEMM_TEST_DROP_COPIES)
     with pytest.raises(cuda.YuukaError) as e:
         sess.verify([rows], mode=cuda.ACCEPT_NONE)
-    assert e.value.status == cuda.ERR_DEVICE
+    assert e.value.status == cuda.ERR_DEVICE and f"(code {code})" in str(e.value)
     again = sess.verify([rows], mode=cuda.ACCEPT_NONE, want_logits=True).logits[0]
     assert np.array_equal(again.view(np.uint32), good.view(np.uint32))
     assert np.array_equal(product(), want)

@@ -1844,14 +1844,27 @@ static uint64_t rows_partial_floats(const RParams & p, int m, int n_out) {
     return (uint64_t)parts * m * n_out;
 }
 // From 17 rows, where passes of sixteen would begin to decode the weights more than once; K of at most 64 superblocks (the
-// masks of RowCut). Up to 24 rows a matrix of under 1024 records has too little to decode for that to matter: 700 x 2048
-// takes 15.7 us in two passes and 17.5 here at 17 rows, 16.9 and 17.6 at 24. (Launches that fold a norm or SwiGLU into their
-// epilogue, steps of up to 32 rows, stay with the passes.)
-static bool rows_route(int m, int n_out, int n_in) {
-    return m > MMA_ROWS && n_in <= 64 * 256 && (m > 24 || (int64_t)((n_out + 15) / 16) * (n_in / 256) >= 1024);
+// masks of RowCut). (Launches that fold a norm or SwiGLU into their epilogue, steps of up to 32 rows, stay with the passes.)
+// Over 256 to 32768 x 512 to 9216 of the four types it takes 0.54 to 1.3 of the time of the passes at 17 rows (mean 0.87) and
+// 0.39 to 1.06 at 36. What it is slower at stays with the passes:
+// - matrices of few tiles and a long K, which its ranges of K (at most eight) leave too long (256 x 9216: 20.1 us against 17.0
+//   at 17 rows, 4096 columns 11.2 against 13.5);
+// - two to four tiles per SM, where its CTAs would have four warps, one per scheduler, which wait for their own records, and no
+//   ranges of K (plan_rows' cost of one range, 4 nsb + 2, against that of two). Q8_0, which is decoded twice at little cost, up
+//   to 32 rows (6144 x 2048: 19.4 against 15.2 at 17; 9216 x 2560: 24.6 against 21.2 at 20), Q4_K up to 28 (9216 x 9216: 58.9
+//   against 48.9 at 17); Q5_K and Q6_K 0.95 to 1.1 either way.
+static bool rows_possible(int m, int n_in) { return m > MMA_ROWS && n_in <= 64 * 256; }
+static bool rows_route(const yuuka_device * dev, uint32_t dtype, int m, int n_out, int n_in) {
+    if (!rows_possible(m, n_in)) return false;
+    const int tiles = (n_out + 15) / 16, nsb = n_in / 256, sms = dev->sm_count;
+    if (m <= 20 && 8 * tiles <= sms && nsb >= 32) return false;
+    if (m > (dtype == YUUKA_DTYPE_Q8_0 ? 32 : (dtype == YUUKA_DTYPE_Q4_K ? 28 : 0))) return true;
+    if (nsb < 8 || tiles <= 2 * sms || tiles > 4 * sms) return true;
+    const int tg = (2 * tiles + sms - 1) / sms;  // tiles per CTA with two ranges of K: tg nsb / 2 + 12
+    return tg <= RW_WARPS && (8 - tg) * nsb > 20;
 }
 bool gemm_tiled_rows_swiglu(int rows, int n_in, bool exact_only, bool wide_from_33) {
-    return rows > 32 && rows <= RW_MAX_ROWS && rows_route(rows, 16, n_in) && !gemm_tiled_wide(rows, exact_only, wide_from_33);
+    return rows > 32 && rows <= RW_MAX_ROWS && rows_possible(rows, n_in) && !gemm_tiled_wide(rows, exact_only, wide_from_33);
 }
 
 // What passes of m rows (at most MMA_ROWS) leave in the scratch where their plan cuts K across CTAs.
@@ -1880,7 +1893,7 @@ TiledScratchNeed gemm_tiled_scratch_need(const yuuka_device * dev, uint32_t w_dt
     need.wanted = need.floats;
     for (int m0 = 0; m0 < rows; m0 += RW_MAX_ROWS) {
         const int m = std::min(rows - m0, RW_MAX_ROWS);
-        if (!rows_route(m, n_out, n_in) || (m0 > 0 && m == RW_MAX_ROWS)) continue;
+        if (!rows_route(dev, w_dtype, m, n_out, n_in) || (m0 > 0 && m == RW_MAX_ROWS)) continue;
         RParams p{};
         plan_rows(dev, w_dtype, m, n_out, n_in, p, false, UINT64_MAX);
         need.wanted = std::max(need.wanted, rows_partial_floats(p, m, n_out));
@@ -1899,7 +1912,7 @@ TiledScratchNeed gemm_tiled_scratch_bound(const yuuka_device * dev, uint32_t w_d
     for (int m = 1; m <= std::min(rows, MMA_ROWS); m++)
         for (bool paired : {false, true}) add_pass_need(dev, w_dtype, m, n_out, n_in, paired, need);
     for (int m = MMA_ROWS + 1; m <= std::min(rows, RW_MAX_ROWS); m++) {
-        if (!rows_route(m, n_out, n_in)) continue;
+        if (!rows_possible(m, n_in)) continue;
         RParams p{};
         plan_rows(dev, w_dtype, m, n_out, n_in, p, false, UINT64_MAX);
         need.floats = std::max(need.floats, rows_partial_floats(p, m, n_out));
@@ -2175,7 +2188,9 @@ static int launch_rows_dt(const yuuka_device * dev, cudaStream_t s, const TiledG
         p.next_w = a.next_w;
         p.next_lines = (uint32_t)(a.next_bytes / 128);
     }
-    switch ((m + 3) / 4) {  // product tiles, four rows each
+    // Product tiles, four rows each. 28 and 44 rows go with the next count: a tile more costs some 2 us (18432 x 2560 Q4_K: 27.2
+    // at 24 rows, 31.3 at 25 to 32, 37.5 at 36, 40.6 at 40, 42.3 at 47), an instance for each count four kernels.
+    switch ((m + 3) / 4) {
     case 5:
     case 6: launch_rows_inst<DT, 6>(dev, s, p, xp, m0); break;
     case 7:
@@ -2242,7 +2257,7 @@ static int launch_mma_dt(const yuuka_device * dev, cudaStream_t s, const TiledGe
     bool normed = false;
     for (int m0 = 0; m0 < a.rows; m0 += m) {
         m = a.rows - m0 < RW_MAX_ROWS ? a.rows - m0 : RW_MAX_ROWS;
-        if (rows_route(m, a.n_out, a.n_in) && !folded) {
+        if (!folded && rows_route(dev, a.w_dtype, m, a.n_out, a.n_in)) {
             const int n = launch_rows_dt<DT>(dev, s, a, xp, m0, m);
             normed = n > 1 && m == a.rows && fuse_row_norm(dev, a);
             launches += n;
