@@ -525,11 +525,11 @@ __global__ void __launch_bounds__(REJ_THREADS, 2) rejection_walk_kernel(const Re
     }
 }
 
-// CTAs per sequence: as many as let all sequences run at once (two CTAs on each of 148 SMs), as long as a CTA keeps
+// CTAs per sequence: as many as let all sequences run at once (two CTAs on each SM), as long as a CTA keeps
 // at least 4,096 tokens (two loads per thread and pass; below that the exchanges cost more than the passes they cut).
-static int rejection_cluster(int batch, int vocab) {
+static int rejection_cluster(int sms, int batch, int vocab) {
     int cl = REJ_MAX_CLUSTER;
-    while (cl > 1 && (batch * cl > 2 * 148 || vocab < cl * 4096)) cl >>= 1;
+    while (cl > 1 && (batch * cl > 2 * sms || vocab < cl * 4096)) cl >>= 1;
     return cl;
 }
 
@@ -552,12 +552,12 @@ int rejection_siblings(const int32_t * parent, int batch, int nodes) {
     return most;
 }
 
-int launch_accept_rejection(cudaStream_t s, const float * logits, const float * draft_probs, const float * uniforms, unsigned long long * residual,
+int launch_accept_rejection(cudaStream_t s, int sms, const float * logits, const float * draft_probs, const float * uniforms, unsigned long long * residual,
                             int vocab, float temperature, const RowMeta & rows, const AcceptOut & out) {
     YK_REQUIRE(temperature > 0.0f, YUUKA_ERR_INVALID_ARGUMENT, "rejection sampling needs a temperature above zero");
     YK_REQUIRE(rows.nodes <= REJ_MAX_NODES, YUUKA_ERR_UNSUPPORTED, "rejection sampling: at most %d rows per sequence", REJ_MAX_NODES);
     RejectParams p{logits, draft_probs, uniforms, residual, vocab, 1.0f / temperature, rows, out};
-    switch (rejection_cluster(rows.batch, vocab)) {
+    switch (rejection_cluster(sms, rows.batch, vocab)) {
     case 8: launch_rejection<8>(s, p); break;
     case 4: launch_rejection<4>(s, p); break;
     case 2: launch_rejection<2>(s, p); break;
@@ -656,7 +656,7 @@ extern "C" yuuka_status yuuka_accept_tree(yuuka_stream * stream, const yuuka_buf
             ArgmaxScratch sc{(float *)(d + o_val), (int32_t *)(d + o_idx), chunks};
             launch_accept_greedy(st, (const float *)logits->ptr, vocab, rows, sc, out);
         } else {
-            launch_accept_rejection(st, (const float *)logits->ptr, (const float *)draft_probs->ptr, (const float *)(d + o_uni),
+            launch_accept_rejection(st, stream->dev->sm_count, (const float *)logits->ptr, (const float *)draft_probs->ptr, (const float *)(d + o_uni),
                                     stores ? (unsigned long long *)(d + o_val) : nullptr, vocab, temperature, rows, out);
         }
         if (end) YK_CUDA(cudaEventRecord(end->e, st));

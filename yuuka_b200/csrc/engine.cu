@@ -906,6 +906,7 @@ void run_step(yuuka_session * s, int seq0, int batch, int nodes, uint32_t mode, 
             g.rank = rank;
             g.S = S;
             g.kernel = c.conv_kernel;
+            g.sms = m->dev->sm_count;
             g.eps = c.rms_eps;
             mark(s, YUUKA_OP_GDN_SCAN);
             if (sub == 0) {
@@ -1091,7 +1092,7 @@ void run_step(yuuka_session * s, int seq0, int batch, int nodes, uint32_t mode, 
     if (mode == YUUKA_ACCEPT_GREEDY) {
         s->launches += launch_accept_greedy(st, s->logits, c.vocab, rows, s->argmax, s->acc);
     } else if (mode == YUUKA_ACCEPT_REJECTION) {
-        s->launches += launch_accept_rejection(st, s->logits, s->st_draft_probs, s->d_uniforms, s->st_stores ? s->reject_residual : nullptr,
+        s->launches += launch_accept_rejection(st, m->dev->sm_count, s->logits, s->st_draft_probs, s->d_uniforms, s->st_stores ? s->reject_residual : nullptr,
                                                c.vocab, s->st_temperature, rows, s->acc);
     } else {
         launch_accept_all(st, rows, s->acc);  // forced commit of a chain

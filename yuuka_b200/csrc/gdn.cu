@@ -169,13 +169,13 @@ template <int S>
 static void launch_gdn_front_s(cudaStream_t s, ScanParams & p) {
     const GdnArgs & a = p.a;
     const int units = 2 * a.groups + a.rank, N = p.rows.nodes;
-    constexpr int64_t WAVE = 148 * 24;
+    const int64_t wave = (int64_t)a.sms * 24;
     const int64_t unit_rows = (int64_t)units * N * p.rows.batch;
-    if (unit_rows * (S / 32) <= WAVE) {
+    if (unit_rows * (S / 32) <= wave) {
         p.block_rows = 1;
         launch_k(a.kernel <= 4 ? gdn_front_kernel<S, 4, true> : gdn_front_kernel<S, 8, true>, dim3(units, N, p.rows.batch), S, 0, s, p);
     } else {
-        const int64_t per_warp = (unit_rows + WAVE - 1) / WAVE;
+        const int64_t per_warp = (unit_rows + wave - 1) / wave;
         const int blocks = (int)((N + 4 * per_warp - 1) / (4 * per_warp));
         p.block_rows = (N + blocks - 1) / blocks;
         launch_k(a.kernel <= 4 ? gdn_front_kernel<S, 4, false> : gdn_front_kernel<S, 8, false>,

@@ -110,6 +110,7 @@ struct GdnArgs {
     float * decay;           // [rows][rank]     log: exp(alpha)
     int groups, rank, S, kernel;
     float eps;
+    int sms;                 // SMs of the device
 };
 // conv + norms, the recurrence and the gated RMSNorm; returns the number of kernels launched
 int launch_gdn_scan(cudaStream_t s, const GdnArgs & a, const RowMeta & rows);
@@ -138,7 +139,7 @@ int launch_accept_greedy(cudaStream_t s, const float * logits, int vocab, const 
 // that a node has), or null: from REJ_STORE_SIBLINGS on the walk is faster with it (see the kernel).
 constexpr int REJ_STORE_SIBLINGS = 5;
 int rejection_siblings(const int32_t * parent, int batch, int nodes);
-int launch_accept_rejection(cudaStream_t s, const float * logits, const float * draft_probs, const float * uniforms, unsigned long long * residual,
+int launch_accept_rejection(cudaStream_t s, int sms, const float * logits, const float * draft_probs, const float * uniforms, unsigned long long * residual,
                             int vocab, float temperature, const RowMeta & rows, const AcceptOut & out);
 // Accept every row of a chain (prefill / forced commit): accepted = nodes-1.
 void launch_accept_all(cudaStream_t s, const RowMeta & rows, const AcceptOut & out);
