@@ -59,7 +59,7 @@ def test_umma_route_accumulates(dev):
 @pytest.mark.parametrize("n_out,n_in,rows", [
     (128, 256, 48),      # one CTA of the pair has no rows of its own; one superblock
     (257, 512, 255), (257, 512, 257),   # a row beyond the first pair; a tile one short of full and one row over
-    (1001, 1536, 97),    # K split with rows that 16-byte stores do not divide
+    (1001, 1536, 97),    # both halves of K on one pair of CTAs, an odd count of rows and of outputs
     (1000, 2560, 289),   # K split, two tiles of rows
     (2560, 768, 513),
     (96000, 256, 48),    # more tiles per pair than there are accumulators
@@ -71,5 +71,19 @@ def test_umma_route_at_the_edges_of_its_tiles(dev, n_out, n_in, rows, dtype):
     x = synth.normal_f32(rows * n_in, 1.0, rows).reshape(rows, n_in)
     want = yo.matmul(w, dtype, n_out, n_in, x)
     got = run_gemm(dev, w, dtype, n_out, n_in, x, cuda.PATH_MMA)
+    err, cos = stats(got, want)
+    assert err <= 6e-3 and cos >= 0.999999, (err, cos)
+
+
+@pytest.mark.parametrize("rows", [48, 96])
+@pytest.mark.parametrize("add", [False, True])
+def test_umma_route_sums_parts_of_rows_that_16_byte_stores_do_not_divide(dev, rows, add):
+    """1001 outputs and up to 96 rows: three parts of K, summed one value at a time."""
+    n_out, n_in, dtype = 1001, 1536, synth.Q4_K
+    w = synth.normal_quant(n_out, n_in, dtype, 0.02, 12)
+    x = synth.normal_f32(rows * n_in, 1.0, 13).reshape(rows, n_in)
+    base = synth.normal_f32(rows * n_out, 1.0, 14).reshape(rows, n_out)
+    want = yo.matmul(w, dtype, n_out, n_in, x) + (base if add else 0.0)
+    got = run_gemm(dev, w, dtype, n_out, n_in, x, cuda.PATH_MMA, accumulate=base if add else None)
     err, cos = stats(got, want)
     assert err <= 6e-3 and cos >= 0.999999, (err, cos)

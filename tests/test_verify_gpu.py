@@ -196,7 +196,7 @@ def test_batched_sequences_with_permuted_block_tables(tiny):
 
 
 def test_steps_of_33_to_47_rows_on_the_wide_route_on_request(tiny):
-    """Four sequences x nine rows: three exact 16-row passes by default, one pass of the tensor-memory route with
+    """Four sequences x nine rows: the exact kernel of 17 to 47 rows by default, one pass of the tensor-memory route with
     YUUKA_SESSION_WIDE_FROM_33. Both stay inside the path's logit bound; the flag changes the kernels that run."""
     cfg, gm, om = tiny
     V, B = cfg["vocab"], 4

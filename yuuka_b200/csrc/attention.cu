@@ -5,7 +5,8 @@
 // the Qwen3.5 layout is applied (model/qwen35/forward.go:188-220; replaces
 // attention_prefill_paged_f32_kernel, kernels/hip/prefill/prefill.hip:683).
 //
-// fp32 arithmetic on CUDA cores; K and V rows are decoded from the pool format.
+// attention_mma_kernel multiplies on tensor cores; attention_partial_kernel, fp32 arithmetic on CUDA cores over rows decoded
+// from the pool format, takes its place with YUUKA_CUDA_ATTN_FP32=1.
 #include <cuda_fp16.h>
 
 #include <cfloat>

@@ -777,8 +777,6 @@ void reserve_gemm(yuuka_session * s, const Tensor & w, int rows) {
 
 enum LogitRows { LOGITS_NONE, LOGITS_LAST, LOGITS_ALL };
 
-// Prompt tokens run through the step kernels in chains of up to this many rows (the row masks are 64 bits
-// wide); from 48 rows on the GEMMs take the tensor-memory route.
 // Key ranges of a step's attention. About one CTA per SM at capacity (measured at a 1500-token context: 3.11 ms per step,
 // against 3.16 with two or four per SM: fewer partials for the merge kernel outweigh the shorter key ranges). Many sequences
 // of different lengths: key ranges of at most 512 keys, so that the CTAs of a long context spread over the machine instead
@@ -796,8 +794,8 @@ int attention_splits(const yuuka_session * s, int batch, int nodes, int max_tota
     return splits < 1 ? 1 : splits;
 }
 
-// A prompt runs in passes of up to CHAIN_ROWS rows: the GEMMs and row-wise kernels take the whole pass (the
-// tensor-memory GEMM route decodes a weight tile once for up to 512 rows), the mixers work on it in sub-chunks of
+// A prompt runs in passes of up to CHAIN_ROWS rows: the GEMMs and row-wise kernels take the whole pass (from 48 rows on the
+// tensor-memory route, which decodes a weight tile once per tile of up to 256 rows), the mixers work on it in sub-chunks of
 // CHAIN_SUB rows, the limit of their per-step row bookkeeping (64-bit ancestor masks).
 constexpr int CHAIN_ROWS = 512;
 constexpr int CHAIN_SUB = 64;

@@ -1726,7 +1726,7 @@ static void plan_tiled(const yuuka_device * dev, uint32_t dtype, int m, int n_ou
     pl.grid_x = pl.n_groups < per ? pl.n_groups : per;
 }
 
-// Rows from which the tensor-memory route takes over from 16-row passes of the register-fed kernel.
+// Rows from which the tensor-memory route takes over from the register-fed kernels.
 constexpr int UMMA_MIN_ROWS = 48;
 constexpr int UMMA_EARLY_ROWS = 33;  // on request: where three passes of the register-fed route would begin
 constexpr int UMMA_PART_ROWS = 512;  // a launch whose parts of K do not all fit the scratch goes by so many rows
