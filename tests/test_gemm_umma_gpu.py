@@ -87,3 +87,20 @@ def test_umma_route_sums_parts_of_rows_that_16_byte_stores_do_not_divide(dev, ro
     got = run_gemm(dev, w, dtype, n_out, n_in, x, cuda.PATH_MMA, accumulate=base if add else None)
     err, cos = stats(got, want)
     assert err <= 6e-3 and cos >= 0.999999, (err, cos)
+
+
+@pytest.mark.parametrize("dtype", [synth.Q4_K, synth.Q5_K, synth.Q6_K, synth.Q8_0])
+@pytest.mark.parametrize("n_out,n_in", [
+    (520, 2560),     # parts of K on pairs of their own
+    (9220, 2048),    # both halves of K on one pair, and a last block of weight rows that is not full
+    (19200, 512),    # K in one piece, several tiles per pair
+])
+def test_weights_in_tensor_memory_and_in_shared_memory_give_the_same_bits(dev, dtype, n_out, n_in):
+    """Up to 192 rows per tile the decoded weights lie in tensor memory, above in shared memory: the operands are the same
+    numbers, so a row's result does not change with the rows that travel with it. The counts take one to four accumulators."""
+    w = synth.normal_quant(n_out, n_in, dtype, 0.02, 700 + dtype)
+    x = synth.normal_f32(250 * n_in, 1.0, 31).reshape(250, n_in)
+    whole = run_gemm(dev, w, dtype, n_out, n_in, x, cuda.PATH_MMA)
+    for rows in (48, 65, 97, 128, 161, 192, 193):
+        got = run_gemm(dev, w, dtype, n_out, n_in, x[:rows], cuda.PATH_MMA)
+        assert np.array_equal(got, whole[:rows]), (rows, float(np.abs(got - whole[:rows]).max()))

@@ -1761,11 +1761,19 @@ static int umma_kparts(const yuuka_device * dev, int n_out, int n_in, int m) {
     if (ks > cap) ks = cap;
     return ks < 1 ? 1 : ks;
 }
+// Whether the decoded weights of a tile go to tensor memory: they do as long as it holds two accumulators beside four stages.
+// Above, shared memory (two accumulators of 256 columns; with one beside the weights 248320 x 2560 Q6_K takes 531 us at 512 rows
+// either way, and 9216 x 2560 Q4_K, whose halves of K need two, 29 against 24). Q8_0, which has twice the packed words to
+// gather per lane, stays in shared memory where a pair walks few superblocks (2560 x 2560 at 48 rows: 12.1 us against 12.4).
+static bool umma_tmem(uint32_t dtype, int n_tile, int nsb, int kparts) {
+    return n_tile <= UM_TMEM_N && (dtype != YUUKA_DTYPE_Q8_0 || nsb / kparts >= 8);
+}
 // The tiling of the rows with the lowest estimate of cycles: rounds of the pairs x (stages of a tile x cycles per stage +
-// a fixed cost for filling and draining the rings). A stage took 634 / 682 / 774 / 890 cycles at 64 / 128 / 192 / 256
-// activation rows per tile (248320 x 2560 Q6_K): the decode of 8192 weights and its barriers, and 1.3 cycles per row on top.
-constexpr double UMMA_STAGE = 540.0, UMMA_ROW = 1.3, UMMA_TILE = 4000.0;
-static UmmaPlan umma_plan(const yuuka_device * dev, int n_out, int n_in, int m) {
+// a fixed cost for filling and draining the rings). A stage took 442 / 554 / 670 cycles at 64 / 128 / 192 activation rows per
+// tile with the weights in tensor memory (248320 x 2560 Q4_K), 634 / 682 / 774 / 890 at 64 / 128 / 192 / 256 in shared memory
+// (Q6_K): the decode of 8192 weights and its barriers, and so many cycles per row on top.
+constexpr double UMMA_STAGE = 540.0, UMMA_ROW = 1.3, UMMA_TMEM_STAGE = 330.0, UMMA_TMEM_ROW = 1.8, UMMA_TILE = 4000.0;
+static UmmaPlan umma_plan(const yuuka_device * dev, uint32_t dtype, int n_out, int n_in, int m) {
     const int m_blocks = (n_out + 2 * UM_ROWS - 1) / (2 * UM_ROWS), nsb = n_in / 256, pairs = dev->sm_count / 2;
     UmmaPlan best{0, 0, umma_kparts(dev, n_out, n_in, m), false};
     if (best.kparts == 2) {
@@ -1778,7 +1786,8 @@ static UmmaPlan umma_plan(const yuuka_device * dev, int n_out, int n_in, int m) 
         const int n_tile = ((m + tiles - 1) / tiles + 31) / 32 * 32;
         if ((m + n_tile - 1) / n_tile != tiles) continue;  // the same cut as a smaller count
         const int rounds = (m_blocks * tiles * best.kparts + pairs - 1) / pairs;
-        const double cost = rounds * (stages * (UMMA_STAGE + UMMA_ROW * n_tile) + UMMA_TILE);
+        const bool tmem = umma_tmem(dtype, n_tile, nsb, best.kparts);
+        const double cost = rounds * (stages * (tmem ? UMMA_TMEM_STAGE + UMMA_TMEM_ROW * n_tile : UMMA_STAGE + UMMA_ROW * n_tile) + UMMA_TILE);
         if (cost < best_cost) {
             best_cost = cost;
             best.n_tile = n_tile;
@@ -1880,7 +1889,7 @@ TiledScratchNeed gemm_tiled_scratch_need(const yuuka_device * dev, uint32_t w_dt
     TiledScratchNeed need;
     if (!tiled_supported(w_dtype, n_in)) return need;
     if (gemm_tiled_wide(rows, false, false)) {
-        const int parts = umma_plan(dev, n_out, n_in, rows).kparts;
+        const int parts = umma_plan(dev, w_dtype, n_out, n_in, rows).kparts;
         if (parts > 1) {
             need.floats = (uint64_t)parts * std::min(rows, UMMA_PART_ROWS) * n_out;
             need.wanted = (uint64_t)parts * rows * n_out;
@@ -2083,7 +2092,7 @@ static bool umma_parts_fit(const TiledGemmArgs & a, int kparts) {
 template <int DT>
 static int launch_umma_dt(const yuuka_device * dev, cudaStream_t s, const TiledGemmArgs & a, const __half * xh) {
     using S = UmmaStage<DT>;
-    const UmmaPlan pl = umma_plan(dev, a.n_out, a.n_in, a.rows);
+    const UmmaPlan pl = umma_plan(dev, DT, a.n_out, a.n_in, a.rows);
     UParams p{};
     p.kc = decode_consts(DT);
     p.w = a.w;
@@ -2107,15 +2116,23 @@ static int launch_umma_dt(const yuuka_device * dev, cudaStream_t s, const TiledG
     }
     alignas(64) CUtensorMap xmap;
     make_x_map(&xmap, xh, a.rows, a.n_in, pl.n_tile / 2);
-    const size_t fixed = (size_t)UM_RAW_STAGES * S::RAW_BYTES + (size_t)UM_DW * HalfRecord<DT>::TAB + 1024,
-                 stage = (size_t)UM_A_BYTES + (size_t)pl.n_tile * 64;
-    p.stages = UM_MAX_STAGES;
-    while (fixed + p.stages * stage + 1024 > dev->prop.sharedMemPerBlockOptin && p.stages > 2) p.stages--;
-    const size_t smem = fixed + p.stages * stage;
-    YK_REQUIRE(smem + 1024 <= dev->prop.sharedMemPerBlockOptin, YUUKA_ERR_INTERNAL, "umma gemm: stage buffers do not fit shared memory");
-    YK_CUDA(cudaFuncSetAttribute(gemm_umma_kernel<DT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    const bool tmem = umma_tmem(DT, pl.n_tile, p.nsb, pl.kparts);
+    // tensor memory: accumulators of n_tile columns, then at least four weight stages; or two or four accumulators alone
+    p.acc_cols = tmem ? (uint32_t)pl.n_tile : (pl.n_tile <= UM_MAX_N / 2 ? UM_MAX_N / 2 : UM_MAX_N);
+    p.n_acc = tmem ? std::min<uint32_t>(UM_MAX_ACC, (512 - 4 * UM_A_COLS) / p.acc_cols) : 512u / p.acc_cols;
+    p.stages = tmem ? std::min<uint32_t>(UM_MAX_STAGES, (512 - p.n_acc * p.acc_cols) / UM_A_COLS) : UM_MAX_STAGES;
+    const size_t stage = (size_t)(tmem ? 0 : UM_A_BYTES) + (size_t)pl.n_tile * 64, tabs = (size_t)UM_DW * HalfRecord<DT>::TAB + 1024,
+                 room = dev->prop.sharedMemPerBlockOptin - 1024;
+    auto bytes = [&] { return tabs + p.stages * stage + p.raw_stages * (size_t)S::RAW_BYTES; };
+    p.raw_stages = tmem ? UM_MAX_RAW : 2;
+    while (bytes() > room && p.raw_stages > 2) p.raw_stages--;
+    while (bytes() > room && p.stages > 2) p.stages--;
+    const size_t smem = bytes();
+    YK_REQUIRE(smem <= room, YUUKA_ERR_INTERNAL, "umma gemm: stage buffers do not fit shared memory");
+    auto kern = tmem ? gemm_umma_kernel<DT, true> : gemm_umma_kernel<DT, false>;
+    YK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     const int items = p.m_blocks * p.n_tiles * p.kparts, pairs = dev->sm_count / 2;
-    launch_k_cluster(gemm_umma_kernel<DT>, dim3(2 * (items < pairs ? items : pairs)), UM_THREADS, smem, s, 2, p, xmap);
+    launch_k_cluster(kern, dim3(2 * (items < pairs ? items : pairs)), UM_THREADS, smem, s, 2, p, xmap);
     YK_CUDA(cudaGetLastError());
     if (pl.kparts == 1) return 1;
     if (fuse_row_norm(dev, a)) {
@@ -2236,7 +2253,7 @@ static int launch_mma_dt(const yuuka_device * dev, cudaStream_t s, const TiledGe
         launches++;
     }
     if (wide) {
-        const int parts = umma_plan(dev, a.n_out, a.n_in, a.rows).kparts;
+        const int parts = umma_plan(dev, DT, a.n_out, a.n_in, a.rows).kparts;
         if (a.rows > UMMA_PART_ROWS && parts > 1 && !umma_parts_fit(a, parts)) {
             // (the fixed scratch of yuuka_gemm_quant_static, nearly filled by the activations)
             for (int m0 = 0; m0 < a.rows; m0 += UMMA_PART_ROWS) {
@@ -2376,7 +2393,8 @@ static void preload_dt() {
     YK_CUDA(cudaFuncGetAttributes(&fa, gemm_tiled_mma_kernel<DT, 4, false>));
     YK_CUDA(cudaFuncGetAttributes(&fa, gemm_tiled_fp32_kernel<DT, float>));
     YK_CUDA(cudaFuncGetAttributes(&fa, gemm_tiled_fp32_kernel<DT, __nv_bfloat16>));
-    YK_CUDA(cudaFuncGetAttributes(&fa, gemm_umma_kernel<DT>));
+    YK_CUDA(cudaFuncGetAttributes(&fa, gemm_umma_kernel<DT, false>));
+    YK_CUDA(cudaFuncGetAttributes(&fa, gemm_umma_kernel<DT, true>));
 }
 void gemm_tiled_preload_kernels() {
     cudaFuncAttributes fa;

@@ -8,15 +8,21 @@
 // this route does not have the register-fed route's exactness), 64 columns at a time, and fetches half of the
 // tile's activation rows (their fp16 hi halves, a tensor-map copy). The even CTA issues the MMAs of both; each CTA reads its own half of D back.
 //
+// Where the decoded weights lie. Up to 192 activation rows per tile tensor memory has room for two accumulators and four
+// stages of weights beside them, and the decode warps store there (tcgen05.st, the A operand of the MMA): the weights then pass
+// through shared memory once, packed, instead of three times. Wider tiles keep the stages in shared memory, since their two
+// accumulators fill tensor memory (one accumulator beside the weights was no faster: its epilogue runs alone). The operands are
+// the same numbers either way, and so are the results.
+//
 // What bounds it, and why this tile. At M = 128 per CTA a stage of 64 columns keeps the tensor pipe busy for two cycles
 // per activation row of the tile. Its activations come from L2, which feeds all SMs 46 bytes per cycle each
 // (13 TB/s measured): one CTA alone on 256 activation rows needs 64 bytes per cycle, a pair that shares them 32. The decode
-// of a stage (8192 weights per SM) takes 500 to 600 cycles with its barriers, so tiles
-// of up to about 200 rows are bound by the decode and wider ones by both. Tensor memory holds two accumulators of 256 columns: the
+// of a stage (8192 weights per SM) with its barriers and the products share tensor memory (or shared memory): a stage takes
+// 330 cycles and 1.8 per row (540 and 1.3). Tensor memory holds two accumulators at least: the
 // epilogue of a tile runs on warps of its own while the next tile is decoded and multiplied.
-// Calls on a B200, before (one CTA per 128 rows, 512 activation rows) and after: 9216 x 2560 Q4_K at 576 rows 115 -> 39 us,
-// 18432 x 2560 at 512 rows 55 -> 46 us; 248320 x 2560 Q6_K at 48 rows 367 -> 195 us (2.7 TB/s of weights), at 512 rows
-// 623 -> 530 us (1.2 PFLOP/s).
+// Calls on a B200, with the weights in shared memory and in tensor memory: 248320 x 2560 Q6_K 187 -> 154 us at 48 rows (3.4 TB/s
+// of weights), 250 -> 222 at 192, 693 -> 590 at 544 (three tiles of 192; 1.2 PFLOP/s); 9216 x 2560 Q4_K at 576 rows
+// 38.5 -> 35 us; 9216 x 2560 Q6_K 20.2 -> 17.6 at 48 rows, 21.5 -> 19.0 at 192; 18432 x 2560 Q4_K at 576 rows 50.5 -> 47.
 //
 // Roles of a CTA's warps: sixteen decode warps (two per 16-row tile), four epilogue warps, one warp that copies packed
 // weights (one bulk copy per record, a superblock of all eight tiles per stage, ahead of everything else), one that copies
@@ -33,8 +39,10 @@ constexpr int UM_ROWS = 128;     // weight rows per CTA; a pair has 256
 constexpr int UM_KC = 64;        // columns per stage
 constexpr int UM_MAX_N = 256;    // activation rows per tile
 constexpr int UM_MAX_STAGES = 6;
-constexpr int UM_MAX_ACC = 4;  // accumulators of up to 128 columns; two of up to 256
-constexpr int UM_RAW_STAGES = 2; // superblocks of packed weights in shared memory
+constexpr int UM_MAX_ACC = 4;    // accumulators
+constexpr int UM_A_COLS = UM_KC / 2;  // tensor-memory columns of a weight stage: 128 lanes (rows) x 64 columns of fp16
+constexpr int UM_TMEM_N = 192;   // activation rows per tile up to which the weight stages are in tensor memory
+constexpr int UM_MAX_RAW = 4;    // superblocks of packed weights in shared memory
 constexpr int UM_TILES = 8;      // 16-row tiles per CTA
 constexpr int UM_DW = 16;        // decode warps, two per tile: a half of every record each
 constexpr int UM_EW = 4;         // epilogue warps, one per quarter of the tensor-memory lanes
@@ -60,7 +68,8 @@ struct UParams {
     int n_tile, n_tiles;  // activation rows per tile (a multiple of 32), tiles
     int m_blocks;         // blocks of 256 weight rows
     uint32_t idesc;
-    uint32_t stages;      // ring depth
+    uint32_t stages, raw_stages;  // ring depths
+    uint32_t acc_cols, n_acc;     // columns of an accumulator, and how many there are (then the weight stages, if they are there)
     int drop_copies;      // test hook: the even CTA's activations are never copied
 };
 
@@ -73,8 +82,15 @@ __device__ __forceinline__ uint64_t umma_desc_sw128(uint32_t smem_addr) {
 // where 16-byte piece c (eight columns) of row r of a stage lies in that layout
 __device__ __forceinline__ uint32_t sw128(int r, int c) { return (uint32_t)(r * 128 + ((c ^ (r & 7)) << 4)); }
 
+__device__ __forceinline__ void tmem_store16(uint32_t dst, const uint32_t (&r)[16]) {  // 16 lanes x 32 columns: four 16 x 16 fp16 A fragments
+    asm volatile(
+        "tcgen05.st.sync.aligned.16x256b.x4.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};" ::"r"(dst),
+        "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]),
+        "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
+        : "memory");
+}
 // ---------------------------------------------------------------------------
-// Decode of half a record: 16 rows x 128 columns, two stages of 64, by one warp. fetch() takes the warp's share of a
+// Decode of half a record: 16 rows x 128 columns, two stages of 64, by one warp, into shared memory. fetch() takes the warp's share of a
 // record out of shared memory; header() turns the block headers into fp16 scales in the warp's own table; store<c>()
 // writes 64 columns (sub-blocks 2c, 2c + 1 of the half) as fp16(s * q - min): lane (g, t) holds rows g and g + 8 and eight
 // columns of each sub-block. Rows of odd g take the two sub-blocks in the other order: the lanes of a store then hit
@@ -257,6 +273,131 @@ template <> struct HalfRecord<YUUKA_DTYPE_Q8_0> {
     }
 };
 
+// The same for tensor memory: a lane takes from shared memory what its part of the fragments is, and 64 columns go out in one
+// store (a quarter of the instructions, and none of the bytes that pass through shared memory twice). The values are the same.
+// The words of a packed record that lane (g, t) takes for tensor memory: of a 32-column sub-block columns 4t .. 4t + 3 and 16 + 4t ..
+// + 3 (its part of two 16 x 16 fragments). `pieces`: 32 pieces of 16 bytes, one per lane (g, t') of the register-fed kernel, which
+// takes columns 8t' .. 8t' + 7 of two sub-blocks as words x y and z w: the columns at 4t are a word of piece t / 2, those at 16 + 4t
+// the same word two pieces on.
+__device__ __forceinline__ uint4 fetch_quads(const uint8_t * pieces, int lane) {
+    const uint32_t * w = reinterpret_cast<const uint32_t *>(pieces + (lane >> 2) * 64 + (lane & 2) * 8 + (lane & 1) * 4);
+    return make_uint4(w[0], w[8], w[2], w[10]);
+}
+
+template <int DT> struct TmemRecord;
+template <> struct TmemRecord<YUUKA_DTYPE_Q4_K> : HalfRecordK4<YUUKA_DTYPE_Q4_K> {
+    __device__ void fetch(const uint8_t * rec, int lane, int half) {
+        qg = fetch_quads(rec + half * 512, lane);
+        qh = fetch_quads(rec + (2 + half) * 512, lane);
+        hdr = reinterpret_cast<const uint4 *>(rec)[128 + (lane & 15)];
+    }
+    template <int C> __device__ void store(int lane, const uint8_t * tab, const DecodeConsts & kc, uint32_t dst) const {
+        const int g = lane >> 2;
+        const uint32_t v[2][2] = {{C ? qg.z : qg.x, C ? qg.w : qg.y}, {C ? qh.z : qh.x, C ? qh.w : qh.y}};
+        uint32_t r[16];
+#pragma unroll
+        for (int n = 0; n < 2; n++) {  // sub-block 2C + n: low or high nibbles
+            const uint32_t mask = n ? kc.mf0 : kc.m0f;
+#pragma unroll
+            for (int rr = 0; rr < 2; rr++) {
+                const uint2 s = reinterpret_cast<const uint2 *>(tab + (g + 8 * rr) * DS)[2 * C + n];
+                const uint32_t m = reinterpret_cast<const uint32_t *>(tab + MN_OFF + (g + 8 * rr) * 16)[2 * C + n];
+#pragma unroll
+                for (int h = 0; h < 2; h++) {
+                    r[8 * n + 4 * h + 2 * rr] = nibble_h2(v[rr][h], mask, kc.magic, s.x, s.y, m);
+                    r[8 * n + 4 * h + 2 * rr + 1] = nibble_h2(v[rr][h] >> 8, mask, kc.magic, s.x, s.y, m);
+                }
+            }
+        }
+        tmem_store16(dst, r);
+    }
+};
+template <> struct TmemRecord<YUUKA_DTYPE_Q5_K> : HalfRecordK4<YUUKA_DTYPE_Q5_K> {
+    uint4 hi;  // as in HalfRecord, by quads
+    __device__ void fetch(const uint8_t * rec, int lane, int half) {
+        qg = fetch_quads(rec + half * 512, lane);
+        qh = fetch_quads(rec + (2 + half) * 512, lane);
+        hdr = reinterpret_cast<const uint4 *>(rec)[160 + (lane & 15)];
+        hi = fetch_quads(rec + 2048, lane);
+        if (half) hi = make_uint4(hi.x >> 4, hi.y >> 4, hi.z >> 4, hi.w >> 4);
+    }
+    template <int C> __device__ void store(int lane, const uint8_t * tab, const DecodeConsts & kc, uint32_t dst) const {
+        const int g = lane >> 2;
+        const uint32_t v[2][2] = {{C ? qg.z : qg.x, C ? qg.w : qg.y}, {C ? qh.z : qh.x, C ? qh.w : qh.y}};
+        const uint32_t hb[2][2] = {{hi.x, hi.y}, {hi.z, hi.w}};
+        uint32_t r[16];
+#pragma unroll
+        for (int n = 0; n < 2; n++) {  // sub-block 2C + n: low or high nibbles; its bit 2C + n of each byte goes to bit 4 or 8
+            const uint32_t mask = n ? kc.mf0 : kc.m0f, hm = n ? kc.h8 : kc.h4;
+            const int up = n ? 7 - 2 * C : 4 - 2 * C, down = n ? 1 + 2 * C : 4 + 2 * C;
+#pragma unroll
+            for (int rr = 0; rr < 2; rr++) {
+                const uint2 s = reinterpret_cast<const uint2 *>(tab + (g + 8 * rr) * DS)[2 * C + n];
+                const uint32_t m = reinterpret_cast<const uint32_t *>(tab + MN_OFF + (g + 8 * rr) * 16)[2 * C + n];
+#pragma unroll
+                for (int h = 0; h < 2; h++) {
+                    r[8 * n + 4 * h + 2 * rr] = nibble_h2(v[rr][h], mask, and_or(hb[rr][h] << up, hm, kc.magic), s.x, s.y, m);
+                    r[8 * n + 4 * h + 2 * rr + 1] = nibble_h2(v[rr][h] >> 8, mask, and_or(hb[rr][h] >> down, hm, kc.magic), s.x, s.y, m);
+                }
+            }
+        }
+        tmem_store16(dst, r);
+    }
+};
+template <> struct TmemRecord<YUUKA_DTYPE_Q6_K> : HalfRecord<YUUKA_DTYPE_Q6_K> {  // (its pieces are quads already)
+    template <int C> __device__ void store(int lane, const uint8_t * tab, const DecodeConsts & kc, uint32_t dst) const {
+        const int g = lane >> 2;
+        const uint32_t qm = C ? kc.mf0 : kc.m0f, hm = C ? kc.h8 : kc.h4;
+        uint32_t r[16];
+#pragma unroll
+        for (int hsel = 0; hsel < 2; hsel++) {  // sub-block 2C + hsel
+            const int lsh = 4 - 2 * hsel, rsh = 4 + 2 * hsel;
+#pragma unroll
+            for (int rr = 0; rr < 2; rr++) {
+                const uint4 l4 = rr ? lh : lg;
+                const uint2 b2 = rr ? hh : hg, m2 = reinterpret_cast<const uint2 *>(tab + MN_OFF + (g + 8 * rr) * MN)[2 * C + hsel];
+                const uint4 s2 = reinterpret_cast<const uint4 *>(tab + (g + 8 * rr) * DS)[2 * C + hsel];
+#pragma unroll
+                for (int h = 0; h < 2; h++) {
+                    const uint32_t v0 = h ? (hsel ? l4.w : l4.y) : (hsel ? l4.z : l4.x), b0 = h ? b2.y : b2.x;
+                    const uint32_t s = h ? s2.z : s2.x, c = h ? s2.w : s2.y, m = h ? m2.y : m2.x;
+                    r[8 * hsel + 4 * h + 2 * rr] = nibble_h2(v0, qm, and_or(b0 << lsh, hm, kc.magic), s, c, m);
+                    r[8 * hsel + 4 * h + 2 * rr + 1] = nibble_h2(v0 >> 8, qm, and_or(b0 >> rsh, hm, kc.magic), s, c, m);
+                }
+            }
+        }
+        tmem_store16(dst, r);
+    }
+};
+template <> struct TmemRecord<YUUKA_DTYPE_Q8_0> : HalfRecord<YUUKA_DTYPE_Q8_0> {
+    __device__ void fetch(const uint8_t * rec, int lane, int half) {
+        g0 = fetch_quads(rec + (2 * half) * 512, lane);
+        g1 = fetch_quads(rec + (2 * half + 1) * 512, lane);
+        h0 = fetch_quads(rec + (4 + 2 * half) * 512, lane);
+        h1 = fetch_quads(rec + (5 + 2 * half) * 512, lane);
+        d = reinterpret_cast<const uint2 *>(rec + 4096 + (lane & 15) * 16)[half];
+    }
+    template <int C> __device__ void store(int lane, const uint8_t * tab, const DecodeConsts &, uint32_t dst) const {
+        const int g = lane >> 2;
+        uint32_t r[16];
+#pragma unroll
+        for (int n = 0; n < 2; n++) {  // block 2C + n
+#pragma unroll
+            for (int rr = 0; rr < 2; rr++) {
+                const uint4 q = rr ? (C ? h1 : h0) : (C ? g1 : g0);
+                const uint32_t s = reinterpret_cast<const uint32_t *>(tab + (g + 8 * rr) * DS)[2 * C + n];
+#pragma unroll
+                for (int h = 0; h < 2; h++) {
+                    const uint32_t v = (n ? (h ? q.w : q.z) : (h ? q.y : q.x)) ^ 0x80808080u;
+                    r[8 * n + 4 * h + 2 * rr] = h2_mul(h2_sub(bytes02_h2(v), H2_1152), s);
+                    r[8 * n + 4 * h + 2 * rr + 1] = h2_mul(h2_sub(bytes13_h2(v), H2_1152), s);
+                }
+            }
+        }
+        tmem_store16(dst, r);
+    }
+};
+
 __device__ __forceinline__ uint32_t smem_u32(const void * p) { return (uint32_t)__cvta_generic_to_shared(p); }
 constexpr uint32_t WAIT_LIMIT = 1u << 22, WAIT_LIMIT_TEST = 1u << 8;  // polls of some 4 us each: 17 s; with the test hook 1 ms
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, uint32_t limit) {
@@ -312,6 +453,14 @@ __device__ __forceinline__ void umma_commit_pair(uint32_t bar) {
                  : "memory");
 }
 
+__device__ __forceinline__ void umma_f16_pair_tmem(uint32_t d, uint32_t a, uint64_t db, uint32_t idesc, uint32_t accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::2.kind::f16 [%0], [%1], %2, %3, {%5, %5, %5, %5, %5, %5, %5, %5}, p;\n\t}"
+        :
+        : "r"(d), "r"(a), "l"(db), "r"(idesc), "r"(accumulate), "r"(0u)
+        : "memory");
+}
 __device__ __forceinline__ bool elect_one() {
     uint32_t e;
     asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(e));
@@ -385,7 +534,8 @@ struct Ring {
     }
 };
 
-template <int DT>
+// TMEM: the decoded weights lie in tensor memory, behind the accumulators, instead of in shared memory.
+template <int DT, bool TMEM>
 __global__ void __launch_bounds__(UM_THREADS, 1) gemm_umma_kernel(const UParams p, const __grid_constant__ CUtensorMap xmap) {
     using C = Codec<DT>;
     using S = UmmaStage<DT>;
@@ -393,21 +543,21 @@ __global__ void __launch_bounds__(UM_THREADS, 1) gemm_umma_kernel(const UParams 
     uint8_t * smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);  // the swizzled stages need 1024-byte alignment
     __shared__ __align__(8) uint64_t empty_bar[UM_MAX_STAGES];  // the tensor pipe has read the stage
     __shared__ __align__(8) uint64_t full_bar[UM_MAX_STAGES];   // this CTA's weights and activations are in the stage (even CTA: both CTAs')
-    __shared__ __align__(8) uint64_t raw_full[UM_RAW_STAGES], raw_empty[UM_RAW_STAGES];
+    __shared__ __align__(8) uint64_t raw_full[UM_MAX_RAW], raw_empty[UM_MAX_RAW];
     __shared__ __align__(8) uint64_t acc_full[UM_MAX_ACC], acc_empty[UM_MAX_ACC]; // accumulators: finished by the MMAs, read by the epilogue
     __shared__ uint32_t tmem_slot, odd_note[UM_MAX_STAGES];  // (the notes' contents are not read)
     const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;  // (uniform for the compiler too)
     const uint32_t rank = blockIdx.x & 1u;  // clusters are pairs along x
-    const uint32_t half_n = (uint32_t)p.n_tile >> 1, b_bytes = half_n * 128u, stage_bytes = UM_A_BYTES + b_bytes;
+    const uint32_t half_n = (uint32_t)p.n_tile >> 1, b_bytes = half_n * 128u, a_bytes = TMEM ? 0u : (uint32_t)UM_A_BYTES, stage_bytes = a_bytes + b_bytes;
     uint8_t * raw = smem + (size_t)p.stages * stage_bytes;
-    uint8_t * tabs = raw + (size_t)UM_RAW_STAGES * S::RAW_BYTES;
+    uint8_t * tabs = raw + (size_t)p.raw_stages * S::RAW_BYTES;
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < UM_MAX_STAGES; s++) {
             mbar_init(smem_u32(&empty_bar[s]), 1);
             mbar_init(smem_u32(&full_bar[s]), UM_TILES + 1);
         }
-        for (int s = 0; s < UM_RAW_STAGES; s++) {
+        for (int s = 0; s < UM_MAX_RAW; s++) {
             mbar_init(smem_u32(&raw_full[s]), 1);
             mbar_init(smem_u32(&raw_empty[s]), UM_DW);
         }
@@ -426,7 +576,7 @@ __global__ void __launch_bounds__(UM_THREADS, 1) gemm_umma_kernel(const UParams 
     cluster_sync_all();  // both CTAs' barriers are set up
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t taddr = tmem_slot, smem_base = smem_u32(smem);
-    const uint32_t acc_cols = p.n_tile <= UM_MAX_N / 2 ? UM_MAX_N / 2 : UM_MAX_N, n_acc = 512u / acc_cols;  // accumulators
+    const uint32_t acc_cols = p.acc_cols, n_acc = p.n_acc, a_base = taddr + n_acc * acc_cols;
     const int n_tiles16 = (p.N + 15) >> 4;
     const size_t rec_row = (size_t)p.nsb * C::REC;
     const uint32_t limit = p.drop_copies ? WAIT_LIMIT_TEST : WAIT_LIMIT;
@@ -456,7 +606,7 @@ __global__ void __launch_bounds__(UM_THREADS, 1) gemm_umma_kernel(const UParams 
                                      smem_u32(raw + (size_t)ring.at * S::RAW_BYTES) + (uint32_t)(lane * C::REC)),
                                  "l"(src + (size_t)sb * C::REC), "r"((uint32_t)C::REC), "r"(bar)
                                  : "memory");
-                ring.next(UM_RAW_STAGES);
+                ring.next(p.raw_stages);
             }
         }
     } else if (warp == UM_WARP_X) {
@@ -473,7 +623,7 @@ __global__ void __launch_bounds__(UM_THREADS, 1) gemm_umma_kernel(const UParams 
                     asm volatile(
                         "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
                         :
-                        : "r"(smem_base + ring.at * stage_bytes + UM_A_BYTES), "l"(&xmap), "r"(col), "r"(row), "r"(bar)
+                        : "r"(smem_base + ring.at * stage_bytes + a_bytes), "l"(&xmap), "r"(col), "r"(row), "r"(bar)
                         : "memory");
                 }
                 __syncwarp();
@@ -483,7 +633,7 @@ __global__ void __launch_bounds__(UM_THREADS, 1) gemm_umma_kernel(const UParams 
     } else if (warp == UM_WARP_MMA && rank == 0) {
         // ---------------- MMAs of the pair ----------------
         Ring ring, acc;
-        const uint64_t da0 = umma_desc_sw128(smem_base), db0 = umma_desc_sw128(smem_base + UM_A_BYTES);
+        const uint64_t da0 = umma_desc_sw128(smem_base), db0 = umma_desc_sw128(smem_base + a_bytes);
         const uint32_t step = stage_bytes >> 4;
         for (UmmaWork wk(p); wk.valid() && !expired; wk.next()) {
             if (!wait(acc_empty[acc.at], acc.phase ^ 1u)) break;
@@ -504,8 +654,10 @@ __global__ void __launch_bounds__(UM_THREADS, 1) gemm_umma_kernel(const UParams 
                 const uint64_t da = da0 + (uint64_t)(ring.at * step), db = db0 + (uint64_t)(ring.at * step);
                 if (elect_one()) {
 #pragma unroll
-                    for (int j = 0; j < UM_KC / 16; j++)
-                        umma_f16_pair(d, da + (uint64_t)(j * 2), db + (uint64_t)(j * 2), p.idesc, j > 0 ? 1u : keep);
+                    for (int j = 0; j < UM_KC / 16; j++) {
+                        if constexpr (TMEM) umma_f16_pair_tmem(d, a_base + ring.at * UM_A_COLS + (uint32_t)(j * 8), db + (uint64_t)(j * 2), p.idesc, j > 0 ? 1u : keep);
+                        else umma_f16_pair(d, da + (uint64_t)(j * 2), db + (uint64_t)(j * 2), p.idesc, j > 0 ? 1u : keep);
+                    }
                     umma_commit_pair(smem_u32(&empty_bar[ring.at]));
                 }
                 __syncwarp();
@@ -529,6 +681,10 @@ __global__ void __launch_bounds__(UM_THREADS, 1) gemm_umma_kernel(const UParams 
                     acc.next(n_acc);
                 }
                 if (!wait(full_bar[ring.at], ring.phase)) break;
+                if constexpr (TMEM) {  // the decode warps' stores come before the note
+                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                }
                 if (lane == 0) note_leader(smem_u32(&odd_note[ring.at]), smem_u32(&full_bar[ring.at]));
                 __syncwarp();
                 ring.next(p.stages);
@@ -536,7 +692,9 @@ __global__ void __launch_bounds__(UM_THREADS, 1) gemm_umma_kernel(const UParams 
         }
     } else if (warp < UM_DW) {
         // ---------------- decode ----------------
-        const int tile = warp >> 1, half = warp & 1;  // stages 2 half, 2 half + 1 of every superblock
+        // Stages 2 half, 2 half + 1 of every superblock. (In tensor memory a warp reaches the 32 lanes of its number mod 4: two tiles.)
+        const int tile = TMEM ? 2 * (warp & 3) + ((warp >> 2) & 1) : warp >> 1, half = TMEM ? warp >> 3 : warp & 1;
+        const uint32_t lanes = (uint32_t)(tile * 16) << 16;
         uint8_t * tab = tabs + warp * HalfRecord<DT>::TAB;
         const DecodeConsts kc = p.kc;
         Ring ring, rr;
@@ -546,17 +704,24 @@ __global__ void __launch_bounds__(UM_THREADS, 1) gemm_umma_kernel(const UParams 
         }
         for (UmmaWork wk(p); wk.valid() && !expired; wk.next()) {
             for (int n = wk.sb_end(p) - wk.sb_begin(p); n > 0; n--) {
-                HalfRecord<DT> r;
+                std::conditional_t<TMEM, TmemRecord<DT>, HalfRecord<DT>> r;
                 if (!wait(raw_full[rr.at], rr.phase)) break;
                 r.fetch(raw + (size_t)rr.at * S::RAW_BYTES + tile * C::REC, lane, half);
                 r.header(lane, half, tab);
                 __syncwarp();  // the table is complete, and every lane has its part of the record
                 if (lane == 0) mbar_arrive(smem_u32(&raw_empty[rr.at]));
-                rr.next(UM_RAW_STAGES);
+                rr.next(p.raw_stages);
                 auto chunk = [&](auto c) {
                     if (expired || !wait(empty_bar[ring.at], ring.phase ^ 1u)) return;
-                    r.template store<decltype(c)::value>(lane, tab, kc, smem + (size_t)ring.at * stage_bytes + tile * 16 * 128);
-                    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                    if constexpr (TMEM) {
+                        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                        r.template store<decltype(c)::value>(lane, tab, kc, a_base + ring.at * UM_A_COLS + lanes);
+                        asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+                        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                    } else {
+                        r.template store<decltype(c)::value>(lane, tab, kc, smem + (size_t)ring.at * stage_bytes + tile * 16 * 128);
+                        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                    }
                     __syncwarp();
                     if (lane == 0) mbar_arrive(smem_u32(&full_bar[ring.at]));
                     ring.next(p.stages);
