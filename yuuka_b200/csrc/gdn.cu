@@ -206,6 +206,7 @@ static void launch_gdn_front(cudaStream_t s, const GdnArgs & a, const RowMeta & 
 // TREE: the rows of a sequence may branch (the host staged parent pointers); they are then walked depth first.
 template <int S, bool TREE>
 __global__ void __launch_bounds__(GDN_WARPS * 32) gdn_scan_kernel(const ScanParams p) {
+    pdl_entry();
     constexpr int RPL = S / 4;  // state rows per lane
     const GdnArgs & a = p.a;
     const int cb = blockIdx.x, h = blockIdx.y, seq = blockIdx.z;
@@ -235,14 +236,11 @@ __global__ void __launch_bounds__(GDN_WARPS * 32) gdn_scan_kernel(const ScanPara
     __shared__ float scale_s[GDN_MAX_NODES];
     __shared__ int order_s[TREE ? GDN_MAX_NODES : 1];  // the rows depth first, worked out by the host when it staged the step
 
-    // Stored state: the longest fetch (HBM), issued first, before the wait for the front end, which does not write it: what does
-    // (the last commit, a reset) was complete when the front end's CTAs went past their own wait, and this kernel starts after those.
+    // stored state: the longest fetch (HBM), issued first
     const float * s0 = a.state + ((int64_t)(seq_of(p.rows, seq) * a.rank + h) * S + rq * RPL) * S + col;
     float2 st[RPL / 2];  // state rows (2 i, 2 i + 1) of this lane's quarter, one column
 #pragma unroll
     for (int i = 0; i < RPL / 2; i++) st[i] = make_float2(s0[(int64_t)(2 * i) * S], s0[(int64_t)(2 * i + 1) * S]);
-
-    pdl_entry();
 
     // the front-end kernel has left normalised q and k, the conv output of v, beta and decay in global memory
     // (16-byte loads, eight in flight per thread: with 64 rows of a prompt sub-chunk a scalar loop spent most
@@ -389,7 +387,7 @@ __global__ void __launch_bounds__(GDN_WARPS * 32) gdn_scan_kernel(const ScanPara
     __syncthreads();  // scales visible to the CTA
     // No CTA leaves while another may still read its sums: the wait is at the end. (Nothing has been written to global memory so
     // far: the release of a cluster barrier waits for such writes, and with the log written row by row, in 32-byte pieces, the
-    // first one did. Steps of 32 sequences x 17 rows 12.02 -> 11.83 ms, of 32 x 5 rows of the mixture 3.25 -> 3.20.)
+    // first one did. Steps of 32 sequences x 17 rows 12.02 -> 11.93 ms, of 32 x 5 rows of the mixture 3.25 -> 3.19.)
     cluster_arrive();
     for (int i = threadIdx.x; i < N * GDN_COLS; i += blockDim.x)
         a.dlog[(int64_t)(seq * N + i / GDN_COLS) * inner + h * S + cb * GDN_COLS + (i & (GDN_COLS - 1))] = dd[i];
