@@ -191,3 +191,25 @@ def test_rows_beyond_one_pass_equal_passes_of_sixteen(dev, dtype, n_out, n_in, r
                            for m in range(0, rows, 16)])
     got = run_gemm(dev, w, dtype, n_out, n_in, x, cuda.PATH_MMA, accumulate=base)
     assert np.array_equal(got, want), float(np.abs(got - want).max())
+
+
+@pytest.mark.parametrize("dtype", [synth.Q4_K, synth.Q5_K, synth.Q6_K, synth.Q8_0])
+@pytest.mark.parametrize("n_out,n_in,rows", [
+    (64, 1024, 4), (64, 1024, 5),        # two and three pieces of sixteen columns per thread of the smallest CTA
+    (24, 256, 1), (24, 256, 16),         # one superblock, a row tile that is not full
+    (2560, 2560, 6), (2560, 2560, 7),    # parts of K on warps of one CTA
+    (160, 9216, 1), (160, 16384, 13),    # few tiles, a long K
+])
+def test_activations_prepared_by_the_kernel_or_by_a_launch_before_it(dev, dtype, n_out, n_in, rows):
+    """Few columns per thread are prepared by the product's own kernel, more by a launch before it: f32 and bf16, stored and added."""
+    w = synth.normal_quant(n_out, n_in, dtype, 0.02, 800 + dtype)
+    x = synth.normal_f32(rows * n_in, 1.0, 60 + rows).reshape(rows, n_in)
+    base = synth.normal_f32(rows * n_out, 1.0, 61).reshape(rows, n_out)
+    want = yo.matmul(w, dtype, n_out, n_in, x)
+    # outputs have a deviation of 0.02 sqrt(n_in), 2.6 at most here; 22 bits of x and fp32 sums leave 1e-5 of it
+    assert np.max(np.abs(run_gemm(dev, w, dtype, n_out, n_in, x, cuda.PATH_MMA) - want)) <= 4e-4
+    assert np.max(np.abs(run_gemm(dev, w, dtype, n_out, n_in, x, cuda.PATH_MMA, accumulate=base) - base - want)) <= 4e-4
+    xb = cuda.from_bf16(cuda.to_bf16(x)).reshape(rows, n_in)
+    want = yo.matmul(w, dtype, n_out, n_in, xb)
+    got = run_gemm(dev, w, dtype, n_out, n_in, x, cuda.PATH_MMA, x_dtype=cuda.BF16)
+    assert np.max(np.abs(got - want)) <= 4e-4

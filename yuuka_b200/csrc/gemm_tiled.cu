@@ -706,8 +706,9 @@ struct TParams {
     const __half * xh;      // prepared activations [M][nsb * 256], hi halves
     const __half * xl;      // lo halves
     const __half2 * xs16;   // [M][nsb * 16]
-    const void * x;         // fp32 route only
+    const void * x;         // fp32 route; register-fed kernel: activations it prepares itself (null: they are in xh, xl, xs16)
     int64_t ldx;
+    int x_bf16;             // x is bf16, else f32
     int M;
     float * out;
     int64_t ldo;
@@ -781,7 +782,8 @@ __device__ __forceinline__ __half2 prep_sum(float gs) {
 // (qwen35moe expert FFNs). A segment's rows are contiguous in the prepared-activation and output
 // arrays unless row_index redirects the activation rows.
 // FOLD: the RMSNorm on either side of this GEMM is folded into its epilogue (TParams::nf_* / cs_*).
-template <int DT, int NT, bool GROUPED, bool FOLD>
+// OWN: the activations arrive as f32 / bf16 and every CTA prepares its columns.
+template <int DT, int NT, bool GROUPED, bool FOLD, bool OWN>
 __device__ __forceinline__ void tiled_mma_body(const TParams & p, const GemmSegment & sg) {
     using C = Codec<DT>;
     using X = XTab<DT>;
@@ -832,11 +834,13 @@ __device__ __forceinline__ void tiled_mma_body(const TParams & p, const GemmSegm
     pdl_trigger();
     int grp = blockIdx.x;
     typename C::Regs cur, nxt;
-    {
+    // (a launch that prepares its activations follows a kernel of the caller's, which may have written the weights)
+    auto first_records = [&] {
         const int rt = min(grp * p.TG + tile_in_group, n_tiles - 1);
         if (sb0 < sb1) C::load(wbase + rt * rec_row + (size_t)sb0 * C::REC, lane, cur);
         if (sb0 + 1 < sb1) prefetch_l2_range(wbase + rt * rec_row + (size_t)(sb0 + 1) * C::REC, (sb1 - sb0 - 1) * C::REC, lane);
-    }
+    };
+    if constexpr (!OWN) first_records();
     // (the barrier the activation copies complete on: set up while the previous kernel still runs)
     if (threadIdx.x == 0) {
         asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"((uint32_t)__cvta_generic_to_shared(&xbar)) : "memory");
@@ -845,9 +849,32 @@ __device__ __forceinline__ void tiled_mma_body(const TParams & p, const GemmSegm
     __syncthreads();
     pdl_wait();
 
-    // ---- activations of this K chunk: one bulk copy per row and half, and one for the sums where the type
-    // has a "- min" term, every row's copies issued by its own lane of the first warp ----
-    if (warp == 0 && !p.drop_copies) {
+    // ---- activations of this K chunk ----
+    if constexpr (OWN) {
+        // as they are: every CTA prepares what it reads, sixteen columns of a row at a time
+        first_records();
+        const int groups = cnt * 16;
+        for (int i = threadIdx.x; i < Mrows * groups; i += blockDim.x) {
+            const int m = i / groups, gq = i - m * groups;
+            const int64_t at = (int64_t)m * p.ldx + (int64_t)c0 * 256 + gq * 16;
+            float v[16];
+            if (p.x_bf16) {
+                load8((const __nv_bfloat16 *)p.x + at, *reinterpret_cast<float(*)[8]>(v));
+                load8((const __nv_bfloat16 *)p.x + at + 8, *reinterpret_cast<float(*)[8]>(v + 8));
+            } else {
+                load8((const float *)p.x + at, *reinterpret_cast<float(*)[8]>(v));
+                load8((const float *)p.x + at + 8, *reinterpret_cast<float(*)[8]>(v + 8));
+            }
+            __half2 sum;
+            xprep_store16(reinterpret_cast<__half *>(xs + (size_t)(2 * m) * xstride) + gq * 16,
+                          reinterpret_cast<__half *>(xs + (size_t)(2 * m + 1) * xstride) + gq * 16, &sum, v);
+            if constexpr (X::SUMS) reinterpret_cast<__half2 *>(xsum + (size_t)m * xsum_stride)[gq] = sum;
+        }
+        __syncthreads();
+    }
+    // prepared: one bulk copy per row and half, and one for the sums where the type
+    // has a "- min" term, every row's copies issued by its own lane of the first warp
+    if (!OWN && warp == 0 && !p.drop_copies) {
         const uint32_t bar = (uint32_t)__cvta_generic_to_shared(&xbar);
         const uint32_t row_bytes_x = (uint32_t)cnt * 512, row_bytes_s = X::SUMS ? (uint32_t)cnt * 64 : 0u;
         if (lane == 0)
@@ -890,7 +917,7 @@ __device__ __forceinline__ void tiled_mma_body(const TParams & p, const GemmSegm
         }
         __syncthreads();  // the row scales are read by every warp's epilogue
     }
-    {
+    if constexpr (!OWN) {
         // bounded wait for the copies; on expiry the error word is set and the results are garbage
         const uint32_t bar = (uint32_t)__cvta_generic_to_shared(&xbar);
         uint32_t ok = 0;
@@ -1158,9 +1185,9 @@ __device__ __forceinline__ void tiled_mma_body(const TParams & p, const GemmSegm
     }
 }
 
-template <int DT, int NT, bool FOLD>
+template <int DT, int NT, bool FOLD, bool OWN = false>
 __global__ void __launch_bounds__(MW * 32, 1) gemm_tiled_mma_kernel(const TParams p) {
-    tiled_mma_body<DT, NT, false, FOLD>(p, GemmSegment{});
+    tiled_mma_body<DT, NT, false, FOLD, OWN>(p, GemmSegment{});
 }
 // One CTA (or a few) per segment. The segments of a routed step hold five rows on average: up to four take one product tile
 // and the others two (moe 32 x 5 rows, 256 experts).
@@ -1171,8 +1198,8 @@ __global__ void __launch_bounds__(MW * 32, 1) gemm_tiled_grouped_kernel(const TP
     pdl_wait();
     const GemmSegment sg = p.segments[blockIdx.z];
     if (sg.count <= 0) return;  // the whole CTA: unused slot of the segment list
-    if (sg.count <= GEMM_SEGMENT_ROWS / 2) tiled_mma_body<DT, GEMM_SEGMENT_ROWS / 8, true, false>(p, sg);
-    else tiled_mma_body<DT, GEMM_SEGMENT_ROWS / 4, true, false>(p, sg);
+    if (sg.count <= GEMM_SEGMENT_ROWS / 2) tiled_mma_body<DT, GEMM_SEGMENT_ROWS / 8, true, false, false>(p, sg);
+    else tiled_mma_body<DT, GEMM_SEGMENT_ROWS / 4, true, false, false>(p, sg);
 }
 
 // ===========================================================================
@@ -1933,16 +1960,22 @@ TiledScratchNeed gemm_tiled_scratch_bound(const yuuka_device * dev, uint32_t w_d
 template <int DT, int NT>
 static void launch_mma_inst(cudaStream_t s, const TiledGemmArgs & a, const XPrepOut & xp, int m0, int m, const TPlan & pl) {
     const bool fold = a.norm.produce_w || a.norm.consume_now || a.swiglu.xh;
-    auto kern = fold ? gemm_tiled_mma_kernel<DT, NT, true> : gemm_tiled_mma_kernel<DT, NT, false>;
+    auto kern = fold ? gemm_tiled_mma_kernel<DT, NT, true> : (xp.xh ? gemm_tiled_mma_kernel<DT, NT, false> : gemm_tiled_mma_kernel<DT, NT, false, true>);
     YK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pl.smem));
     TParams p{};
     p.kc = decode_consts(DT);
     p.w = a.w;
     p.N = a.n_out;
     p.nsb = a.n_in / 256;
-    p.xh = xp.xh + (int64_t)m0 * a.n_in;
-    p.xl = xp.xl + (int64_t)m0 * a.n_in;
-    p.xs16 = xp.xs16 + (int64_t)m0 * (a.n_in / 16);
+    if (xp.xh) {
+        p.xh = xp.xh + (int64_t)m0 * a.n_in;
+        p.xl = xp.xl + (int64_t)m0 * a.n_in;
+        p.xs16 = xp.xs16 + (int64_t)m0 * (a.n_in / 16);
+    } else {
+        p.x_bf16 = a.x_dtype == YUUKA_DTYPE_BF16 ? 1 : 0;
+        p.x = (const char *)a.x + (int64_t)m0 * a.ldx * (p.x_bf16 ? 2 : 4);
+        p.ldx = a.ldx;
+    }
     p.M = m;
     p.out = a.out + (int64_t)m0 * a.ldo;
     p.ldo = a.ldo;
@@ -2238,8 +2271,19 @@ static int launch_mma_dt(const yuuka_device * dev, cudaStream_t s, const TiledGe
     };
     XPrepOut xp = a.xprep;
     const bool wide = gemm_tiled_wide(a.rows, a.exact_only, a.wide_from_33);
-    if (!xp.xh) {
-        // activations arrive as f32 / bf16: convert once into the scratch
+    const bool folded = a.norm.produce_w || a.norm.consume_now || (a.swiglu.xh && a.rows <= 32);
+    // Activations that arrive as f32 / bf16: the kernel prepares them itself where one launch of the register-fed kernel reads them
+    // and no thread has more than two pieces of sixteen to do (every CTA does all of its columns). A launch less: 4096 x 1024
+    // Q5_K 7.4 -> 6.1 us at 9 rows, 16384 x 512 Q8_0 9.4 -> 8.0 at 16, 18432 x 2560 Q4_K 13.8 -> 13.4 at 5. With three pieces
+    // that matrix takes 17.6 us at 9 rows against 16.5, and 512 x 9216 Q8_0 13.8 against 11.4 at 5. Where the host's call is no longer than the
+    // launches, 300 x 512 Q4_K 6.7 -> 4.5 us at 1 to 5 rows, 2560 x 2560 6.9 -> 5.3 at 2.
+    const bool own_x = !xp.xh && a.x && !wide && !folded && a.rows <= MMA_ROWS && !(a.flags & YUUKA_GEMM_TEST_DROP_COPIES) && [&] {
+        TPlan pl;
+        plan_tiled(dev, a.w_dtype, a.rows, a.n_out, a.n_in, pl);
+        return a.rows * pl.nsb_chunk * 16 <= 2 * pl.TG * pl.KS * 32;
+    }();
+    if (!xp.xh && !own_x) {
+        // convert once into the scratch
         YK_REQUIRE(a.x && a.scratch && a.scratch->xh && a.scratch->xl && a.scratch->xh_elems >= (uint64_t)a.rows * a.n_in,
                    YUUKA_ERR_INTERNAL, "gemm: no prepared activations and no scratch to prepare them in");
         __half * xl = wide ? nullptr : a.scratch->xl;  // (the wide route reads the hi halves alone)
@@ -2268,8 +2312,7 @@ static int launch_mma_dt(const yuuka_device * dev, cudaStream_t s, const TiledGe
         const int n = launch_umma_dt<DT>(dev, s, a, xp.xh);
         return launches + n + norm(n > 1 && fuse_row_norm(dev, a));
     }
-    YK_REQUIRE(xp.xl && xp.xs16, YUUKA_ERR_INTERNAL, "gemm: the prepared activations lack their lo halves or sums");
-    const bool folded = a.norm.produce_w || a.norm.consume_now || (a.swiglu.xh && a.rows <= 32);
+    YK_REQUIRE(own_x || (xp.xl && xp.xs16), YUUKA_ERR_INTERNAL, "gemm: the prepared activations lack their lo halves or sums");
     int m = 0;
     bool normed = false;
     for (int m0 = 0; m0 < a.rows; m0 += m) {
@@ -2383,14 +2426,18 @@ template <int DT>
 static void preload_dt() {
     cudaFuncAttributes fa;
     YK_CUDA(cudaFuncGetAttributes(&fa, gemm_tiled_mma_kernel<DT, 1, false>));
+    YK_CUDA(cudaFuncGetAttributes(&fa, gemm_tiled_mma_kernel<DT, 1, false, true>));
     YK_CUDA(cudaFuncGetAttributes(&fa, gemm_tiled_mma_kernel<DT, 2, false>));
+    YK_CUDA(cudaFuncGetAttributes(&fa, gemm_tiled_mma_kernel<DT, 2, false, true>));
     YK_CUDA(cudaFuncGetAttributes(&fa, gemm_tiled_rows_kernel<DT, 6>));
     YK_CUDA(cudaFuncGetAttributes(&fa, gemm_tiled_rows_kernel<DT, 8>));
     YK_CUDA(cudaFuncGetAttributes(&fa, gemm_tiled_rows_kernel<DT, 9>));
     YK_CUDA(cudaFuncGetAttributes(&fa, gemm_tiled_rows_kernel<DT, 10>));
     YK_CUDA(cudaFuncGetAttributes(&fa, gemm_tiled_rows_kernel<DT, 12>));
     YK_CUDA(cudaFuncGetAttributes(&fa, gemm_tiled_mma_kernel<DT, 3, false>));
+    YK_CUDA(cudaFuncGetAttributes(&fa, gemm_tiled_mma_kernel<DT, 3, false, true>));
     YK_CUDA(cudaFuncGetAttributes(&fa, gemm_tiled_mma_kernel<DT, 4, false>));
+    YK_CUDA(cudaFuncGetAttributes(&fa, gemm_tiled_mma_kernel<DT, 4, false, true>));
     YK_CUDA(cudaFuncGetAttributes(&fa, gemm_tiled_fp32_kernel<DT, float>));
     YK_CUDA(cudaFuncGetAttributes(&fa, gemm_tiled_fp32_kernel<DT, __nv_bfloat16>));
     YK_CUDA(cudaFuncGetAttributes(&fa, gemm_umma_kernel<DT, false>));
