@@ -259,9 +259,6 @@ inline void launch_k_cluster(void (*kern)(KArgs...), dim3 grid, dim3 block, size
 __device__ __forceinline__ void cluster_sync_all() {
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
-// The same barrier in two parts: every thread of the cluster arrives, later every thread waits.
-__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
-__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
 // A double in the shared memory of CTA `rank` of this cluster, at the address `p` has in this CTA.
 __device__ __forceinline__ double ld_cluster_f64(const double * p, unsigned rank) {
     const uint32_t local = (uint32_t)__cvta_generic_to_shared(p);

@@ -353,6 +353,7 @@ __global__ void __launch_bounds__(GDN_WARPS * 32) gdn_scan_kernel(const ScanPara
         if (rq == 0) {
             o_s[node * GDN_COLS + cl] = o;
             dd[node * GDN_COLS + cl] = d;
+            a.dlog[(int64_t)(seq * N + node) * inner + h * S + col] = d;
         }
         if (TREE && node == 0) {
 #pragma unroll
@@ -384,13 +385,7 @@ __global__ void __launch_bounds__(GDN_WARPS * 32) gdn_scan_kernel(const ScanPara
         const float mean = (float)(tot / (double)S);
         scale_s[node] = (float)(1.0 / sqrt((double)(mean + a.eps)));
     }
-    __syncthreads();  // scales visible to the CTA
-    // No CTA leaves while another may still read its sums: the wait is at the end. (Nothing has been written to global memory so
-    // far: the release of a cluster barrier waits for such writes, and with the log written row by row, in 32-byte pieces, the
-    // first one did. 24 layers of 32 sequences x 17 rows 3.61 -> 3.53 ms with the front end, the step 12.02 -> 11.93.)
-    cluster_arrive();
-    for (int i = threadIdx.x; i < N * GDN_COLS; i += blockDim.x)
-        a.dlog[(int64_t)(seq * N + i / GDN_COLS) * inner + h * S + cb * GDN_COLS + (i & (GDN_COLS - 1))] = dd[i];
+    cluster_sync_all();  // scales visible to the CTA; no CTA leaves while another may still read its sums
 #pragma unroll
     for (int k = 0; k < ZPT; k++) {
         const int i = threadIdx.x + k * (GDN_WARPS * 32);
@@ -402,10 +397,7 @@ __global__ void __launch_bounds__(GDN_WARPS * 32) gdn_scan_kernel(const ScanPara
             else o_s[i] = t;
         }
     }
-    if (hi_only) {
-        cluster_wait();
-        return;
-    }
+    if (hi_only) return;
     __syncthreads();
     for (int gi = threadIdx.x; gi < N * (GDN_COLS >> 4); gi += blockDim.x) {
         const int node = gi / (GDN_COLS >> 4), part = gi - node * (GDN_COLS >> 4);
@@ -419,7 +411,6 @@ __global__ void __launch_bounds__(GDN_WARPS * 32) gdn_scan_kernel(const ScanPara
         for (int i = 0; i < 4; i++) dst[i] = make_float4(g16[4 * i], g16[4 * i + 1], g16[4 * i + 2], g16[4 * i + 3]);
         if (a.prep.xh) xprep_store16(a.prep.xh + r * inner + c0, a.prep.xl + r * inner + c0, a.prep.xs16 + r * (inner >> 4) + (c0 >> 4), g16);
     }
-    cluster_wait();
 }
 
 int launch_gdn_scan(cudaStream_t s, const GdnArgs & a, const RowMeta & rows) {
