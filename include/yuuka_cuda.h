@@ -130,7 +130,8 @@ YUUKA_API yuuka_status yuuka_buffer_copy(yuuka_stream * stream, yuuka_buffer * d
  * GGUF row layout of w_dtype (replaces yuuka_gemv_batch, yuuka_hip.h:291-300,
  * and YUUKA_OP_LM_HEAD). x_dtype is F32 or BF16. Byte offsets select
  * sub-ranges of the buffers. flags: bit 0 adds the product to out instead of
- * overwriting it (GEMV_RESIDUAL, yuuka_hip.h:398-401).
+ * overwriting it (GEMV_RESIDUAL, yuuka_hip.h:398-401). On the mma route out may
+ * lie over x (the call has read x before it writes).
  * The call keeps one scratch area per device (prepared activations, split-K
  * partial sums and arrival counters) that it grows with cudaMalloc when a larger
  * shape arrives. Host threads may call concurrently (the growth is serialized), but

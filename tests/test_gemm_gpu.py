@@ -213,3 +213,36 @@ def test_activations_prepared_by_the_kernel_or_by_a_launch_before_it(dev, dtype,
     want = yo.matmul(w, dtype, n_out, n_in, xb)
     got = run_gemm(dev, w, dtype, n_out, n_in, x, cuda.PATH_MMA, x_dtype=cuda.BF16)
     assert np.max(np.abs(got - want)) <= 4e-4
+
+
+@pytest.mark.parametrize("dtype", [synth.Q4_K, synth.Q5_K, synth.Q6_K, synth.Q8_0])
+@pytest.mark.parametrize("n_out,n_in,rows", [
+    (2560, 2560, 2), (2560, 2560, 5),    # in place as a whole, by both forms of the preparation
+    (24, 256, 1), (300, 512, 3), (4096, 1024, 4), (2560, 2560, 9), (520, 1024, 20), (520, 512, 64),
+])
+def test_an_output_that_lies_over_the_activations(dev, dtype, n_out, n_in, rows):
+    """The activations are read before anything is stored, wherever the two ranges meet. The product is then not the one to
+    prepare them, so this also compares the two ways to do that, to the last bit."""
+    w = synth.normal_quant(n_out, n_in, dtype, 0.02, 900 + dtype)
+    x = synth.normal_f32(rows * n_in, 1.0, 71 + rows).reshape(rows, n_in)
+    stream = dev.stream()
+    raw = dev.upload(w)
+    wb = dev.alloc(cuda.tiled_bytes(dtype, n_out, n_in) + 256)
+    cuda.tile_weights(stream, wb, raw, dtype, n_out, n_in)
+    out_bytes = rows * n_out * 4
+    for x_dtype in (cuda.F32, cuda.BF16):
+        data = np.ascontiguousarray(cuda.to_bf16(x) if x_dtype == cuda.BF16 else x).view(np.uint8).ravel()
+        want = run_gemm(dev, w, dtype, n_out, n_in, x, cuda.PATH_MMA, x_dtype=x_dtype).view(np.uint32).ravel()
+        # one at the start of the other, the output from the last 16 bytes of x on, x from the last 16 of the output on
+        for out_at, x_at in ((0, 0), (data.size - 16, 0), (0, (out_bytes - 1) // 16 * 16)):
+            both = dev.alloc(max(out_at + out_bytes, x_at + data.size))
+            for call in (cuda.gemm_quant, cuda.gemm_quant_static):
+                both.write(data, x_at)
+                call(stream, both, both, wb, n_in, n_out, rows, dtype, x_dtype, cuda.PATH_MMA, cuda.GEMM_TILED, out_at, x_at)
+                stream.synchronize()
+                got = both.read(np.uint32, rows * n_out, out_at)
+                assert np.array_equal(got, want), (x_dtype, out_at, x_at, call.__name__)
+            both.free()
+    for b in (raw, wb):
+        b.free()
+    stream.destroy()

@@ -2277,7 +2277,11 @@ static int launch_mma_dt(const yuuka_device * dev, cudaStream_t s, const TiledGe
     // Q5_K 7.4 -> 6.1 us at 9 rows, 16384 x 512 Q8_0 9.4 -> 8.0 at 16, 18432 x 2560 Q4_K 13.8 -> 13.4 at 5. With three pieces
     // that matrix takes 17.6 us at 9 rows against 16.5, and 512 x 9216 Q8_0 13.8 against 11.4 at 5. Where the host's call is no longer than the
     // launches, 300 x 512 Q4_K 6.7 -> 4.5 us at 1 to 5 rows, 2560 x 2560 6.9 -> 5.3 at 2.
-    const bool own_x = !xp.xh && a.x && !wide && !folded && a.rows <= MMA_ROWS && !(a.flags & YUUKA_GEMM_TEST_DROP_COPIES) && [&] {
+    // (Not where `out` lies over x: the first CTAs to finish would store over columns that others have still to read.)
+    const char * x0 = (const char *)a.x, * out0 = (const char *)a.out;
+    const bool apart = out0 + (((int64_t)a.rows - 1) * a.ldo + a.n_out) * 4 <= x0 ||
+                       x0 + (((int64_t)a.rows - 1) * a.ldx + a.n_in) * (a.x_dtype == YUUKA_DTYPE_F32 ? 4 : 2) <= out0;
+    const bool own_x = !xp.xh && a.x && apart && !wide && !folded && a.rows <= MMA_ROWS && !(a.flags & YUUKA_GEMM_TEST_DROP_COPIES) && [&] {
         TPlan pl;
         plan_tiled(dev, a.w_dtype, a.rows, a.n_out, a.n_in, pl);
         return a.rows * pl.nsb_chunk * 16 <= 2 * pl.TG * pl.KS * 32;

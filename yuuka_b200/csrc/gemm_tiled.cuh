@@ -80,7 +80,7 @@ struct NormFuse {
 struct TiledGemmArgs {
     const uint8_t * w = nullptr;  // tiled layout
     uint32_t w_dtype = 0;
-    const void * x = nullptr;     // f32 / bf16 activations (fp32 route, or to be prepared into the scratch)
+    const void * x = nullptr;     // f32 / bf16 activations (fp32 route, or to be prepared: into the scratch, or by the kernel itself)
     XPrepOut xprep;               // prepared activations [rows][n_in], if a producer already made them
     uint32_t x_dtype = YUUKA_DTYPE_F32;
     int64_t ldx = 0;
