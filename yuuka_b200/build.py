@@ -56,6 +56,11 @@ def build_synth(force: bool = False, verbose: bool = False) -> str:
     return SYNTH_LIB
 
 
+def ptxas_report(source: str) -> str:
+    """Where the assembler's report on a source file's kernels is kept."""
+    return os.path.join(HERE, "build", os.path.basename(source) + ".txt")
+
+
 def cuda_sources() -> list[str]:
     return sorted(glob.glob(os.path.join(CSRC, "*.cu")))
 
@@ -75,16 +80,16 @@ def build_cuda(force: bool = False, verbose: bool = False, ptxas_v: bool = False
         objs.append(o)
         if not force and not _stale(o, [s] + [d for d in deps if not d.endswith(".cu")]):
             continue
-        cmd = [_nvcc(), *NVCC_FLAGS, "-I", os.path.join(ROOT, "include"), "-I", CSRC, "-c", s, "-o", o]
-        if ptxas_v:
-            cmd.insert(1, "-Xptxas=-v")
+        cmd = [_nvcc(), "-Xptxas=-v", *NVCC_FLAGS, "-I", os.path.join(ROOT, "include"), "-I", CSRC, "-c", s, "-o", o]
         if verbose:
             print(" ".join(cmd))
         procs.append((s, subprocess.Popen(cmd, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)))
     failed = False
     for s, p in procs:
         out, _ = p.communicate()
-        if p.returncode != 0 or ptxas_v or (verbose and out.strip()):
+        with open(ptxas_report(s), "w") as f:  # registers and spills of every kernel
+            f.write(out)
+        if p.returncode != 0 or ptxas_v or (verbose and "warning" in out):
             print(f"--- {os.path.basename(s)}\n{out}")
         failed |= p.returncode != 0
     if failed:

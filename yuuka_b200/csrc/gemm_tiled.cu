@@ -834,13 +834,11 @@ __device__ __forceinline__ void tiled_mma_body(const TParams & p, const GemmSegm
     pdl_trigger();
     int grp = blockIdx.x;
     typename C::Regs cur, nxt;
-    // (a launch that prepares its activations follows a kernel of the caller's, which may have written the weights)
-    auto first_records = [&] {
+    if constexpr (!OWN) {
         const int rt = min(grp * p.TG + tile_in_group, n_tiles - 1);
         if (sb0 < sb1) C::load(wbase + rt * rec_row + (size_t)sb0 * C::REC, lane, cur);
         if (sb0 + 1 < sb1) prefetch_l2_range(wbase + rt * rec_row + (size_t)(sb0 + 1) * C::REC, (sb1 - sb0 - 1) * C::REC, lane);
-    };
-    if constexpr (!OWN) first_records();
+    }
     // (the barrier the activation copies complete on: set up while the previous kernel still runs)
     if (threadIdx.x == 0) {
         asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"((uint32_t)__cvta_generic_to_shared(&xbar)) : "memory");
@@ -851,8 +849,12 @@ __device__ __forceinline__ void tiled_mma_body(const TParams & p, const GemmSegm
 
     // ---- activations of this K chunk ----
     if constexpr (OWN) {
-        // as they are: every CTA prepares what it reads, sixteen columns of a row at a time
-        first_records();
+        // as they are: every CTA prepares what it reads, sixteen columns of a row at a time. (The weights' first loads come
+        // after the wait here: the kernel before is the caller's, and may have written the weights. Shared with the lines above as a
+        // lambda they cost the other instances registers: the experts of a mixture, 32 x 5 rows, 1.63 -> 1.70 ms a step.)
+        const int rt = min(grp * p.TG + tile_in_group, n_tiles - 1);
+        if (sb0 < sb1) C::load(wbase + rt * rec_row + (size_t)sb0 * C::REC, lane, cur);
+        if (sb0 + 1 < sb1) prefetch_l2_range(wbase + rt * rec_row + (size_t)(sb0 + 1) * C::REC, (sb1 - sb0 - 1) * C::REC, lane);
         const int groups = cnt * 16;
         for (int i = threadIdx.x; i < Mrows * groups; i += blockDim.x) {
             const int m = i / groups, gq = i - m * groups;
