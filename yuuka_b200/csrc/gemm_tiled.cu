@@ -2275,10 +2275,13 @@ static int launch_mma_dt(const yuuka_device * dev, cudaStream_t s, const TiledGe
     const bool wide = gemm_tiled_wide(a.rows, a.exact_only, a.wide_from_33);
     const bool folded = a.norm.produce_w || a.norm.consume_now || (a.swiglu.xh && a.rows <= 32);
     // Activations that arrive as f32 / bf16: the kernel prepares them itself where one launch of the register-fed kernel reads them
-    // and no thread has more than two pieces of sixteen to do (every CTA does all of its columns). A launch less: 4096 x 1024
-    // Q5_K 7.4 -> 6.1 us at 9 rows, 16384 x 512 Q8_0 9.4 -> 8.0 at 16, 18432 x 2560 Q4_K 13.8 -> 13.4 at 5. With three pieces
-    // that matrix takes 17.6 us at 9 rows against 16.5, and 512 x 9216 Q8_0 13.8 against 11.4 at 5. Where the host's call is no longer than the
-    // launches, 300 x 512 Q4_K 6.7 -> 4.5 us at 1 to 5 rows, 2560 x 2560 6.9 -> 5.3 at 2.
+    // and no thread has more than two pieces of sixteen to do (every CTA does all of its columns): a launch less. Calls one after
+    // another, the launch before and this: 300 x 512 Q4_K 5.9 -> 3.7 us at 1 to 7 rows, 2560 x 2560 6.4 -> 5.2 at 2 and 7.8 -> 7.4 at 5,
+    // 4096 x 1024 Q5_K 6.2 -> 4.9 at 7, 16384 x 512 Q8_0 9.6 -> 8.1 at 16, 18432 x 2560 Q4_K 14.3 -> 13.9 at 5. Between two and three
+    // pieces it depends: 4096 x 1024 Q6_K at 12 rows gains a sixth, 2560 x 4096 Q4_K at 5 rows loses 5 % (8.25 -> 8.69 us).
+    // The loop of this instance is 2 to 8 % slower for Q5_K and Q8_0 beyond four rows, so a warp that walks many records keeps the
+    // launch: 151936 x 2048 Q8_0 (40 records) 79 us instead of 85 at 7 rows, 248320 x 2560 Q5_K (70) 142 instead of 147 at 5;
+    // 40960 x 2560 (20) 36 us both ways, 100000 x 1280 Q8_0 (15) 35 -> 34 at 6.
     // (Not where `out` lies over x: the first CTAs to finish would store over columns that others have still to read.)
     const char * x0 = (const char *)a.x, * out0 = (const char *)a.out;
     const bool apart = out0 + (((int64_t)a.rows - 1) * a.ldo + a.n_out) * 4 <= x0 ||
@@ -2286,6 +2289,8 @@ static int launch_mma_dt(const yuuka_device * dev, cudaStream_t s, const TiledGe
     const bool own_x = !xp.xh && a.x && apart && !wide && !folded && a.rows <= MMA_ROWS && !(a.flags & YUUKA_GEMM_TEST_DROP_COPIES) && [&] {
         TPlan pl;
         plan_tiled(dev, a.w_dtype, a.rows, a.n_out, a.n_in, pl);
+        const int records = (pl.n_groups + pl.grid_x - 1) / pl.grid_x * pl.nsb_chunk / pl.KS;  // of a warp
+        if ((DT == YUUKA_DTYPE_Q5_K || DT == YUUKA_DTYPE_Q8_0) && a.rows > 4 && records > 16) return false;
         return a.rows * pl.nsb_chunk * 16 <= 2 * pl.TG * pl.KS * 32;
     }();
     if (!xp.xh && !own_x) {
