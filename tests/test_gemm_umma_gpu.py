@@ -89,18 +89,39 @@ def test_umma_route_sums_parts_of_rows_that_16_byte_stores_do_not_divide(dev, ro
     assert err <= 6e-3 and cos >= 0.999999, (err, cos)
 
 
-@pytest.mark.parametrize("dtype", [synth.Q4_K, synth.Q5_K, synth.Q6_K, synth.Q8_0])
-@pytest.mark.parametrize("n_out,n_in", [
-    (520, 2560),     # parts of K on pairs of their own
-    (9220, 2048),    # both halves of K on one pair, and a last block of weight rows that is not full
-    (19200, 512),    # K in one piece, several tiles per pair
+MANY, ALWAYS = [synth.Q5_K, synth.Q8_0], [synth.Q4_K, synth.Q6_K]  # superblocks per pair that tensor memory takes
+
+
+@pytest.mark.parametrize("n_out,n_in,shared_rows,rows,dtypes", [
+    # parts of K on pairs of their own: tiles of 256 rows, and of 32 and 64
+    (520, 2560, 900, (48, 128, 193), ALWAYS),
+    # the same with enough superblocks per pair for all types: one tile of 256, three of 96 and 128
+    (1100, 16384, 250, (257, 320), ALWAYS + MANY),
+    # both halves of K on one pair, a last block of weight rows that is not full: two tiles of 224, and of 32 to 160 (four,
+    # three and two accumulators)
+    (9220, 4096, 448, (48, 97, 160, 193, 320), ALWAYS + MANY),
+    # K in one piece, several tiles per pair: 256 rows, and 64 to 192 (Q8_0 only of 64 and 160, where six stages fit)
+    (19200, 3072, 250, (48, 65, 128, 160, 192), ALWAYS + MANY),
+    (19200, 512, 250, (48, 97, 192), ALWAYS),
+    # few superblocks per pair: Q5_K and Q8_0 stay in shared memory
+    (19200, 512, 250, (48, 192), MANY),
 ])
-def test_weights_in_tensor_memory_and_in_shared_memory_give_the_same_bits(dev, dtype, n_out, n_in):
-    """Up to 192 rows per tile the decoded weights lie in tensor memory, above in shared memory: the operands are the same
-    numbers, so a row's result does not change with the rows that travel with it. The counts take one to four accumulators."""
-    w = synth.normal_quant(n_out, n_in, dtype, 0.02, 700 + dtype)
-    x = synth.normal_f32(250 * n_in, 1.0, 31).reshape(250, n_in)
-    whole = run_gemm(dev, w, dtype, n_out, n_in, x, cuda.PATH_MMA)
-    for rows in (48, 65, 97, 128, 161, 192, 193):
-        got = run_gemm(dev, w, dtype, n_out, n_in, x[:rows], cuda.PATH_MMA)
-        assert np.array_equal(got, whole[:rows]), (rows, float(np.abs(got - whole[:rows]).max()))
+def test_weights_in_tensor_memory_and_in_shared_memory_give_the_same_bits(dev, n_out, n_in, shared_rows, rows, dtypes):
+    """Up to 192 rows per tile the decoded weights lie in tensor memory (Q5_K and Q8_0 where a pair walks many superblocks), above in
+    shared memory: the operands are the same numbers, so a row's result does not change with the rows that travel with it. (The
+    tilings named are those of 148 SMs.)"""
+    for dtype in dtypes:
+        w = synth.normal_quant(n_out, n_in, dtype, 0.02, 700 + dtype)
+        x = synth.normal_f32(shared_rows * n_in, 1.0, 31).reshape(shared_rows, n_in)
+        x = np.concatenate([x, x])
+        shared = run_gemm(dev, w, dtype, n_out, n_in, x[:shared_rows], cuda.PATH_MMA)
+        want = yo.matmul(w, dtype, n_out, n_in, x[:8])
+        # A weight s q - m rounds s, m, s q and the result to fp16, x once: each 2e-4 (rms) of a number whose deviation is at most 2.3
+        # times the weight's (m is near two of them), five together at most 1e-3 of an output's deviation, 0.02 sqrt(n_in). The
+        # largest of 1.5e5 such errors is 4.5 times that; twice as much is allowed.
+        assert np.max(np.abs(shared[:8] - want)) <= 9e-3 * 0.02 * n_in ** 0.5
+        for m in rows:
+            got = run_gemm(dev, w, dtype, n_out, n_in, x[:m], cuda.PATH_MMA)
+            same = min(m, shared_rows)
+            assert np.array_equal(got[:same], shared[:same]), (dtype, m, float(np.abs(got[:same] - shared[:same]).max()))
+            assert np.array_equal(got[same:], shared[:m - same]), (dtype, m)

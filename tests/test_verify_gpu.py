@@ -708,6 +708,7 @@ def test_prompt_that_fills_a_session_shorter_than_its_chunks(tiny, n, kv):
     (synth.Q8_0, 6144, 4096, 20, 4), (synth.Q5_K, 256, 9216, 20, 1), (synth.Q5_K, 256, 9216, 21, 4),
     (synth.Q4_K, 512, 16640, 20, 1),                                  # more superblocks than the cuts have bits
     (synth.Q8_0, 700, 2048, 48, 3), (synth.Q8_0, 700, 2048, 300, 3),  # tensor memory, one and several tiles of rows
+    (synth.Q4_K, 700, 2048, 48, 3), (synth.Q6_K, 9220, 2048, 300, 3), # the same with the weights in tensor memory too
 ])
 def test_an_expired_wait_in_each_gemm_kernel_leaves_the_device_usable(tiny, dtype, n_out, n_in, n, code):
     """Without their activations the kernels give up, a step reports it with the code of the kernel that the route has

@@ -1775,7 +1775,8 @@ bool gemm_tiled_wide(int rows, bool exact_only, bool wide_from_33) {
 // How a launch of the tensor-memory kernel is cut: m activation rows into n_tiles tiles of n_tile rows, K into kparts.
 struct UmmaPlan {
     int n_tile, n_tiles, kparts;
-    bool halves;
+    bool halves;  // one pair takes both halves of K
+    bool tmem;    // the decoded weights lie in tensor memory
 };
 // K parts: enough pairs of CTAs to fill the machine when the matrix has few blocks of rows, at least two superblocks each.
 // Two parts do not pay for the launch that sums them (9216 x 2560 at 576 rows: 47 us against 39): one pair then takes both
@@ -1790,21 +1791,34 @@ static int umma_kparts(const yuuka_device * dev, int n_out, int n_in, int m) {
     if (ks > cap) ks = cap;
     return ks < 1 ? 1 : ks;
 }
-// Whether the decoded weights of a tile go to tensor memory: they do as long as it holds two accumulators beside four stages.
-// Above, shared memory (two accumulators of 256 columns; with one beside the weights 248320 x 2560 Q6_K takes 531 us at 512 rows
-// either way, and 9216 x 2560 Q4_K, whose halves of K need two, 29 against 24). Q8_0, which has twice the packed words to
-// gather per lane, stays in shared memory where a pair walks few superblocks (2560 x 2560 at 48 rows: 12.1 us against 12.4).
-static bool umma_tmem(uint32_t dtype, int n_tile, int nsb, int kparts) {
-    return n_tile <= UM_TMEM_N && (dtype != YUUKA_DTYPE_Q8_0 || nsb / kparts >= 8);
+// Whether the decoded weights of a tile go to tensor memory. It has to hold two accumulators beside four stages: up to 192 rows
+// per tile. (With one accumulator 248320 x 2560 Q6_K takes 531 us at 512 rows either way, and 9216 x 2560 Q4_K, whose halves of K
+// need two, 29 against 24.) Q4_K and Q6_K never lose there: over matrices of 512 to 248320 rows with 1 to 36 superblocks and 48 to
+// 576 activation rows Q6_K gains 3 to 21 %, Q4_K up to 13 %. Q6_K's words lie as the fragments need them; the others are gathered
+// (fetch_quads), 8 words a lane and half record for Q4_K, 12 for Q5_K, 16 for Q8_0, and those two need a pair that walks many
+// superblocks. Q5_K: below twelve mostly 1 to 2 % slower (2560 x 4096 at 160 rows 16.3 -> 16.7 us; none at ten), from there faster
+// (18432 x 3072 at 192 rows 1 %, 9216 x 2560 at 576 5 %, 248320 x 2560 at 160 5 %). Q8_0: below sixteen 1 to 4 % slower
+// (2560 x 2560 at 160 rows 14.1 -> 14.6), from there faster with six stages of weights (248320 x 2560 at 48 rows 159 -> 149,
+// 9216 x 2560 at 576 35.3 -> 34.1) and with four where tiles share weights of up to sixteen superblocks (65536 x 2560 at 576 rows
+// 6 %), but not with four alone on its weights or over a long K (18432 x 9216 at 128 rows 52.7 -> 58.1, at 352 rows 111 -> 117).
+static uint32_t umma_accumulators(int n_tile) { return std::min<uint32_t>(UM_MAX_ACC, (512 - 4 * UM_A_COLS) / n_tile); }
+static uint32_t umma_tmem_stages(int n_tile) { return std::min<uint32_t>(UM_MAX_STAGES, (512 - umma_accumulators(n_tile) * n_tile) / UM_A_COLS); }
+static bool umma_tmem(uint32_t dtype, int n_tile, int tiles, int rounds, int nsb, int kparts) {
+    if (n_tile > UM_TMEM_N) return false;
+    const int walked = rounds * nsb / kparts;
+    if (dtype == YUUKA_DTYPE_Q5_K) return walked >= 12;
+    if (dtype == YUUKA_DTYPE_Q8_0) return walked >= 16 && (umma_tmem_stages(n_tile) == UM_MAX_STAGES || (tiles > 1 && nsb / kparts <= 16));
+    return true;
 }
 // The tiling of the rows with the lowest estimate of cycles: rounds of the pairs x (stages of a tile x cycles per stage +
-// a fixed cost for filling and draining the rings). A stage took 442 / 554 / 670 cycles at 64 / 128 / 192 activation rows per
+// a fixed cost for filling and draining the rings). It picks the fastest tiling, or one within 2 % of it, of all four types over
+// 16 matrices and eleven row counts from 48 to 576. A stage took 442 / 554 / 670 cycles at 64 / 128 / 192 activation rows per
 // tile with the weights in tensor memory (248320 x 2560 Q4_K), 634 / 682 / 774 / 890 at 64 / 128 / 192 / 256 in shared memory
 // (Q6_K): the decode of 8192 weights and its barriers, and so many cycles per row on top.
 constexpr double UMMA_STAGE = 540.0, UMMA_ROW = 1.3, UMMA_TMEM_STAGE = 330.0, UMMA_TMEM_ROW = 1.8, UMMA_TILE = 4000.0;
 static UmmaPlan umma_plan(const yuuka_device * dev, uint32_t dtype, int n_out, int n_in, int m) {
     const int m_blocks = (n_out + 2 * UM_ROWS - 1) / (2 * UM_ROWS), nsb = n_in / 256, pairs = dev->sm_count / 2;
-    UmmaPlan best{0, 0, umma_kparts(dev, n_out, n_in, m), false};
+    UmmaPlan best{0, 0, umma_kparts(dev, n_out, n_in, m), false, false};
     if (best.kparts == 2) {
         best.kparts = 1;
         best.halves = true;
@@ -1815,12 +1829,13 @@ static UmmaPlan umma_plan(const yuuka_device * dev, uint32_t dtype, int n_out, i
         const int n_tile = ((m + tiles - 1) / tiles + 31) / 32 * 32;
         if ((m + n_tile - 1) / n_tile != tiles) continue;  // the same cut as a smaller count
         const int rounds = (m_blocks * tiles * best.kparts + pairs - 1) / pairs;
-        const bool tmem = umma_tmem(dtype, n_tile, nsb, best.kparts);
+        const bool tmem = umma_tmem(dtype, n_tile, tiles, rounds, nsb, best.kparts);
         const double cost = rounds * (stages * (tmem ? UMMA_TMEM_STAGE + UMMA_TMEM_ROW * n_tile : UMMA_STAGE + UMMA_ROW * n_tile) + UMMA_TILE);
         if (cost < best_cost) {
             best_cost = cost;
             best.n_tile = n_tile;
             best.n_tiles = tiles;
+            best.tmem = tmem;
         }
     }
     return best;
@@ -2151,11 +2166,11 @@ static int launch_umma_dt(const yuuka_device * dev, cudaStream_t s, const TiledG
     }
     alignas(64) CUtensorMap xmap;
     make_x_map(&xmap, xh, a.rows, a.n_in, pl.n_tile / 2);
-    const bool tmem = umma_tmem(DT, pl.n_tile, p.nsb, pl.kparts);
+    const bool tmem = pl.tmem;
     // tensor memory: accumulators of n_tile columns, then at least four weight stages; or two or four accumulators alone
     p.acc_cols = tmem ? (uint32_t)pl.n_tile : (pl.n_tile <= UM_MAX_N / 2 ? UM_MAX_N / 2 : UM_MAX_N);
-    p.n_acc = tmem ? std::min<uint32_t>(UM_MAX_ACC, (512 - 4 * UM_A_COLS) / p.acc_cols) : 512u / p.acc_cols;
-    p.stages = tmem ? std::min<uint32_t>(UM_MAX_STAGES, (512 - p.n_acc * p.acc_cols) / UM_A_COLS) : UM_MAX_STAGES;
+    p.n_acc = tmem ? umma_accumulators(pl.n_tile) : 512u / p.acc_cols;
+    p.stages = tmem ? umma_tmem_stages(pl.n_tile) : UM_MAX_STAGES;
     const size_t stage = (size_t)(tmem ? 0 : UM_A_BYTES) + (size_t)pl.n_tile * 64, tabs = (size_t)UM_DW * HalfRecord<DT>::TAB + 1024,
                  room = dev->prop.sharedMemPerBlockOptin - 1024;
     auto bytes = [&] { return tabs + p.stages * stage + p.raw_stages * (size_t)S::RAW_BYTES; };

@@ -11,7 +11,8 @@
 // Where the decoded weights lie. Up to 192 activation rows per tile tensor memory has room for two accumulators and four
 // stages of weights beside them, and the decode warps store there (tcgen05.st, the A operand of the MMA): the weights then pass
 // through shared memory once, packed, instead of three times. Wider tiles keep the stages in shared memory, since their two
-// accumulators fill tensor memory (one accumulator beside the weights was no faster: its epilogue runs alone). The operands are
+// accumulators fill tensor memory (one accumulator beside the weights was no faster: its epilogue runs alone), and so do Q5_K and
+// Q8_0 where a pair walks few superblocks (umma_tmem). The operands are
 // the same numbers either way, and so are the results.
 //
 // What bounds it, and why this tile. At M = 128 per CTA a stage of 64 columns keeps the tensor pipe busy for two cycles
@@ -278,7 +279,8 @@ template <> struct HalfRecord<YUUKA_DTYPE_Q8_0> {
 // The words of a packed record that lane (g, t) takes for tensor memory: of a 32-column sub-block columns 4t .. 4t + 3 and 16 + 4t ..
 // + 3 (its part of two 16 x 16 fragments). `pieces`: 32 pieces of 16 bytes, one per lane (g, t') of the register-fed kernel, which
 // takes columns 8t' .. 8t' + 7 of two sub-blocks as words x y and z w: the columns at 4t are a word of piece t / 2, those at 16 + 4t
-// the same word two pieces on.
+// the same word two pieces on. (Lanes g, g + 2, g + 4 and g + 6 of a load meet on one bank: sixteen wavefronts instead of four for
+// the 512 bytes. A record order without that would have every other kernel read it otherwise.)
 __device__ __forceinline__ uint4 fetch_quads(const uint8_t * pieces, int lane) {
     const uint32_t * w = reinterpret_cast<const uint32_t *>(pieces + (lane >> 2) * 64 + (lane & 2) * 8 + (lane & 1) * 4);
     return make_uint4(w[0], w[8], w[2], w[10]);
