@@ -199,7 +199,7 @@ def test_rows_beyond_one_pass_equal_passes_of_sixteen(dev, dtype, n_out, n_in, r
     (24, 256, 1), (24, 256, 16),         # one superblock, a row tile that is not full
     (2560, 2560, 6), (2560, 2560, 7),    # parts of K on warps of one CTA
     (160, 9216, 1), (160, 16384, 13),    # few tiles, a long K
-    (40960, 2048, 5), (40960, 2304, 5),  # 16 and 18 records per warp: Q5_K and Q8_0 change over
+    (65536, 1792, 5), (65536, 2048, 5),  # 14 and 16 records per warp: Q5_K and Q8_0 change over
 ])
 def test_activations_prepared_by_the_kernel_or_by_a_launch_before_it(dev, dtype, n_out, n_in, rows):
     """Few columns per thread are prepared by the product's own kernel, more by a launch before it: f32 and bf16, stored and added."""

@@ -2294,9 +2294,9 @@ static int launch_mma_dt(const yuuka_device * dev, cudaStream_t s, const TiledGe
     // another, the launch before and this: 300 x 512 Q4_K 5.9 -> 3.7 us at 1 to 7 rows, 2560 x 2560 6.4 -> 5.2 at 2 and 7.8 -> 7.4 at 5,
     // 4096 x 1024 Q5_K 6.2 -> 4.9 at 7, 16384 x 512 Q8_0 9.6 -> 8.1 at 16, 18432 x 2560 Q4_K 14.3 -> 13.9 at 5. Between two and three
     // pieces it depends: 4096 x 1024 Q6_K at 12 rows gains a sixth, 2560 x 4096 Q4_K at 5 rows loses 5 % (8.25 -> 8.69 us).
-    // The loop of this instance is 2 to 8 % slower for Q5_K and Q8_0 beyond four rows, so a warp that walks many records keeps the
-    // launch: 151936 x 2048 Q8_0 (40 records) 79 us instead of 85 at 7 rows, 248320 x 2560 Q5_K (70) 142 instead of 147 at 5;
-    // 40960 x 2560 (20) 36 us both ways, 100000 x 1280 Q8_0 (15) 35 -> 34 at 6.
+    // Q5_K and Q8_0 beyond four rows lose where a warp walks sixteen records or more, and keep the launch there: 248320 x 2560 Q5_K
+    // (70 records) 142 us instead of 147 at 5 rows, 151936 x 2048 Q8_0 (36) 79 instead of 85 at 7, 65536 x 2048 Q8_0 (16) 36.2
+    // instead of 37.9 at 5; 40960 x 2560 Q8_0 (15) 36 both ways, 113664 x 1280 Q8_0 (15) 36.5 -> 35.3 at 6.
     // (Not where `out` lies over x: the first CTAs to finish would store over columns that others have still to read.)
     const char * x0 = (const char *)a.x, * out0 = (const char *)a.out;
     const bool apart = out0 + (((int64_t)a.rows - 1) * a.ldo + a.n_out) * 4 <= x0 ||
@@ -2305,7 +2305,7 @@ static int launch_mma_dt(const yuuka_device * dev, cudaStream_t s, const TiledGe
         TPlan pl;
         plan_tiled(dev, a.w_dtype, a.rows, a.n_out, a.n_in, pl);
         const int records = (pl.n_groups + pl.grid_x - 1) / pl.grid_x * pl.nsb_chunk / pl.KS;  // of a warp
-        if ((DT == YUUKA_DTYPE_Q5_K || DT == YUUKA_DTYPE_Q8_0) && a.rows > 4 && records > 16) return false;
+        if ((DT == YUUKA_DTYPE_Q5_K || DT == YUUKA_DTYPE_Q8_0) && a.rows > 4 && records >= 16) return false;
         return a.rows * pl.nsb_chunk * 16 <= 2 * pl.TG * pl.KS * 32;
     }();
     if (!xp.xh && !own_x) {
