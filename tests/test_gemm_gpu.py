@@ -200,6 +200,8 @@ def test_rows_beyond_one_pass_equal_passes_of_sixteen(dev, dtype, n_out, n_in, r
     (2560, 2560, 6), (2560, 2560, 7),    # parts of K on warps of one CTA
     (160, 9216, 1), (160, 16384, 13),    # few tiles, a long K
     (65536, 1792, 5), (65536, 2048, 5),  # 14 and 16 records per warp: Q5_K and Q8_0 change over
+    (10208, 2816, 16),                   # Q4_K, Q5_K: K in ranges of 4, 4 and 3 superblocks on CTAs of their own
+    (20000, 4352, 1), (20000, 4352, 4),  # the same with several groups per CTA, for every type: 6, 6 and 5
 ])
 def test_activations_prepared_by_the_kernel_or_by_a_launch_before_it(dev, dtype, n_out, n_in, rows):
     """Few columns per thread are prepared by the product's own kernel, more by a launch before it: f32 and bf16, stored and added."""
@@ -220,6 +222,7 @@ def test_activations_prepared_by_the_kernel_or_by_a_launch_before_it(dev, dtype,
 @pytest.mark.parametrize("n_out,n_in,rows", [
     (2560, 2560, 2), (2560, 2560, 5),    # in place as a whole, by both forms of the preparation
     (24, 256, 1), (300, 512, 3), (4096, 1024, 4), (2560, 2560, 9), (520, 1024, 20), (520, 512, 64),
+    (10208, 2816, 16), (20000, 4352, 4),  # K in three ranges on CTAs of their own, the last one shorter
 ])
 def test_an_output_that_lies_over_the_activations(dev, dtype, n_out, n_in, rows):
     """The activations are read before anything is stored, wherever the two ranges meet. The product is then not the one to
@@ -247,3 +250,13 @@ def test_an_output_that_lies_over_the_activations(dev, dtype, n_out, n_in, rows)
     for b in (raw, wb):
         b.free()
     stream.destroy()
+
+
+@pytest.mark.parametrize("dtype", [synth.Q4_K, synth.Q5_K, synth.Q6_K, synth.Q8_0])
+def test_six_rows_and_seven_give_the_same_bits(dev, dtype):
+    """K of 2560 x 2560 is cut alike for both, and six rows are prepared by the product's kernel, seven by a launch before it."""
+    n_out, n_in = 2560, 2560
+    w = synth.normal_quant(n_out, n_in, dtype, 0.02, 1000 + dtype)
+    x = synth.normal_f32(7 * n_in, 1.0, 81).reshape(7, n_in)
+    seven = run_gemm(dev, w, dtype, n_out, n_in, x, cuda.PATH_MMA)
+    assert np.array_equal(run_gemm(dev, w, dtype, n_out, n_in, x[:6], cuda.PATH_MMA), seven[:6])
