@@ -165,8 +165,9 @@ YUUKA_API yuuka_status yuuka_gemm_quant(yuuka_stream * stream,
  * This call allocates and frees nothing, on the device or through a library.
  *  - Same arguments, routes and bit-identical results as yuuka_gemm_quant with
  *    YUUKA_GEMM_TILED, which flags must carry.
- *  - The scratch holds the prepared fp16 activations (rows * n_in * 2.25 bytes),
- *    the split-K partial sums and 4096 arrival counters. A shape that needs more
+ *  - The scratch has room for the prepared fp16 activations (rows * n_in * 2.25
+ *    bytes; calls of few columns per thread leave it unused and prepare them in
+ *    shared memory), the split-K partial sums and 4096 arrival counters. A shape that needs more
  *    than YUUKA_GEMM_STATIC_SCRATCH_BYTES returns YUUKA_ERR_UNSUPPORTED and
  *    launches nothing; yuuka_last_error() names the bytes needed.
  *  - The first call on each device does the set-up (it looks up the array's
